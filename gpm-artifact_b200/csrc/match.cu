@@ -26,17 +26,10 @@
 #include <type_traits>
 #include <vector>
 
-#include "common.cuh"
+#include "match.cuh"
 
-constexpr int kMaxQ = 64;     // query vertices (sub_ceci/configuration/config.h:12)
 constexpr int kNarrowQ = 16;  // plans up to this size take the narrow kernels
-
-struct gpm_query {
-  int n = 0;
-  int32_t labels[kMaxQ];
-  unsigned long long adjmask[kMaxQ];  // bit j set iff query edge (i, j)
-  int deg[kMaxQ];
-};
+constexpr int kMaxWeights = 2;  // vertices of a factored plan that are counted as a set size
 
 namespace gpm {
 
@@ -53,6 +46,18 @@ struct QueryPlanT {
   Mask back_pos[Q];   // bitmask of earlier positions that must be adjacent (parent excluded)
   int32_t label[Q];   // label of the vertex at each position
   int mindeg[Q];      // query degree at each position
+  // Weight vertices (factored plans, counts only): nw query vertices that
+  // take no position.  Weight vertex i is adjacent to the positions w_nb[i]
+  // alone, so the images it can take under an embedding of the positions are
+  // a set whose size multiplies the count.  w_lv[i]: the last of those
+  // positions; w_same[i]: the positions before the last one that carry its
+  // label and are not its neighbours (their images are taken out of the set
+  // when they lie in it); w_close[i]: the same for the last position (0: other
+  // label, 1: to be tested, 2: same neighbours, hence always in the set).
+  int nw;
+  int w_lv[kMaxWeights], w_close[kMaxWeights];
+  int32_t w_label[kMaxWeights];
+  Mask w_nb[kMaxWeights], w_same[kMaxWeights];
 };
 using QueryPlan = QueryPlanT<kNarrowQ>;
 using WidePlan = QueryPlanT<kMaxQ>;
@@ -68,6 +73,14 @@ static void narrow_plan(const WidePlan &w, QueryPlanT<Q> *p) {
     p->back_pos[k] = (typename QueryPlanT<Q>::Mask)w.back_pos[k];
     p->label[k] = w.label[k];
     p->mindeg[k] = w.mindeg[k];
+  }
+  p->nw = w.nw;
+  for (int i = 0; i < w.nw; ++i) {
+    p->w_lv[i] = w.w_lv[i];
+    p->w_close[i] = w.w_close[i];
+    p->w_label[i] = w.w_label[i];
+    p->w_nb[i] = (typename QueryPlanT<Q>::Mask)w.w_nb[i];
+    p->w_same[i] = (typename QueryPlanT<Q>::Mask)w.w_same[i];
   }
 }
 
@@ -85,22 +98,6 @@ __device__ __forceinline__ bool has_edge(const int64_t *__restrict__ off, const 
     if (x < key) lo = mid + 1; else hi = mid - 1;
   }
   return false;
-}
-
-// [s, e): v's neighbours with label l inside its label-partitioned list,
-// relative to off[v].  L == 0: the lists are not partitioned (labels >= 64),
-// the whole list is scanned and the label test filters.
-__device__ __forceinline__ void seg_range(const int64_t *__restrict__ off, const int32_t *__restrict__ loff, int L,
-                                          int32_t v, int l, int64_t *s, int64_t *e) {
-  if (L == 0) {
-    *s = 0;
-    *e = off[v + 1] - off[v];
-  } else if (l < 0 || l >= L) {
-    *s = *e = 0;
-  } else {
-    *s = loff[(int64_t)v * (L + 1) + l];
-    *e = loff[(int64_t)v * (L + 1) + l + 1];
-  }
 }
 
 // Is x in a's neighbours with label l?  Binary search inside a's label
@@ -162,15 +159,167 @@ struct MatchGraph {
   HubIndex hub;
 };
 
+// The images of one embedding that a query vertex is tested against:
+// positions 0 .. n-3 in emb, except that the last two of a pooled pair, z at
+// n'-2 and y at n'-1 of the n' mapped positions, are the caller's lane's own.
+struct Images {
+  const int32_t *emb;
+  int32_t z, y;
+  int par, pre;
+  __device__ __forceinline__ int32_t at(int j) const { return j == pre ? y : j == par ? z : emb[j]; }
+};
+
+// Is v (label l) a neighbour of every image of the positions in nb?
+template <class Mask>
+__device__ __forceinline__ bool adjacent_all(const MatchGraph &G, const Images &im, Mask nb, int l, int32_t v) {
+  for (; nb; nb &= nb - 1)
+    if (!adjacent(G.hub, G.off, G.adj, G.ladj, G.loff, G.L, im.at(low_bit(nb)), l, v)) return false;
+  return true;
+}
+
+// The shortest label-l segment among the images of the positions in nb:
+// start in ladj, length, and the position it belongs to.
+template <class Mask>
+__device__ __forceinline__ void shortest_segment(const MatchGraph &G, const Images &im, Mask nb, int l, int *src,
+                                                 long long *st, long long *len) {
+  *src = -1;
+  *st = *len = 0;
+  for (; nb; nb &= nb - 1) {
+    const int j = low_bit(nb);
+    const int32_t a = im.at(j);
+    int64_t s, e;
+    seg_range(G.off, G.loff, G.L, a, l, &s, &e);
+    if (*src < 0 || e - s < *len) {
+      *src = j;
+      *st = G.off[a] + s;
+      *len = e - s;
+    }
+  }
+}
+
+// Embeddings completing positions 0 .. n-4 (emb) with the lane's (z, y) at
+// positions (n-3, n-2) -- lanes t < k hold a pair each, pairs from several
+// parents z pooled -- and some last vertex.  Returned summed over the lanes
+// of the warp by the caller (TRACK: counted into *found instead).  WGT: every
+// embedding counts prod_i (the set size of weight vertex i), w0 / w1 being
+// the lane's sizes before the last position's image is taken out (1 where the
+// plan has no such weight vertex).
+template <bool TRACK, int Q, bool WGT>
+__device__ __forceinline__ unsigned long long close_pairs(const QueryPlanT<Q> &q, const MatchGraph &G,
+                                                          const int32_t *emb, int32_t z, int32_t y, int k,
+                                                          unsigned long long w0, unsigned long long w1,
+                                                          unsigned long long limit, unsigned long long *found,
+                                                          int32_t *__restrict__ emb_out) {
+  using Mask = typename QueryPlanT<Q>::Mask;
+  const unsigned lane = lane_id();
+  const int last = q.n - 1, pre = q.n - 2, par = q.n - 3;
+  const int llab = q.label[last];
+  const Mask lmask = q.back_pos[last] | ((Mask)1 << q.parent_pos[last]);
+  unsigned long long c = 0;
+  // lane t: its candidate's shortest segment for the last vertex
+  int src = -1;
+  long long st = 0, len = 0;
+  if ((int)lane < k) shortest_segment(G, Images{emb, z, y, par, pre}, lmask, llab, &src, &st, &len);
+  if (WGT && (w0 == 0 || w1 == 0)) len = 0;
+  flat_segments(G.ladj, st, len, [&](int t, bool valid, int32_t x) {
+    const int srct = __shfl_sync(0xffffffffu, src, t);
+    const int32_t yt = __shfl_sync(0xffffffffu, y, t), zt = __shfl_sync(0xffffffffu, z, t);
+    unsigned long long wt0 = 1, wt1 = 1;
+    if (WGT) {
+      wt0 = __shfl_sync(0xffffffffu, w0, t);
+      wt1 = __shfl_sync(0xffffffffu, w1, t);
+    }
+    const Images im{emb, zt, yt, par, pre};
+    bool ok = false;
+    if (valid) {
+      ok = (G.L > 0 || G.labels[x] == llab) && x != yt && x != zt;
+      for (int j = 0; ok && j < par; ++j) ok = emb[j] != x;
+      ok = ok && adjacent_all(G, im, lmask & ~((Mask)1 << srct), llab, x);
+    }
+    if (WGT) {
+      if (ok) {
+        if (q.w_close[0] == 2 || (q.w_close[0] == 1 && adjacent_all(G, im, q.w_nb[0], llab, x))) --wt0;
+        if (q.nw > 1 && (q.w_close[1] == 2 || (q.w_close[1] == 1 && adjacent_all(G, im, q.w_nb[1], llab, x)))) --wt1;
+        c += wt0 * wt1;
+      }
+      return;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, ok);
+    if (TRACK && m) {
+      unsigned long long at = 0;
+      if (lane == 0) at = atomicAdd(found, (unsigned long long)__popc(m));
+      at = __shfl_sync(0xffffffffu, at, 0);
+      const unsigned long long slot = at + __popc(m & ((1u << lane) - 1u));
+      if (emb_out && ok && slot < limit) {
+        int32_t *row = emb_out + slot * (unsigned long long)q.n;
+        for (int j = 0; j < par; ++j) row[q.order[j]] = emb[j];
+        row[q.order[par]] = zt;
+        row[q.order[pre]] = yt;
+        row[q.order[last]] = x;
+      }
+    }
+    c += lane == 0 ? (unsigned long long)__popc(m) : 0ull;
+  });
+  return c;
+}
+
+// Size of weight vertex i's set for the lane's pair (z, y): its raw size less
+// the images of w_same[i] that lie in it.
+template <int Q>
+__device__ __forceinline__ unsigned long long weight_of(const QueryPlanT<Q> &q, const MatchGraph &G, const Images &im,
+                                                        int i, unsigned long long raw) {
+  if (i >= q.nw) return 1ull;
+  for (typename QueryPlanT<Q>::Mask m = q.w_same[i]; m; m &= m - 1)
+    if (adjacent_all(G, im, q.w_nb[i], q.w_label[i], im.at(low_bit(m)))) --raw;
+  return raw;
+}
+
+// Plans of three positions, starting from (root, second vertex) pairs: lane t
+// < k of the warp holds the pair (z, y).  32 pairs are closed together, so
+// short segments do not leave lanes idle (R-MAT 17 to 21: most pairs of a
+// triangle or diamond query close over fewer than 32 entries).  cnt: 32 ints
+// of the warp's shared memory.  Each lane returns its part of the count.
+template <int Q, bool WGT>
+__device__ __forceinline__ unsigned long long match_pairs3(const QueryPlanT<Q> &q, const MatchGraph &G, int32_t z,
+                                                           int32_t y, int k, int32_t *cnt) {
+  using Mask = typename QueryPlanT<Q>::Mask;
+  const unsigned lane = lane_id();
+  unsigned long long w[2] = {1, 1};
+  if (WGT) {
+    const Images own{nullptr, z, y, 0, 1};
+#pragma unroll
+    for (int i = 0; i < kMaxWeights; ++i) {
+      if (i >= q.nw) break;
+      int src = -1;
+      long long st = 0, len = 0;
+      if ((int)lane < k) shortest_segment(G, own, q.w_nb[i], q.w_label[i], &src, &st, &len);
+      cnt[lane] = 0;
+      __syncwarp();
+      flat_segments(G.ladj, st, len, [&](int t, bool valid, int32_t x) {
+        const int srct = __shfl_sync(0xffffffffu, src, t);
+        const int32_t yt = __shfl_sync(0xffffffffu, y, t), zt = __shfl_sync(0xffffffffu, z, t);
+        if (valid && (G.L > 0 || G.labels[x] == q.w_label[i]) &&
+            adjacent_all(G, Images{nullptr, zt, yt, 0, 1}, q.w_nb[i] & ~((Mask)1 << srct), q.w_label[i], x))
+          atomicAdd(&cnt[t], 1);
+      });
+      __syncwarp();
+      w[i] = (int)lane < k ? weight_of(q, G, own, i, (unsigned long long)(unsigned)cnt[lane]) : 0ull;
+      __syncwarp();
+    }
+  }
+  return close_pairs<false, Q, WGT>(q, G, nullptr, z, y, k, w[0], w[1], ~0ull, nullptr, nullptr);
+}
+
 // The embeddings extending one partial embedding `row` (positions 0 .. t-1
 // mapped, t >= 2: a (root, second vertex) pair, or a row of a breadth-first
-// extension), by one warp; lane 0 returns the count (TRACK: counted into
-// *found instead, see k_match).  chunk >= 0 restricts position t's
-// candidates to the `span` entries from `chunk` on (tasks split by the batch
-// path); buf is the warp's shared
+// extension), by one warp; the count is the sum over the lanes (TRACK:
+// counted into *found instead, see k_match).  chunk >= 0 restricts position
+// t's candidates to the `span` entries from `chunk` on (tasks split by the
+// batch path); buf is the warp's shared
 // buffer of Q rows of 32 candidates (rows d - 2 for positions 2 .. n-2,
-// the last two for the pool of position n-2's survivors).
-template <bool TRACK, int Q>
+// the last two for the pool of position n-2's survivors).  WGT: the plan's
+// weight vertices are counted (set sizes, QueryPlanT).
+template <bool TRACK, int Q, bool WGT>
 __device__ __forceinline__ unsigned long long match_task(const QueryPlanT<Q> &q, const MatchGraph &G,
                                                          const int32_t *__restrict__ row, int t, int64_t chunk,
                                                          int64_t span,
@@ -189,10 +338,9 @@ __device__ __forceinline__ unsigned long long match_task(const QueryPlanT<Q> &q,
   int64_t pos[Q], end[Q];
   Mask chk[Q];
   int bcnt[Q], bcur[Q];
-  const int last = q.n - 1, pre = q.n - 2;
-  const int llab = q.label[last];
-  const Mask lmask = q.back_pos[last] | ((Mask)1 << q.parent_pos[last]);
+  const int pre = q.n - 2;
   unsigned long long c = 0;
+  unsigned long long raw0 = 1, raw1 = 1;  // raw set sizes of the weight vertices whose positions are mapped
 
   // candidate segment of position d: the shortest label segment among the
   // mapped query-neighbours, the others left to check (chk)
@@ -238,79 +386,53 @@ __device__ __forceinline__ unsigned long long match_task(const QueryPlanT<Q> &q,
     return __popc(m);
   };
 
-  // embeddings completing positions 0 .. n-4 with (z, y) at positions
-  // (n-3, n-2) (lane t < k holds pair t: pairs from several parents z are
-  // pooled) and some last vertex
-  auto close = [&](int32_t z, int32_t y, int k) {
-    const int par = pre - 1;
-    // lane t: its candidate's shortest segment for the last vertex
-    int src = -1;
-    long long st = 0, len = 0;
-    if ((int)lane < k) {
-      for (Mask bm = lmask; bm; bm &= bm - 1) {
-        const int j = low_bit(bm);
-        const int32_t a = j == pre ? y : j == par ? z : emb[j];
-        int64_t s, e;
-        seg_range(off, loff, L, a, llab, &s, &e);
-        if (src < 0 || e - s < len) {
-          src = j;
-          st = off[a] + s;
-          len = e - s;
-        }
-      }
-    }
-    long long inc = len;  // inclusive prefix over the lanes
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const long long v = __shfl_up_sync(0xffffffffu, inc, o);
-      if ((int)lane >= o) inc += v;
-    }
-    const long long total = __shfl_sync(0xffffffffu, inc, 31);
-    for (long long base = 0; base < total; base += 32) {
-      const long long idx = base + lane;
-      // t = first lane whose inclusive prefix exceeds idx
-      int lo = 0, hi = 31;
-#pragma unroll
-      for (int r = 0; r < 5; ++r) {
-        const int mid = (lo + hi) >> 1;
-        const long long pm = __shfl_sync(0xffffffffu, inc, mid);
-        if (pm > idx) hi = mid; else lo = mid + 1;
-      }
-      const int t = lo;
-      const long long pt = __shfl_sync(0xffffffffu, inc, t), lt = __shfl_sync(0xffffffffu, len, t);
-      const long long stt = __shfl_sync(0xffffffffu, st, t);
-      const int srct = __shfl_sync(0xffffffffu, src, t);
-      const int32_t yt = __shfl_sync(0xffffffffu, y, t), zt = __shfl_sync(0xffffffffu, z, t);
+  // raw set size of weight vertex i: the common neighbours with its label of
+  // the images of w_nb[i] (all in emb)
+  auto raw_size = [&](int i) -> unsigned long long {
+    const Images im{emb, 0, 0, Q, Q};
+    int src;
+    long long st, len;
+    shortest_segment(G, im, q.w_nb[i], q.w_label[i], &src, &st, &len);
+    unsigned long long got = 0;
+    for (long long b = 0; b < len; b += 32) {
       bool ok = false;
-      int32_t x = 0;
-      if (idx < total) {
-        x = __ldg(ladj + stt + (idx - (pt - lt)));
-        ok = (L > 0 || labels[x] == llab) && x != yt && x != zt;
-        for (int j = 0; ok && j < par; ++j) ok = emb[j] != x;
-        for (Mask bm = lmask & ~((Mask)1 << srct); ok && bm; bm &= bm - 1) {
-          const int j = low_bit(bm);
-          ok = adjacent(hub, off, adj, ladj, loff, L, j == pre ? yt : j == par ? zt : emb[j], llab, x);
-        }
+      if (b + lane < len) {
+        const int32_t x = __ldg(ladj + st + b + lane);
+        ok = (L > 0 || labels[x] == q.w_label[i]) &&
+             adjacent_all(G, im, q.w_nb[i] & ~((Mask)1 << src), q.w_label[i], x);
       }
-      const unsigned m = __ballot_sync(0xffffffffu, ok);
-      if (TRACK && m) {
-        unsigned long long at = 0;
-        if (lane == 0) at = atomicAdd(found, (unsigned long long)__popc(m));
-        at = __shfl_sync(0xffffffffu, at, 0);
-        const unsigned long long slot = at + __popc(m & ((1u << lane) - 1u));
-        if (emb_out && ok && slot < limit) {
-          int32_t *row = emb_out + slot * (unsigned long long)q.n;
-          for (int j = 0; j < par; ++j) row[q.order[j]] = emb[j];
-          row[q.order[par]] = zt;
-          row[q.order[pre]] = yt;
-          row[q.order[last]] = x;
-        }
-      }
-      c += lane == 0 ? (unsigned long long)__popc(m) : 0ull;
+      got += __popc(__ballot_sync(0xffffffffu, ok));
     }
+    return got;
+  };
+  // the weight vertices whose last position is d, once emb[d] is mapped;
+  // false: one of their sets is empty
+  auto weigh = [&](int d) -> bool {
+    bool some = true;
+    if (q.nw > 0 && q.w_lv[0] == d) {
+      raw0 = raw_size(0);
+      some = raw0 != 0;
+    }
+    if (q.nw > 1 && q.w_lv[1] == d) {
+      raw1 = raw_size(1);
+      some = some && raw1 != 0;
+    }
+    return some;
+  };
+  auto close = [&](int32_t z, int32_t y, int k) {
+    unsigned long long w0 = 1, w1 = 1;
+    if (WGT && (int)lane < k) {
+      const Images im{emb, z, y, pre - 1, pre};
+      w0 = weight_of(q, G, im, 0, raw0);
+      w1 = weight_of(q, G, im, 1, raw1);
+    }
+    c += close_pairs<TRACK, Q, WGT>(q, G, emb, z, y, k, w0, w1, limit, found, emb_out);
   };
 
   for (int j = 0; j < t; ++j) emb[j] = row[j];
+  if (WGT)
+    for (int j = 0; j < t; ++j)
+      if (!weigh(j)) return 0;
   if (pre == t - 1) {  // the row already maps position n-2
     close(emb[pre - 1], emb[pre], 1);
     return c;
@@ -349,7 +471,14 @@ __device__ __forceinline__ unsigned long long match_task(const QueryPlanT<Q> &q,
       continue;
     }
     if (bcur[d] < bcnt[d]) {
-      emb[d] = buf[d - 2][bcur[d]++];
+      const int32_t x = buf[d - 2][bcur[d]++];
+      // pending pairs carry the set sizes of the images before this one
+      if (WGT && ((q.nw > 0 && q.w_lv[0] == d) || (q.nw > 1 && q.w_lv[1] == d))) {
+        flush();
+        emb[d] = x;
+        if (!weigh(d)) continue;
+      }
+      emb[d] = x;
       ++d;
       open(d);
       bcnt[d] = bcur[d] = 0;
@@ -380,6 +509,9 @@ __device__ __forceinline__ unsigned long long match_task(const QueryPlanT<Q> &q,
 // 48 registers the compiler picks unbounded (5 CTAs per SM)
 #define GPM_MATCH_MIN_BLOCKS 6
 #endif
+#ifndef GPM_MATCH_WGT_BLOCKS
+#define GPM_MATCH_WGT_BLOCKS 4  // factored plans
+#endif
 // Candidate rows of the wide kernels (Q > kNarrowQ): Q rows of 32 ids per
 // warp in dynamic shared memory (64 KB per CTA at Q = 64).
 template <int Q>
@@ -393,8 +525,8 @@ __device__ __forceinline__ int32_t (*warp_rows(int32_t (*narrow)[32]))[32] {
   return Q <= kNarrowQ ? narrow : reinterpret_cast<int32_t(*)[32]>(match_dyn + (threadIdx.x >> 5) * Q * 32);
 }
 
-template <bool TRACK, int Q>
-__global__ void __launch_bounds__(kMatchWarps * 32, Q <= kNarrowQ ? GPM_MATCH_MIN_BLOCKS : 2)
+template <bool TRACK, int Q, bool WGT>
+__global__ void __launch_bounds__(kMatchWarps * 32, Q > kNarrowQ ? 2 : WGT ? GPM_MATCH_WGT_BLOCKS : GPM_MATCH_MIN_BLOCKS)
     k_match(QueryPlanT<Q> q, MatchGraph G, const int32_t *__restrict__ rows, int t, int64_t n,
             unsigned long long *__restrict__ cursor, unsigned long long *__restrict__ out, unsigned long long limit,
             unsigned long long *found, int32_t *__restrict__ emb_out) {
@@ -402,13 +534,20 @@ __global__ void __launch_bounds__(kMatchWarps * 32, Q <= kNarrowQ ? GPM_MATCH_MI
   int32_t(*buf)[32] = warp_rows<Q>(sbuf[threadIdx.x >> 5]);
   const unsigned lane = lane_id();
   unsigned long long c = 0;
+  const bool pool = !TRACK && q.n == 3 && t == 2;  // 32 pairs at a time
   while (true) {
     unsigned long long r = 0;
-    if (lane == 0) r = atomicAdd(cursor, 1ull);
+    if (lane == 0) r = atomicAdd(cursor, pool ? 32ull : 1ull);
     r = __shfl_sync(0xffffffffu, r, 0);
     if (r >= (unsigned long long)n) break;
     if (TRACK && *(volatile unsigned long long *)found >= limit) break;
-    c += match_task<TRACK, Q>(q, G, rows + (int64_t)r * t, t, -1, 0, buf, limit, found, emb_out);
+    if (pool) {
+      const int k = (int)min((long long)32, (long long)n - (long long)r);
+      const int2 p = (int)lane < k ? reinterpret_cast<const int2 *>(rows)[r + lane] : make_int2(0, 0);
+      c += match_pairs3<Q, WGT>(q, G, p.x, p.y, k, buf[0]);
+    } else {
+      c += match_task<TRACK, Q, WGT>(q, G, rows + (int64_t)r * t, t, -1, 0, buf, limit, found, emb_out);
+    }
   }
   if (TRACK) return;
   c = warp_sum(c);
@@ -560,11 +699,52 @@ __global__ void k_label_offsets(int64_t n, const int64_t *__restrict__ off, cons
   }
 }
 
-static int plan_query(const gpm_query *q, const std::vector<int64_t> &label_freq, WidePlan *p) {
-  const int n = q->n;
+// Matching order of the query vertices in `in` (a connected set): the given
+// root first, then repeatedly the unplaced vertex with most placed neighbours
+// (ties: vertices of `soon` first, then higher degree).  Returns the number
+// of vertices placed (fewer than popcount(in) when `in` is not connected).
+static int match_order(const gpm_query *q, unsigned long long in, int root, unsigned long long soon, int *order) {
+  unsigned long long placed = 1ull << root;
+  int k = 1;
+  for (order[0] = root; placed != in; ++k) {
+    int b = -1, bs = 0, bd = -1;
+    for (unsigned long long m = in & ~placed; m; m &= m - 1) {
+      const int u = __builtin_ctzll(m);
+      const int s = __builtin_popcountll(q->adjmask[u] & placed);
+      const int d = q->deg[u] + ((soon >> u) & 1 ? kMaxQ : 0);
+      if (s > bs || (s == bs && s > 0 && d > bd)) {
+        b = u;
+        bs = s;
+        bd = d;
+      }
+    }
+    if (bs <= 0) break;
+    order[k] = b;
+    placed |= 1ull << b;
+  }
+  return k;
+}
+
+// The plan that maps order[0 .. n) in that order.
+static void fill_plan(const gpm_query *q, const int *order, int n, WidePlan *p) {
   memset(p, 0, sizeof *p);
   p->n = n;
-  bool placed[kMaxQ] = {false};
+  for (int k = 0; k < n; ++k) {
+    const int u = order[k];
+    p->order[k] = u;
+    p->label[k] = q->labels[u];
+    p->mindeg[k] = q->deg[u];
+    p->parent_pos[k] = -1;
+    for (int j = 0; j < k; ++j) {
+      if (!((q->adjmask[u] >> order[j]) & 1u)) continue;
+      if (p->parent_pos[k] < 0) p->parent_pos[k] = j;
+      else p->back_pos[k] |= 1ull << j;
+    }
+  }
+}
+
+static int plan_query(const gpm_query *q, const std::vector<int64_t> &label_freq, WidePlan *p) {
+  const int n = q->n;
   int best = 0;
   auto freq = [&](int u) -> int64_t {
     int32_t l = q->labels[u];
@@ -572,49 +752,105 @@ static int plan_query(const gpm_query *q, const std::vector<int64_t> &label_freq
   };
   for (int u = 1; u < n; ++u)
     if (freq(u) < freq(best) || (freq(u) == freq(best) && q->deg[u] > q->deg[best])) best = u;
-  p->order[0] = best;
-  placed[best] = true;
-  for (int k = 1; k < n; ++k) {
-    int b = -1, bs = -1, bd = -1;
-    for (int u = 0; u < n; ++u) {
-      if (placed[u]) continue;
-      int s = 0;
-      for (int w = 0; w < n; ++w) s += placed[w] && ((q->adjmask[u] >> w) & 1u);
-      if (s > bs || (s == bs && q->deg[u] > bd)) {
-        b = u;
-        bs = s;
-        bd = q->deg[u];
-      }
-    }
-    if (bs <= 0) return fail(GPM_EUNSUPPORTED, "query graph must be connected");
-    p->order[k] = b;
-    placed[b] = true;
-  }
-  for (int k = 0; k < n; ++k) {
-    int u = p->order[k];
-    p->label[k] = q->labels[u];
-    p->mindeg[k] = q->deg[u];
-    p->parent_pos[k] = -1;
-    p->back_pos[k] = 0;
-    for (int j = 0; j < k; ++j) {
-      if (!((q->adjmask[u] >> p->order[j]) & 1u)) continue;
-      if (p->parent_pos[k] < 0) p->parent_pos[k] = j;
-      else p->back_pos[k] |= 1ull << j;
-    }
-  }
+  int order[kMaxQ];
+  if (match_order(q, n >= 64 ? ~0ull : (1ull << n) - 1, best, 0, order) < n)
+    return fail(GPM_EUNSUPPORTED, "query graph must be connected");
+  fill_plan(q, order, n, p);
   return GPM_OK;
 }
 
-// Label-partitioned copy of a labelled graph's lists (cached per graph).
-struct LabelCsr {
-  int L = 0;  // partitions (max label + 1); 0: labels too wide, lists copied as they are
-  DevBuf<int32_t> ladj, loff;
-  // adjacency bitmaps of the vertices with at least hub_min neighbours
-  DevBuf<int32_t> hub_slot;
-  DevBuf<uint32_t> hub_bm;
-  int64_t hub_words = 0;
-  int hubs = 0, hub_min = 0;
-};
+// A cheaper plan of a counted query, where there is one: one or two vertices,
+// adjacent neither to each other nor to the vertex mapped last, take no
+// position; the number of images they can take is a set size that multiplies
+// the count, so the embeddings that differ only there are never walked one by
+// one.  (The diamond query becomes, per edge, two set sizes.  R-MAT 17, a
+// batch of a triangle, a diamond, a house and a 4-cycle: 1.67 s walked, 14.8
+// ms with the sets and match_cycle.cu's 4-cycles.)  Every choice of such
+// vertices and of a root is compared with the plan at hand by the number of
+// partial embeddings and of entries scanned that an average graph with these
+// label frequencies would give: each position multiplies by the mean label
+// segment (walks meet hubs, hence kSkew times the mean) and each further back
+// edge by kClose.
+static void factor_query(const gpm_query *q, const std::vector<int64_t> &label_freq, int64_t n, int64_t nnz,
+                         WidePlan *p) {
+  const int nq = q->n;
+  if (nq < 4 || nq > kNarrowQ || n <= 0) return;
+  constexpr double kSkew = 4.0, kClose = 0.1;
+  auto freq = [&](int32_t l) { return (l >= 0 && (size_t)l < label_freq.size()) ? (double)label_freq[l] : 0.0; };
+  auto seg = [&](int32_t l) { return kSkew * (double)nnz / (double)n * freq(l) / (double)n; };
+  auto cost_of = [&](const WidePlan &w) {
+    double e = freq(w.label[0]), cost = 0;
+    for (int k = 1; k < w.n; ++k) {
+      cost += e * (1.0 + seg(w.label[k]));
+      e *= seg(w.label[k]);
+      for (unsigned long long m = w.back_pos[k]; m; m &= m - 1) e *= kClose;
+      for (int i = 0; i < w.nw; ++i)
+        if (w.w_lv[i] == k) cost += e * (1.0 + seg(w.w_label[i]));
+    }
+    return cost;
+  };
+  const unsigned long long all = (1ull << nq) - 1;
+  double best = cost_of(*p);
+  WidePlan cand, keep = *p;
+  // weight vertices wm (at most two, pairwise not adjacent, of different
+  // labels) with the vertex c mapped last
+  auto consider = [&](unsigned long long wm, int c) {
+    const unsigned long long pre = all & ~wm & ~(1ull << c);
+    unsigned long long soon = 0;
+    for (unsigned long long m = wm; m; m &= m - 1) soon |= q->adjmask[__builtin_ctzll(m)];
+    if (__builtin_popcountll(pre) < 2 || !(q->adjmask[c] & pre)) return;
+    // larger queries: the rarest root alone
+    int rare = -1;
+    if (nq > 8)
+      for (unsigned long long m = pre; m; m &= m - 1) {
+        const int u = __builtin_ctzll(m);
+        if (rare < 0 || freq(q->labels[u]) < freq(q->labels[rare])) rare = u;
+      }
+    for (unsigned long long rm = pre; rm; rm &= rm - 1) {
+      const int root = __builtin_ctzll(rm);
+      if (rare >= 0 && root != rare) continue;
+      int order[kMaxQ];
+      int k = match_order(q, pre, root, soon, order);
+      if (k < __builtin_popcountll(pre)) return;  // not connected
+      order[k++] = c;
+      fill_plan(q, order, k, &cand);
+      bool ok = true;
+      for (unsigned long long m = wm; m; m &= m - 1) {
+        const int u = __builtin_ctzll(m), i = cand.nw++;
+        cand.w_label[i] = q->labels[u];
+        for (int j = 0; j + 1 < k; ++j) {
+          if ((q->adjmask[u] >> order[j]) & 1u) {
+            cand.w_nb[i] |= 1ull << j;
+            cand.w_lv[i] = j;
+          } else if (q->labels[order[j]] == q->labels[u]) {
+            cand.w_same[i] |= 1ull << j;
+          }
+        }
+        if (q->labels[c] == q->labels[u]) cand.w_close[i] = q->adjmask[u] == q->adjmask[c] ? 2 : 1;
+        // the set is sized when position w_lv is mapped, before the pooled pairs
+        ok = ok && cand.w_nb[i] && cand.w_lv[i] <= std::max(1, k - 3);
+      }
+      if (!ok) continue;
+      const double cost = cost_of(cand);
+      if (cost < best) {
+        best = cost;
+        keep = cand;
+      }
+    }
+  };
+  for (int w = 0; w < nq; ++w)
+    for (int c = 0; c < nq; ++c) {
+      if (c == w || ((q->adjmask[w] >> c) & 1u)) continue;
+      consider(1ull << w, c);
+      for (int v = w + 1; v < nq && nq <= 8; ++v) {
+        if (v == c || ((q->adjmask[v] >> w) & 1u) || ((q->adjmask[v] >> c) & 1u) || q->labels[v] == q->labels[w])
+          continue;
+        consider(1ull << w | 1ull << v, c);
+      }
+    }
+  *p = keep;
+}
+
 void free_label_csr(LabelCsr *p) { delete p; }
 
 __global__ void k_label_range(int64_t n, const int32_t *__restrict__ labels, int *__restrict__ mm) {
@@ -749,11 +985,27 @@ static int ensure_label_csr(gpm_graph *g) {
   return GPM_OK;
 }
 
+// h[l] = vertices with label l < nl.  Up to kHistBins labels are counted in
+// shared memory first (a few labels would otherwise meet in a few global
+// counters: R-MAT 19, 8 labels, 149 us).
+constexpr int kHistBins = 256;
 __global__ void k_label_hist(int64_t n, const int32_t *__restrict__ labels, int nl, unsigned long long *__restrict__ h) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    int32_t l = labels[i];
-    if (l >= 0 && l < nl) atomicAdd(&h[l], 1ull);
+  __shared__ unsigned sh[kHistBins];
+  const bool local = nl <= kHistBins;
+  if (local) {
+    for (int i = threadIdx.x; i < nl; i += blockDim.x) sh[i] = 0u;
+    __syncthreads();
   }
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t l = labels[i];
+    if (l < 0 || l >= nl) continue;
+    if (local) atomicAdd(&sh[l], 1u);
+    else atomicAdd(&h[l], 1ull);
+  }
+  if (!local) return;
+  __syncthreads();
+  for (int i = threadIdx.x; i < nl; i += blockDim.x)
+    if (sh[i]) atomicAdd(&h[i], (unsigned long long)sh[i]);
 }
 
 }  // namespace gpm
@@ -804,20 +1056,27 @@ static int launch_match(const QueryPlanT<Q> &plan, const MatchGraph &G, const in
                         unsigned long long *cursor, unsigned long long *out, bool track, unsigned long long limit,
                         unsigned long long *found, int32_t *emb) {
   constexpr int smem = match_dyn_smem<Q>();
-  static PerDevice match_grid;
-  const int grid = match_grid.get([] {
-    if (smem > 0) {
-      cudaFuncSetAttribute(k_match<false, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      cudaFuncSetAttribute(k_match<true, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    }
+  constexpr bool kWgt = Q <= kNarrowQ;  // wide plans are not factored
+  static PerDevice match_grid, wgt_grid;
+  auto grid_of = [](auto kernel) {
+    if (smem > 0) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_match<false, Q>, kMatchWarps * 32, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kMatchWarps * 32, smem);
     return std::max(1, per_sm) * num_sms();
+  };
+  const int grid = match_grid.get([&] {
+    if (smem > 0) cudaFuncSetAttribute(k_match<true, Q, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return grid_of(k_match<false, Q, false>);
   });
   if (track)
-    k_match<true, Q><<<grid, kMatchWarps * 32, smem>>>(plan, G, rows, t, nrows, cursor, out, limit, found, emb);
+    k_match<true, Q, false>
+        <<<grid, kMatchWarps * 32, smem>>>(plan, G, rows, t, nrows, cursor, out, limit, found, emb);
+  else if (kWgt && plan.nw)
+    k_match<false, Q, kWgt><<<wgt_grid.get([&] { return grid_of(k_match<false, Q, kWgt>); }), kMatchWarps * 32, smem>>>(
+        plan, G, rows, t, nrows, cursor, out, limit, found, nullptr);
   else
-    k_match<false, Q><<<grid, kMatchWarps * 32, smem>>>(plan, G, rows, t, nrows, cursor, out, limit, found, nullptr);
+    k_match<false, Q, false>
+        <<<grid, kMatchWarps * 32, smem>>>(plan, G, rows, t, nrows, cursor, out, limit, found, nullptr);
   GPM_LAUNCH_CHECK();
   return GPM_OK;
 }
@@ -890,6 +1149,7 @@ static int match_run(gpm_graph *g, const gpm_query *q, unsigned long long limit,
   }
   WidePlan plan;
   GPM_TRY(plan_query(q, freq, &plan));
+  if (!track) factor_query(q, freq, g->n, g->nnz, &plan);
   DevBuf<unsigned long long> found;
   DevBuf<int32_t> demb;
   GPM_TRY(found.reserve(1));
@@ -916,6 +1176,18 @@ static int match_run(gpm_graph *g, const gpm_query *q, unsigned long long limit,
   const int blocks = (int)std::min<int64_t>((g->n * 32 + 255) / 256, (int64_t)num_sms() * 16);
   DevBuf<unsigned long long> d, npairs;
   GPM_TRY(d.reserve(1));
+  if (!track && is_cycle4(q, lc)) {
+    CyclePlan cp;
+    bool fits = false;
+    GPM_TRY(cycle_plan(g, lc, q, &cp, &lc->cycle, &fits));
+    if (fits) {
+      GPM_CUDA(cudaMemset(d.p, 0, 8));
+      GPM_TRY(cycle_launch(g, lc, cp, lc->cycle, nullptr, d.p, 0));
+      unsigned long long total = 0;
+      GPM_CUDA(cudaMemcpy(&total, d.p, 8, cudaMemcpyDeviceToHost));
+      return finish(total);
+    }
+  }
   GPM_TRY(npairs.reserve(1));
   GPM_CUDA(cudaMemset(npairs.p, 0, 8));
   // (root, second vertex) pairs: counted, then materialised
@@ -997,7 +1269,11 @@ struct gpm_match_batch {
   gpm_graph *g = nullptr;
   int nq = 0, nm = 1;
   int qcap = 16;  // plan width of the launch: 16, or 64 when a query has more than 16 vertices
+  bool weighted = false;  // some plan is factored (plan width 16 only)
   std::vector<gpm::WidePlan> plans;
+  // 4-cycle queries (their index) and the scratch they take one after another
+  std::vector<std::pair<int, gpm::CyclePlan>> cycles;
+  gpm::CycleSpace *cycle = nullptr;
   std::vector<gpm::DevBuf<int2>> pairs;  // per query (empty for 1- and 2-vertex queries)
   std::vector<int64_t> npairs;
   // per query: its task rows (the pairs, or their breadth-first extension
@@ -1017,6 +1293,7 @@ struct gpm_match_batch {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   ~gpm_match_batch() {
+    gpm::free_cycle_space(cycle);
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
   }
@@ -1024,8 +1301,12 @@ struct gpm_match_batch {
 
 namespace gpm {
 
-template <int Q>
-__global__ void __launch_bounds__(kMatchWarps * 32, Q <= kNarrowQ ? GPM_MATCH_MIN_BLOCKS : 2)
+// Tasks name a row of their query's list: with chunk >= -1 one row (chunk >= 0:
+// that chunk of its first unmapped position's candidates), with chunk <= -2
+// the -1 - chunk rows from there on, (root, second vertex) pairs of a
+// three-position plan that are closed together.
+template <int Q, bool WGT>
+__global__ void __launch_bounds__(kMatchWarps * 32, Q > kNarrowQ ? 2 : WGT ? GPM_MATCH_WGT_BLOCKS : GPM_MATCH_MIN_BLOCKS)
     k_match_batch(const QueryPlanT<Q> *__restrict__ plans, const int4 *__restrict__ qrows, MatchGraph G,
                   const int4 *__restrict__ tasks, int64_t ntasks, int64_t span, const int32_t *__restrict__ member,
                   int nm, unsigned long long *__restrict__ cursor, unsigned long long *__restrict__ out) {
@@ -1054,8 +1335,16 @@ __global__ void __launch_bounds__(kMatchWarps * 32, Q <= kNarrowQ ? GPM_MATCH_MI
     const int32_t *rows = reinterpret_cast<const int32_t *>(((unsigned long long)(unsigned)qr.y << 32) |
                                                              (unsigned)qr.x);
     const int32_t *row = rows + (((int64_t)t.y << 32) | (unsigned)t.x) * qr.z;
-    const unsigned long long c = match_task<false, Q>(splan[w], G, row, qr.z, t.w < 0 ? -1 : (int64_t)t.w * span,
-                                                      span, buf, ~0ull, nullptr, nullptr);
+    unsigned long long c;
+    if (t.w <= -2) {
+      const int k = -1 - t.w;
+      const int2 p = (int)lane < k ? reinterpret_cast<const int2 *>(row)[lane] : make_int2(0, 0);
+      c = match_pairs3<Q, WGT>(splan[w], G, p.x, p.y, k, buf[0]);
+    } else {
+      c = match_task<false, Q, WGT>(splan[w], G, row, qr.z, t.w < 0 ? -1 : (int64_t)t.w * span, span, buf, ~0ull,
+                                    nullptr, nullptr);
+    }
+    c = warp_sum(c);
     if (lane == 0 && c) atomicAdd(&out[(int64_t)t.z * nm + (member ? member[row[0]] : 0)], c);
   }
 }
@@ -1081,6 +1370,12 @@ __global__ void k_row_tasks(WidePlan q, const int32_t *__restrict__ rows, int64_
     cnt[i] = span > 0 ? max((int64_t)1, (best + span - 1) / span) : 1;
   }
 }
+// 32 pairs per task (three-position plans): chunk field -1 - pairs
+__global__ void k_pair_tasks(int64_t nrows, int query, int4 *__restrict__ tasks) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; 32 * i < nrows; i += (int64_t)gridDim.x * blockDim.x)
+    tasks[i] = make_int4((int)(uint32_t)(32 * i), (int)((32 * i) >> 32), query,
+                         -1 - (int)min((int64_t)32, nrows - 32 * i));
+}
 __global__ void k_expand_tasks(int64_t nrows, const int64_t *__restrict__ first, const int64_t *__restrict__ cnt,
                                int query, int split, int4 *__restrict__ tasks) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nrows; i += (int64_t)gridDim.x * blockDim.x)
@@ -1095,6 +1390,19 @@ __global__ void k_small_counts(int64_t n, const int32_t *__restrict__ labels, in
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < tot; i += (int64_t)gridDim.x * blockDim.x) {
     if (pairs) atomicAdd(&dst[member ? member[pairs[i].x] : 0], 1ull);
     else if (labels[i] == label) atomicAdd(&dst[member ? member[i] : 0], 1ull);
+  }
+}
+
+// *cross = 1 when an edge joins vertices of two members
+__global__ void k_member_cross(int64_t n, const int64_t *__restrict__ off, const int32_t *__restrict__ adj,
+                               const int32_t *__restrict__ member, int *__restrict__ cross) {
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t v = warp; v < n; v += nw) {
+    const int32_t m = member[v];
+    bool bad = false;
+    for (int64_t k = off[v] + lane_id(); k < off[v + 1]; k += 32) bad = bad || member[adj[k]] != m;
+    if (bad) *cross = 1;
   }
 }
 
@@ -1129,9 +1437,17 @@ static int batch_tasks(gpm_match_batch *b, int64_t span) {
   // position t of a row is split into chunks only when the depth-first walk
   // takes it (t <= n - 2; a row of depth n - 1 is closed at once)
   auto splits = [&](int k) { return span > 0 && b->depth[k] <= b->plans[k].n - 2; };
+  // pairs of three-position plans are closed 32 at a time (not with several
+  // members: the pairs of a task may have roots of different ones)
+  auto pooled = [&](int k) { return b->plans[k].n == 3 && b->depth[k] == 2 && b->nm == 1; };
   for (int k = 0; k < b->nq; ++k) {
     const int64_t np = b->nrows[k];
     if (b->plans[k].n < 3 || np == 0) continue;
+    if (pooled(k)) {
+      cnt_total[k] = (np + 31) / 32;
+      total += cnt_total[k];
+      continue;
+    }
     GPM_TRY(cnt[k].reserve(np));
     GPM_TRY(first[k].reserve(np + 1));
     k_row_tasks<<<blocks, 256>>>(b->plans[k], b->rows[k], np, b->depth[k], g->off.p, lc->loff.p, lc->L,
@@ -1153,7 +1469,8 @@ static int batch_tasks(gpm_match_batch *b, int64_t span) {
   for (int k = 0; k < b->nq; ++k) {
     if (!cnt_total[k]) continue;
     // each query's tasks at its own offset: shift the scan by `at`
-    k_expand_tasks<<<blocks, 256>>>(b->nrows[k], first[k].p, cnt[k].p, k, splits(k), b->tasks.p + at);
+    if (pooled(k)) k_pair_tasks<<<blocks, 256>>>(b->nrows[k], k, b->tasks.p + at);
+    else k_expand_tasks<<<blocks, 256>>>(b->nrows[k], first[k].p, cnt[k].p, k, splits(k), b->tasks.p + at);
     GPM_LAUNCH_CHECK();
     at += cnt_total[k];
   }
@@ -1164,14 +1481,14 @@ static int batch_tasks(gpm_match_batch *b, int64_t span) {
   return GPM_OK;
 }
 
-template <int Q>
+template <int Q, bool WGT>
 static int batch_grid() {
   static PerDevice grid;
   return grid.get([] {
     constexpr int smem = match_dyn_smem<Q>();
-    if (smem > 0) cudaFuncSetAttribute(k_match_batch<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (smem > 0) cudaFuncSetAttribute(k_match_batch<Q, WGT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_match_batch<Q>, kMatchWarps * 32, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_match_batch<Q, WGT>, kMatchWarps * 32, smem);
     return std::max(1, per_sm) * num_sms();
   });
 }
@@ -1182,18 +1499,22 @@ static int batch_launch(gpm_match_batch *b, cudaStream_t st) {
   const size_t bytes = sizeof(unsigned long long) * b->nq * b->nm;
   GPM_CUDA(cudaMemcpyAsync(b->out.p, b->base.p, bytes, cudaMemcpyDeviceToDevice, st));
   GPM_CUDA(cudaMemsetAsync(b->cursor.p, 0, 8, st));
+  const int32_t *member = b->nm > 1 ? b->member.p : nullptr;
+  for (const auto &c : b->cycles)
+    GPM_TRY(cycle_launch(g, lc, c.second, b->cycle, member, b->out.p + (size_t)c.first * b->nm, st));
   if (b->ntasks == 0) return GPM_OK;
   const MatchGraph G{g->off.p, g->adj.p, lc->ladj.p, lc->loff.p, g->labels.p, lc->L,
                      HubIndex{lc->hub_slot.p, lc->hub_bm.p, lc->hub_words}};
-  const int32_t *member = b->nm > 1 ? b->member.p : nullptr;
-  if (b->qcap <= kNarrowQ)
-    k_match_batch<kNarrowQ><<<b->grid, kMatchWarps * 32, 0, st>>>(
-        reinterpret_cast<const QueryPlan *>(b->dplans.p), b->drows.p, G, b->tasks.p, b->ntasks, b->span, member,
-        b->nm, b->cursor.p, b->out.p);
+  auto launch = [&](auto kernel, auto plans, int smem) {
+    kernel<<<b->grid, kMatchWarps * 32, smem, st>>>(plans, b->drows.p, G, b->tasks.p, b->ntasks, b->span, member, b->nm,
+                                                    b->cursor.p, b->out.p);
+  };
+  if (b->qcap > kNarrowQ)
+    launch(k_match_batch<kMaxQ, false>, reinterpret_cast<const WidePlan *>(b->dplans.p), match_dyn_smem<kMaxQ>());
+  else if (b->weighted)
+    launch(k_match_batch<kNarrowQ, true>, reinterpret_cast<const QueryPlan *>(b->dplans.p), 0);
   else
-    k_match_batch<kMaxQ><<<b->grid, kMatchWarps * 32, match_dyn_smem<kMaxQ>(), st>>>(
-        reinterpret_cast<const WidePlan *>(b->dplans.p), b->drows.p, G, b->tasks.p, b->ntasks, b->span, member,
-        b->nm, b->cursor.p, b->out.p);
+    launch(k_match_batch<kNarrowQ, false>, reinterpret_cast<const QueryPlan *>(b->dplans.p), 0);
   GPM_LAUNCH_CHECK();
   return GPM_OK;
 }
@@ -1275,11 +1596,35 @@ int gpm_match_batch_create(gpm_graph *g, int nq, const gpm_query *const *queries
                      HubIndex{lc->hub_slot.p, lc->hub_bm.p, lc->hub_words}};
   DevBuf<unsigned long long> np;
   if ((s = np.reserve(1))) return bail(s);
+  // a factored plan may start at another root, whose member is the same one
+  // when no edge joins two members
+  bool factor = true;
+  if (b->nm > 1 && g->n > 0) {
+    DevBuf<int> cross;
+    int hcross = 0;
+    if ((s = cross.reserve(1))) return bail(s);
+    GPM_CUDA(cudaMemset(cross.p, 0, sizeof(int)));
+    k_member_cross<<<(int)std::min<int64_t>((g->n * 32 + 255) / 256, (int64_t)num_sms() * 16), 256>>>(
+        g->n, g->off.p, g->adj.p, b->member.p, cross.p);
+    GPM_CUDA(cudaMemcpy(&hcross, cross.p, sizeof(int), cudaMemcpyDeviceToHost));
+    factor = hcross == 0;
+  }
   const int blocks = (int)std::min<int64_t>((g->n * 32 + 255) / 256, (int64_t)num_sms() * 16);
   const int sblocks = (int)std::min<int64_t>((g->n + 255) / 256 + 1, (int64_t)num_sms() * 8);
   for (int k = 0; k < nq; ++k) {
     WidePlan &p = b->plans[k];
     if ((s = plan_query(queries[k], freq, &p))) return bail(s);
+    if (factor && b->qcap <= kNarrowQ) factor_query(queries[k], freq, g->n, g->nnz, &p);
+    b->weighted = b->weighted || p.nw > 0;
+    if (factor && is_cycle4(queries[k], lc)) {
+      CyclePlan cp;
+      bool fits = false;
+      if ((s = cycle_plan(g, lc, queries[k], &cp, &b->cycle, &fits))) return bail(s);
+      if (fits) {
+        b->cycles.emplace_back(k, cp);
+        continue;
+      }
+    }
     if (p.n == 1) {
       if (g->n) k_small_counts<<<sblocks, 256>>>(g->n, g->labels.p, p.label[0], nullptr, 0,
                                                   b->nm > 1 ? b->member.p : nullptr, b->base.p + (size_t)k * b->nm);
@@ -1318,10 +1663,10 @@ int gpm_match_batch_create(gpm_graph *g, int nq, const gpm_query *const *queries
     std::vector<QueryPlan> narrow(nq);
     for (int k = 0; k < nq; ++k) narrow_plan(b->plans[k], &narrow[k]);
     GPM_CUDA(cudaMemcpy(b->dplans.p, narrow.data(), plan_bytes * nq, cudaMemcpyHostToDevice));
-    b->grid = batch_grid<kNarrowQ>();
+    b->grid = b->weighted ? batch_grid<kNarrowQ, true>() : batch_grid<kNarrowQ, false>();
   } else {
     GPM_CUDA(cudaMemcpy(b->dplans.p, b->plans.data(), plan_bytes * nq, cudaMemcpyHostToDevice));
-    b->grid = batch_grid<kMaxQ>();
+    b->grid = batch_grid<kMaxQ, false>();
   }
   if ((s = batch_tasks(b, 0))) return bail(s);
   *out = b;
