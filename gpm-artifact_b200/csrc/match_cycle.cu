@@ -9,7 +9,7 @@
 // vertex of c's label class, the walk a - d - c adds up the counters it meets.
 // The work is the wedges, not the embeddings (R-MAT 19, labels 0 0 3 1: 0.6 G
 // wedges; 145-178 ms by the depth-first walk, which tests every wedge for its
-// closing edge, 4.9 ms here, 3.4 of it in k_cycle_big: 0.6 G increments and as
+// closing edge, 3.4 ms here, most of it in k_cycle_big: 0.6 G increments and as
 // many loads and clears at 180 G/s, bound by shared-memory atomics).
 //
 // Counters are indexed by the rank inside the label class in descending degree
@@ -89,7 +89,10 @@ __device__ __forceinline__ unsigned long long wedge_bound(const CycleArgs &A, in
 }
 
 // Roots with wedges on both sides into the queue of their size; a warp takes
-// 32 roots and queues them with one atomic per queue.  The side with fewer
+// 32 roots and queues them with one atomic per queue.  Roots come in descending
+// degree order, so a warp takes every (nroots / 32)-th of them: 32 neighbours
+// would give all hubs to a few warps (R-MAT 19, labels 0 0 3 1: 1.3-2.1 ms; the
+// whole call 5.6 ms then, 3.4 ms now).  The side with fewer
 // wedges is the one that is counted (its counters are written and cleared).
 __global__ void k_cycle_split(CycleArgs A, const int32_t *__restrict__ roots, int64_t nroots, int2 *__restrict__ small,
                               int2 *__restrict__ big, int *__restrict__ sizes) {
@@ -97,11 +100,12 @@ __global__ void k_cycle_split(CycleArgs A, const int32_t *__restrict__ roots, in
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const bool same = A.lb == A.ld;
-  for (int64_t r0 = warp * 32; r0 < nroots; r0 += nw * 32) {
+  const int64_t groups = (nroots + 31) / 32;
+  for (int64_t r0 = warp; r0 < groups; r0 += nw) {
     int2 mine = make_int2(0, 0);
     int which = 0;  // 1 small, 2 big
-    for (int j = 0; j < 32 && r0 + j < nroots; ++j) {
-      const int32_t v = roots[r0 + j];
+    for (int j = 0; j < 32 && r0 + j * groups < nroots; ++j) {
+      const int32_t v = roots[r0 + j * groups];
       const unsigned long long wb = wedge_bound(A, v, A.lb, lane), wd = same ? wb : wedge_bound(A, v, A.ld, lane);
       if ((int)lane == j && min(wb, wd) > 0) {
         mine = make_int2(v, wd < wb);
