@@ -56,17 +56,29 @@ struct ArenaScope {
   Arena *prev;
 };
 
+// Every other allocation comes from a process-wide pool of freed blocks, per
+// device.  Freeing waits for the device, as cudaFree does, so a block in the
+// pool is idle and may go to any thread and stream; at most kPoolBytes are
+// kept per device, all of them are given back when an allocation fails or
+// plans are dropped, and larger remainders go straight to cudaFree.  (A first
+// triangle count on R-MAT 22 made 56 cudaMalloc and 37 cudaFree calls: 27 of
+// its 37 ms.)
+void *pool_get(size_t bytes, size_t *cap, int *dev);  // nullptr: out of memory (cudaGetLastError not cleared)
+void pool_put(void *p, size_t cap, int dev);
+void pool_trim();  // the current device's cached blocks back to the driver
+
 // Owning device allocation; move-only.
 template <typename T>
 struct DevBuf {
   T *p = nullptr;
   size_t n = 0;
-  Arena *arena = nullptr;  // pool the block came from (nullptr: cudaMalloc)
-  size_t cap = 0;          // bytes of a pooled block
+  Arena *arena = nullptr;  // arena the block came from (nullptr: the process-wide pool)
+  size_t cap = 0;          // bytes of the block
+  int dev = 0;             // its device (process-wide pool)
   DevBuf() = default;
   DevBuf(const DevBuf &) = delete;
   DevBuf &operator=(const DevBuf &) = delete;
-  DevBuf(DevBuf &&o) noexcept : p(o.p), n(o.n), arena(o.arena), cap(o.cap) {
+  DevBuf(DevBuf &&o) noexcept : p(o.p), n(o.n), arena(o.arena), cap(o.cap), dev(o.dev) {
     o.p = nullptr;
     o.n = 0;
     o.arena = nullptr;
@@ -78,6 +90,7 @@ struct DevBuf {
       n = o.n;
       arena = o.arena;
       cap = o.cap;
+      dev = o.dev;
       o.p = nullptr;
       o.n = 0;
       o.arena = nullptr;
@@ -88,7 +101,7 @@ struct DevBuf {
   void reset() {
     if (p) {
       if (arena) arena_put(arena, p, cap);
-      else cudaFree(p);
+      else pool_put(p, cap, dev);
     }
     p = nullptr;
     n = 0;
@@ -106,13 +119,9 @@ struct DevBuf {
       n = count ? count : 1;
       return GPM_OK;
     }
-    cudaError_t e = cudaMalloc((void **)&p, bytes);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      p = nullptr;
-      return fail(GPM_ENOMEM, "cudaMalloc(" + std::to_string(bytes) + " B) failed: " +
-                                  cudaGetErrorString(e));
-    }
+    p = static_cast<T *>(pool_get(bytes, &cap, &dev));
+    if (!p) return fail(GPM_ENOMEM, "cudaMalloc(" + std::to_string(bytes) + " B) failed: " +
+                                        cudaGetErrorString(cudaGetLastError()));
     n = count ? count : 1;
     return GPM_OK;
   }

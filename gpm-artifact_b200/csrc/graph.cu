@@ -590,6 +590,7 @@ int gpm_graph_drop_plans(gpm_graph *g) {
   if (!g) return fail(GPM_EINVAL, "NULL graph");
   GPM_CUDA(cudaDeviceSynchronize());  // no kernel may still read what is freed
   drop_plans(g);
+  pool_trim();
   return GPM_OK;
 }
 

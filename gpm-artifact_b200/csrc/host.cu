@@ -16,6 +16,7 @@
 #include <fstream>
 #include <limits>
 #include <map>
+#include <mutex>
 #include <sstream>
 #include <string>
 #include <vector>
@@ -84,6 +85,87 @@ ArenaScope::ArenaScope() : prev(tl_active) {
   tl_active = &tl_arena;
 }
 ArenaScope::~ArenaScope() { tl_active = prev; }
+
+struct BlockPool {
+  static constexpr int kDevices = 64;
+  static constexpr size_t kPoolBytes = (size_t)4 << 30;  // cached bytes per device
+  std::mutex mu;
+  std::multimap<size_t, void *> blocks[kDevices];  // size -> idle block
+  size_t bytes[kDevices] = {};
+};
+// never destroyed: buffers of static and thread-local objects may be freed
+// after the end of main
+static BlockPool &block_pool() {
+  static BlockPool *p = new BlockPool();
+  return *p;
+}
+// sizes are rounded up by at most an eighth, so that blocks of nearly equal
+// requests serve one another
+static size_t pool_size(size_t bytes) {
+  size_t step = 512;
+  while (step * 16 <= bytes) step *= 2;
+  return (bytes + step - 1) / step * step;
+}
+
+static void pool_trim_device(int dev) {
+  BlockPool &P = block_pool();
+  std::vector<void *> gone;
+  {
+    std::lock_guard<std::mutex> lock(P.mu);
+    for (auto &b : P.blocks[dev]) gone.push_back(b.second);
+    P.blocks[dev].clear();
+    P.bytes[dev] = 0;
+  }
+  for (void *p : gone) cudaFree(p);
+}
+
+void pool_trim() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < BlockPool::kDevices) pool_trim_device(dev);
+}
+
+void *pool_get(size_t bytes, size_t *cap, int *dev) {
+  BlockPool &P = block_pool();
+  const size_t want = pool_size(bytes);
+  void *p = nullptr;
+  *dev = 0;
+  if (cudaGetDevice(dev) != cudaSuccess) return nullptr;
+  const bool pooled = *dev >= 0 && *dev < BlockPool::kDevices;
+  if (pooled) {
+    std::lock_guard<std::mutex> lock(P.mu);
+    auto &blocks = P.blocks[*dev];
+    auto it = blocks.lower_bound(want);
+    if (it != blocks.end() && it->first <= want + want / 4) {
+      p = it->second;
+      *cap = it->first;
+      P.bytes[*dev] -= it->first;
+      blocks.erase(it);
+      return p;
+    }
+  }
+  *cap = want;
+  if (cudaMalloc(&p, want) == cudaSuccess) return p;
+  if (!pooled) return nullptr;
+  cudaGetLastError();
+  pool_trim_device(*dev);
+  return cudaMalloc(&p, want) == cudaSuccess ? p : nullptr;
+}
+
+void pool_put(void *p, size_t cap, int dev) {
+  BlockPool &P = block_pool();
+  int cur = -1;
+  // as with cudaFree, work in flight on the device ends first
+  if (dev >= 0 && dev < BlockPool::kDevices && cudaGetDevice(&cur) == cudaSuccess && cur == dev &&
+      cudaDeviceSynchronize() == cudaSuccess) {
+    std::lock_guard<std::mutex> lock(P.mu);
+    if (P.bytes[dev] + cap <= BlockPool::kPoolBytes) {
+      P.blocks[dev].emplace(cap, p);
+      P.bytes[dev] += cap;
+      return;
+    }
+  }
+  cudaFree(p);
+}
 
 int ensure_device() {
   int n = 0;
