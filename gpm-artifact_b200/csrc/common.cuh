@@ -200,6 +200,29 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
+// Warp tasks of a queue sorted heaviest first, handed out by an atomic cursor:
+// the first `lone` one at a time, the others in runs of kTaskRun.  All grabs
+// meet in one word of L2, about one per clock, so a million small tasks taken
+// singly cost a third of a millisecond whatever they do (Erdos-Renyi, 10^6
+// vertices of mean degree 12: 588 us per triangle count, 334 us in runs;
+// R-MAT 22: 4.94 -> 4.86 ms).
+constexpr int kTaskRun = 8;
+struct WarpTasks {
+  int t = -1;
+  // the next task (at or past the queue's end when there is none)
+  __device__ __forceinline__ int next(int *cursor, int lone, unsigned lane) {
+    if (t < lone || ((t + 1 - lone) & (kTaskRun - 1)) == 0) {
+      int u = 0;
+      if (lane == 0) u = atomicAdd(cursor, 1);
+      u = __shfl_sync(0xffffffffu, u, 0);
+      t = u < lone ? u : lone + (u - lone) * kTaskRun;
+    } else {
+      ++t;
+    }
+    return t;
+  }
+};
+
 // ---------------------------------------------------------------- graph handle
 struct TcPlan;
 struct RankPlan;
@@ -215,6 +238,8 @@ struct gpm_graph {
   int64_t n = 0;
   int64_t nnz = 0;
   int32_t max_deg = 0;
+  uint64_t sum_deg2 = 0;  // sum of the squared list lengths
+  double hash_us = 0;     // estimated time of gpm_tc's counts with the hash kernel (tc.cu)
   int oriented = 0;
   int relabeled = 0;
   int device = 0;

@@ -163,10 +163,9 @@ __global__ void __launch_bounds__(kSmallWarps * 32)
   unsigned long long c = 0;
   for (int i = lane; i < kSmallSlots; i += 32) tab[i] = make_int2(-1, 0);
   __syncwarp();
+  WarpTasks queue;
   while (true) {
-    int t = 0;
-    if (lane == 0) t = atomicAdd(&sizes[2], 1);
-    t = __shfl_sync(0xffffffffu, t, 0);
+    const int t = queue.next(&sizes[2], 0, lane);
     if (t >= n) break;
     const int2 task = tasks[t];
     const int32_t self = A.skip_root ? A.lrank[task.x] : -1;

@@ -267,10 +267,9 @@ __global__ void __launch_bounds__(256, GPM_TC_RANK_MIN_BLOCKS)
   const int wid = threadIdx.x >> 5;
   const unsigned lane = threadIdx.x & 31;
   uint32_t *region = rsm + wid * kWarpWords;
+  WarpTasks queue;
   while (true) {
-    int t = 0;
-    if (lane == 0) t = atomicAdd(&counters[1], 1);
-    t = __shfl_sync(0xffffffffu, t, 0);
+    const int t = queue.next(&counters[1], gridDim.x * kRWarps * 8, lane);
     if (t >= n_warp) break;
     const int32_t x = warp_tasks[t];
     c += owner_task<false, REC>(x, roff, radj, radj4, poff, pseg, plong, pshort, region, kWarpWords,
