@@ -148,31 +148,38 @@ int build_csr_device(gpm_graph *g, int64_t n, int64_t m, const int32_t *d_src,
   return GPM_OK;
 }
 
-__global__ void k_degrees(int64_t n, const int64_t *__restrict__ off, int32_t *__restrict__ deg) {
+// out[0] = max list length, out[1] = sum of the squared lengths
+__global__ void k_degrees(int64_t n, const int64_t *__restrict__ off, unsigned long long *__restrict__ out) {
+  unsigned long long mx = 0, sq = 0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    deg[i] = (int32_t)(off[i + 1] - off[i]);
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const unsigned long long d = (unsigned long long)(off[i + 1] - off[i]);
+    mx = max(mx, d);
+    sq += d * d;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  sq = warp_sum(sq);
+  if (lane_id() == 0 && mx) {
+    atomicMax(&out[0], mx);
+    atomicAdd(&out[1], sq);
+  }
 }
 
 int compute_max_degree(gpm_graph *g, cudaStream_t st) {
-  if (g->n == 0) {
-    g->max_deg = 0;
-    return GPM_OK;
-  }
-  DevBuf<int32_t> deg, mx;
-  GPM_TRY(deg.reserve(g->n));
-  GPM_TRY(mx.reserve(1));
-  k_degrees<<<grid_for(g->n), 256, 0, st>>>(g->n, g->off.p, deg.p);
+  g->max_deg = 0;
+  g->sum_deg2 = 0;
+  if (g->n == 0) return GPM_OK;
+  DevBuf<unsigned long long> mx;
+  GPM_TRY(mx.reserve(2));
+  GPM_CUDA(cudaMemsetAsync(mx.p, 0, 16, st));
+  k_degrees<<<std::min(grid_for(g->n), num_sms() * 2), 256, 0, st>>>(g->n, g->off.p, mx.p);
   GPM_LAUNCH_CHECK();
-  size_t tmp = 0;
-  GPM_CUDA(cub::DeviceReduce::Max(nullptr, tmp, deg.p, mx.p, (int)g->n, st));
-  DevBuf<char> t;
-  GPM_TRY(t.reserve(tmp));
-  GPM_CUDA(cub::DeviceReduce::Max(t.p, tmp, deg.p, mx.p, (int)g->n, st));
-  int32_t h = 0;
-  GPM_CUDA(cudaMemcpyAsync(&h, mx.p, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+  unsigned long long h[2] = {0, 0};
+  GPM_CUDA(cudaMemcpyAsync(h, mx.p, sizeof h, cudaMemcpyDeviceToHost, st));
   GPM_CUDA(cudaStreamSynchronize(st));
-  g->max_deg = h;
+  g->max_deg = (int32_t)h[0];
+  g->sum_deg2 = h[1];
   return GPM_OK;
 }
 
@@ -382,6 +389,7 @@ using namespace gpm;
 
 namespace gpm {
 void drop_plans(gpm_graph *g) {
+  g->hash_us = 0;
   free_tc_plan(g->tc);
   g->tc = nullptr;
   free_rank_plan(g->rank);

@@ -273,20 +273,25 @@ __device__ unsigned long long warp_task(int32_t u, const int64_t *__restrict__ o
   return c;
 }
 
-__global__ void __launch_bounds__(256) k_tc_hash(const int64_t *__restrict__ off,
-                                                 const int32_t *__restrict__ adj,
-                                                 const int32_t *__restrict__ cta_tasks, int n_cta,
-                                                 const int32_t *__restrict__ warp_tasks, int n_warp,
-                                                 int *__restrict__ counters,
-                                                 unsigned long long *__restrict__ out) {
-  extern __shared__ __align__(16) char smem[];
-  __shared__ int s_task;
+// The CTA's part of the count over both queues.  `even`: no list is longer
+// than kEvenDegree, so the tail tasks cost about the same; they are dealt out
+// in turn while each warp has at most kTaskRun of them (their cost is a few
+// memory latencies, less than the cursor's), and taken from the cursor in runs
+// of kTaskRun otherwise (ER, 10^6 vertices of mean degree 12: 621 -> 339 us).
+// Uneven tasks come one at a time: R-MAT 16 took 688 us in runs, 463 singly.
+constexpr int kEvenDegree = 48;
+__device__ __forceinline__ unsigned long long hash_tasks(const int64_t *__restrict__ off,
+                                                         const int32_t *__restrict__ adj,
+                                                         const int32_t *__restrict__ cta_tasks, int n_cta,
+                                                         const int32_t *__restrict__ warp_tasks, int n_warp,
+                                                         int *__restrict__ counters, bool even, char *smem,
+                                                         int *s_task) {
   unsigned long long c = 0;
   // hub queue: one task per CTA at a time
-  while (true) {
-    if (threadIdx.x == 0) s_task = atomicAdd(&counters[0], 1);
+  while (n_cta > 0) {
+    if (threadIdx.x == 0) *s_task = atomicAdd(&counters[0], 1);
     __syncthreads();
-    int t = s_task;
+    int t = *s_task;
     __syncthreads();
     if (t >= n_cta) break;
     c += cta_task(cta_tasks[t], off, adj, smem);
@@ -294,15 +299,59 @@ __global__ void __launch_bounds__(256) k_tc_hash(const int64_t *__restrict__ off
   // tail queue: one task per warp at a time
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   char *region = smem + warp * kWarpBytes;
-  while (true) {
-    int t = 0;
-    if (lane == 0) t = atomicAdd(&counters[1], 1);
-    t = __shfl_sync(0xffffffffu, t, 0);
-    if (t >= n_warp) break;
-    c += warp_task(warp_tasks[t], off, adj, region);
+  const int warps = gridDim.x * kWarps;
+  if (even && (int64_t)n_warp <= (int64_t)warps * kTaskRun) {
+    for (int t = blockIdx.x * kWarps + warp; t < n_warp; t += warps) c += warp_task(warp_tasks[t], off, adj, region);
+  } else {
+    WarpTasks queue;
+    while (true) {
+      const int t = queue.next(&counters[1], even ? 0 : n_warp, lane);
+      if (t >= n_warp) break;
+      c += warp_task(warp_tasks[t], off, adj, region);
+    }
   }
+  return c;
+}
+
+// The CTA's sum of c in thread 0.
+__device__ __forceinline__ unsigned long long cta_sum(unsigned long long c) {
+  __shared__ unsigned long long s_part[kWarps];
   c = warp_sum(c);
-  if (lane == 0 && c) atomicAdd(out, c);
+  if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = c;
+  __syncthreads();
+  c = 0;
+  if (threadIdx.x == 0)
+    for (int w = 0; w < kWarps; ++w) c += s_part[w];
+  return c;
+}
+
+// state: two cursors, the number of CTAs that have ended, and the sum, all
+// zero before the launch; the last CTA writes *out and leaves them zero, so a
+// repeated count is this launch alone (ER, 16,384 vertices: 26 us per count
+// before, with two memsets and one atomic per warp and task).
+struct HashState {
+  int cursor[2], done, pad;
+  unsigned long long sum;
+};
+__global__ void __launch_bounds__(256) k_tc_hash(const int64_t *__restrict__ off,
+                                                 const int32_t *__restrict__ adj,
+                                                 const int32_t *__restrict__ cta_tasks, int n_cta,
+                                                 const int32_t *__restrict__ warp_tasks, int n_warp,
+                                                 HashState *__restrict__ state, int even,
+                                                 unsigned long long *__restrict__ out) {
+  extern __shared__ __align__(16) char smem[];
+  __shared__ int s_task;
+  const unsigned long long c =
+      cta_sum(hash_tasks(off, adj, cta_tasks, n_cta, warp_tasks, n_warp, state->cursor, even != 0, smem, &s_task));
+  if (threadIdx.x == 0) {
+    if (c) atomicAdd(&state->sum, c);
+    __threadfence();
+    if (atomicAdd(&state->done, 1) == (int)gridDim.x - 1) {
+      __threadfence();
+      *out = atomicExch(&state->sum, 0ull);
+      state->cursor[0] = state->cursor[1] = state->done = 0;
+    }
+  }
 }
 
 // Task split by degree (the reference's USE_WARP / USE_CTA thresholds).
@@ -340,11 +389,13 @@ int tc_build_plan(gpm_graph *g, int warp_min, int cta_min, cudaStream_t st) {
   p->cta_min = cta_min;
   int64_t n = g->n;
   int s = GPM_OK;
-  if ((s = p->cta_tasks.reserve(n)) || (s = p->warp_tasks.reserve(n)) || (s = p->counters.reserve(4)) ||
+  static_assert(sizeof(HashState) == 6 * sizeof(int), "plan counters hold a HashState");
+  if ((s = p->cta_tasks.reserve(n)) || (s = p->warp_tasks.reserve(n)) || (s = p->counters.reserve(6)) ||
       (s = p->sizes.reserve(2))) {
     delete p;
     return s;
   }
+  cudaMemsetAsync(p->counters.p, 0, 6 * sizeof(int), st);
   cudaMemsetAsync(p->sizes.p, 0, 2 * sizeof(int), st);
   if (n > 0) {
     int grid = (int)std::min<int64_t>((n + 255) / 256, (int64_t)num_sms() * 8);
@@ -364,7 +415,7 @@ int tc_build_plan(gpm_graph *g, int warp_min, int cta_min, cudaStream_t st) {
 }
 
 int tc_launch(gpm_graph *g, int variant, cudaStream_t st, unsigned long long *d_out) {
-  GPM_CUDA(cudaMemsetAsync(d_out, 0, sizeof(unsigned long long), st));
+  if (variant != GPM_TC_HASH || g->nnz == 0) GPM_CUDA(cudaMemsetAsync(d_out, 0, sizeof(unsigned long long), st));
   if (g->nnz == 0) return GPM_OK;
   if (variant == GPM_TC_BSEARCH || variant == GPM_TC_MERGE) {
     GPM_TRY(ensure_src(g, st));
@@ -381,14 +432,38 @@ int tc_launch(gpm_graph *g, int variant, cudaStream_t st, unsigned long long *d_
     GPM_TRY(tc_build_plan(g, 2, 101, st));
     TcPlan *p = g->tc;
     if (p->cta_min - 1 > kWarpChunk) return fail(GPM_EINVAL, "warp tasks exceed the warp table");
-    GPM_CUDA(cudaMemsetAsync(p->counters.p, 0, 4 * sizeof(int), st));
-    k_tc_hash<<<tc_hash_grid(), 256, TC_SMEM, st>>>(g->off.p, g->adj.p, p->cta_tasks.p, p->n_cta,
-                                                    p->warp_tasks.p, p->n_warp, p->counters.p, d_out);
+    const int64_t blocks = (int64_t)p->n_cta + ((int64_t)p->n_warp + kWarps - 1) / kWarps;
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(tc_hash_grid(), blocks));
+    k_tc_hash<<<grid, 256, TC_SMEM, st>>>(g->off.p, g->adj.p, p->cta_tasks.p, p->n_cta, p->warp_tasks.p, p->n_warp,
+                                          reinterpret_cast<HashState *>(p->counters.p), g->max_deg <= kEvenDegree, d_out);
     GPM_LAUNCH_CHECK();
     return GPM_OK;
   }
   if (variant == GPM_TC_BITMAP) return rank_launch(g, st, d_out);
   return fail(GPM_EINVAL, "unknown triangle-count variant " + std::to_string(variant));
+}
+
+// gpm_tc's kernel.  The rank plan's repeated counts are the faster ones on
+// every graph of some size, but the plan has to be built first.  Microseconds
+// (hash count; rank count; its first count, plan included): R-MAT 14: 145, 83,
+// 654; R-MAT 17: 965, 181, 1163; R-MAT 18: 2298, 223, 1486; R-MAT 20: 13755,
+// 874, 3695; Chung-Lu 300,007 x 24: 445, 195, 1051; ER 10^6 x 12: 621, 588,
+// 2915.  So a count builds the plan at once where the hash kernel would
+// clearly take longer than that (the sum of squared degrees follows its time
+// within a factor of two, 5 ps each), and otherwise when the counts made on
+// this graph with the hash kernel have cost as much as the plan.
+static int tc_auto_launch(gpm_graph *g, cudaStream_t st, unsigned long long *d_out) {
+  if (!g->rank && g->nnz > 0) {
+    const double hash_us = 10 + 5e-6 * (double)g->sum_deg2, plan_us = 300 + 2.5e-4 * (double)g->nnz;
+    if (hash_us < 40 || g->hash_us + hash_us < plan_us) {
+      g->hash_us += hash_us;
+      return tc_launch(g, GPM_TC_HASH, st, d_out);
+    }
+  }
+  const int s = tc_launch(g, GPM_TC_BITMAP, st, d_out);
+  if (s != GPM_ENOMEM && s != GPM_EUNSUPPORTED) return s;
+  g->hash_us = -1e30;  // not tried again
+  return tc_launch(g, GPM_TC_HASH, st, d_out);  // no room for the plan, or beyond its descriptors
 }
 
 }  // namespace gpm
@@ -408,8 +483,7 @@ int gpm_tc(gpm_graph *g, int mode, uint64_t *out) {
   if (!g || !out) return fail(GPM_EINVAL, "gpm_tc: NULL argument");
   if (mode != GPM_V_CENTRIC && mode != GPM_E_CENTRIC) return fail(GPM_EINVAL, "Wrong Calculation Mode.");
   GPM_TRY(g->result.reserve(8));
-  int variant = mode == GPM_V_CENTRIC ? GPM_TC_HASH : GPM_TC_BSEARCH;
-  GPM_TRY(tc_launch(g, variant, 0, (unsigned long long *)g->result.p));
+  GPM_TRY(tc_auto_launch(g, 0, (unsigned long long *)g->result.p));
   GPM_CUDA(cudaMemcpy(out, g->result.p, sizeof(uint64_t), cudaMemcpyDeviceToHost));
   return GPM_OK;
 }
@@ -528,27 +602,9 @@ __global__ void __launch_bounds__(256) k_tc_hash_noalloc(const int64_t *__restri
                                                          unsigned long long *__restrict__ out) {
   extern __shared__ __align__(16) char smem[];
   __shared__ int s_task;
-  const int n_cta = sizes[0], n_warp = sizes[1];
-  unsigned long long c = 0;
-  while (true) {
-    if (threadIdx.x == 0) s_task = atomicAdd(&counters[0], 1);
-    __syncthreads();
-    int t = s_task;
-    __syncthreads();
-    if (t >= n_cta) break;
-    c += cta_task(cta_tasks[t], off, adj, smem);
-  }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  char *region = smem + warp * kWarpBytes;
-  while (true) {
-    int t = 0;
-    if (lane == 0) t = atomicAdd(&counters[1], 1);
-    t = __shfl_sync(0xffffffffu, t, 0);
-    if (t >= n_warp) break;
-    c += warp_task(warp_tasks[t], off, adj, region);
-  }
-  c = warp_sum(c);
-  if (lane == 0 && c) atomicAdd(out, c);
+  const unsigned long long c =
+      cta_sum(hash_tasks(off, adj, cta_tasks, sizes[0], warp_tasks, sizes[1], counters, false, smem, &s_task));
+  if (threadIdx.x == 0 && c) atomicAdd(out, c);
 }
 
 }  // namespace gpm

@@ -182,9 +182,10 @@ int gpm_graph_work(gpm_graph *g, uint64_t *wedge_work, uint64_t *pair_work);
 /* TCSolver (src/TCSolver.cuh:9-121): sum over stored edges u->v of
  * |N(u) & N(v)|.  On an oriented graph this is the triangle count (the
  * reference's Engine::RunTC orients first, src/Engine.h:47-56).
- * mode: GPM_V_CENTRIC / GPM_E_CENTRIC choose the default variant
- * (GPM_TC_HASH / GPM_TC_BSEARCH) when variant == GPM_TC_AUTO and no trained
- * scheduler is attached. */
+ * mode: GPM_V_CENTRIC or GPM_E_CENTRIC, the reference's two kernels; both
+ * give the same count, and both run the kernel that suits the graph: the
+ * GPM_TC_HASH kernel for small graphs and first counts, GPM_TC_BITMAP once its
+ * plan pays (src/TCSolver.cuh chooses by mode alone). */
 int gpm_tc(gpm_graph *g, int mode, uint64_t *out);
 /* Explicit variant, asynchronous: writes the count to device memory d_out
  * (8 bytes) on stream; no host synchronisation; capturable. */
