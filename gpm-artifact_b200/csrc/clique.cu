@@ -14,8 +14,15 @@
 //   * tasks with |L| <= 64: one warp, rows are uint64 held in shared memory,
 //     one lane per starting row;
 //   * tasks with 64 < |L| <= 2048: one CTA, rows of W = ceil(|L|/32) words
-//     in shared memory (or a per-CTA global slab when they do not fit), each
-//     warp walks rows with the bitset spread over its lanes.
+//     in shared memory (or a per-CTA global slab when they do not fit).
+// Building the rows is most of the work of a 4-clique count (R-MAT 20: 4.2 G
+// list entries looked up in L, 1.4 G row words ANDed afterwards), so an entry
+// is looked up in a hash table of L's positions, a row whose list is much
+// longer than the rest of L looks that rest up in the list instead, and hubs
+// answer for the top ranks from a bitmap.  R-MAT 20, 4-cliques: 24.1 ms with a
+// binary search of L per entry, 13.2 ms with table and search, 7.6 ms with the
+// bitmaps too (6.5 ms CTA tasks, issue-bound with 11 of 32 lanes active in the
+// AND loops; 1.1 ms warp tasks).
 // Graphs whose stored edges do not all point upward in rank order, or with
 // an out-list longer than 2048, use an edge-centric kernel shaped like the
 // reference (materialised lists in per-warp global scratch).
@@ -32,15 +39,25 @@ namespace gpm {
 constexpr int kCqWarpMax = 64;      // warp tasks: |L| <= 64
 constexpr int kCqCtaMax = 2048;     // CTA tasks: |L| <= 2048 (W <= 64)
 constexpr int kCqMaxK = 8;
-#ifndef GPM_CQ_SMEM_KB
-// 32 KB: 5 CTAs per SM (registers allow 5; 48 KB allowed 4).  R-MAT 20 with
-// the lane-parallel last levels: 4-cliques 24.1 ms, 5-cliques 188 ms against
-// 27.0 / 194 ms at 48 KB and 24.3 / 195 ms at 40 KB (motif batch replay 809
-// against 835 ms).  Earlier, 48 KB beat 96 KB (2 CTAs per SM) by 1.6x.
-// Tasks whose rows do not fit use their CTA's global slab.
-#define GPM_CQ_SMEM_KB 32
-#endif
-constexpr size_t kCqSmem = GPM_CQ_SMEM_KB * 1024;  // dynamic shared memory per CTA
+// A row's list is searched for the rest of L when it is more than this many
+// times longer: a search is some ten dependent loads, a lookup one or two
+// shared-memory reads.
+constexpr int kCqSearch = 6;
+// Vertices with at least kCqCoreMin neighbours above them among the top kCqCore ranks
+// keep those as a bitmap (2 KB): whether they are adjacent to the rest of L
+// is then one bit test per member.
+constexpr int64_t kCqCore = 16384;
+constexpr int kCqCoreMin = 64;
+struct CqCore {
+  const int32_t *rowid;  // nullptr: no bitmaps
+  const uint32_t *rows;
+  int32_t base;
+  int words;
+};
+// CTA tasks whose layout (cq_layout) fits in kCqSmemSmall run in 256-thread CTAs, several per SM; larger ones in
+// 512-thread CTAs with kCqSmemBig, two per SM, and beyond that in a slab.
+constexpr size_t kCqSmemSmall = 44 * 1024, kCqSmemBig = 112 * 1024;
+constexpr int kCqSmallThreads = 256, kCqBigThreads = 512;
 
 static int grid_for(int64_t work, int block = 256) {
   int64_t g = (work + block - 1) / block;
@@ -48,16 +65,30 @@ static int grid_for(int64_t work, int block = 256) {
   return (int)std::max<int64_t>(1, std::min(g, cap));
 }
 
-// position of key in sorted L[0..d), or -1
-__device__ __forceinline__ int find_pos(const int32_t *L, int d, int32_t key) {
-  int lo = 0, hi = d - 1;
+// Positions of L's keys in an open-addressing table of 2^logcap slots (P =
+// uint8_t or uint16_t, all ones = empty); the key itself is read from L.
+template <class P>
+__device__ __forceinline__ int find_pos(const P *tab, int logcap, const int32_t *L, int32_t key) {
+  const uint32_t mask = (1u << logcap) - 1u;
+  uint32_t h = ((uint32_t)key * 2654435769u) >> (32 - logcap);
+  while (true) {
+    const int p = tab[h];
+    if (p == (int)(P)~(P)0) return -1;
+    if (L[p] == key) return p;
+    h = (h + 1) & mask;
+  }
+}
+
+// Is key in the sorted list a[0 .. n)?
+__device__ __forceinline__ bool in_list(const int32_t *__restrict__ a, int64_t n, int32_t key) {
+  int64_t lo = 0, hi = n - 1;
   while (lo <= hi) {
-    int mid = (lo + hi) >> 1;
-    int32_t x = L[mid];
-    if (x == key) return mid;
+    const int64_t mid = (lo + hi) >> 1;
+    const int32_t x = __ldg(a + mid);
+    if (x == key) return true;
     if (x < key) lo = mid + 1; else hi = mid - 1;
   }
-  return -1;
+  return false;
 }
 
 // first index in sorted a[0..n) with a[i] > key
@@ -108,68 +139,94 @@ __device__ unsigned long long local_count64(const unsigned long long *rows, unsi
   return c;
 }
 
+// Shared memory of a warp task.  Row i's list part that can meet L is radj[st[i]
+// .. st[i] + len[i]); scan[i] / pair[i]: inclusive prefixes of the entries to
+// look up in L, and of the pairs (i, j > i) to search in row i's list.
+struct CqWarp {
+  unsigned long long rows[kCqWarpMax];
+  int64_t st[kCqWarpMax];
+  int32_t L[kCqWarpMax], len[kCqWarpMax], scan[kCqWarpMax], pair[kCqWarpMax];
+  uint8_t tab[256];
+};
+
+// first i of 64 with pre[i] > x (pre inclusive, x < pre[63])
+__device__ __forceinline__ int segment_of(const int32_t *pre, int x) {
+  int lo = 0;
+#pragma unroll
+  for (int s = 32; s; s >>= 1)
+    if (pre[lo + s - 1] <= x) lo += s;
+  return lo;
+}
+
 __device__ unsigned long long clique_warp_task(int32_t u, int k, const int64_t *__restrict__ roff,
-                                               const int32_t *__restrict__ radj, int32_t *L,
-                                               unsigned long long *rows) {
+                                               const int32_t *__restrict__ radj, CqWarp &sm) {
   const unsigned lane = lane_id();
   const int64_t s0 = roff[u];
   const int d = (int)(roff[u + 1] - s0);
-  for (int i = lane; i < d; i += 32) {
-    L[i] = radj[s0 + i];
-    rows[i] = 0ull;
+  reinterpret_cast<uint2 *>(sm.tab)[lane] = make_uint2(~0u, ~0u);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int i = (int)lane + 32 * h;
+    if (i < d) sm.L[i] = radj[s0 + i];
+    sm.rows[i] = 0ull;
   }
   __syncwarp();
-  const int32_t kmax = L[d - 1];
-  // row i: members of L inside N+(L[i]) (all > L[i]); only N+(L[i]) up to
-  // kmax can hit.  Lane j finds the scan ranges of rows j and j + 32 (one
-  // binary search each, in parallel), then the ranges are laid end to end
-  // and every lane takes one entry of the concatenation per round, so short
-  // lists do not leave lanes idle.
-  long long sa = 0, la = 0, sb = 0, lb = 0;
-  if ((int)lane < d) {
-    const int32_t v = L[lane];
-    sa = roff[v];
-    la = upper_bound_g(radj + sa, roff[v + 1] - sa, kmax);
-  }
-  if ((int)lane + 32 < d) {
-    const int32_t v = L[lane + 32];
-    sb = roff[v];
-    lb = upper_bound_g(radj + sb, roff[v + 1] - sb, kmax);
-  }
-  long long ia = la, ib = lb;  // inclusive prefixes over rows 0..31 and 32..63
+  const int32_t kmax = sm.L[d - 1];
+  int carry_s = 0, carry_p = 0;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const long long va = __shfl_up_sync(0xffffffffu, ia, o), vb = __shfl_up_sync(0xffffffffu, ib, o);
-    if ((int)lane >= o) {
-      ia += va;
-      ib += vb;
+  for (int h = 0; h < 2; ++h) {
+    const int i = (int)lane + 32 * h;
+    int ns = 0, np = 0;
+    if (i < d) {
+      const int32_t v = sm.L[i];
+      // position i under v's hash; bytes are claimed through their word
+      uint32_t slot = ((uint32_t)v * 2654435769u) >> 24;
+      while (true) {
+        unsigned *word = reinterpret_cast<unsigned *>(sm.tab) + (slot >> 2);
+        const unsigned sh = (slot & 3) * 8, old = *(volatile unsigned *)word;
+        if (((old >> sh) & 255u) == 255u) {
+          if (atomicCAS(word, old, (old & ~(255u << sh)) | ((unsigned)i << sh)) == old) break;
+        } else {
+          slot = (slot + 1) & 255u;
+        }
+      }
+      const int64_t s = roff[v];
+      const int len = (int)upper_bound_g(radj + s, roff[v + 1] - s, kmax), rest = d - 1 - i;
+      sm.st[i] = s;
+      sm.len[i] = len;
+      if (rest * kCqSearch < len) np = rest;
+      else ns = len;
     }
-  }
-  const long long ta = __shfl_sync(0xffffffffu, ia, 31), total = ta + __shfl_sync(0xffffffffu, ib, 31);
-  for (long long base = 0; base < total; base += 32) {
-    const long long idx = base + lane;
-    const bool hi = idx >= ta;
-    const long long key = hi ? idx - ta : idx;
-    int lo = 0, up = 31;
 #pragma unroll
-    for (int r = 0; r < 5; ++r) {
-      const int mid = (lo + up) >> 1;
-      const long long pa = __shfl_sync(0xffffffffu, ia, mid), pb = __shfl_sync(0xffffffffu, ib, mid);
-      if ((hi ? pb : pa) > key) up = mid; else lo = mid + 1;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int vs = __shfl_up_sync(0xffffffffu, ns, o), vp = __shfl_up_sync(0xffffffffu, np, o);
+      if ((int)lane >= o) {
+        ns += vs;
+        np += vp;
+      }
     }
-    const long long pa = __shfl_sync(0xffffffffu, ia, lo), pb = __shfl_sync(0xffffffffu, ib, lo);
-    const long long ra = __shfl_sync(0xffffffffu, la, lo), rb = __shfl_sync(0xffffffffu, lb, lo);
-    const long long xa = __shfl_sync(0xffffffffu, sa, lo), xb = __shfl_sync(0xffffffffu, sb, lo);
-    if (idx < total) {
-      const int row = lo + (hi ? 32 : 0);
-      const long long t = (hi ? xb : xa) + key - ((hi ? pb : pa) - (hi ? rb : ra));
-      const int p = find_pos(L, d, __ldg(radj + t));
-      if (p >= 0) atomicOr(&rows[row], 1ull << p);
-    }
+    ns += carry_s;
+    np += carry_p;
+    sm.scan[i] = ns;
+    sm.pair[i] = np;
+    carry_s = __shfl_sync(0xffffffffu, ns, 31);
+    carry_p = __shfl_sync(0xffffffffu, np, 31);
+  }
+  __syncwarp();
+  // both kinds of work laid end to end, so short lists leave no lanes idle
+  for (int x = lane; x < carry_s; x += 32) {
+    const int i = segment_of(sm.scan, x);
+    const int p = find_pos(sm.tab, 8, sm.L, __ldg(radj + sm.st[i] + (x - (sm.scan[i] - sm.len[i]))));
+    if (p >= 0) atomicOr(&sm.rows[i], 1ull << p);
+  }
+  for (int x = lane; x < carry_p; x += 32) {
+    const int i = segment_of(sm.pair, x);
+    const int j = d - (sm.pair[i] - x);
+    if (in_list(radj + sm.st[i], sm.len[i], sm.L[j])) atomicOr(&sm.rows[i], 1ull << j);
   }
   __syncwarp();
   unsigned long long c = 0;
-  for (int i = lane; i < d; i += 32) c += local_count64(rows, rows[i], k - 2);
+  for (int i = lane; i < d; i += 32) c += local_count64(sm.rows, sm.rows[i], k - 2);
   __syncwarp();
   return c;
 }
@@ -298,87 +355,381 @@ __device__ unsigned long long warp_count_set(const uint32_t *rows, int W, WarpSe
   return c;
 }
 
+// ------------------------------------------------------------ compaction (5-cliques)
+// The bits of y selected by a mask moved together to the low end, the mask
+// given by its five move words (compress by parallel suffix: H. S. Warren,
+// Hacker's Delight, section 7-4).
+__device__ __forceinline__ void compact_moves(uint32_t m, uint32_t *mv) {
+  uint32_t mk = ~m << 1;
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+    uint32_t mp = mk ^ (mk << 1);
+    mp ^= mp << 2;
+    mp ^= mp << 4;
+    mp ^= mp << 8;
+    mp ^= mp << 16;
+    const uint32_t v = mp & m;
+    mv[i] = v;
+    m = (m ^ v) | (v >> (1 << i));
+    mk &= ~mp;
+  }
+}
+__device__ __forceinline__ uint32_t compact_bits(uint32_t y, const uint32_t *mv) {
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+    const uint32_t t = y & mv[i];
+    y = (y ^ t) | (t >> (1 << i));
+  }
+  return y;
+}
+
+// Rows of up to kCqWarpX members are compacted and counted by one warp.
+// Words of its buffer: move words and bit offsets of W row words, then
+// kCqWarpX rows of kCqWarpX bits and their members.
+constexpr int kCqWarpX = 128;
+__host__ __device__ constexpr size_t cq_warp_words(int W) {
+  return ((size_t)6 * W + 3) / 4 * 4 + kCqWarpX * (kCqWarpX / 32) + kCqWarpX / 2;
+}
+
+// Shared-memory layout of a CTA task in words (16-byte aligned parts).  comp:
+// the warps' buffers, and the CTA's own compacted rows when those are done.
+struct CqLayout {
+  size_t tab, xl, heavy, moves, comp, comp_words, rows, total;
+  int logcap;
+};
+__host__ __device__ inline CqLayout cq_layout(int d, int k, int nwarps, bool rows_in) {
+  CqLayout l;
+  const int W = (d + 31) >> 5;
+  l.logcap = 8;
+  while ((1 << l.logcap) < 4 * d && l.logcap < 12) ++l.logcap;
+  l.tab = ((size_t)d + 3) & ~(size_t)3;
+  l.xl = l.tab + ((size_t)1 << l.logcap) / 2;
+  const size_t list = k == 5 ? (((size_t)d + 1) / 2 + 3) & ~(size_t)3 : 0;
+  l.heavy = l.xl + list;
+  l.moves = l.heavy + list;
+  l.comp = l.moves + (k == 5 ? (6 * (size_t)W + 3) & ~(size_t)3 : 0);
+  l.comp_words = k == 5 ? nwarps * cq_warp_words(W) : 0;
+  l.rows = l.comp + l.comp_words;
+  l.total = l.rows + (rows_in ? (size_t)d * W : 0);
+  return l;
+}
+
+// Members of X = a row of W <= 64 words (lane: words lane, lane + 32), their
+// number, and per word the compaction moves and first position: mem[0 .. m),
+// mv[6 w ..].  One warp; mem == nullptr: the number alone.
+__device__ __forceinline__ int cq_members(const uint32_t *ri, int W, unsigned lane, uint16_t *mem, uint32_t *mv) {
+  int run = 0;
+  for (int w0 = 0; w0 < W; w0 += 32) {
+    const int w = w0 + (int)lane;
+    uint32_t word = w < W ? ri[w] : 0u;
+    const int nb = __popc(word);
+    int inc = nb;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, inc, o);
+      if ((int)lane >= o) inc += v;
+    }
+    if (mem && w < W) {
+      int at = run + inc - nb;
+      mv[6 * w + 5] = at;
+      compact_moves(word, mv + 6 * w);
+      for (; word; word &= word - 1) mem[at++] = (uint16_t)(w * 32 + __ffs(word) - 1);
+    }
+    run += __shfl_sync(0xffffffffu, inc, 31);
+  }
+  return run;
+}
+
+// Rows of the members x0 .. x0 + 31 (lane: x0 + lane) compacted to X's
+// columns: comp + x * stride, stride words of which the last are zero.  The
+// columns fill up word by word at the same pace in every lane.
+__device__ __forceinline__ void cq_compact(const uint32_t *rows, const uint32_t *ri, int W, const uint16_t *mem, int m,
+                                           int x0, const uint32_t *mv, uint32_t *comp, int stride, unsigned lane) {
+  const int x = x0 + (int)lane;
+  if (x >= m) return;
+  const uint32_t *rl = rows + (int)mem[x] * W;
+  uint32_t *cx = comp + x * stride;
+  unsigned long long acc = 0;
+  int at = 0, fill = 0;  // words written, bits pending
+  for (int w = 0; w < W; ++w) {
+    const uint32_t mask = ri[w];
+    if (!mask) continue;
+    acc |= (unsigned long long)compact_bits(rl[w] & mask, mv + 6 * w) << fill;
+    fill += __popc(mask);
+    if (fill >= 32) {
+      cx[at++] = (uint32_t)acc;
+      acc >>= 32;
+      fill -= 32;
+    }
+  }
+  for (; at < stride; ++at) {
+    cx[at] = (uint32_t)acc;
+    acc = 0;
+  }
+}
+
+// Pairs (a, b) of the compacted rows, a in 32 r + lane, b a member of word w
+// of row a: the common members of both in the NW words from column word q on.
+// All lanes walk the same word and the same columns, so they differ only in
+// how many members their word has.
+template <int NW>
+__device__ __forceinline__ unsigned cq_pairs(const uint32_t *comp, int stride, int m, int r, int w, int q,
+                                             unsigned lane) {
+  const int a = 32 * r + (int)lane;
+  uint32_t own[NW], oth[NW];
+  uint32_t word = 0;
+  if (a < m) {
+    word = comp[a * stride + w];
+#pragma unroll
+    for (int i = 0; i < NW; ++i) own[i] = comp[a * stride + q + i];
+  }
+  unsigned s = 0;
+  for (; word; word &= word - 1) {
+    const uint32_t *cb = comp + (w * 32 + __ffs(word) - 1) * stride + q;
+    if (NW == 4) {
+      const uint4 t = *reinterpret_cast<const uint4 *>(cb);
+      oth[0] = t.x, oth[1] = t.y, oth[2 % NW] = t.z, oth[3 % NW] = t.w;
+    } else {
+      const uint2 t = *reinterpret_cast<const uint2 *>(cb);
+      oth[0] = t.x, oth[1] = t.y;
+    }
+#pragma unroll
+    for (int i = 0; i < NW; ++i) s += __popc(own[i] & oth[i]);
+  }
+  return s;
+}
+
+// One vertex task on a CTA.  SM: the rows are in shared memory (smem), else in
+// the CTA's slab (two halves of slab_half words: rows, compacted rows).  Each
+// thread returns its part of the count.
+template <int KM, bool SM>
 __device__ unsigned long long clique_cta_task(int32_t u, int k, const int64_t *__restrict__ roff,
-                                              const int32_t *__restrict__ radj, char *smem, uint32_t *slab,
-                                              uint32_t *xs) {
+                                              const int32_t *__restrict__ radj, uint32_t *smem, uint32_t *slab, size_t slab_half,
+                                              const CqCore &core, uint32_t *xs) {
   const int tid = threadIdx.x, nthr = blockDim.x, wid = tid >> 5, nw = nthr >> 5;
   const unsigned lane = tid & 31;
   const int64_t s0 = roff[u];
   const int d = (int)(roff[u + 1] - s0);
   const int W = (d + 31) >> 5;
+  const CqLayout lay = cq_layout(d, k, nw, SM);
   int32_t *L = reinterpret_cast<int32_t *>(smem);
-  size_t lbytes = ((size_t)d * 4 + 15) & ~(size_t)15;
-  size_t rbytes = (size_t)d * W * 4;
-  uint32_t *rows = lbytes + rbytes <= kCqSmem ? reinterpret_cast<uint32_t *>(smem + lbytes) : slab;
+  uint16_t *tab = reinterpret_cast<uint16_t *>(smem + lay.tab);
+  uint32_t *rows = SM ? smem + lay.rows : slab;
   for (int i = tid; i < d; i += nthr) L[i] = radj[s0 + i];
-  for (size_t i = tid; i < (size_t)d * W; i += nthr) rows[i] = 0u;
+  for (int i = tid; i < (1 << lay.logcap) / 2; i += nthr) smem[lay.tab + i] = ~0u;
+  for (int i = tid; i < d * W; i += nthr) rows[i] = 0u;
+  __syncthreads();
+  for (int i = tid; i < d; i += nthr) {
+    uint32_t h = ((uint32_t)L[i] * 2654435769u) >> (32 - lay.logcap);
+    while (atomicCAS(reinterpret_cast<unsigned short *>(tab) + h, (unsigned short)0xffff, (unsigned short)i) != 0xffff)
+      h = (h + 1) & ((1u << lay.logcap) - 1u);
+  }
   __syncthreads();
   const int32_t kmax = L[d - 1];
+  int jc = d;  // first position in the core
+  if (core.rowid) {
+    int lo = 0;
+    while (lo < jc) {
+      const int mid = (lo + jc) >> 1;
+      if (L[mid] < core.base) lo = mid + 1; else jc = mid;
+    }
+  }
   // warp wid builds rows wid, wid + nw, ...; the scan ranges of 32 of them at
-  // a time are found in parallel, one lane per row
+  // a time are found in parallel, one lane per row.  With a bitmap row, only
+  // the keys below the core are looked up.
   for (int i0 = wid; i0 < d; i0 += nw * 32) {
     const int mine = i0 + (int)lane * nw;
-    long long ms = 0, mstop = 0;
+    long long ms = 0;
+    int mlen = 0, mrow = -1;
     if (mine < d) {
       const int32_t v = L[mine];
-      ms = roff[v];
-      mstop = ms + upper_bound_g(radj + ms, roff[v + 1] - ms, kmax);
+      if (core.rowid && jc < d) mrow = core.rowid[v];
+      if (mrow < 0 || mine + 1 < jc) {
+        ms = roff[v];
+        mlen = (int)upper_bound_g(radj + ms, roff[v + 1] - ms, mrow < 0 ? kmax : core.base - 1);
+      }
     }
     for (int j = 0; j < 32 && i0 + j * nw < d; ++j) {
-      const int i = i0 + j * nw;
-      const long long s = __shfl_sync(0xffffffffu, ms, j), stop = __shfl_sync(0xffffffffu, mstop, j);
-      uint32_t *ri = rows + (size_t)i * W;
-      for (long long t = s + lane; t < stop; t += 32) {
-        int p = find_pos(L, d, __ldg(radj + t));
+      const int i = i0 + j * nw, len = __shfl_sync(0xffffffffu, mlen, j), row = __shfl_sync(0xffffffffu, mrow, j);
+      const int32_t *__restrict__ list = radj + __shfl_sync(0xffffffffu, ms, j);
+      uint32_t *ri = rows + i * W;
+      const int jend = row < 0 ? d : jc;  // positions from jend on by the bitmap
+      if (row >= 0) {
+        const uint32_t *__restrict__ bits = core.rows + (size_t)row * core.words;
+        const int first = max(i + 1, jc);
+        for (int b = first & ~31; b < d; b += 32) {
+          const int q = b + (int)lane;
+          bool in = false;
+          if (q >= first && q < d) {
+            const unsigned o = (unsigned)(L[q] - core.base);
+            in = (__ldg(bits + (o >> 5)) >> (o & 31)) & 1u;
+          }
+          const unsigned m = __ballot_sync(0xffffffffu, in);
+          if (lane == 0 && m) ri[b >> 5] = m;
+        }
+        __syncwarp();
+        if (i + 1 >= jc) continue;
+      }
+      if ((jend - 1 - i) * kCqSearch < len) {  // the rest of L searched in the list, a word of the row at a time
+        for (int b = (i + 1) & ~31; b < jend; b += 32) {
+          const int q = b + (int)lane;
+          const unsigned m = __ballot_sync(0xffffffffu, q > i && q < jend && in_list(list, len, L[q]));
+          if (lane == 0 && m) ri[b >> 5] |= m;
+        }
+        continue;
+      }
+      int t = lane;
+      for (; t + 32 < len; t += 64) {
+        const int32_t x0 = __ldg(list + t), x1 = __ldg(list + t + 32);
+        const int p0 = find_pos(tab, lay.logcap, L, x0);
+        if (p0 >= 0) atomicOr(&ri[p0 >> 5], 1u << (p0 & 31));
+        const int p1 = find_pos(tab, lay.logcap, L, x1);
+        if (p1 >= 0) atomicOr(&ri[p1 >> 5], 1u << (p1 & 31));
+      }
+      if (t < len) {
+        const int p = find_pos(tab, lay.logcap, L, __ldg(list + t));
         if (p >= 0) atomicOr(&ri[p >> 5], 1u << (p & 31));
       }
     }
   }
   __syncthreads();
   unsigned long long c = 0;
-  // each lane accumulates the popcounts of its own words; the warp sum is the count
-  for (int i = wid; i < d; i += nw) c += warp_count_set(rows, W, wrow(rows, W, i, lane), k - 2, xs, lane);
+  if (KM == 4) {
+    // a thread per row word: its members l, each ANDed with the row from l's
+    // word on (row_l has no bits below l)
+    for (int x = tid; x < d * W; x += nthr) {
+      uint32_t word = rows[x];
+      if (!word) continue;
+      const int i = x / W, w = x - i * W;
+      unsigned s = 0;
+      for (; word; word &= word - 1) {
+        const uint32_t *rl = rows + (w * 32 + __ffs(word) - 1) * W;
+        for (int ww = w; ww < W; ++ww) s += __popc(rows[i * W + ww] & rl[ww]);
+      }
+      c += s;
+    }
+  } else if (KM == 5) {
+    // For each row i, the triangles of the local DAG inside X = row_i: the
+    // rows of X's members are compacted to X's columns (|X| bits in place of
+    // |L|, R-MAT 20: 91 of 350 for |L| in 257 .. 512), then every member pair
+    // ANDs compacted rows.  Rows of up to kCqWarpX members by one warp each;
+    // the others are listed and taken by the whole CTA afterwards.  R-MAT 19 /
+    // 20: 71 / 188 ms on full-width rows, 22.3 / 66 ms compacted.
+    uint16_t *xl = reinterpret_cast<uint16_t *>(smem + lay.xl);
+    uint16_t *heavy = reinterpret_cast<uint16_t *>(smem + lay.heavy);
+    __shared__ int s_heavy;
+    if (tid == 0) s_heavy = 0;
+    __syncthreads();
+    {
+      uint32_t *wmv = smem + lay.comp + wid * cq_warp_words(W);
+      uint32_t *cr = wmv + (6 * W + 3) / 4 * 4;
+      uint16_t *mem = reinterpret_cast<uint16_t *>(cr + kCqWarpX * (kCqWarpX / 32));
+      for (int i = wid; i < d; i += nw) {
+        const uint32_t *ri = rows + i * W;
+        int m = cq_members(ri, W, lane, nullptr, nullptr);
+        if (m < 3) continue;
+        if (m > kCqWarpX) {
+          if (lane == 0) heavy[atomicAdd(&s_heavy, 1)] = (uint16_t)i;
+          continue;
+        }
+        cq_members(ri, W, lane, mem, wmv);
+        __syncwarp();
+        const int stride = m <= 64 ? 2 : 4, strips = (m + 31) >> 5;
+        for (int x0 = 0; x0 < m; x0 += 32) cq_compact(rows, ri, W, mem, m, x0, wmv, cr, stride, lane);
+        __syncwarp();
+        unsigned s = 0;
+        for (int w = 0; w < strips; ++w)
+          for (int r = 0; r <= w; ++r)
+            s += m <= 64 ? cq_pairs<2>(cr, 2, m, r, w, 0, lane) : cq_pairs<4>(cr, 4, m, r, w, 0, lane);
+        c += s;
+        __syncwarp();
+      }
+    }
+    __syncthreads();
+    const int nh = s_heavy;
+    __syncthreads();  // s_heavy becomes |X| below
+    uint32_t *mv = smem + lay.moves;
+    for (int hi = 0; hi < nh; ++hi) {
+      const uint32_t *ri = rows + heavy[hi] * W;
+      if (wid == 0) {
+        const int m = cq_members(ri, W, lane, xl, mv);
+        if (lane == 0) s_heavy = m;
+      }
+      __syncthreads();
+      const int m = s_heavy, strips = (m + 31) >> 5, stride = (strips + 3) & ~3;
+      // the slab holds what the warps' buffers have no room for
+      uint32_t *comp = (size_t)m * stride <= lay.comp_words ? smem + lay.comp : slab + slab_half;
+      for (int r = wid; r < strips; r += nw) cq_compact(rows, ri, W, xl, m, 32 * r, mv, comp, stride, lane);
+      __syncthreads();
+      // (r <= w, four column words from 4 (w / 4) on): small w first, they have most columns
+      unsigned s = 0;
+      int t = 0;
+      for (int w = 0; w < strips; ++w)
+        for (int q = w & ~3; q < strips; q += 4)
+          for (int r = 0; r <= w; ++r, ++t)
+            if (t % nw == wid) s += cq_pairs<4>(comp, stride, m, r, w, q, lane);
+      c += s;
+      __syncthreads();
+    }
+  } else {
+    // each lane accumulates the popcounts of its own words; the warp sum is the count
+    for (int i = wid; i < d; i += nw) c += warp_count_set(rows, W, wrow(rows, W, i, lane), k - 2, xs, lane);
+  }
   __syncthreads();
   return c;
 }
 
-__global__ void __launch_bounds__(256) k_clique_local(int k, const int64_t *__restrict__ roff,
-                                                      const int32_t *__restrict__ radj,
-                                                      const int32_t *__restrict__ cta_tasks, int n_cta,
-                                                      const int32_t *__restrict__ warp_tasks, int n_warp,
-                                                      int *__restrict__ counters, uint32_t *__restrict__ slabs,
-                                                      size_t slab_words, const int32_t *__restrict__ gid,
-                                                      unsigned long long *__restrict__ acc, int stride, int slot) {
-  extern __shared__ __align__(16) char csm[];
+// CTA tasks [t0, t1) of the queue, heaviest first.  KM: 4, 5, or 0 for the
+// other clique sizes.  BIG: rows may be in the slab.
+template <int KM, bool BIG>
+__global__ void __launch_bounds__(BIG ? kCqBigThreads : kCqSmallThreads)
+    k_clique_cta(int k, const int64_t *__restrict__ roff, const int32_t *__restrict__ radj,
+                 const int32_t *__restrict__ tasks, int ntasks, int *__restrict__ cursor, uint32_t *__restrict__ slabs,
+                 size_t slab_half, CqCore core, const int32_t *__restrict__ gid, unsigned long long *__restrict__ acc,
+                 int stride, int slot) {
+  extern __shared__ __align__(16) uint32_t csm[];
   __shared__ int s_task;
-  __shared__ uint32_t sxs[8][64];  // each warp's staged set (wsum_pairs)
+  __shared__ uint32_t sxs[KM == 0 ? (BIG ? kCqBigThreads : kCqSmallThreads) / 32 : 1][64];  // staged sets (wsum_pairs)
   const int wid = threadIdx.x >> 5;
   const unsigned lane = threadIdx.x & 31;
-  uint32_t *slab = slabs + (size_t)blockIdx.x * slab_words;
+  constexpr size_t words = (BIG ? kCqSmemBig : kCqSmemSmall) / 4;
+  uint32_t *slab = slabs + (size_t)blockIdx.x * 2 * slab_half;
+  uint32_t *xs = sxs[KM == 0 ? wid : 0];
   while (true) {
-    if (threadIdx.x == 0) s_task = atomicAdd(&counters[0], 1);
+    if (threadIdx.x == 0) s_task = atomicAdd(cursor, 1);
     __syncthreads();
     int t = s_task;
     __syncthreads();
-    if (t >= n_cta) break;
-    const int32_t u = cta_tasks[t];
-    unsigned long long c = warp_sum(clique_cta_task(u, k, roff, radj, csm, slab, sxs[wid]));
-    if (lane == 0 && c) atomicAdd(&acc[(size_t)stride * (gid ? gid[u] : 0) + slot], c);
-  }
-  int32_t *L = reinterpret_cast<int32_t *>(csm + wid * (kCqWarpMax * 12));
-  unsigned long long *rows = reinterpret_cast<unsigned long long *>(csm + wid * (kCqWarpMax * 12) + kCqWarpMax * 4);
-  while (true) {
-    int t = 0;
-    if (lane == 0) t = atomicAdd(&counters[1], 1);
-    t = __shfl_sync(0xffffffffu, t, 0);
-    if (t >= n_warp) break;
-    const int32_t u = warp_tasks[t];
-    unsigned long long c = warp_sum(clique_warp_task(u, k, roff, radj, L, rows));
+    if (t >= ntasks) break;
+    const int32_t u = tasks[t];
+    unsigned long long c;
+    if (BIG && cq_layout((int)(roff[u + 1] - roff[u]), k, kCqBigThreads / 32, true).total > words)
+      c = clique_cta_task<KM, false>(u, k, roff, radj, csm, slab, slab_half, core, xs);
+    else
+      c = clique_cta_task<KM, true>(u, k, roff, radj, csm, slab, slab_half, core, xs);
+    c = warp_sum(c);
     if (lane == 0 && c) atomicAdd(&acc[(size_t)stride * (gid ? gid[u] : 0) + slot], c);
   }
 }
 
-__global__ void k_clique_tasks(int64_t n, const int64_t *__restrict__ roff, int k, int warp_max,
+__global__ void __launch_bounds__(256) k_clique_warp(int k, const int64_t *__restrict__ roff,
+                                                     const int32_t *__restrict__ radj,
+                                                     const int32_t *__restrict__ tasks, int ntasks,
+                                                     int *__restrict__ cursor, const int32_t *__restrict__ gid,
+                                                     unsigned long long *__restrict__ acc, int stride, int slot) {
+  __shared__ CqWarp sm[8];
+  const unsigned lane = threadIdx.x & 31;
+  WarpTasks queue;
+  while (true) {
+    const int t = queue.next(cursor, gridDim.x * 16, lane);
+    if (t >= ntasks) break;
+    const int32_t u = tasks[t];
+    unsigned long long c = warp_sum(clique_warp_task(u, k, roff, radj, sm[threadIdx.x >> 5]));
+    if (lane == 0 && c) atomicAdd(&acc[(size_t)stride * (gid ? gid[u] : 0) + slot], c);
+  }
+}
+
+__global__ void k_clique_tasks(int64_t n, const int64_t *__restrict__ roff, int k, int warp_max, int small_max,
                                uint32_t *__restrict__ ckey,
                                int32_t *__restrict__ cval, uint32_t *__restrict__ wkey, int32_t *__restrict__ wval,
                                int *__restrict__ sizes) {
@@ -389,6 +740,7 @@ __global__ void k_clique_tasks(int64_t n, const int64_t *__restrict__ roff, int 
       int i = atomicAdd(&sizes[0], 1);
       ckey[i] = ~(uint32_t)d;
       cval[i] = (int32_t)u;
+      if (d > small_max) atomicAdd(&sizes[2], 1);
     } else {
       int i = atomicAdd(&sizes[1], 1);
       wkey[i] = ~(uint32_t)d;
@@ -485,14 +837,42 @@ __global__ void __launch_bounds__(256) k_clique_edge(int64_t nnz, int k, const i
 }
 
 // ------------------------------------------------------------ host
-static int clique_local_grid() {
-  static PerDevice grid;
-  return grid.get([] {
-    cudaFuncSetAttribute(k_clique_local, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCqSmem);
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_clique_local, 256, kCqSmem);
-    return std::max(1, per_sm) * num_sms();
+template <class K>
+static int cq_grid(K kernel, int threads, size_t smem) {
+  if (smem) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
+  return std::max(1, per_sm) * num_sms();
+}
+
+// The kernels of clique size k: f(small CTA kernel, big CTA kernel).
+template <class F>
+static void cq_kernels(int k, F f) {
+  if (k == 4) f(k_clique_cta<4, false>, k_clique_cta<4, true>);
+  else if (k == 5) f(k_clique_cta<5, false>, k_clique_cta<5, true>);
+  else f(k_clique_cta<0, false>, k_clique_cta<0, true>);
+}
+
+struct CqGrids {
+  int small, big, warp;
+};
+static CqGrids cq_grids(int k) {
+  static PerDevice small[3], big[3], warp;
+  const int i = k == 4 ? 0 : k == 5 ? 1 : 2;
+  CqGrids g;
+  cq_kernels(k, [&](auto s, auto b) {
+    g.small = small[i].get([&] { return cq_grid(s, kCqSmallThreads, kCqSmemSmall); });
+    g.big = big[i].get([&] { return cq_grid(b, kCqBigThreads, kCqSmemBig); });
   });
+  g.warp = warp.get([] { return cq_grid(k_clique_warp, 256, 0); });
+  return g;
+}
+
+// Largest |L| whose layout fits the small CTAs.
+static int cq_small_max(int k) {
+  int d = kCqWarpMax;
+  while (d < kCqCtaMax && cq_layout(d + 1, k, kCqSmallThreads / 32, true).total * 4 <= kCqSmemSmall) ++d;
+  return d;
 }
 
 // Plan: task queues (heaviest first) and row slabs; the run is launches only.
@@ -520,11 +900,12 @@ int clique_plan_build(CliquePlan *p, int64_t n, const int64_t *roff, const int32
   GPM_TRY(wval.reserve(n));
   GPM_TRY(p->ctasks.reserve(n));
   GPM_TRY(p->wtasks.reserve(n));
-  GPM_TRY(sizes.reserve(2));
-  GPM_TRY(p->counters.reserve(2));
-  GPM_CUDA(cudaMemsetAsync(sizes.p, 0, 2 * sizeof(int), st));
-  k_clique_tasks<<<grid_for(n), 256, 0, st>>>(n, roff, k, warp_max, ckey.p, cval.p, wkey.p, wval.p, sizes.p);
-  int h[2];
+  GPM_TRY(sizes.reserve(3));
+  GPM_TRY(p->counters.reserve(3));
+  GPM_CUDA(cudaMemsetAsync(sizes.p, 0, 3 * sizeof(int), st));
+  k_clique_tasks<<<grid_for(n), 256, 0, st>>>(n, roff, k, warp_max, cq_small_max(k), ckey.p, cval.p, wkey.p, wval.p,
+                                              sizes.p);
+  int h[3];
   GPM_CUDA(cudaMemcpyAsync(h, sizes.p, sizeof h, cudaMemcpyDeviceToHost, st));
   GPM_CUDA(cudaStreamSynchronize(st));
   for (int which = 0; which < 2; ++which) {
@@ -542,22 +923,74 @@ int clique_plan_build(CliquePlan *p, int64_t n, const int64_t *roff, const int32
   }
   p->n_cta = h[0];
   p->n_warp = h[1];
-  // per-CTA slabs for rows that do not fit in shared memory
-  p->grid = clique_local_grid();
-  size_t W = (size_t)(max_deg + 31) / 32;
-  p->slab_words = (size_t)max_deg * W * 4 + (size_t)max_deg * 4 > kCqSmem ? (size_t)max_deg * W : 1;
-  GPM_TRY(p->slabs.reserve(p->slab_words * p->grid));
+  p->n_big = h[2];
+  if (p->n_cta > 0) {
+    int64_t nkeys = 0;
+    GPM_CUDA(cudaMemcpyAsync(&nkeys, roff + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    GPM_CUDA(cudaStreamSynchronize(st));
+    const int s = core_rows_build(n, roff, radj, nkeys, kCqCore, kCqCoreMin, p->rowid, &p->core, st);
+    if (s == GPM_ENOMEM) p->core = CoreRows();  // counted without them
+    else GPM_TRY(s);
+  }
+  // per-CTA slabs of the big CTAs: rows, and compacted rows, that do not fit
+  // in shared memory
+  const size_t W = (size_t)(max_deg + 31) / 32;
+  const CqGrids grids = cq_grids(k);
+  p->big_grid = std::max(1, std::min(grids.big, p->n_big));
+  if (p->n_big > 0 && p->n_big < p->n_cta + p->n_warp && !p->side &&
+      (cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking) != cudaSuccess ||
+       cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming) != cudaSuccess ||
+       cudaEventCreateWithFlags(&p->join, cudaEventDisableTiming) != cudaSuccess)) {
+    cudaGetLastError();
+    return fail(GPM_ECUDA, "clique plan: side stream");
+  }
+  const CqLayout big = cq_layout(max_deg, k, kCqBigThreads / 32, true);
+  const size_t comp_max = (size_t)max_deg * ((W + 3) & ~(size_t)3);
+  const bool spill = p->n_big && (big.total * 4 > kCqSmemBig || (k == 5 && comp_max > kCqBigThreads / 32 * cq_warp_words(1)));
+  p->slab_words = comp_max;
+  GPM_TRY(p->slabs.reserve(spill ? 2 * p->slab_words * p->big_grid : 1));
+  if (p->n_cta > p->n_big && k == 5) {
+    // small CTAs: compacted rows beyond the warps' buffers
+    const int sd = std::min(max_deg, cq_small_max(k));
+    p->small_slab = (size_t)sd * (((sd + 31) / 32 + 3) & ~3);
+    GPM_TRY(p->small_slabs.reserve(2 * p->small_slab * grids.small));
+  } else {
+    GPM_TRY(p->small_slabs.reserve(1));
+  }
   GPM_CUDA(cudaStreamSynchronize(st));
   return GPM_OK;
 }
 
 int clique_plan_run(CliquePlan *p, cudaStream_t st) {
   if (p->n_cta + p->n_warp == 0) return GPM_OK;
-  GPM_CUDA(cudaMemsetAsync(p->counters.p, 0, 2 * sizeof(int), st));
-  k_clique_local<<<p->grid, 256, kCqSmem, st>>>(p->k, p->roff, p->radj, p->ctasks.p, p->n_cta, p->wtasks.p,
-                                                p->n_warp, p->counters.p, p->slabs.p, p->slab_words, p->gid, p->acc,
-                                                p->stride, p->slot);
+  GPM_CUDA(cudaMemsetAsync(p->counters.p, 0, 3 * sizeof(int), st));
+  const CqGrids grids = cq_grids(p->k);
+  const int nsmall = p->n_cta - p->n_big;
+  const CqCore core{p->core.n_rows ? p->rowid.p : nullptr, p->core.rows.p, p->core.base, p->core.words};
+  // the large tasks may be few: they run beside the others
+  cudaStream_t bst = st;
+  if (p->side) {
+    bst = p->side;
+    GPM_CUDA(cudaEventRecord(p->fork, st));
+    GPM_CUDA(cudaStreamWaitEvent(bst, p->fork, 0));
+  }
+  cq_kernels(p->k, [&](auto small, auto big) {
+    if (p->n_big > 0)
+      big<<<p->big_grid, kCqBigThreads, kCqSmemBig, bst>>>(p->k, p->roff, p->radj, p->ctasks.p, p->n_big,
+                                                           p->counters.p, p->slabs.p, p->slab_words, core, p->gid,
+                                                           p->acc, p->stride, p->slot);
+    if (nsmall > 0)
+      small<<<std::min(grids.small, nsmall), kCqSmallThreads, kCqSmemSmall, st>>>(
+          p->k, p->roff, p->radj, p->ctasks.p + p->n_big, nsmall, p->counters.p + 1, p->small_slabs.p, p->small_slab,
+          core, p->gid, p->acc, p->stride, p->slot);
+  });
   GPM_LAUNCH_CHECK();
+  if (bst != st) GPM_CUDA(cudaEventRecord(p->join, bst));
+  if (p->n_warp > 0)
+    k_clique_warp<<<std::min(grids.warp, (p->n_warp + 7) / 8), 256, 0, st>>>(
+        p->k, p->roff, p->radj, p->wtasks.p, p->n_warp, p->counters.p + 2, p->gid, p->acc, p->stride, p->slot);
+  GPM_LAUNCH_CHECK();
+  if (bst != st) GPM_CUDA(cudaStreamWaitEvent(st, p->join, 0));
   return GPM_OK;
 }
 

@@ -1,6 +1,7 @@
 // motif.cuh -- motif pipeline over one graph or a disjoint union of graphs.
 #pragma once
 #include "common.cuh"
+#include "tc_rank.cuh"
 
 namespace gpm {
 
@@ -36,13 +37,29 @@ struct CliquePlan {
   int64_t n = 0;
   const int64_t *roff = nullptr;
   const int32_t *radj = nullptr;
-  int k = 0, stride = 0, slot = 0, n_cta = 0, n_warp = 0, grid = 0;
+  int k = 0, stride = 0, slot = 0, n_cta = 0, n_warp = 0;
+  int n_big = 0, big_grid = 0;  // the first n_big CTA tasks take the large CTAs
   const int32_t *gid = nullptr;
   unsigned long long *acc = nullptr;
-  size_t slab_words = 0;
+  size_t slab_words = 0, small_slab = 0;  // words of half a slab (big, small CTAs)
   DevBuf<int32_t> ctasks, wtasks;
   DevBuf<int> counters;
-  DevBuf<uint32_t> slabs;
+  DevBuf<uint32_t> slabs, small_slabs;
+  DevBuf<int32_t> rowid;  // bitmap row of each vertex over the core (core.n_rows > 0)
+  CoreRows core;
+  // the large tasks run beside the others on a stream of the plan's own,
+  // forked from and joined back into the caller's by the two events
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+  CliquePlan() = default;
+  CliquePlan(const CliquePlan &) = delete;
+  CliquePlan &operator=(const CliquePlan &) = delete;
+  ~CliquePlan() {
+    if (join) cudaEventSynchronize(join);
+    if (side) cudaStreamDestroy(side);
+    if (fork) cudaEventDestroy(fork);
+    if (join) cudaEventDestroy(join);
+  }
 };
 int clique_plan_build(CliquePlan *p, int64_t n, const int64_t *roff, const int32_t *radj, int max_deg, int k,
                       const int32_t *gid, unsigned long long *acc, int stride, int slot, cudaStream_t st,

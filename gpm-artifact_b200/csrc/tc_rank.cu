@@ -1124,10 +1124,21 @@ static int64_t env_or(const char *name, int64_t dflt) {
 // and more than four times the bytes of the rank graph's lists (R-MAT 22:
 // 176 MB of rows against 257 MB of lists).
 static int build_core_rows(gpm_graph *g, RankPlan *p, DevBuf<int32_t> &rowid, int *dense_pct, cudaStream_t st) {
-  const int64_t n = g->n;
   const int64_t K = env_or("GPM_TC_CORE", GPM_RANK_CORE);
   const int64_t min_keys = std::max<int64_t>(1, env_or("GPM_TC_CORE_MIN", GPM_RANK_CORE_MIN));
   *dense_pct = (int)std::max<int64_t>(0, env_or("GPM_TC_DENSE_PCT", GPM_RANK_DENSE_PCT));
+  CoreRows c;
+  GPM_TRY(core_rows_build(g->n, g->rg->roff.p, g->rg->radj.p, (int64_t)g->rg->radj.n, K, (int)min_keys, rowid, &c, st));
+  if (!c.n_rows) return GPM_OK;
+  p->core_base = c.base;
+  p->row_words = c.words;
+  p->n_rows = c.n_rows;
+  p->rows = std::move(c.rows);
+  return GPM_OK;
+}
+
+int core_rows_build(int64_t n, const int64_t *roff, const int32_t *radj, int64_t nkeys, int64_t K, int min_keys,
+                    DevBuf<int32_t> &rowid, CoreRows *out, cudaStream_t st) {
   if (K <= 0 || n <= 0 || n > INT32_MAX - 128) return GPM_OK;
   const int32_t core_base = (int32_t)(std::max<int64_t>(0, n - K) & ~(int64_t)127);
   const int64_t row_words = ((n - core_base + 127) >> 7) << 2;
@@ -1138,24 +1149,22 @@ static int build_core_rows(gpm_graph *g, RankPlan *p, DevBuf<int32_t> &rowid, in
   GPM_TRY(rowid.reserve(n));
   GPM_TRY(nrows.reserve(1));
   GPM_CUDA(cudaMemsetAsync(nrows.p, 0, sizeof(int), st));
-  k_core_rowid<<<grid_for(n), 256, 0, st>>>(n, g->rg->roff.p, g->rg->radj.p, core_base, (int)min_keys, rowid.p,
-                                            nrows.p);
+  k_core_rowid<<<grid_for(n), 256, 0, st>>>(n, roff, radj, core_base, min_keys, rowid.p, nrows.p);
   GPM_LAUNCH_CHECK();
   int h = 0;
   GPM_CUDA(cudaMemcpyAsync(&h, nrows.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   GPM_CUDA(cudaStreamSynchronize(st));
   if (h <= 0) return GPM_OK;
   const size_t bytes = (size_t)h * (size_t)row_words * 4;
-  if (bytes > std::max<size_t>((size_t)1 << 30, 16 * (size_t)g->rg->radj.n)) return GPM_OK;
+  if (bytes > std::max<size_t>((size_t)1 << 30, 16 * (size_t)nkeys)) return GPM_OK;
   if (bytes / 16 >= ((size_t)1 << 31)) return GPM_OK;  // a dense descriptor indexes the rows' uint4 in 31 bits
-  GPM_TRY(p->rows.reserve((size_t)h * (size_t)row_words));
-  GPM_CUDA(cudaMemsetAsync(p->rows.p, 0, bytes, st));
-  k_core_rows<<<grid_for(n * 32), 256, 0, st>>>(n, g->rg->roff.p, g->rg->radj.p, core_base, rowid.p,
-                                                (int)row_words, p->rows.p);
+  GPM_TRY(out->rows.reserve((size_t)h * (size_t)row_words));
+  GPM_CUDA(cudaMemsetAsync(out->rows.p, 0, bytes, st));
+  k_core_rows<<<grid_for(n * 32), 256, 0, st>>>(n, roff, radj, core_base, rowid.p, (int)row_words, out->rows.p);
   GPM_LAUNCH_CHECK();
-  p->core_base = core_base;
-  p->row_words = (int)row_words;
-  p->n_rows = h;
+  out->base = core_base;
+  out->words = (int)row_words;
+  out->n_rows = h;
   return GPM_OK;
 }
 

@@ -83,6 +83,20 @@ using Seg = int2;
 __host__ __device__ __forceinline__ int seg_keys(Seg s) { return (int)((uint32_t)s.y >> 2); }
 __host__ __device__ __forceinline__ int seg_rows(Seg s) { return (int)(((s.y & 3) + ((uint32_t)s.y >> 2) + 3) >> 2); }
 
+// Bitmaps over the top K ranks [base, n) (base a multiple of 128): row
+// rowid[v] holds, as `words` 32-bit words, the keys >= base of a vertex v that
+// has at least min_keys of them (rowid[v] = -1: no row).  n_rows stays 0 when no
+// vertex qualifies, or the rows would take more than 1 GiB and more than four
+// times the lists.
+struct CoreRows {
+  int32_t base = INT32_MAX;
+  int words = 0;
+  int64_t n_rows = 0;
+  DevBuf<uint32_t> rows;
+};
+int core_rows_build(int64_t n, const int64_t *roff, const int32_t *radj, int64_t nkeys, int64_t K, int min_keys,
+                    DevBuf<int32_t> &rowid, CoreRows *out, cudaStream_t st);
+
 // Core bitmaps of an owner x whose keys all lie in the core (min N(x) >=
 // core_base): N(x) as bits from base = min N(x) rounded down to 128, so
 // bitmap word i lines up with word (base - core_base) / 32 + i of every core
