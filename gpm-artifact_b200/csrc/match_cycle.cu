@@ -9,8 +9,8 @@
 // vertex of c's label class, the walk a - d - c adds up the counters it meets.
 // The work is the wedges, not the embeddings (R-MAT 19, labels 0 0 3 1: 0.6 G
 // wedges; 145-178 ms by the depth-first walk, which tests every wedge for its
-// closing edge, 3.4 ms here, most of it in k_cycle_big: 0.6 G increments and as
-// many loads and clears at 180 G/s, bound by shared-memory atomics).
+// closing edge, 3.3 ms here, 2.7 of it in k_cycle_big: 0.8 G increments, loads
+// and clears, bound by the latency of lists and counters at 32 warps per SM).
 //
 // Counters are indexed by the rank inside the label class in descending degree
 // order.  A walk ends at a vertex in proportion to its degree, so the ranks
@@ -23,18 +23,19 @@
 #include <algorithm>
 
 #include "match.cuh"
+#include "wedge.cuh"
 
 namespace gpm {
 
 constexpr int kSmallWarps = 8, kSmallSlots = 512;
 constexpr unsigned long long kSmallBound = kSmallSlots / 2;
-constexpr int kBigThreads = 512, kBigWarps = kBigThreads / 32, kBigPerSm = 2;
+constexpr int kBigThreads = 512, kBigPerSm = 2;
 constexpr int kHot = 24576;                 // shared counters of a CTA (96 KB, two CTAs per SM)
-constexpr int kLongSeg = 64;                // segments streamed by the whole warp
 constexpr int64_t kTailBytes = 4ll << 30;   // most global memory for the counters of ranks >= kHot
 
 struct CycleSpace {
-  DevBuf<int2> small, big;      // tasks: (vertex, 1 when the d side is counted first)
+  DevBuf<int2> small;           // tasks: (vertex, 1 when the d side is counted first)
+  DevBuf<int4> big;             // the same, then the wedges of the counted and of the other side (capped)
   DevBuf<int> sizes;            // [0] small tasks, [1] big tasks, [2], [3] their cursors
   DevBuf<unsigned> tail;        // grid x (class size - kHot), all zero between launches
   int64_t tail_len = 0;         // counters per CTA
@@ -69,7 +70,7 @@ __device__ __forceinline__ void middles(const CycleArgs &A, int32_t v, int l, in
   *m = o[1] - o[0];
 }
 // label-lc segment of middle b: first entry and length
-__device__ __forceinline__ void ends(const CycleArgs &A, int32_t b, long long *st, long long *len) {
+__device__ __forceinline__ void ends(const CycleArgs &A, int32_t b, long long *st, int *len) {
   const int32_t *o = A.loff + (int64_t)b * (A.L + 1) + A.lc;
   const int32_t s = o[0];
   *st = A.off[b] + s;
@@ -95,20 +96,21 @@ __device__ __forceinline__ unsigned long long wedge_bound(const CycleArgs &A, in
 // whole call 5.6 ms then, 3.4 ms now).  The side with fewer
 // wedges is the one that is counted (its counters are written and cleared).
 __global__ void k_cycle_split(CycleArgs A, const int32_t *__restrict__ roots, int64_t nroots, int2 *__restrict__ small,
-                              int2 *__restrict__ big, int *__restrict__ sizes) {
+                              int4 *__restrict__ big, int *__restrict__ sizes) {
   const unsigned lane = lane_id();
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const bool same = A.lb == A.ld;
   const int64_t groups = (nroots + 31) / 32;
   for (int64_t r0 = warp; r0 < groups; r0 += nw) {
-    int2 mine = make_int2(0, 0);
+    int4 mine = make_int4(0, 0, 0, 0);
     int which = 0;  // 1 small, 2 big
     for (int j = 0; j < 32 && r0 + j * groups < nroots; ++j) {
       const int32_t v = roots[r0 + j * groups];
       const unsigned long long wb = wedge_bound(A, v, A.lb, lane), wd = same ? wb : wedge_bound(A, v, A.ld, lane);
       if ((int)lane == j && min(wb, wd) > 0) {
-        mine = make_int2(v, wd < wb);
+        const unsigned long long cap = 0x7fffffffull;
+        mine = make_int4(v, wd < wb, (int)min(min(wb, wd), cap), (int)min(max(wb, wd), cap));
         which = min(wb, wd) <= kSmallBound ? 1 : 2;
       }
     }
@@ -119,34 +121,20 @@ __global__ void k_cycle_split(CycleArgs A, const int32_t *__restrict__ roots, in
       int at = 0;
       if (lane == 0) at = atomicAdd(&sizes[q - 1], __popc(m));
       at = __shfl_sync(0xffffffffu, at, 0);
-      if (which == q) (q == 1 ? small : big)[at + __popc(m & ((1u << lane) - 1u))] = mine;
+      at += __popc(m & ((1u << lane) - 1u));
+      if (which == q && q == 1) small[at] = make_int2(mine.x, mine.y);
+      if (which == q && q == 2) big[at] = mine;
     }
   }
 }
 
-// f(rank of c) for every wedge v - b - c of up to 32 middles b = ladj[s ..
-// s + m): long segments by the whole warp, the others laid end to end.
+// f(rank of c) for every wedge v - b - c of up to 32 middles b = ladj[s .. s + m)
 template <class F>
 __device__ __forceinline__ void walk_wedges(const CycleArgs &A, int64_t s, int m, unsigned lane, F f) {
-  long long st = 0, len = 0;
+  long long st = 0;
+  int len = 0;
   if ((int)lane < m) ends(A, __ldg(A.ladj + s + lane), &st, &len);
-  for (unsigned lm = __ballot_sync(0xffffffffu, len >= kLongSeg); lm; lm &= lm - 1) {
-    const int t = __ffs(lm) - 1;
-    const long long ts = __shfl_sync(0xffffffffu, st, t), te = ts + __shfl_sync(0xffffffffu, len, t);
-    long long i = ts + lane;
-    for (; i + 96 < te; i += 128) {
-      const int32_t x0 = __ldg(A.lrk + i), x1 = __ldg(A.lrk + i + 32), x2 = __ldg(A.lrk + i + 64),
-                    x3 = __ldg(A.lrk + i + 96);
-      f(x0);
-      f(x1);
-      f(x2);
-      f(x3);
-    }
-    for (; i < te; i += 32) f(__ldg(A.lrk + i));
-  }
-  flat_segments(A.lrk, st, len >= kLongSeg ? 0 : len, [&](int, bool valid, int32_t x) {
-    if (valid) f(x);
-  });
+  warp_segments(A.lrk, st, len, lane, f);
 }
 
 __device__ __forceinline__ uint32_t small_slot(int32_t key) { return ((uint32_t)key * 2654435769u) >> (32 - 9); }
@@ -212,13 +200,15 @@ __global__ void __launch_bounds__(kSmallWarps * 32)
 }
 
 __global__ void __launch_bounds__(kBigThreads, kBigPerSm)
-    k_cycle_big(CycleArgs A, const int2 *__restrict__ tasks, int *__restrict__ sizes, unsigned *__restrict__ tails,
+    k_cycle_big(CycleArgs A, const int4 *__restrict__ tasks, int *__restrict__ sizes, unsigned *__restrict__ tails,
                 int64_t tail_len, const int32_t *__restrict__ member, unsigned long long *__restrict__ out) {
   extern __shared__ __align__(16) unsigned hot[];
   __shared__ int s_task;
+  __shared__ WedgeWalk s_walk;
   unsigned *tail = tails + (int64_t)blockIdx.x * tail_len;
   const unsigned lane = lane_id();
-  const int wid = threadIdx.x >> 5;
+  int turn = 0;
+  if (threadIdx.x == 0) s_walk.s[0].next = s_walk.s[0].nlong = 0;
   const int n = sizes[1];
   const bool same = A.lb == A.ld;
   unsigned long long c = 0;
@@ -229,36 +219,32 @@ __global__ void __launch_bounds__(kBigThreads, kBigPerSm)
     const int t = s_task;
     __syncthreads();
     if (t >= n) break;
-    const int2 task = tasks[t];
+    const int4 task = tasks[t];
     const int32_t self = A.skip_root ? A.lrank[task.x] : -1;
-    // f over the wedges of side l, the middles dealt to the warps in runs of
-    // up to 32
-    auto side = [&](int l, auto f) {
+    // f over the wedges of side l
+    auto side = [&](int l, int wedges, auto f) {
       int64_t s;
       int m;
       middles(A, task.x, l, &s, &m);
-      const int run = max(1, min(32, (m + kBigWarps - 1) / kBigWarps));
-      for (int i = wid * run; i < m; i += kBigWarps * run) walk_wedges(A, s + i, min(run, m - i), lane, f);
+      cta_wedges(A.lrk, m, (unsigned long long)wedges, s_walk, &turn,
+                 [&](int i, long long *st, int *len) { ends(A, __ldg(A.ladj + s + i), st, len); }, f);
     };
     const int first = task.y ? A.ld : A.lb;
     if (same) {
-      side(first, [&](int32_t x) {
+      side(first, task.z, [&](int32_t x) {
         if (x == self) return;
         c += 2ull * (x < kHot ? atomicAdd(&hot[x], 1u) : atomicAdd(&tail[x - kHot], 1u));
       });
-      __syncthreads();
     } else {
-      side(first, [&](int32_t x) {
+      side(first, task.z, [&](int32_t x) {
         if (x == self) return;
         if (x < kHot) atomicAdd(&hot[x], 1u);
         else atomicAdd(&tail[x - kHot], 1u);
       });
-      __syncthreads();
-      side(task.y ? A.lb : A.ld, [&](int32_t x) { c += x < kHot ? hot[x] : __ldcg(&tail[x - kHot]); });
-      __syncthreads();
+      side(task.y ? A.lb : A.ld, task.w, [&](int32_t x) { c += x < kHot ? hot[x] : __ldcg(&tail[x - kHot]); });
     }
     // back to zero: the same walk again
-    side(first, [&](int32_t x) {
+    side(first, task.z, [&](int32_t x) {
       if (x < kHot) hot[x] = 0u;
       else tail[x - kHot] = 0u;
     });
@@ -267,7 +253,6 @@ __global__ void __launch_bounds__(kBigThreads, kBigPerSm)
       if (lane == 0 && c) atomicAdd(&out[member[task.x]], c);
       c = 0;
     }
-    __syncthreads();
   }
   c = warp_sum(c);
   if (lane == 0 && c) atomicAdd(out, c);
@@ -401,7 +386,8 @@ int cycle_plan(gpm_graph *g, LabelCsr *lc, const gpm_query *q, CyclePlan *p, Cyc
     s->tail_len = tail_len;
   }
   if ((int64_t)s->big.n < nroots) {
-    DevBuf<int2> small, big;
+    DevBuf<int2> small;
+    DevBuf<int4> big;
     if (small.reserve(nroots) != GPM_OK || big.reserve(nroots) != GPM_OK) return GPM_OK;
     s->small = std::move(small);
     s->big = std::move(big);

@@ -23,7 +23,6 @@
 // each sorted list is the degree-oriented DAG.  Every kernel takes an
 // optional per-vertex graph id so one launch serves a disjoint union of many
 // graphs (batch.cu) with per-graph accumulators.
-#include <cooperative_groups.h>
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -32,10 +31,9 @@
 #include "common.cuh"
 #include "motif.cuh"
 #include "tc_rank.cuh"
+#include "wedge.cuh"
 
 namespace gpm {
-
-namespace cg = cooperative_groups;
 
 static int grid_for(int64_t work, int block = 256) {
   int64_t g = (work + block - 1) / block;
@@ -263,7 +261,6 @@ __global__ void k_c4_tasks(int64_t n, const int64_t *__restrict__ roff, const in
         const int i = atomicAdd(&sizes[2], 1);
         big_tasks[i] = (int32_t)x;
         big_b[i] = b;
-        atomicMax(&sizes[3], (int)dx);
       } else if (b > (unsigned long long)warp_bound) {
         cta_tasks[atomicAdd(&sizes[0], 1)] = (int32_t)x;
       } else {
@@ -343,47 +340,35 @@ __global__ void __launch_bounds__(256) k_c4(const int64_t *__restrict__ roff, co
 }
 
 // ------------------------------------------------------------ giant 4-cycle tasks
-// A task whose 2-hop bound passes big_min has far more distinct y than any
-// shared-memory table holds (nearly every wedge ends at its own y).  Its key
-// range [base, x) is cut into chunks that fit dense counters in shared memory
-// -- 16-bit halves of 32-bit words while x has fewer than 65536 neighbours
-// below it, so no count can carry into the next key.  Each a in N(x), a < x,
-// keeps a cursor into its sorted list, so a chunk walks only its own segment
-// [cur, first y >= hi) and records where it stopped.  Every increment adds
-// the counter's old value to the sum (C(c+1,2) - C(c,2) = c), so a chunk needs
-// no scan.  A dense chunk is then cleared by a vector memset, a sparse one by
-// re-walking the recorded segments.
-// Neighbours are handed out highest rank (longest list) first through a
-// shared counter, one atomic per warp, to lane groups of P = 1..32 lanes (P
-// grows as x has fewer neighbours below it); each lane reads four keys per
-// 16-byte load.  Lists longer than twice the task's mean go first, to whole
-// warps.  Tasks with a bound of at most kC4HashMax skip the chunks and count
-// in one pass in a hash table over the same memory (below).
-// CTA shape: one 1024-thread CTA with 200 KB of counters per SM measured
-// ahead of two 512-thread CTAs with 100 or 110 KB each.
-#ifndef GPM_C4_BIG_THREADS
-#define GPM_C4_BIG_THREADS 1024
-#endif
-#ifndef GPM_C4_BIG_KB
-#define GPM_C4_BIG_KB 200
-#endif
-constexpr int kC4BigThreads = GPM_C4_BIG_THREADS;
-constexpr int kC4BigSmem = GPM_C4_BIG_KB * 1024;
-constexpr int kC4BigWords = kC4BigSmem / 4;
+// A task whose 2-hop bound passes big_min has far more distinct y than a hash
+// table of k_c4's holds (nearly every wedge ends at its own y).  Its counters
+// are indexed by y directly, a window of keys at a time, in shared memory --
+// 16-bit halves of 32-bit words while x has fewer than 65536 neighbours below
+// it, so no count can carry into the next key.  Ranks ascend with degree and y
+// lies below x, so the window just below x takes most wedges (R-MAT 18: 91 %
+// end within 50,000 of x, Chung-Lu 200,000: 61 %).  A task that spans more than
+// kC4Windows windows has shared counters for the first alone and counts the
+// `cold_len` keys below it in the CTA's own array in global memory.  Every
+// increment adds the counter's old value to the sum (C(c+1,2) - C(c,2) = c),
+// so no scan is needed.
+// The walk (wedge.cuh) clips each list to the window by binary search and takes
+// 1.2 G warp instructions for the 0.85 G wedges of R-MAT 18, where lane groups
+// with a cursor per list took 2.2 G (3.88 ms; 3.4 ms now; batch of 48
+// Chung-Lu graphs 13.95 -> 11.8 ms).  It is bound by the latency of the lists
+// and of the counters' old values at 48 warps per SM.  CTA shapes, R-MAT 18 /
+// batch: 2 x 768 threads, 100 KB each 3.4 / 11.8 ms; 1 x 1024, 200 KB 3.2 /
+// 14.5; 3 x 512, 66 KB 4.6 / 12.8; 4 x 384, 49 KB 6.4 / 14.4.  Windows: 8
+// against 4 at R-MAT 18 (six windows): 3.4 / 4.5 ms.
+constexpr int kC4BigThreads = 768, kC4BigPerSm = 2;
+constexpr int kC4HotWords = 25600;  // 100 KB per CTA
+constexpr int kC4BigSmem = kC4HotWords * 4;
+constexpr int kC4Windows = 8;
+constexpr int64_t kC4ColdBytes = 16ll << 30;  // most global memory for cold counters
 
-struct C4Chunk {
-  const int32_t *radj;
-  int64_t nnz;  // radj length: 16-byte loads only inside it
-  int sh;
-  int32_t lo, hi;
-};
-
-// Hash mode: a task whose bound is at most kC4HashMax counts in one pass in an
-// open-addressing table over the same shared memory, slots of (key + 1,
-// count) with 0 = empty, so a cleared array is an empty table and the dense
-// chunks find it zeroed.  The bound caps the distinct keys below the slot
-// count, so every probe sequence ends.
-constexpr unsigned kC4HashSlots = kC4BigWords / 2;
+// Tasks whose bound is at most kC4HashMax count in an open-addressing table
+// over the same shared memory, slots of (key + 1, count) with 0 = empty.  The
+// bound caps the distinct keys below the slot count, so every probe ends.
+constexpr unsigned kC4HashSlots = kC4HotWords / 2;
 constexpr unsigned long long kC4HashMax = kC4HashSlots * 6 / 10;
 __device__ __forceinline__ unsigned c4_hash_add(unsigned *cw, unsigned key1) {
   unsigned h = (unsigned)(((unsigned long long)(key1 * 2654435761u) * kC4HashSlots) >> 32);
@@ -399,203 +384,99 @@ __device__ __forceinline__ unsigned c4_hash_add(unsigned *cw, unsigned key1) {
   return 0u;
 }
 
-// One step of a group of P lanes over a segment at j (< e): lane gl takes the
-// four keys at (j rounded down to 4) + 4 gl.  Keys at or after j that are
-// below hi and before e form a prefix of the step (the list is sorted); they
-// are counted into cw.  Returns the stop position (first key >= hi, or e)
-// when the segment ends inside the step, else -1.
-template <bool HASH>
-__device__ __forceinline__ int64_t c4_step(const C4Chunk &q, unsigned *cw, int64_t j, int64_t e, unsigned gl,
-                                           unsigned gfirst, unsigned gmask, unsigned gbits,
-                                           unsigned long long &c, unsigned &nw) {
-  const int64_t jb = j & ~(int64_t)3;
-  const int64_t p0 = jb + 4 * (int64_t)gl;
-  int32_t v[4];
-  if (p0 + 4 <= q.nnz) {
-    const int4 t = __ldg(reinterpret_cast<const int4 *>(q.radj + p0));
-    v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
-  } else {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = p0 + k < q.nnz ? __ldg(q.radj + p0 + k) : INT32_MAX;
+__device__ __forceinline__ int64_t first_at_least(const int32_t *__restrict__ a, int64_t lo, int64_t hi, int64_t key) {
+  while (lo < hi) {
+    const int64_t mid = (lo + hi) >> 1;
+    if (__ldg(a + mid) < key) lo = mid + 1; else hi = mid;
   }
-  const unsigned hmask = q.sh ? 0xffffu : 0xffffffffu;
-  const int64_t dj = j - p0, de = e - p0;
-  const int skip = dj <= 0 ? 0 : dj >= 4 ? 4 : (int)dj;  // keys of this lane before j
-  const int lim = de <= 0 ? 0 : de >= 4 ? 4 : (int)de;   // keys of this lane before e
-  int n_ok = 0;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const bool ok = k >= skip && k < lim && v[k] < q.hi;
-    if (ok) {
-      const unsigned key = (unsigned)(v[k] - q.lo);
-      if (HASH) {
-        c += c4_hash_add(cw, key + 1);
-      } else {
-        const unsigned w = key >> q.sh, s = (key & (unsigned)q.sh) << 4;
-        const unsigned old = atomicAdd(&cw[w], 1u << s);
-        c += (old >> s) & hmask;
-      }
-      ++n_ok;
-    }
-  }
-  nw += n_ok;
-  const bool out = skip + n_ok < 4;  // this lane saw the end of the segment
-  const unsigned has = (__ballot_sync(gmask, out) >> gfirst) & gbits;
-  if (!has) return -1;
-  const int rel = __shfl_sync(gmask, 4 * (int)gl + skip + n_ok, (int)gfirst + __ffs(has) - 1);
-  return jb + rel;
+  return lo;
 }
 
-__global__ void __launch_bounds__(kC4BigThreads, 1024 / kC4BigThreads)
+__global__ void __launch_bounds__(kC4BigThreads, kC4BigPerSm)
     k_c4_big(const int64_t *__restrict__ roff, const int64_t *__restrict__ split, const int32_t *__restrict__ radj,
-             int64_t nnz, const int32_t *__restrict__ gid, const int64_t *__restrict__ gbase,
-             const int32_t *__restrict__ tasks, const unsigned long long *__restrict__ task_b, int n_tasks,
-             int *__restrict__ counters, int64_t *__restrict__ scratch, int64_t scratch_len,
-             unsigned long long *__restrict__ acc) {
-  extern __shared__ __align__(16) unsigned cw[];
-  __shared__ int s_task, s_nlong, s_next, s_lnext;
-  __shared__ unsigned s_nw[2];
-  __shared__ unsigned long long s_sum;
-  // per-CTA scratch: cursor pairs (two arrays, swapped per chunk), list ends
-  // (bitwise-not for long lists), long-list indices
-  int64_t *cur = scratch + (int64_t)blockIdx.x * 4 * scratch_len;
-  int64_t *nxt = cur + scratch_len;
-  int64_t *end = nxt + scratch_len;
-  int32_t *lng = reinterpret_cast<int32_t *>(end + scratch_len);
+             const int32_t *__restrict__ gid, const int64_t *__restrict__ gbase, const int32_t *__restrict__ tasks,
+             const unsigned long long *__restrict__ task_b, int n_tasks, int *__restrict__ counters,
+             unsigned *__restrict__ colds, int64_t cold_len, unsigned long long *__restrict__ acc) {
+  extern __shared__ __align__(16) unsigned hot[];
+  __shared__ int s_task;
+  __shared__ WedgeWalk s_walk;
+  unsigned *cold = colds + (int64_t)blockIdx.x * cold_len;
   const unsigned lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < kC4BigWords; i += blockDim.x) cw[i] = 0u;
-  C4Chunk q;
-  q.radj = radj;
-  q.nnz = nnz;
+  int turn = 0;
+  if (threadIdx.x == 0) s_walk.s[0].next = s_walk.s[0].nlong = 0;
+  for (int i = threadIdx.x; i < kC4HotWords; i += blockDim.x) hot[i] = 0u;
   while (true) {
-    if (threadIdx.x == 0) {
-      s_task = atomicAdd(&counters[2], 1);
-      s_nlong = 0;
-      s_sum = 0;
-      s_next = 0;
-      s_lnext = 0;
-      s_nw[0] = s_nw[1] = 0;
-    }
+    if (threadIdx.x == 0) s_task = atomicAdd(&counters[2], 1);
     __syncthreads();
     const int t = s_task;
+    __syncthreads();
     if (t >= n_tasks) break;
     const int32_t x = tasks[t];
+    const unsigned long long W = task_b[t];
     const int g = graph_of(gid, x);
-    const int64_t base = gbase ? gbase[g] : 0;
+    const int32_t base = gbase ? (int32_t)gbase[g] : 0;
     const int64_t a0 = roff[x];
     const int dx = (int)(split[x] - a0);
-    q.sh = dx < 65536 ? 1 : 0;
-    int P = 1;
-    while (P < 32 && (int64_t)P * 2 * dx <= (int64_t)blockDim.x * 2) P *= 2;
-    const long long mean = (long long)(task_b[t] / (unsigned long long)dx);
-    const long long long_min = max(64ll * P, 2 * mean);
-    for (int i = threadIdx.x; i < dx; i += blockDim.x) {
-      const int32_t a = radj[a0 + i];
-      const int64_t s = roff[a], e = roff[a + 1];
-      cur[i] = s;
-      const bool lg = P < 32 && e - s > long_min;
-      end[i] = lg ? ~e : e;
-      if (lg) lng[atomicAdd(&s_nlong, 1)] = i;
-    }
-    __syncthreads();
-    const int nlong = s_nlong;
-    const bool hash = task_b[t] <= kC4HashMax;  // one pass over [base, x) in the hash table
-    const int64_t keys = hash ? (int64_t)x - base : (int64_t)kC4BigWords << q.sh;
-    const unsigned gl = lane & (P - 1);
-    const unsigned gfirst = lane & ~(unsigned)(P - 1);
-    const unsigned gmask = P == 32 ? 0xffffffffu : (((1u << P) - 1) << gfirst);
-    const unsigned gbits = P == 32 ? 0xffffffffu : ((1u << P) - 1);
+    const int sh = dx < 65536 ? 1 : 0;
+    const unsigned mask = sh ? 0xffffu : 0xffffffffu;
+    // cold keys of this task
+    const int64_t cl = (int64_t)x - base <= (int64_t)kC4Windows * (kC4HotWords << sh) ? 0 : cold_len << sh;
     unsigned long long c = 0;
-    int parity = 0;
-    for (int64_t lo = base; lo < x; lo += keys, parity ^= 1) {
-      q.lo = (int32_t)lo;
-      q.hi = (int32_t)(lo + keys < (int64_t)x ? lo + keys : (int64_t)x);
-      unsigned nw = 0;
-      // long lists first, one warp each, handed out through s_lnext
-      while (true) {
-        int li = 0;
-        if (lane == 0) li = atomicAdd(&s_lnext, 1);
-        li = __shfl_sync(0xffffffffu, li, 0);
-        if (li >= nlong) break;
-        const int i = lng[li];
-        const int64_t e = ~end[i];
-        int64_t j = cur[i];
-        while (j < e) {
-          const int64_t stop = hash ? c4_step<true>(q, cw, j, e, lane, 0, 0xffffffffu, 0xffffffffu, c, nw)
-                                    : c4_step<false>(q, cw, j, e, lane, 0, 0xffffffffu, 0xffffffffu, c, nw);
-          if (stop >= 0) {
-            j = stop;
-            break;
-          }
-          j = (j & ~(int64_t)3) + 128;
-        }
-        if (lane == 0) nxt[i] = j < e ? j : e;
-      }
-      // short lists: flattened walk, one step or one refill per iteration
-      {
-        int i = -1;
-        int64_t j = 0, e = 0;
-        while (true) {
-          if (j >= e) {
-            if (i >= 0 && gl == 0) nxt[i] = j;
-            int ni = 0;
-            if (gl == 0) {  // one shared atomic for all group leaders of the warp that need an a
-              const cg::coalesced_group ct = cg::coalesced_threads();
-              int base = 0;
-              if (ct.thread_rank() == 0) base = atomicAdd(&s_next, (int)ct.size());
-              ni = ct.shfl(base, 0) + (int)ct.thread_rank();
-            }
-            ni = __shfl_sync(gmask, ni, gfirst);
-            if (ni >= dx) break;
-            i = dx - 1 - ni;  // highest rank (longest lists) first
-            e = end[i];
-            j = cur[i];
-            if (e < 0) {  // long list: walked above
-              i = -1;
-              j = e = 0;
-            }
-            continue;
-          }
-          const int64_t stop = hash ? c4_step<true>(q, cw, j, e, gl, gfirst, gmask, gbits, c, nw)
-                                    : c4_step<false>(q, cw, j, e, gl, gfirst, gmask, gbits, c, nw);
-          if (stop >= 0) j = e = stop;
-          else j = (j & ~(int64_t)3) + 4 * P;
-        }
-      }
-      nw = warp_sum(nw);
-      if (lane == 0 && nw) atomicAdd(&s_nw[parity], nw);
+    if (W <= kC4HashMax) {
+      cta_wedges(radj, dx, W, s_walk, &turn,
+                 [&](int i, long long *st, int *len) {
+                   const int32_t a = radj[a0 + i];
+                   *st = roff[a];
+                   *len = (int)(first_at_least(radj, *st, roff[a + 1], x) - *st);
+                 },
+                 [&](int32_t y) { c += c4_hash_add(hot, (unsigned)(y - base) + 1u); });
+      uint4 *v = reinterpret_cast<uint4 *>(hot);
+      for (int i = threadIdx.x; i < kC4HotWords / 4; i += blockDim.x) v[i] = make_uint4(0u, 0u, 0u, 0u);
       __syncthreads();
-      // clear: memset when dense, else re-walk [cur, nxt)
-      const bool dense = hash || (unsigned long long)s_nw[parity] * 4 > (unsigned long long)kC4BigWords;
-      if (threadIdx.x == 0) {
-        s_next = 0;
-        s_lnext = 0;
-        s_nw[parity ^ 1] = 0;
-      }
-      if (dense) {
-        uint4 *v = reinterpret_cast<uint4 *>(cw);
-        for (int k = threadIdx.x; k < kC4BigWords / 4; k += blockDim.x) v[k] = make_uint4(0u, 0u, 0u, 0u);
-      } else {
-        for (int i = threadIdx.x; i < dx; i += blockDim.x) {
-          const int64_t j1 = nxt[i];
-          for (int64_t j = cur[i]; j < j1; ++j) cw[(unsigned)(__ldg(radj + j) - q.lo) >> q.sh] = 0u;
+    }
+    for (int32_t hi = W <= kC4HashMax ? base : x; hi > base;) {
+      const int32_t hot0 = (int32_t)max((int64_t)base, (int64_t)hi - ((int64_t)kC4HotWords << sh));
+      const int32_t lo = (int32_t)max((int64_t)base, (int64_t)hot0 - cl);
+      // entries of N(a) in [lo, h) for the i-th neighbour a of x
+      auto part = [&](int h) {
+        return [=](int i, long long *st, int *len) {
+          const int32_t a = radj[a0 + i];
+          int64_t s = roff[a];
+          const int64_t e = first_at_least(radj, s, roff[a + 1], h);
+          if (lo > base) s = first_at_least(radj, s, e, lo);
+          *st = s;
+          *len = (int)(e - s);
+        };
+      };
+      cta_wedges(radj, dx, W, s_walk, &turn, part(hi), [&](int32_t y) {
+        if (y >= hot0) {
+          const unsigned o = (unsigned)(y - hot0), s = (o & (unsigned)sh) << 4;
+          c += (atomicAdd(&hot[o >> sh], 1u << s) >> s) & mask;
+        } else {
+          const unsigned o = (unsigned)(y - lo), s = (o & (unsigned)sh) << 4;
+          c += (atomicAdd(&cold[o >> sh], 1u << s) >> s) & mask;
         }
+      });
+      // back to zero: the hot words by a memset when the wedges are many, the
+      // rest by the same walk
+      const bool sweep = W * 4 >= (unsigned long long)kC4HotWords;
+      if (sweep) {
+        const int words = ((hi - hot0) >> sh) + 1;
+        uint4 *v = reinterpret_cast<uint4 *>(hot);
+        for (int i = threadIdx.x; 4 * i < words; i += blockDim.x)
+          if (i < kC4HotWords / 4) v[i] = make_uint4(0u, 0u, 0u, 0u);
       }
-      __syncthreads();
-      int64_t *tmp = cur;
-      cur = nxt;
-      nxt = tmp;
+      if (!sweep || hot0 > lo)
+        cta_wedges(radj, dx, W, s_walk, &turn, part(sweep ? hot0 : hi), [&](int32_t y) {
+          if (y >= hot0) hot[(unsigned)(y - hot0) >> sh] = 0u;
+          else cold[(unsigned)(y - lo) >> sh] = 0u;
+        });
+      else
+        __syncthreads();
+      hi = lo;
     }
     c = warp_sum(c);
-    if (lane == 0 && c) atomicAdd(&s_sum, c);
-    __syncthreads();
-    if (threadIdx.x == 0 && s_sum) atomicAdd(&acc[8 * g + 6], s_sum);
-    // cur and nxt swap once per chunk: restore the base layout for the next task
-    if (cur != scratch + (int64_t)blockIdx.x * 4 * scratch_len) {
-      int64_t *tmp = cur;
-      cur = nxt;
-      nxt = tmp;
-    }
+    if (lane == 0 && c) atomicAdd(&acc[8 * g + 6], c);
   }
 }
 
@@ -703,7 +584,7 @@ int motif_plan_build(const MotifInput &in, MotifPlan *p, cudaStream_t st) {
   GPM_TRY(p->te.reserve(std::max<int64_t>(in.nnz, 1)));
   // queues of the per-edge triangle pass and of the 4-cycle pass
   DevBuf<int> sizes;
-  GPM_TRY(sizes.reserve(6));
+  GPM_TRY(sizes.reserve(5));
   GPM_TRY(p->te_ct.reserve(n));
   GPM_TRY(p->te_wt.reserve(n));
   GPM_TRY(p->c4_ct.reserve(n));
@@ -714,7 +595,7 @@ int motif_plan_build(const MotifInput &in, MotifPlan *p, cudaStream_t st) {
   GPM_TRY(bb.reserve(n));
   GPM_TRY(p->te_counters.reserve(2));
   GPM_TRY(p->c4_counters.reserve(4));
-  GPM_CUDA(cudaMemsetAsync(sizes.p, 0, 6 * sizeof(int), st));
+  GPM_CUDA(cudaMemsetAsync(sizes.p, 0, 5 * sizeof(int), st));
   if (n > 0) {
     k_te_tasks<<<grid_for(n), 256, 0, st>>>(n, roff, p->split.p, std::min(in.te_cta_min, kTeWarpCap / 2), p->te_ct.p, p->te_wt.p, sizes.p);
     if (in.size == 4) {
@@ -728,7 +609,7 @@ int motif_plan_build(const MotifInput &in, MotifPlan *p, cudaStream_t st) {
                                                    p->c4_ct.p, p->c4_wt.p, bt.p, bb.p, sizes.p + 2);
     }
   }
-  int h[6];
+  int h[5];
   GPM_CUDA(cudaMemcpyAsync(h, sizes.p, sizeof h, cudaMemcpyDeviceToHost, st));
   GPM_CUDA(cudaStreamSynchronize(st));
   p->te_nc = h[0];
@@ -756,11 +637,20 @@ int motif_plan_build(const MotifInput &in, MotifPlan *p, cudaStream_t st) {
     int per_sm = 0;
     GPM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_c4_big, kC4BigThreads, kC4BigSmem));
     p->c4_big_grid = std::max(1, per_sm) * num_sms();
-    p->c4_scratch = std::max(h[5], 1);
-    // per CTA: cursors, next cursors, list ends (int64 each), long-list indices (int32, padded)
-    GPM_TRY(p->c4_cur.reserve((size_t)p->c4_scratch * 4 * p->c4_big_grid));
-    if ((reinterpret_cast<uintptr_t>(in.radj) & 15) != 0)
-      return fail(GPM_EINVAL, "motif: adjacency not 16-byte aligned");
+    p->c4_big_grid = std::min(p->c4_big_grid, p->c4_nb);
+    // cold counters for every key below the shared ones of the largest member
+    // (none where all members span few windows), as far as memory goes (fewer:
+    // more passes over the lists)
+    size_t free_b = 0, total_b = 0;
+    GPM_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    int64_t room = std::min<int64_t>(kC4ColdBytes, (int64_t)(free_b / 4)) / 4 / p->c4_big_grid;
+    if (const char *e = getenv("GPM_C4_COLD_LEN")) room = std::min<int64_t>(room, std::max(0ll, atoll(e)));
+    p->c4_cold_len = in.max_graph_n <= (int64_t)kC4Windows * kC4HotWords ? 0 : std::min(room, in.max_graph_n);
+    while (p->c4_cold.reserve((size_t)p->c4_cold_len * p->c4_big_grid) != GPM_OK) {
+      if (p->c4_cold_len == 0) return GPM_ENOMEM;
+      p->c4_cold_len = p->c4_cold_len < 4096 ? 0 : p->c4_cold_len / 2;
+    }
+    GPM_CUDA(cudaMemsetAsync(p->c4_cold.p, 0, sizeof(unsigned) * (size_t)p->c4_cold_len * p->c4_big_grid, st));
     GPM_CUDA(cudaStreamSynchronize(st));
   }
   {
@@ -779,8 +669,8 @@ static int c4_launch(MotifPlan *p, cudaStream_t st) {
   const MotifInput &in = p->in;
   if (p->c4_nb > 0)
     k_c4_big<<<p->c4_big_grid, kC4BigThreads, kC4BigSmem, st>>>(
-        in.roff, p->split.p, in.radj, in.nnz, in.gid, in.gbase, p->c4_bt.p, p->c4_bb.p, p->c4_nb, p->c4_counters.p,
-        p->c4_cur.p, p->c4_scratch, p->acc.p);
+        in.roff, p->split.p, in.radj, in.gid, in.gbase, p->c4_bt.p, p->c4_bb.p, p->c4_nb, p->c4_counters.p,
+        p->c4_cold.p, p->c4_cold_len, p->acc.p);
   if (p->c4_nc + p->c4_nw > 0)
     k_c4<<<p->c4_grid, 256, 0, st>>>(in.roff, p->split.p, in.radj, in.gid, in.gbase, p->c4_ct.p, p->c4_nc,
                                      p->c4_wt.p, p->c4_nw, p->c4_counters.p, p->acc.p);
