@@ -134,7 +134,7 @@ __device__ __forceinline__ void walk_wedges(const CycleArgs &A, int64_t s, int m
   long long st = 0;
   int len = 0;
   if ((int)lane < m) ends(A, __ldg(A.ladj + s + lane), &st, &len);
-  warp_segments(A.lrk, st, len, lane, f);
+  warp_segments(A.lrk, st, len, 0, lane, [&](int32_t x, long long, int) { f(x); });
 }
 
 __device__ __forceinline__ uint32_t small_slot(int32_t key) { return ((uint32_t)key * 2654435769u) >> (32 - 9); }
@@ -227,7 +227,8 @@ __global__ void __launch_bounds__(kBigThreads, kBigPerSm)
       int m;
       middles(A, task.x, l, &s, &m);
       cta_wedges(A.lrk, m, (unsigned long long)wedges, s_walk, &turn,
-                 [&](int i, long long *st, int *len) { ends(A, __ldg(A.ladj + s + i), st, len); }, f);
+                 [&](int i, long long *st, int *len) { ends(A, __ldg(A.ladj + s + i), st, len); },
+                 [&](int32_t x, long long, int) { f(x); });
     };
     const int first = task.y ? A.ld : A.lb;
     if (same) {

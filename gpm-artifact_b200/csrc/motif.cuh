@@ -78,7 +78,7 @@ struct MotifPlan {
   DevBuf<unsigned> te;
   DevBuf<int32_t> te_ct, te_wt, c4_ct, c4_wt, c4_bt;
   DevBuf<unsigned long long> c4_bb;  // giant 4-cycle tasks and their 2-hop bounds, largest first
-  int te_nc = 0, te_nw = 0, c4_nc = 0, c4_nw = 0, c4_nb = 0, te_grid = 0, c4_grid = 0, c4_big_grid = 0;
+  int te_nc = 0, te_nw = 0, te_nl = 0, c4_nc = 0, c4_nw = 0, c4_nb = 0, te_grid = 0, c4_grid = 0, c4_big_grid = 0;
   DevBuf<unsigned> c4_cold;  // cold counters of the giant tasks, c4_cold_len per CTA, zero between launches
   int64_t c4_cold_len = 0;
   DevBuf<int> te_counters, c4_counters;

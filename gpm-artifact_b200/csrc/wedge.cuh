@@ -9,31 +9,34 @@ namespace gpm {
 constexpr int kWedgeLong = 64;    // segments of at least this many entries are streamed by the whole warp
 constexpr int kWedgePiece = 256;  // and, shared by the CTA, in pieces of this many
 
-// f(entry) for data[s .. e), the warp's lanes side by side.
+// Below, f(entry, position, segment) is called for entries data[position] of a
+// numbered segment.
+
+// data[s .. e) of segment `seg`, the warp's lanes side by side
 template <class F>
-__device__ __forceinline__ void warp_stream(const int32_t *__restrict__ data, long long s, long long e, unsigned lane,
-                                            F f) {
+__device__ __forceinline__ void warp_stream(const int32_t *__restrict__ data, long long s, long long e, int seg,
+                                            unsigned lane, F f) {
   long long i = s + lane;
   for (; i + 96 < e; i += 128) {
     const int32_t x0 = __ldg(data + i), x1 = __ldg(data + i + 32), x2 = __ldg(data + i + 64),
                   x3 = __ldg(data + i + 96);
-    f(x0);
-    f(x1);
-    f(x2);
-    f(x3);
+    f(x0, i, seg);
+    f(x1, i + 32, seg);
+    f(x2, i + 64, seg);
+    f(x3, i + 96, seg);
   }
-  for (; i < e; i += 32) f(__ldg(data + i));
+  for (; i < e; i += 32) f(__ldg(data + i), i, seg);
 }
 
-// f(entry) for every entry of the lanes' segments data[st .. st + len): long
-// ones one after another, the others laid end to end over the lanes.
+// Every entry of the lanes' segments data[st .. st + len), lane t's numbered seg0
+// + t: long ones one after another, the others laid end to end over the lanes.
 template <class F>
-__device__ __forceinline__ void warp_segments(const int32_t *__restrict__ data, long long st, int len, unsigned lane,
-                                              F f) {
+__device__ __forceinline__ void warp_segments(const int32_t *__restrict__ data, long long st, int len, int seg0,
+                                              unsigned lane, F f) {
   for (unsigned lm = __ballot_sync(0xffffffffu, len >= kWedgeLong); lm; lm &= lm - 1) {
     const int t = __ffs(lm) - 1;
     const long long ts = __shfl_sync(0xffffffffu, st, t);
-    warp_stream(data, ts, ts + __shfl_sync(0xffffffffu, len, t), lane, f);
+    warp_stream(data, ts, ts + __shfl_sync(0xffffffffu, len, t), seg0 + t, lane, f);
   }
   const int n = len >= kWedgeLong ? 0 : len;
   int inc = n;
@@ -51,7 +54,7 @@ __device__ __forceinline__ void warp_segments(const int32_t *__restrict__ data, 
     for (int r = 16; r; r >>= 1)
       if (__shfl_sync(0xffffffffu, inc, lo + r - 1) <= idx) lo += r;
     const long long ft = __shfl_sync(0xffffffffu, first, lo & 31);
-    if (idx < total) f(__ldg(data + ft + idx));
+    if (idx < total) f(__ldg(data + ft + idx), ft + idx, seg0 + lo);
   }
 }
 
@@ -61,12 +64,12 @@ struct WedgeWalk {
   struct {
     int next, nlong;
     long long st[kLong];
-    int len[kLong];
+    int len[kLong], seg[kLong];
   } s[2];
 };
 
-// f(entry) for every entry of the segments seg(i) -> (start, length) of m
-// middles, W entries in all (an estimate will do), by the CTA.  Runs of
+// Every entry of the segments seg(i) -> (start, length), i < m, of m middles, W
+// entries in all (an estimate will do), by the CTA.  Runs of
 // middles go to the warps through a shared counter; a segment that holds more
 // than 1/64 of the work would keep one warp busy while the others wait at the
 // barrier, so those are listed and shared out in pieces.  (Dealt out in fixed
@@ -96,11 +99,12 @@ __device__ __forceinline__ void cta_wedges(const int32_t *__restrict__ data, int
       if (at < WedgeWalk::kLong) {
         q.st[at] = st;
         q.len[at] = len;
+        q.seg[at] = i + (int)lane;
         len = 0;
       }
     }
     __syncwarp();
-    warp_segments(data, st, len, lane, f);
+    warp_segments(data, st, len, i, lane, f);
   }
   __syncthreads();
   const int nlong = min(q.nlong, WedgeWalk::kLong);
@@ -110,7 +114,7 @@ __device__ __forceinline__ void cta_wedges(const int32_t *__restrict__ data, int
     const int len = q.len[j], pieces = (len + kWedgePiece - 1) / kWedgePiece;
     for (; piece < pieces; piece += nw) {
       const int b = piece * kWedgePiece;
-      warp_stream(data, st + b, st + min(len, b + kWedgePiece), lane, f);
+      warp_stream(data, st + b, st + min(len, b + kWedgePiece), q.seg[j], lane, f);
     }
     piece -= pieces;
   }
