@@ -33,8 +33,6 @@
 // 4-lane groups.  Owners with more than `cta_min` keys are CTA tasks, the
 // rest warp tasks; both queues are sorted heaviest first and drained by a
 // persistent grid.
-#include <cooperative_groups.h>
-#include <cooperative_groups/reduce.h>
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -47,8 +45,6 @@
 #include "tc_rank.cuh"
 
 namespace gpm {
-
-namespace cg = cooperative_groups;
 
 constexpr int kRWarps = 8;
 constexpr int kCtaWords = kRankCtaWords;
@@ -376,16 +372,83 @@ __global__ void k_rank_inverse(int64_t n, const int32_t *__restrict__ order, con
 constexpr int kSortCap = 1024;
 constexpr int kGatherWarps = 8;
 
-__device__ __forceinline__ int32_t warp_bitonic32(int32_t key, unsigned lane) {
+// Bitonic sort of 32 E keys in the registers of a warp: key i is k[i / 32] of
+// lane i % 32, so exchanges over 32 or more are between registers and the
+// others one shuffle.
+template <int E>
+__device__ __forceinline__ void warp_bitonic(int32_t (&k)[E], unsigned lane) {
 #pragma unroll
-  for (int k = 2; k <= 32; k <<= 1)
+  for (int kk = 2; kk <= 32 * E; kk <<= 1)
 #pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      const int32_t other = __shfl_xor_sync(0xffffffffu, key, j);
-      const bool asc = (lane & k) == 0, low = (lane & j) == 0;
-      key = (low == asc) ? min(key, other) : max(key, other);
+    for (int j = kk >> 1; j > 0; j >>= 1) {
+      if (j >= 32) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          const int p = e ^ (j >> 5);
+          if (p < e) continue;
+          const int32_t lo = min(k[e], k[p]), hi = max(k[e], k[p]);
+          const bool asc = ((32 * e) & kk) == 0;
+          k[e] = asc ? lo : hi;
+          k[p] = asc ? hi : lo;
+        }
+      } else {
+        const bool low = (lane & j) == 0;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          const int32_t other = __shfl_xor_sync(0xffffffffu, k[e], j);
+          const bool asc = kk >= 32 ? ((32 * e) & kk) == 0 : (lane & kk) == 0;
+          k[e] = (low == asc) ? min(k[e], other) : max(k[e], other);
+        }
+      }
     }
-  return key;
+}
+template <int E>
+__device__ __forceinline__ void warp_sort_regs(const int32_t *src, int32_t *dst, int len, unsigned lane) {
+  int32_t k[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) k[e] = 32 * e + (int)lane < len ? src[32 * e + lane] : INT_MAX;
+  warp_bitonic<E>(k, lane);
+  __syncwarp();
+#pragma unroll
+  for (int e = 0; e < E; ++e)
+    if (32 * e + (int)lane < len) dst[32 * e + lane] = k[e];
+}
+
+// src[0 .. len) sorted into dst by one warp, len <= kSortCap; buf: kSortCap
+// ids of shared memory (may be src).  Up to 512 ids in registers (with the
+// shared-memory network for everything above 32 the relabel of R-MAT 22 took
+// 2.36 ms in k_rank_gather_sort).
+__device__ __forceinline__ void warp_sort(const int32_t *src, int32_t *dst, int len, int32_t *buf, unsigned lane) {
+  if (len <= 32) {
+    warp_sort_regs<1>(src, dst, len, lane);
+  } else if (len <= 64) {
+    warp_sort_regs<2>(src, dst, len, lane);
+  } else if (len <= 128) {
+    warp_sort_regs<4>(src, dst, len, lane);
+  } else if (len <= 256) {
+    warp_sort_regs<8>(src, dst, len, lane);
+  } else if (len <= 512) {
+    warp_sort_regs<16>(src, dst, len, lane);
+  } else {
+    const int p = kSortCap;
+    for (int i = lane; i < p; i += 32) buf[i] = i < len ? src[i] : INT_MAX;
+    __syncwarp();
+    for (int k = 2; k <= p; k <<= 1)
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        for (int i = lane; i < p; i += 32) {
+          const int ixj = i ^ j;
+          if (ixj > i) {
+            const int32_t a = buf[i], b = buf[ixj];
+            if ((a > b) == ((i & k) == 0)) {
+              buf[i] = b;
+              buf[ixj] = a;
+            }
+          }
+        }
+        __syncwarp();
+      }
+    for (int i = lane; i < len; i += 32) dst[i] = buf[i];
+  }
 }
 
 __global__ void __launch_bounds__(kGatherWarps * 32)
@@ -419,30 +482,7 @@ __global__ void __launch_bounds__(kGatherWarps * 32)
       if (lane == 0) big[atomicAdd(nbig, 1)] = (int32_t)r;
       continue;
     }
-    if (len <= 32) {
-      const int32_t key = warp_bitonic32((int64_t)lane < len ? buf[lane] : INT_MAX, lane);
-      if ((int64_t)lane < len) out[o + lane] = key;
-    } else {
-      int p = 64;
-      while (p < len) p <<= 1;
-      for (int i = (int)len + lane; i < p; i += 32) buf[i] = INT_MAX;
-      __syncwarp();
-      for (int k = 2; k <= p; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-          for (int i = lane; i < p; i += 32) {
-            const int ixj = i ^ j;
-            if (ixj > i) {
-              const int32_t a = buf[i], b = buf[ixj];
-              if ((a > b) == ((i & k) == 0)) {
-                buf[i] = b;
-                buf[ixj] = a;
-              }
-            }
-          }
-          __syncwarp();
-        }
-      for (int64_t i = lane; i < len; i += 32) out[o + i] = buf[i];
-    }
+    warp_sort(buf, out + o, (int)len, buf, lane);
     __syncwarp();
   }
 }
@@ -497,82 +537,160 @@ __device__ __forceinline__ int64_t upper_bound_key(const int32_t *__restrict__ a
   return lo;
 }
 
+// What the placement needs of a vertex, in one 32-byte sector: its list
+// (start, len) and the smallest and largest key of it, its first 16-byte row
+// in radj4, and its core bitmap row (-1: none).
+struct __align__(32) VertexInfo {
+  uint32_t start;
+  int32_t len, kmin, kmax, row4, rowid;
+  int32_t pad[2];
+};
+__global__ void k_vertex_info(int64_t n, const int64_t *__restrict__ roff, const int32_t *__restrict__ radj,
+                              const int64_t *__restrict__ roff4, const int32_t *__restrict__ rowid,
+                              VertexInfo *__restrict__ info) {
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t s = roff[v], e = roff[v + 1];
+    VertexInfo f;
+    f.start = (uint32_t)s;
+    f.len = (int32_t)(e - s);
+    f.kmin = e > s ? radj[s] : 0;
+    f.kmax = e > s ? radj[e - 1] : 0;
+    f.row4 = (int32_t)(roff4[v] >> 2);
+    f.rowid = rowid ? rowid[v] : -1;
+    f.pad[0] = f.pad[1] = 0;
+    info[v] = f;
+  }
+}
+
 // Every stored edge k = (u, radj[k]) placed in one pass: the endpoint with
 // the longer list owns it (ties to u), the other is its partner; the segment
 // is the part of the partner's list inside [min, max] of the owner's list
 // (empty, hence left out, also when the owner has fewer than 2 keys and so
 // closes no triangle through the edge).  It goes into the owner's room
 // [poff[x], poff[x+1]) -- one slot per incident edge, so it always fits --
-// long segments from the front (cursor plong[x]), short ones from the back
-// (cursor pshort[x]), as ranges of radj4.  With radj4 non-null the pass also
-// copies each list u into it (with its INT32_MAX padding).  upward: every list holds only ids above its vertex,
-// so when u owns the edge, min N(u) <= v < every id of N(v) and the lower
-// search is skipped.  The lanes of a warp that share an (owner, class) take
-// their slots with one atomic (hub owners get most of theirs from their own
-// list, i.e. from one warp).
+// long segments from the front (cursor lcnt[x]), short ones from the back
+// (cursor scnt[x]), as ranges of radj4; a cursor's upper half adds up the keys
+// that will be streamed.  With radj4 non-null the pass also copies each list u
+// into it (with its INT32_MAX padding).  upward: every list holds only ids
+// above its vertex, so when u owns the edge, min N(u) <= v < every id of N(v)
+// and the lower search is skipped.
+// A warp takes 32 consecutive edges at a time (ustart[c]: the vertex of edge 32
+// c), in edge order over the grid, so that an owner's segments arrive about in
+// the order of their partners and the count kernel finds their lists near one
+// another.  Edges that u owns take their slots with one atomic per run of
+// lanes of the same u; the others have owners of their own.  (R-MAT 22: 4.2 ms
+// with a warp per vertex, a labelled partition of the lanes by owner and a
+// third atomic for the work.  Blocks of 32 vertices per warp: 3.0 ms, but the
+// count then took 4.4 ms in place of 4.25, and R-MAT 20 waited for the warps
+// with 32 hubs.)
+__global__ void k_chunk_starts(int64_t n, const int64_t *__restrict__ roff, int32_t *__restrict__ ustart) {
+  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x)
+    for (int64_t c = (roff[u] + 31) >> 5; 32 * c < roff[u + 1]; ++c) ustart[c] = (int32_t)u;
+}
 __global__ void k_partner_place(int64_t n, const int64_t *__restrict__ roff, const int32_t *__restrict__ radj,
-                                const int64_t *__restrict__ roff4, int32_t *__restrict__ radj4, int upward,
-                                int long_min, const uint8_t *__restrict__ cfg,
-                                const int64_t *__restrict__ poff, int32_t *__restrict__ plong,
-                                int32_t *__restrict__ pshort, Seg *__restrict__ pseg,
-                                unsigned long long *__restrict__ work, int32_t core_base,
-                                const int32_t *__restrict__ rowid, int row_words, int dense_pct,
+                                const int32_t *__restrict__ ustart, const VertexInfo *__restrict__ info,
+                                int32_t *__restrict__ radj4, int upward, int long_min,
+                                const uint8_t *__restrict__ cfg, const int64_t *__restrict__ poff,
+                                unsigned long long *__restrict__ lcnt, unsigned long long *__restrict__ scnt,
+                                Seg *__restrict__ pseg, int32_t core_base, int row_words, int dense_pct,
                                 int32_t *__restrict__ pdense, int *__restrict__ too_long) {
-  int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t u = warp; u < n; u += nw) {
-    int64_t s = roff[u], e = roff[u + 1], du = e - s;
-    if (radj4) {  // u's list into radj4 with its padding, one 16-byte row per lane
-      int4 *row = reinterpret_cast<int4 *>(radj4 + roff4[u]);
-      for (int64_t r = lane_id(); 4 * r < du; r += 32) {
-        const int64_t b = s + 4 * r;
-        row[r] = make_int4(radj[b], b + 1 < e ? radj[b + 1] : INT32_MAX, b + 2 < e ? radj[b + 2] : INT32_MAX,
-                           b + 3 < e ? radj[b + 3] : INT32_MAX);
+  const unsigned lane = lane_id(), below = (1u << lane) - 1u;
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int64_t nnz = roff[n], chunks = (nnz + 31) >> 5;
+  for (int64_t c0 = warp; c0 < chunks; c0 += nw) {
+    const int64_t k = 32 * c0 + lane;
+    const bool valid = k < nnz;
+    // the vertex of edge k: the last one whose list starts at or before k
+    int32_t t = -1;
+    if (valid) {
+      int32_t lo = ustart[c0], hi = c0 + 1 < chunks ? ustart[c0 + 1] : (int32_t)n - 1;
+      while (lo < hi) {
+        const int32_t mid = lo + ((hi - lo + 1) >> 1);
+        if (roff[mid] <= k) lo = mid; else hi = mid - 1;
+      }
+      t = lo;
+    }
+    // lanes of the same u are a run; its first lane and its lanes
+    const int32_t before = __shfl_up_sync(0xffffffffu, t, 1);
+    const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || t != before);
+    const int head = 31 - __clz(heads & (below | (1u << lane)));
+    const unsigned after = heads & ~(below | (1u << lane));
+    const unsigned run = (after ? (1u << (__ffs(after) - 1)) - 1u : ~0u) & ~((1u << head) - 1u);
+    bool own_u = false, lng = false, seg = false;
+    int32_t owner = 0;
+    Seg sg = make_int2(0, 0);
+    unsigned units = 0;
+    if (valid) {
+      const int32_t u = t, v = radj[k];
+      const VertexInfo U = info[u], V = info[v];
+      if (radj4) {
+        int32_t *row = radj4 + 4 * (int64_t)U.row4;
+        const int at = (int)(k - (int64_t)U.start);
+        row[at] = v;
+        if (at == U.len - 1)
+          for (int i = U.len; i & 3; ++i) row[i] = INT32_MAX;
+      }
+      own_u = V.len <= U.len;
+      owner = own_u ? u : v;
+      const int32_t kmin = own_u ? U.kmin : V.kmin, kmax = own_u ? U.kmax : V.kmax;
+      const VertexInfo P = own_u ? V : U;
+      if ((own_u ? U.len : V.len) >= 2 && P.len > 0) {
+        const int64_t ps = P.start, pe = ps + P.len;
+        // upward: when v owns the edge, every id of N(u) up to v sits at or
+        // before slot k, and min N(v) > v, so the search starts past k
+        const int64_t lo = upward && own_u ? ps : lower_bound_key(radj, upward ? k + 1 : ps, pe, kmin);
+        const int64_t len = (P.kmax <= kmax ? pe : upper_bound_key(radj, lo, pe, kmax)) - lo;
+        if (len > 0) {
+          seg = true;
+          // dense: a core owner and a partner with a core row, the keys at
+          // least dense_pct % of the owner's words to AND (k_tc_dense counts
+          // it; the count kernel only skips its descriptor)
+          int64_t row = -1;  // dense: the uint4 index of the partner's row words from the owner's base
+          if (P.rowid >= 0 && kmin >= core_base &&
+              100 * len >= (int64_t)dense_pct * core_and_words(kmin, kmax))
+            row = (int64_t)P.rowid * (row_words >> 2) + (((kmin & ~127) - core_base) >> 7);
+          units = row >= 0 ? 0u : (unsigned)len;
+          lng = row >= 0 || len >= owner_long_min(cfg, owner, long_min);
+          const int64_t lo4 = lo - ps;  // the same keys in radj4
+          if (len >= (1 << 29)) *too_long = 1;  // no 8-byte descriptor for it
+          sg = row >= 0 ? make_int2((int)(-1 - row), (int)(len << 2))
+                        : make_int2((int)(P.row4 + (lo4 >> 2)), (int)((len << 2) | (lo4 & 3)));
+          if (row >= 0) atomicAdd(&pdense[owner], 1);
+        }
       }
     }
-    for (int64_t k = s + lane_id(); k < e; k += 32) {
-      int32_t v = radj[k];
-      int64_t vs = roff[v], ve = roff[v + 1], dv = ve - vs;
-      bool own_u = dv <= du;
-      int32_t owner = own_u ? (int32_t)u : v;
-      int64_t os = own_u ? s : vs, oe = own_u ? e : ve;
-      int64_t ps = own_u ? vs : s, pe = own_u ? ve : e;
-      if (oe - os < 2) continue;
-      // upward: when v owns the edge, every id of N(u) up to v sits at or
-      // before slot k, and min N(v) > v, so the search starts past k
-      const int64_t lo = upward ? (own_u ? ps : lower_bound_key(radj, k + 1, pe, radj[os]))
-                                : lower_bound_key(radj, ps, pe, radj[os]);
-      const int64_t len = upper_bound_key(radj, lo, pe, radj[oe - 1]) - lo;
-      if (len == 0) continue;
-      const int32_t partner = own_u ? v : (int32_t)u;
-      // dense: a core owner and a partner with a core row, the keys at least
-      // dense_pct % of the owner's words to AND (k_tc_dense counts it; the
-      // count kernel only skips its descriptor)
-      int64_t row = -1;  // dense: the uint4 index of the partner's row words from the owner's base
-      if (rowid && radj[os] >= core_base) {
-        const int32_t kmin = radj[os], r = rowid[partner];
-        if (r >= 0 && 100 * len >= (int64_t)dense_pct * core_and_words(kmin, radj[oe - 1]))
-          row = (int64_t)r * (row_words >> 2) + (((kmin & ~127) - core_base) >> 7);
-      }
-      const int64_t units = row >= 0 ? 0 : len;
-      const bool lng = row >= 0 || len >= owner_long_min(cfg, owner, long_min);
-      cg::coalesced_group grp =
-          cg::labeled_partition(cg::coalesced_threads(), ((unsigned long long)(uint32_t)owner << 1) | lng);
-      int base = 0;
-      if (grp.thread_rank() == 0) base = atomicAdd(lng ? &plong[owner] : &pshort[owner], (int)grp.size());
-      const int64_t slot = grp.shfl(base, 0) + (int64_t)grp.thread_rank();
-      const int64_t pos = lng ? poff[owner] + slot : poff[owner + 1] - 1 - slot;
-      const int64_t lo4 = lo - roff[partner] + roff4[partner];  // the same keys in radj4
-      if (len >= (1 << 29)) *too_long = 1;  // no 8-byte descriptor for it
-      pseg[pos] = row >= 0 ? make_int2((int)(-1 - row), (int)(len << 2))
-                           : make_int2((int)(lo4 >> 2), (int)((len << 2) | (lo4 & 3)));
-      const unsigned long long w = cg::reduce(grp, (unsigned long long)units + 1ull, cg::plus<unsigned long long>());
-      if (grp.thread_rank() == 0) atomicAdd(&work[owner], w);
-      if (rowid) {
-        const int nd = __popc(grp.ballot(row >= 0));
-        if (nd && grp.thread_rank() == 0) atomicAdd(&pdense[owner], nd);
+    // slots of the edges that u owns: long and short ones, run by run
+    int64_t slot = 0;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const bool take = seg && own_u && lng == (c == 0);
+      const unsigned m = __ballot_sync(0xffffffffu, take) & run;
+      if (take) {
+        const unsigned sum = __reduce_add_sync(m, units);
+        const int lead = __ffs(m) - 1;
+        unsigned long long at = 0;
+        if ((int)lane == lead)
+          at = atomicAdd(c == 0 ? &lcnt[owner] : &scnt[owner],
+                         ((unsigned long long)sum << 32) | (unsigned)__popc(m));
+        slot = (int64_t)(unsigned)__shfl_sync(m, at, lead) + __popc(m & below);
       }
     }
+    if (seg && !own_u)
+      slot = (int64_t)(unsigned)atomicAdd(lng ? &lcnt[owner] : &scnt[owner], ((unsigned long long)units << 32) | 1ull);
+    if (seg) pseg[lng ? poff[owner] + slot : poff[owner + 1] - 1 - slot] = sg;
+  }
+}
+// The cursors taken apart: segments of each class, and the owner's work (keys
+// streamed plus one per segment)
+__global__ void k_place_counts(int64_t n, const unsigned long long *__restrict__ lcnt,
+                               const unsigned long long *__restrict__ scnt, int32_t *__restrict__ plong,
+                               int32_t *__restrict__ pshort, unsigned long long *__restrict__ work) {
+  for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
+    const unsigned long long l = lcnt[x], s = scnt[x];
+    plong[x] = (int32_t)(uint32_t)l;
+    pshort[x] = (int32_t)(uint32_t)s;
+    work[x] = (l >> 32) + (s >> 32) + (uint32_t)l + (uint32_t)s;
   }
 }
 // Dense core rows: rowid[v] = a row number when v has at least min_keys
@@ -771,68 +889,16 @@ static int rank_order(gpm_graph *g, const int32_t *indeg, const int32_t *gid, in
   return GPM_OK;
 }
 
-// dst[0 .. len) sorted in place by one warp (len <= kSortCap): a register
-// bitonic network up to 32 ids, else a shared-memory network in buf.
-__device__ __forceinline__ void warp_sort_list(int32_t *dst, int64_t len, int32_t *buf, unsigned lane) {
-  if (len <= 1) return;
-  if (len <= 32) {
-    const int32_t key = warp_bitonic32((int64_t)lane < len ? dst[lane] : INT_MAX, lane);
-    if ((int64_t)lane < len) dst[lane] = key;
-    return;
-  }
-  int p = 64;
-  while (p < len) p <<= 1;
-  for (int i = lane; i < p; i += 32) buf[i] = i < len ? dst[i] : INT_MAX;
-  __syncwarp();
-  for (int k = 2; k <= p; k <<= 1)
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = lane; i < p; i += 32) {
-        const int ixj = i ^ j;
-        if (ixj > i) {
-          const int32_t a = buf[i], b = buf[ixj];
-          if ((a > b) == ((i & k) == 0)) {
-            buf[i] = b;
-            buf[ixj] = a;
-          }
-        }
-      }
-      __syncwarp();
-    }
-  for (int64_t i = lane; i < len; i += 32) dst[i] = buf[i];
-  __syncwarp();
-}
-
 // Upward lists of a symmetric graph, gathered chunk by chunk: for source
 // vertex v, the ranks of its neighbours above rank[v], appended (unsorted)
 // into tmp at v's own symmetric offset -- room for all of v's neighbours, so
 // no count pass is needed first.  A vertex with at most kHubBlock neighbours
-// is one warp's task; a longer list is cut into kHubBlock-entry block tasks
+// is one warp's task; a longer list is cut into kHubPiece-entry block tasks
 // (queued here, run by k_up_gather_hub) so that no warp scans a hub's whole
 // list alone.
 constexpr int kHubBlock = 1024;
+constexpr int kHubPiece = 256;
 static_assert(kHubBlock <= kSortCap, "a non-hub list must fit the sort buffer");
-
-__device__ __forceinline__ int64_t gather_upward(int32_t r, int64_t s, int64_t e, const int32_t *__restrict__ rank,
-                                                 const int32_t *__restrict__ adj, int32_t *dst,
-                                                 unsigned long long *cursor, unsigned lane) {
-  int64_t len = 0;
-  for (int64_t base = s; base < e; base += 32) {
-    const int64_t k = base + lane;
-    const int32_t x = k < e ? rank[adj[k]] : -1;
-    const bool keep = k < e && x > r;
-    const unsigned m = __ballot_sync(0xffffffffu, keep);
-    if (m == 0) continue;
-    int64_t at = len;
-    if (cursor) {  // shared with the hub's other block tasks
-      unsigned long long b = 0;
-      if (lane == 0) b = atomicAdd(cursor, (unsigned long long)__popc(m));
-      at = (int64_t)__shfl_sync(0xffffffffu, b, 0);
-    }
-    if (keep) dst[at + __popc(m & ((1u << lane) - 1u))] = x;
-    len += __popc(m);
-  }
-  return len;
-}
 
 __global__ void __launch_bounds__(kGatherWarps * 32)
     k_up_gather(int64_t v0, int64_t v1, const int32_t *__restrict__ rank, const int64_t *__restrict__ off,
@@ -844,37 +910,75 @@ __global__ void __launch_bounds__(kGatherWarps * 32)
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t v = v0 + warp; v < v1; v += nw) {
-    const int64_t s = off[v], e = off[v + 1];
-    if (e - s > kHubBlock) {
-      const int nb = (int)((e - s + kHubBlock - 1) / kHubBlock);
+    const int64_t s = off[v];
+    const int64_t deg = off[v + 1] - s;
+    if (deg > kHubBlock) {
+      const int nb = (int)((deg + kHubPiece - 1) / kHubPiece);
+      int at = 0;
       if (lane == 0) {
         hubcnt[v] = 0;
-        const int at = atomicAdd(nhubq, nb);
-        for (int b = 0; b < nb; ++b) hubq[at + b] = make_int2((int)v, b);
+        at = atomicAdd(nhubq, nb);
       }
+      at = __shfl_sync(0xffffffffu, at, 0);
+      for (int b = lane; b < nb; b += 32) hubq[at + b] = make_int2((int)v, b);
       continue;
     }
     const int32_t r = rank[v];
-    const int64_t len = gather_upward(r, s, e, rank, adj, tmp + s, nullptr, lane);
+    int len = 0;
+    for (int b = 0; b < (int)deg; b += 32) {
+      const bool in = b + (int)lane < (int)deg;
+      const int32_t x = in ? rank[adj[s + b + lane]] : -1;
+      const bool keep = x > r;
+      const unsigned m = __ballot_sync(0xffffffffu, keep);
+      if (keep) buf[len + __popc(m & ((1u << lane) - 1u))] = x;
+      len += __popc(m);
+    }
     if (lane == 0) kept[r] = len;
     __syncwarp();
-    warp_sort_list(tmp + s, len, buf, lane);  // len <= kHubBlock = kSortCap
+    if (len) warp_sort(buf, tmp + s, len, buf, lane);
+    __syncwarp();
   }
 }
 
+// One piece of a hub's list per warp: its kHubPiece entries at once, one
+// atomic for their place in the hub's list.  (Pieces of 1024 entries with an
+// atomic per 32 took 42 us per chunk of the upload, one warp's chain of
+// latencies.)
 __global__ void k_up_gather_hub(const int2 *__restrict__ hubq, const int *__restrict__ nhubq,
                                 const int32_t *__restrict__ rank, const int64_t *__restrict__ off,
                                 const int32_t *__restrict__ adj, int32_t *__restrict__ tmp,
                                 unsigned long long *__restrict__ hubcnt) {
-  const unsigned lane = lane_id();
+  const unsigned lane = lane_id(), below = (1u << lane) - 1u;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const int nt = *nhubq;
+  constexpr int E = kHubPiece / 32;
   for (int64_t t = warp; t < nt; t += nw) {
     const int2 task = hubq[t];
-    const int64_t s = off[task.x], e = off[task.x + 1];
-    const int64_t b0 = s + (int64_t)task.y * kHubBlock, b1 = min(e, b0 + kHubBlock);
-    gather_upward(rank[task.x], b0, b1, rank, adj, tmp + s, &hubcnt[task.x], lane);
+    const int64_t s = off[task.x], b0 = s + (int64_t)task.y * kHubPiece;
+    const int cnt = (int)min((int64_t)kHubPiece, off[task.x + 1] - b0);
+    const int32_t r = rank[task.x];
+    int32_t x[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) x[e] = 32 * e + (int)lane < cnt ? adj[b0 + 32 * e + lane] : -1;
+#pragma unroll
+    for (int e = 0; e < E; ++e) x[e] = x[e] >= 0 ? rank[x[e]] : -1;
+    unsigned m[E];
+    int total = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      m[e] = __ballot_sync(0xffffffffu, x[e] > r);
+      total += __popc(m[e]);
+    }
+    if (total == 0) continue;
+    unsigned long long at = 0;
+    if (lane == 0) at = atomicAdd(&hubcnt[task.x], (unsigned long long)total);
+    int64_t o = s + (int64_t)__shfl_sync(0xffffffffu, at, 0);
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      if (x[e] > r) tmp[o + __popc(m[e] & below)] = x[e];
+      o += __popc(m[e]);
+    }
   }
 }
 
@@ -907,7 +1011,9 @@ __global__ void __launch_bounds__(kGatherWarps * 32)
       if (len > kSortCap) {
         if (lane == 0) big[atomicAdd(nbig, 1)] = (int32_t)r;
       } else {
-        warp_sort_list(src, len, buf, lane);
+        warp_sort(src, radj + o, (int)len, buf, lane);
+        __syncwarp();
+        continue;
       }
     }
     for (int64_t i = lane; i < len; i += 32) radj[o + i] = src[i];
@@ -935,8 +1041,8 @@ int build_upward_rank_graph(gpm_graph *g, cudaStream_t st, const int64_t *h_off,
   DevBuf<int> nbig, nhubq;
   DevBuf<unsigned long long> hubcnt;
   DevBuf<int2> hubq;
-  // hub block tasks: at most nsym / kHubBlock + (number of hubs) of them
-  const int64_t maxq = nsym / kHubBlock + nsym / (kHubBlock + 1) + 1;
+  // hub block tasks: at most nsym / kHubPiece + (number of hubs) of them
+  const int64_t maxq = nsym / kHubPiece + nsym / (kHubBlock + 1) + 1;
   if ((s = r->order.reserve(n)) || (s = rank.reserve(n)) || (s = kept.reserve(n)) || (s = r->roff.reserve(n + 1)) ||
       (s = inc.reserve(n)) || (s = r->rinc.reserve(n + 1)) || (s = tmp.reserve(std::max<int64_t>(nsym, 1))) ||
       (s = big.reserve(n)) || (s = nbig.reserve(1)) ||
@@ -1191,9 +1297,12 @@ int rank_plan_new(gpm_graph *g, int cta_min, int long_min, const uint8_t *cfg, c
   DevBuf<unsigned long long> work;
   if ((s = work.reserve(n))) return bail(s);
   cudaMemcpyAsync(p->poff.p, g->rg->rinc.p, sizeof(int64_t) * (n + 1), cudaMemcpyDeviceToDevice, st);
-  cudaMemsetAsync(p->plong.p, 0, sizeof(int32_t) * n, st);
-  cudaMemsetAsync(p->pshort.p, 0, sizeof(int32_t) * n, st);
-  cudaMemsetAsync(work.p, 0, sizeof(unsigned long long) * n, st);
+  DevBuf<unsigned long long> lcnt, scnt;
+  DevBuf<VertexInfo> info;
+  if ((s = lcnt.reserve(n)) || (s = scnt.reserve(n)) || (s = info.reserve(n))) return bail(s);
+  cudaMemsetAsync(lcnt.p, 0, sizeof(unsigned long long) * n, st);
+  cudaMemsetAsync(scnt.p, 0, sizeof(unsigned long long) * n, st);
+  if (g->rg->radj.n >= ((size_t)1 << 32)) return bail(fail(GPM_EUNSUPPORTED, "triangle plan: 2^32 keys or more"));
   // 8-byte segment descriptors address radj4 by 16-byte rows in 31 bits
   if ((int64_t)(g->rg->radj4.n / 4) >= ((int64_t)1 << 31))
     return bail(fail(GPM_EUNSUPPORTED, "triangle plan: more than 2^33 padded keys"));
@@ -1210,10 +1319,15 @@ int rank_plan_new(gpm_graph *g, int cta_min, int long_min, const uint8_t *cfg, c
   DevBuf<int> sizes;
   if ((s = sizes.reserve(5))) return bail(s);
   cudaMemsetAsync(sizes.p, 0, 5 * sizeof(int), st);
-  k_partner_place<<<grid_for(n * 32), 256, 0, st>>>(n, roff, radj, g->rg->roff4.p, fill ? g->rg->radj4.p : nullptr,
-                                                     g->rg->upward, long_min, cfg, p->poff.p, p->plong.p, p->pshort.p,
-                                                     p->pseg.p, work.p, p->core_base, p->n_rows ? rowid.p : nullptr,
-                                                     p->row_words, dense_pct, p->pdense.p, sizes.p + 4);
+  k_vertex_info<<<grid_for(n), 256, 0, st>>>(n, roff, radj, g->rg->roff4.p, p->n_rows ? rowid.p : nullptr, info.p);
+  const int64_t keys = (int64_t)g->rg->radj.n;
+  DevBuf<int32_t> ustart;
+  if ((s = ustart.reserve((keys + 31) / 32))) return bail(s);
+  k_chunk_starts<<<grid_for(n), 256, 0, st>>>(n, roff, ustart.p);
+  k_partner_place<<<grid_for(keys), 256, 0, st>>>(n, roff, radj, ustart.p, info.p, fill ? g->rg->radj4.p : nullptr, g->rg->upward,
+                                               long_min, cfg, p->poff.p, lcnt.p, scnt.p, p->pseg.p, p->core_base,
+                                               p->row_words, dense_pct, p->pdense.p, sizes.p + 4);
+  k_place_counts<<<grid_for(n), 256, 0, st>>>(n, lcnt.p, scnt.p, p->plong.p, p->pshort.p, work.p);
   GPM_LAUNCH_CHECK();
   if (p->n_rows) {  // the dense segments moved out of the long ones
     DevBuf<int64_t> cnt;
