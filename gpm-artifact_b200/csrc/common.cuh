@@ -239,6 +239,8 @@ struct gpm_graph {
   int64_t nnz = 0;
   int32_t max_deg = 0;
   uint64_t sum_deg2 = 0;  // sum of the squared list lengths
+  bool symmetric = false; // every stored entry has its reverse (built so, not oriented since)
+  gpm::DevBuf<int32_t> odeg;  // oriented from a symmetric graph: each vertex's degree there (in + out degree now)
   double hash_us = 0;     // estimated time of gpm_tc's counts with the hash kernel (tc.cu)
   int oriented = 0;
   int relabeled = 0;

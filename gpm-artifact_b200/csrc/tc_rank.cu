@@ -346,11 +346,12 @@ __global__ void k_indeg(int64_t nnz, const int32_t *__restrict__ adj, int32_t *_
     atomicAdd(&indeg[adj[i]], 1);
 }
 // sort key: (graph id, in + out degree); the stable sort breaks ties by id.
-// indeg == nullptr: the stored graph is symmetric, out-degree orders alike
+// deg: that degree where it is known; indeg == deg == nullptr: the stored graph
+// is symmetric, out-degree orders alike
 __global__ void k_rank_keys(int64_t n, const int64_t *__restrict__ off, const int32_t *__restrict__ indeg,
-                            const int32_t *__restrict__ gid, uint64_t *__restrict__ key, int32_t *__restrict__ val) {
+                            const int32_t *__restrict__ deg, const int32_t *__restrict__ gid, uint64_t *__restrict__ key, int32_t *__restrict__ val) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    uint64_t d = (uint64_t)(uint32_t)((off[i + 1] - off[i]) + (indeg ? indeg[i] : 0));
+    uint64_t d = deg ? (uint64_t)(uint32_t)deg[i] : (uint64_t)(uint32_t)((off[i + 1] - off[i]) + (indeg ? indeg[i] : 0));
     key[i] = gid ? ((uint64_t)(uint32_t)gid[i] << 32) | d : d;
     val[i] = (int32_t)i;
   }
@@ -487,11 +488,13 @@ __global__ void __launch_bounds__(kGatherWarps * 32)
   }
 }
 
-// incident edges of rank r: its out-degree plus the in-degree of order[r]
+// incident edges of rank r: its out-degree plus the in-degree of order[r], as
+// k_rank_keys knows them
 __global__ void k_incident(int64_t n, const int32_t *__restrict__ order, const int64_t *__restrict__ rdeg,
-                           const int32_t *__restrict__ indeg, int64_t *__restrict__ inc) {
+                           const int32_t *__restrict__ indeg, const int32_t *__restrict__ deg,
+                           int64_t *__restrict__ inc) {
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
-    inc[r] = rdeg[r] + indeg[order[r]];
+    inc[r] = deg ? deg[order[r]] : indeg ? rdeg[r] + indeg[order[r]] : 2 * rdeg[r];
 }
 
 __global__ void k_big_bounds(int nbig, const int32_t *__restrict__ big, const int64_t *__restrict__ roff,
@@ -763,25 +766,32 @@ __global__ void k_padded_len(int64_t n, const int64_t *__restrict__ roff, int64_
     len4[v] = (roff[v + 1] - roff[v] + 3) & ~(int64_t)3;
 }
 
-// dense tasks: owners with dense segments, key = ~(their words to AND)
+// sort keys of the task queues: ~work, work capped to 32 bits, so that an
+// ascending sort of four passes puts heavy tasks first
+__device__ __forceinline__ uint32_t task_key(unsigned long long work) {
+  return ~(uint32_t)min(work, 0xffffffffull);
+}
+
+// dense tasks: owners with dense segments, by their words to AND
 __global__ void k_dense_tasks(int64_t n, const int64_t *__restrict__ roff, const int32_t *__restrict__ radj,
-                              const int32_t *__restrict__ pdense, unsigned long long *__restrict__ key,
+                              const int32_t *__restrict__ pdense, uint32_t *__restrict__ key,
                               int32_t *__restrict__ val, int *__restrict__ size) {
   for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
     if (pdense[x] == 0) continue;
     const int i = atomicAdd(size, 1);
-    key[i] = ~((unsigned long long)pdense[x] * (unsigned long long)core_and_words(radj[roff[x]], radj[roff[x + 1] - 1]));
+    key[i] = task_key((unsigned long long)pdense[x] *
+                      (unsigned long long)core_and_words(radj[roff[x]], radj[roff[x + 1] - 1]));
     val[i] = (int32_t)x;
   }
 }
 
-// tasks: owners with partners; key = ~work so an ascending sort puts heavy first
+// tasks: owners with partners, by their work
 __global__ void k_rank_tasks(int64_t n, const int64_t *__restrict__ roff, const int32_t *__restrict__ plong,
                              const int32_t *__restrict__ pshort,
                              const unsigned long long *__restrict__ work, int cta_min,
                              const uint8_t *__restrict__ cfg, const int32_t *__restrict__ pdense,
-                             int32_t *__restrict__ donly, unsigned long long *__restrict__ ckey,
-                             int32_t *__restrict__ cval, unsigned long long *__restrict__ wkey,
+                             int32_t *__restrict__ donly, uint32_t *__restrict__ ckey,
+                             int32_t *__restrict__ cval, uint32_t *__restrict__ wkey,
                              int32_t *__restrict__ wval, int *__restrict__ sizes) {
   for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
     if (plong[x] + pshort[x] == 0) {  // nothing to stream
@@ -791,11 +801,11 @@ __global__ void k_rank_tasks(int64_t n, const int64_t *__restrict__ roff, const 
     int64_t d = roff[x + 1] - roff[x];
     if (cfg ? cfg[x] / 3 == 1 : d > cta_min) {
       int i = atomicAdd(&sizes[0], 1);
-      ckey[i] = ~work[x];
+      ckey[i] = task_key(work[x]);
       cval[i] = (int32_t)x;
     } else {
       int i = atomicAdd(&sizes[1], 1);
-      wkey[i] = ~work[x];
+      wkey[i] = task_key(work[x]);
       wval[i] = (int32_t)x;
     }
   }
@@ -803,16 +813,15 @@ __global__ void k_rank_tasks(int64_t n, const int64_t *__restrict__ roff, const 
 
 void free_rank_plan(RankPlan *p) { delete p; }
 
-static int sort_pairs_u64(DevBuf<unsigned long long> &k, DevBuf<int32_t> &v, int count, DevBuf<int32_t> &out,
-                          cudaStream_t st) {
+static int sort_tasks(DevBuf<uint32_t> &k, DevBuf<int32_t> &v, int count, DevBuf<int32_t> &out, cudaStream_t st) {
   if (count <= 0) return GPM_OK;
-  DevBuf<unsigned long long> k2;
+  DevBuf<uint32_t> k2;
   GPM_TRY(k2.reserve(count));
   size_t tmp = 0;
-  GPM_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, k.p, k2.p, v.p, out.p, count, 0, 64, st));
+  GPM_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, k.p, k2.p, v.p, out.p, count, 0, 32, st));
   DevBuf<char> t;
   GPM_TRY(t.reserve(tmp));
-  GPM_CUDA(cub::DeviceRadixSort::SortPairs(t.p, tmp, k.p, k2.p, v.p, out.p, count, 0, 64, st));
+  GPM_CUDA(cub::DeviceRadixSort::SortPairs(t.p, tmp, k.p, k2.p, v.p, out.p, count, 0, 32, st));
   return GPM_OK;
 }
 
@@ -868,8 +877,8 @@ static int finish_rank_graph(RankGraph *r, int64_t n, int64_t nnz, const int32_t
 }
 
 // Rank keys of the stored graph sorted: order[rank] = vertex, rank[vertex].
-// indeg == nullptr: a symmetric graph (out-degree orders like in + out).
-static int rank_order(gpm_graph *g, const int32_t *indeg, const int32_t *gid, int ngraphs, int32_t *order,
+// indeg, deg: as k_rank_keys takes them.
+static int rank_order(gpm_graph *g, const int32_t *indeg, const int32_t *deg, const int32_t *gid, int ngraphs, int32_t *order,
                       int32_t *rank, int64_t *rdeg, cudaStream_t st) {
   const int64_t n = g->n;
   int s;
@@ -879,7 +888,7 @@ static int rank_order(gpm_graph *g, const int32_t *indeg, const int32_t *gid, in
   int end_bit = 32;
   if (gid)
     while (end_bit < 64 && (1ll << (end_bit - 32)) < ngraphs) ++end_bit;
-  k_rank_keys<<<grid_for(n), 256, 0, st>>>(n, g->off.p, indeg, gid, key.p, val.p);
+  k_rank_keys<<<grid_for(n), 256, 0, st>>>(n, g->off.p, indeg, deg, gid, key.p, val.p);
   size_t tmp = 0;
   GPM_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, key.p, key2.p, val.p, order, (int)n, 0, end_bit, st));
   DevBuf<char> t;
@@ -1078,7 +1087,7 @@ int build_upward_rank_graph(gpm_graph *g, cudaStream_t st, const int64_t *h_off,
     }
   // 2. ranks from the degrees alone (symmetric input), meanwhile; a
   // vertex's symmetric degree is its incident-edge count in the DAG
-  if ((s = rank_order(g, nullptr, nullptr, 1, r->order.p, rank.p, inc.p, st))) return bail(s);
+  if ((s = rank_order(g, nullptr, nullptr, nullptr, 1, r->order.p, rank.p, inc.p, st))) return bail(s);
   if ((s = scan_i64(n, inc.p, r->rinc.p, st))) return bail(s);
   // 3. each chunk gathered as soon as it has landed: small lists one warp
   // each, hub lists as block tasks over the whole grid
@@ -1132,15 +1141,22 @@ int ensure_rank_graph(gpm_graph *g, cudaStream_t st, const int32_t *gid, int ngr
   DevBuf<int32_t> indeg, rank, big;
   DevBuf<int64_t> rdeg, inc;
   DevBuf<int> nbig;
-  if ((s = indeg.reserve(n)) || (s = r->order.reserve(n)) || (s = rank.reserve(n)) || (s = rdeg.reserve(n)) ||
+  if ((s = r->order.reserve(n)) || (s = rank.reserve(n)) || (s = rdeg.reserve(n)) ||
       (s = inc.reserve(n)) || (s = r->roff.reserve(n + 1)) || (s = r->rinc.reserve(n + 1)) ||
       (s = r->radj.reserve(std::max<int64_t>(nnz, 1))) || (s = big.reserve(n)) || (s = nbig.reserve(1)))
     return bail(s);
-  cudaMemsetAsync(indeg.p, 0, sizeof(int32_t) * n, st);
-  k_indeg<<<grid_for(nnz), 256, 0, st>>>(nnz, g->adj.p, indeg.p);
-  if ((s = rank_order(g, indeg.p, gid, ngraphs, r->order.p, rank.p, rdeg.p, st))) return bail(s);
+  // in-degrees are counted only where the graph's history does not give them
+  // (R-MAT 22: 0.95 ms of atomics)
+  const bool known = g->symmetric || g->odeg.p;
+  const int32_t *deg = g->odeg.p;
+  if (!known) {
+    if ((s = indeg.reserve(n))) return bail(s);
+    cudaMemsetAsync(indeg.p, 0, sizeof(int32_t) * n, st);
+    k_indeg<<<grid_for(nnz), 256, 0, st>>>(nnz, g->adj.p, indeg.p);
+  }
+  if ((s = rank_order(g, indeg.p, deg, gid, ngraphs, r->order.p, rank.p, rdeg.p, st))) return bail(s);
   if ((s = scan_i64(n, rdeg.p, r->roff.p, st))) return bail(s);
-  k_incident<<<grid_for(n), 256, 0, st>>>(n, r->order.p, rdeg.p, indeg.p, inc.p);
+  k_incident<<<grid_for(n), 256, 0, st>>>(n, r->order.p, rdeg.p, indeg.p, deg, inc.p);
   if ((s = scan_i64(n, inc.p, r->rinc.p, st))) return bail(s);
   cudaMemcpyAsync(&r->nin, r->rinc.p + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st);
   // gather + sort in one pass; lists longer than kSortCap get a segmented
@@ -1345,9 +1361,9 @@ int rank_plan_new(gpm_graph *g, int cta_min, int long_min, const uint8_t *cfg, c
   }
   if (fill) g->rg->padded = 1;
   // 3. task queues, heaviest first
-  DevBuf<unsigned long long> ckey, wkey;
+  DevBuf<uint32_t> ckey, wkey;
   DevBuf<int32_t> cval, wval;
-  DevBuf<unsigned long long> dkey;
+  DevBuf<uint32_t> dkey;
   DevBuf<int32_t> dval;
   if ((s = ckey.reserve(n)) || (s = wkey.reserve(n)) || (s = cval.reserve(n)) || (s = wval.reserve(n)) ||
       (s = p->cta_tasks.reserve(n)) || (s = p->warp_tasks.reserve(n)))
@@ -1370,8 +1386,8 @@ int rank_plan_new(gpm_graph *g, int cta_min, int long_min, const uint8_t *cfg, c
   p->n_dense = h[2];
   p->n_dense_only = h[3];
   if (p->n_dense && (s = p->dense_tasks.reserve(p->n_dense))) return bail(s);
-  if ((s = sort_pairs_u64(ckey, cval, h[0], p->cta_tasks, st)) || (s = sort_pairs_u64(wkey, wval, h[1], p->warp_tasks, st)) ||
-      (s = sort_pairs_u64(dkey, dval, h[2], p->dense_tasks, st)))
+  if ((s = sort_tasks(ckey, cval, h[0], p->cta_tasks, st)) || (s = sort_tasks(wkey, wval, h[1], p->warp_tasks, st)) ||
+      (s = sort_tasks(dkey, dval, h[2], p->dense_tasks, st)))
     return bail(s);
   if (p->n_dense) {
     p->dense_smem = (size_t)(p->row_words + 4) * sizeof(uint32_t);
