@@ -21,8 +21,9 @@
 // longer than the rest of L looks that rest up in the list instead, and hubs
 // answer for the top ranks from a bitmap.  R-MAT 20, 4-cliques: 24.1 ms with a
 // binary search of L per entry, 13.2 ms with table and search, 7.6 ms with the
-// bitmaps too (6.5 ms CTA tasks, issue-bound with 11 of 32 lanes active in the
-// AND loops; 1.1 ms warp tasks).
+// bitmaps too, 5.8 ms with the rows ANDed strip by strip (cq_pairs; a row word
+// per thread kept 11 of 32 lanes active): 4.7 ms CTA tasks, 75 % issue-active,
+// and 1.1 ms warp tasks.
 // Graphs whose stored edges do not all point upward in rank order, or with
 // an out-list longer than 2048, use an edge-centric kernel shaped like the
 // reference (materialised lists in per-warp global scratch).
@@ -397,6 +398,8 @@ struct CqLayout {
   size_t tab, xl, heavy, moves, comp, comp_words, rows, total;
   int logcap;
 };
+// Words from one row to the next: cq_pairs reads 4-cliques' rows 16 bytes at a time.
+__host__ __device__ constexpr int cq_stride(int W, int k) { return k == 4 ? (W + 3) & ~3 : W; }
 __host__ __device__ inline CqLayout cq_layout(int d, int k, int nwarps, bool rows_in) {
   CqLayout l;
   const int W = (d + 31) >> 5;
@@ -410,7 +413,7 @@ __host__ __device__ inline CqLayout cq_layout(int d, int k, int nwarps, bool row
   l.comp = l.moves + (k == 5 ? (6 * (size_t)W + 3) & ~(size_t)3 : 0);
   l.comp_words = k == 5 ? nwarps * cq_warp_words(W) : 0;
   l.rows = l.comp + l.comp_words;
-  l.total = l.rows + (rows_in ? (size_t)d * W : 0);
+  l.total = l.rows + (rows_in ? (size_t)d * cq_stride(W, k) : 0);
   return l;
 }
 
@@ -510,14 +513,14 @@ __device__ unsigned long long clique_cta_task(int32_t u, int k, const int64_t *_
   const unsigned lane = tid & 31;
   const int64_t s0 = roff[u];
   const int d = (int)(roff[u + 1] - s0);
-  const int W = (d + 31) >> 5;
+  const int W = (d + 31) >> 5, RS = KM == 4 ? cq_stride(W, 4) : W;
   const CqLayout lay = cq_layout(d, k, nw, SM);
   int32_t *L = reinterpret_cast<int32_t *>(smem);
   uint16_t *tab = reinterpret_cast<uint16_t *>(smem + lay.tab);
   uint32_t *rows = SM ? smem + lay.rows : slab;
   for (int i = tid; i < d; i += nthr) L[i] = radj[s0 + i];
   for (int i = tid; i < (1 << lay.logcap) / 2; i += nthr) smem[lay.tab + i] = ~0u;
-  for (int i = tid; i < d * W; i += nthr) rows[i] = 0u;
+  for (int i = tid; i < d * RS; i += nthr) rows[i] = 0u;
   __syncthreads();
   for (int i = tid; i < d; i += nthr) {
     uint32_t h = ((uint32_t)L[i] * 2654435769u) >> (32 - lay.logcap);
@@ -552,7 +555,7 @@ __device__ unsigned long long clique_cta_task(int32_t u, int k, const int64_t *_
     for (int j = 0; j < 32 && i0 + j * nw < d; ++j) {
       const int i = i0 + j * nw, len = __shfl_sync(0xffffffffu, mlen, j), row = __shfl_sync(0xffffffffu, mrow, j);
       const int32_t *__restrict__ list = radj + __shfl_sync(0xffffffffu, ms, j);
-      uint32_t *ri = rows + i * W;
+      uint32_t *ri = rows + i * RS;
       const int jend = row < 0 ? d : jc;  // positions from jend on by the bitmap
       if (row >= 0) {
         const uint32_t *__restrict__ bits = core.rows + (size_t)row * core.words;
@@ -595,19 +598,15 @@ __device__ unsigned long long clique_cta_task(int32_t u, int k, const int64_t *_
   __syncthreads();
   unsigned long long c = 0;
   if (KM == 4) {
-    // a thread per row word: its members l, each ANDed with the row from l's
-    // word on (row_l has no bits below l)
-    for (int x = tid; x < d * W; x += nthr) {
-      uint32_t word = rows[x];
-      if (!word) continue;
-      const int i = x / W, w = x - i * W;
-      unsigned s = 0;
-      for (; word; word &= word - 1) {
-        const uint32_t *rl = rows + (w * 32 + __ffs(word) - 1) * W;
-        for (int ww = w; ww < W; ++ww) s += __popc(rows[i * W + ww] & rl[ww]);
-      }
-      c += s;
-    }
+    // (strip r, word w >= r, columns from 4 (w / 4) on; row_l has no bits below l)
+    const int strips = W;
+    unsigned s = 0;
+    int t = 0;
+    for (int w = 0; w < strips; ++w)
+      for (int q = w & ~3; q < strips; q += 4)
+        for (int r = 0; r <= w; ++r, ++t)
+          if (t % nw == wid) s += cq_pairs<4>(rows, RS, d, r, w, q, lane);
+    c += s;
   } else if (KM == 5) {
     // For each row i, the triangles of the local DAG inside X = row_i: the
     // rows of X's members are compacted to X's columns (|X| bits in place of
