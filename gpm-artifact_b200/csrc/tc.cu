@@ -354,6 +354,68 @@ __global__ void __launch_bounds__(256) k_tc_hash(const int64_t *__restrict__ off
   }
 }
 
+// ------------------------------------------------------------------ LISTS
+// Graphs whose lists are all short: a lane per stored edge u->v merges the two
+// lists, one or two sectors each.  No tables, queues or plan.  A warp takes
+// `span` consecutive vertices (a power of two up to 32, so that small graphs
+// fill the GPU), their edges end to end over its lanes.  Bound by the latency
+// of the merge's dependent loads, so only for the shortest lists.  ER, count /
+// first count in us, against hash kernel and rank plan: 16,384 x 16 (longest
+// list 15) 17 / 28, 17 / 44, 26 / 375; 100,003 x 20 (20) 71 / 83, 78 / 111, 82 /
+// 495; 10^6 x 12 (13) 160 / 173, 344 / 400, 345 / 1268.  But 10^6 x 32 (30) 952,
+// 920, 654, and Chung-Lu 100,001 x 8 (33) 114, 93, 52.
+constexpr int kListDegree = 24;  // longest list
+__global__ void __launch_bounds__(256) k_tc_lists(int64_t n, int span, const int64_t *__restrict__ off,
+                                                  const int32_t *__restrict__ adj, HashState *__restrict__ state,
+                                                  unsigned long long *__restrict__ out) {
+  const int lane = (int)lane_id();
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  unsigned long long c = 0;
+  for (int64_t u0 = warp * span; u0 < n; u0 += nw * span) {
+    const int64_t u = u0 + lane;
+    const bool in = lane < span && u < n;
+    const int64_t s = in ? off[u] : 0, e = in ? off[u + 1] : INT64_MAX;
+    const int last = (int)min((int64_t)span, n - u0) - 1;
+    const int64_t k0 = __shfl_sync(0xffffffffu, s, 0), k1 = __shfl_sync(0xffffffffu, e, last);
+    for (int64_t base = k0; base < k1; base += 32) {
+      const int64_t k = base + lane;
+      int t = 0;  // u = u0 + t: the first lane whose list ends past k
+#pragma unroll
+      for (int r = 16; r; r >>= 1)
+        if (__shfl_sync(0xffffffffu, e, t + r - 1) <= k) t += r;
+      int64_t i = __shfl_sync(0xffffffffu, s, t & 31);
+      const int64_t i1 = __shfl_sync(0xffffffffu, e, t & 31);
+      if (k >= k1) continue;
+      const int32_t v = __ldg(adj + k);
+      int64_t j = off[v];
+      const int64_t j1 = off[v + 1];
+      if (j >= j1) continue;
+      int32_t x = __ldg(adj + i), y = __ldg(adj + j);
+      unsigned hits = 0;
+      while (true) {
+        hits += x == y;
+        const bool ai = x <= y, aj = y <= x;
+        if (ai && ++i >= i1) break;
+        if (aj && ++j >= j1) break;
+        if (ai) x = __ldg(adj + i);
+        if (aj) y = __ldg(adj + j);
+      }
+      c += hits;
+    }
+  }
+  c = cta_sum(c);
+  if (threadIdx.x == 0) {
+    if (c) atomicAdd(&state->sum, c);
+    __threadfence();
+    if (atomicAdd(&state->done, 1) == (int)gridDim.x - 1) {
+      __threadfence();
+      *out = atomicExch(&state->sum, 0ull);
+      state->done = 0;
+    }
+  }
+}
+
 // Task split by degree (the reference's USE_WARP / USE_CTA thresholds).
 __global__ void k_tc_split(int64_t n, const int64_t *__restrict__ off, int warp_min, int cta_min,
                            int32_t *__restrict__ cta_tasks, int32_t *__restrict__ warp_tasks,
@@ -443,6 +505,23 @@ int tc_launch(gpm_graph *g, int variant, cudaStream_t st, unsigned long long *d_
   return fail(GPM_EINVAL, "unknown triangle-count variant " + std::to_string(variant));
 }
 
+static int lists_launch(gpm_graph *g, cudaStream_t st, unsigned long long *d_out) {
+  if (!g->tc_state.p) {
+    GPM_TRY(g->tc_state.reserve(sizeof(HashState) / sizeof(int)));
+    GPM_CUDA(cudaMemsetAsync(g->tc_state.p, 0, sizeof(HashState), st));
+  }
+  // one vertex per warp until all SMs have 32 warps, then more
+  const int64_t warps = (int64_t)num_sms() * 32;
+  int span = 1;
+  while (span < 32 && (g->n + span - 1) / span > warps) span *= 2;
+  const int64_t blocks = ((g->n + span - 1) / span + kWarps - 1) / kWarps;
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(blocks, (int64_t)num_sms() * 32));
+  k_tc_lists<<<grid, 256, 0, st>>>(g->n, span, g->off.p, g->adj.p, reinterpret_cast<HashState *>(g->tc_state.p),
+                                   d_out);
+  GPM_LAUNCH_CHECK();
+  return GPM_OK;
+}
+
 // gpm_tc's kernel.  The rank plan's repeated counts are the faster ones on
 // every graph of some size, but the plan has to be built first.  Microseconds
 // (hash count; rank count; its first count, plan included): R-MAT 14: 145, 83,
@@ -453,6 +532,7 @@ int tc_launch(gpm_graph *g, int variant, cudaStream_t st, unsigned long long *d_
 // within a factor of two, 5 ps each), and otherwise when the counts made on
 // this graph with the hash kernel have cost as much as the plan.
 static int tc_auto_launch(gpm_graph *g, cudaStream_t st, unsigned long long *d_out) {
+  if (g->nnz > 0 && g->max_deg <= kListDegree) return lists_launch(g, st, d_out);
   if (!g->rank && g->nnz > 0) {
     const double hash_us = 10 + 5e-6 * (double)g->sum_deg2, plan_us = 300 + 2.5e-4 * (double)g->nnz;
     if (hash_us < 40 || g->hash_us + hash_us < plan_us) {
@@ -474,7 +554,10 @@ extern "C" {
 
 int gpm_tc_async(gpm_graph *g, int variant, void *stream, uint64_t *d_out) {
   if (!g || !d_out) return fail(GPM_EINVAL, "gpm_tc_async: NULL argument");
-  if (variant == GPM_TC_AUTO) variant = GPM_TC_BITMAP;
+  if (variant == GPM_TC_AUTO) {
+    if (g->nnz > 0 && g->max_deg <= kListDegree) return lists_launch(g, (cudaStream_t)stream, (unsigned long long *)d_out);
+    variant = GPM_TC_BITMAP;
+  }
   if (variant == GPM_TC_LEARNED) return tc_learned_launch(g, (cudaStream_t)stream, (unsigned long long *)d_out);
   return tc_launch(g, variant, (cudaStream_t)stream, (unsigned long long *)d_out);
 }

@@ -15,6 +15,11 @@ GRAPHS = {
     # more tail tasks than eight per resident warp
     "er200k": lambda: gpm.gen_er(200003, 1400000, seed=3),
     "hubs": lambda: gpm.gen_chung_lu(30001, 2.1, 40.0, seed=4),
+    # short lists around the merging kernel's limit, a last warp of one vertex
+    "er65": lambda: gpm.gen_er(65, 200, seed=5),
+    "er5k": lambda: gpm.gen_er(4737, 40000, seed=6),
+    "clique25": lambda: (25, *(x.astype(np.int32) for x in np.triu_indices(25, 1))),
+    "clique26": lambda: (26, *(x.astype(np.int32) for x in np.triu_indices(26, 1))),
 }
 
 
@@ -35,8 +40,10 @@ def test_every_count_of_a_row(name, oriented):
         assert g.tc(gpm.E_CENTRIC if i % 2 else gpm.V_CENTRIC) == want, i
         g.tc_async(gpm.TC_HASH, stream, out.data_ptr())
         assert int(out.item()) == want, i
-    g.tc_async(gpm.TC_BITMAP, stream, out.data_ptr())
-    assert int(out.item()) == want
+    for variant in (gpm.TC_BITMAP, gpm.TC_AUTO, gpm.TC_AUTO):
+        out.fill_(-1)
+        g.tc_async(variant, stream, out.data_ptr())
+        assert int(out.item()) == want, variant
     g.drop_plans()
     assert g.tc() == want
 
