@@ -150,11 +150,10 @@ struct CqWarp {
   uint8_t tab[256];
 };
 
-// first i of 64 with pre[i] > x (pre inclusive, x < pre[63])
-__device__ __forceinline__ int segment_of(const int32_t *pre, int x) {
+// first i of 2 * half with pre[i] > x (pre inclusive, x < its last)
+__device__ __forceinline__ int segment_of(const int32_t *pre, int half, int x) {
   int lo = 0;
-#pragma unroll
-  for (int s = 32; s; s >>= 1)
+  for (int s = half; s; s >>= 1)
     if (pre[lo + s - 1] <= x) lo += s;
   return lo;
 }
@@ -165,8 +164,8 @@ __device__ unsigned long long clique_warp_task(int32_t u, int k, const int64_t *
   const int64_t s0 = roff[u];
   const int d = (int)(roff[u + 1] - s0);
   reinterpret_cast<uint2 *>(sm.tab)[lane] = make_uint2(~0u, ~0u);
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
+  const int halves = d > 32 ? 2 : 1;
+  for (int h = 0; h < halves; ++h) {
     const int i = (int)lane + 32 * h;
     if (i < d) sm.L[i] = radj[s0 + i];
     sm.rows[i] = 0ull;
@@ -174,8 +173,7 @@ __device__ unsigned long long clique_warp_task(int32_t u, int k, const int64_t *
   __syncwarp();
   const int32_t kmax = sm.L[d - 1];
   int carry_s = 0, carry_p = 0;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
+  for (int h = 0; h < halves; ++h) {
     const int i = (int)lane + 32 * h;
     int ns = 0, np = 0;
     if (i < d) {
@@ -216,12 +214,12 @@ __device__ unsigned long long clique_warp_task(int32_t u, int k, const int64_t *
   __syncwarp();
   // both kinds of work laid end to end, so short lists leave no lanes idle
   for (int x = lane; x < carry_s; x += 32) {
-    const int i = segment_of(sm.scan, x);
+    const int i = segment_of(sm.scan, 16 * halves, x);
     const int p = find_pos(sm.tab, 8, sm.L, __ldg(radj + sm.st[i] + (x - (sm.scan[i] - sm.len[i]))));
     if (p >= 0) atomicOr(&sm.rows[i], 1ull << p);
   }
   for (int x = lane; x < carry_p; x += 32) {
-    const int i = segment_of(sm.pair, x);
+    const int i = segment_of(sm.pair, 16 * halves, x);
     const int j = d - (sm.pair[i] - x);
     if (in_list(radj + sm.st[i], sm.len[i], sm.L[j])) atomicOr(&sm.rows[i], 1ull << j);
   }

@@ -528,21 +528,21 @@ __device__ __forceinline__ int32_t (*warp_rows(int32_t (*narrow)[32]))[32] {
 template <bool TRACK, int Q, bool WGT>
 __global__ void __launch_bounds__(kMatchWarps * 32, Q > kNarrowQ ? 2 : WGT ? GPM_MATCH_WGT_BLOCKS : GPM_MATCH_MIN_BLOCKS)
     k_match(QueryPlanT<Q> q, MatchGraph G, const int32_t *__restrict__ rows, int t, int64_t n,
-            unsigned long long *__restrict__ cursor, unsigned long long *__restrict__ out, unsigned long long limit,
-            unsigned long long *found, int32_t *__restrict__ emb_out) {
+            int pool, unsigned long long *__restrict__ cursor, unsigned long long *__restrict__ out,
+            unsigned long long limit, unsigned long long *found, int32_t *__restrict__ emb_out) {
   __shared__ int32_t sbuf[kMatchWarps][Q <= kNarrowQ ? Q : 1][32];
   int32_t(*buf)[32] = warp_rows<Q>(sbuf[threadIdx.x >> 5]);
   const unsigned lane = lane_id();
   unsigned long long c = 0;
-  const bool pool = !TRACK && q.n == 3 && t == 2;  // 32 pairs at a time
+  // pool: that many pairs at a time (three-position plans)
   while (true) {
     unsigned long long r = 0;
-    if (lane == 0) r = atomicAdd(cursor, pool ? 32ull : 1ull);
+    if (lane == 0) r = atomicAdd(cursor, !TRACK && pool ? (unsigned long long)pool : 1ull);
     r = __shfl_sync(0xffffffffu, r, 0);
     if (r >= (unsigned long long)n) break;
     if (TRACK && *(volatile unsigned long long *)found >= limit) break;
-    if (pool) {
-      const int k = (int)min((long long)32, (long long)n - (long long)r);
+    if (!TRACK && pool) {
+      const int k = (int)min((long long)pool, (long long)n - (long long)r);
       const int2 p = (int)lane < k ? reinterpret_cast<const int2 *>(rows)[r + lane] : make_int2(0, 0);
       c += match_pairs3<Q, WGT>(q, G, p.x, p.y, k, buf[0]);
     } else {
@@ -1049,6 +1049,14 @@ int gpm_query_destroy(gpm_query *q) {
 
 namespace gpm {
 
+// (root, second vertex) pairs of a three-position plan that a warp closes
+// together: as many as leave two tasks for every resident warp (48 per SM), up to
+// 32.  R-MAT 16, 12,000 pairs of a triangle query: 129 us one by one, 191 us
+// in 32s; R-MAT 19 and larger queries have pairs for 32.
+static int pair_pool(int64_t npairs) {
+  return (int)std::min<int64_t>(32, std::max<int64_t>(1, npairs / ((int64_t)num_sms() * 96)));
+}
+
 // One k_match launch over the (root, second vertex) pairs on a persistent
 // grid (occupancy x SMs, per device and plan width).
 template <int Q>
@@ -1064,19 +1072,20 @@ static int launch_match(const QueryPlanT<Q> &plan, const MatchGraph &G, const in
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kMatchWarps * 32, smem);
     return std::max(1, per_sm) * num_sms();
   };
+  const int pool = plan.n == 3 && t == 2 ? pair_pool(nrows) : 0;
   const int grid = match_grid.get([&] {
     if (smem > 0) cudaFuncSetAttribute(k_match<true, Q, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     return grid_of(k_match<false, Q, false>);
   });
   if (track)
     k_match<true, Q, false>
-        <<<grid, kMatchWarps * 32, smem>>>(plan, G, rows, t, nrows, cursor, out, limit, found, emb);
+        <<<grid, kMatchWarps * 32, smem>>>(plan, G, rows, t, nrows, pool, cursor, out, limit, found, emb);
   else if (kWgt && plan.nw)
     k_match<false, Q, kWgt><<<wgt_grid.get([&] { return grid_of(k_match<false, Q, kWgt>); }), kMatchWarps * 32, smem>>>(
-        plan, G, rows, t, nrows, cursor, out, limit, found, nullptr);
+        plan, G, rows, t, nrows, pool, cursor, out, limit, found, nullptr);
   else
     k_match<false, Q, false>
-        <<<grid, kMatchWarps * 32, smem>>>(plan, G, rows, t, nrows, cursor, out, limit, found, nullptr);
+        <<<grid, kMatchWarps * 32, smem>>>(plan, G, rows, t, nrows, pool, cursor, out, limit, found, nullptr);
   GPM_LAUNCH_CHECK();
   return GPM_OK;
 }
@@ -1095,9 +1104,10 @@ static int64_t row_target() { return (int64_t)num_sms() * 256; }
 static int extend_rows(const WidePlan &plan, const MatchGraph &G, DevBuf<int32_t> *store, const int32_t **rows,
                        int64_t *nrows, int *t, int64_t target) {
   if (*nrows == 0 || *nrows >= target || *t >= plan.n - 1) return GPM_OK;
-  size_t free_b = 0, total_b = 0;
-  GPM_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  const unsigned long long budget = std::min<unsigned long long>(2ull << 30, free_b / 8);
+  // up to kRowsAlways without asking the driver for the free memory, which
+  // takes longer than the levels of a small query
+  constexpr unsigned long long kRowsAlways = 64ull << 20;
+  unsigned long long budget = kRowsAlways;
   DevBuf<unsigned long long> cnt;
   GPM_TRY(cnt.reserve(1));
   const int blocks = num_sms() * 8;
@@ -1107,7 +1117,13 @@ static int extend_rows(const WidePlan &plan, const MatchGraph &G, DevBuf<int32_t
     GPM_LAUNCH_CHECK();
     unsigned long long nn = 0;
     GPM_CUDA(cudaMemcpy(&nn, cnt.p, 8, cudaMemcpyDeviceToHost));
-    if (nn * (unsigned long long)(*t + 1) * sizeof(int32_t) > budget) break;
+    const unsigned long long bytes = nn * (unsigned long long)(*t + 1) * sizeof(int32_t);
+    if (bytes > budget && budget == kRowsAlways) {
+      size_t free_b = 0, total_b = 0;
+      GPM_CUDA(cudaMemGetInfo(&free_b, &total_b));
+      budget = std::max<unsigned long long>(budget + 1, std::min<unsigned long long>(2ull << 30, free_b / 8));
+    }
+    if (bytes > budget) break;
     DevBuf<int32_t> next;
     if (nn) {
       GPM_TRY(next.reserve((size_t)nn * (*t + 1)));
@@ -1179,7 +1195,7 @@ static int match_run(gpm_graph *g, const gpm_query *q, unsigned long long limit,
   if (!track && is_cycle4(q, lc)) {
     CyclePlan cp;
     bool fits = false;
-    GPM_TRY(cycle_plan(g, lc, q, &cp, &lc->cycle, &fits));
+    GPM_TRY(cycle_plan(g, lc, q, 0, &cp, &lc->cycle, &fits));
     if (fits) {
       GPM_CUDA(cudaMemset(d.p, 0, 8));
       GPM_TRY(cycle_launch(g, lc, cp, lc->cycle, nullptr, d.p, 0));
@@ -1370,11 +1386,11 @@ __global__ void k_row_tasks(WidePlan q, const int32_t *__restrict__ rows, int64_
     cnt[i] = span > 0 ? max((int64_t)1, (best + span - 1) / span) : 1;
   }
 }
-// 32 pairs per task (three-position plans): chunk field -1 - pairs
-__global__ void k_pair_tasks(int64_t nrows, int query, int4 *__restrict__ tasks) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; 32 * i < nrows; i += (int64_t)gridDim.x * blockDim.x)
-    tasks[i] = make_int4((int)(uint32_t)(32 * i), (int)((32 * i) >> 32), query,
-                         -1 - (int)min((int64_t)32, nrows - 32 * i));
+// `pool` pairs per task (three-position plans): chunk field -1 - pairs
+__global__ void k_pair_tasks(int64_t nrows, int pool, int query, int4 *__restrict__ tasks) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; pool * i < nrows; i += (int64_t)gridDim.x * blockDim.x)
+    tasks[i] = make_int4((int)(uint32_t)(pool * i), (int)((pool * i) >> 32), query,
+                         -1 - (int)min((int64_t)pool, nrows - pool * i));
 }
 __global__ void k_expand_tasks(int64_t nrows, const int64_t *__restrict__ first, const int64_t *__restrict__ cnt,
                                int query, int split, int4 *__restrict__ tasks) {
@@ -1437,14 +1453,15 @@ static int batch_tasks(gpm_match_batch *b, int64_t span) {
   // position t of a row is split into chunks only when the depth-first walk
   // takes it (t <= n - 2; a row of depth n - 1 is closed at once)
   auto splits = [&](int k) { return span > 0 && b->depth[k] <= b->plans[k].n - 2; };
-  // pairs of three-position plans are closed 32 at a time (not with several
+  // pairs of three-position plans are closed several at a time (not with several
   // members: the pairs of a task may have roots of different ones)
   auto pooled = [&](int k) { return b->plans[k].n == 3 && b->depth[k] == 2 && b->nm == 1; };
   for (int k = 0; k < b->nq; ++k) {
     const int64_t np = b->nrows[k];
     if (b->plans[k].n < 3 || np == 0) continue;
     if (pooled(k)) {
-      cnt_total[k] = (np + 31) / 32;
+      const int pool = pair_pool(np);
+      cnt_total[k] = (np + pool - 1) / pool;
       total += cnt_total[k];
       continue;
     }
@@ -1469,7 +1486,7 @@ static int batch_tasks(gpm_match_batch *b, int64_t span) {
   for (int k = 0; k < b->nq; ++k) {
     if (!cnt_total[k]) continue;
     // each query's tasks at its own offset: shift the scan by `at`
-    if (pooled(k)) k_pair_tasks<<<blocks, 256>>>(b->nrows[k], k, b->tasks.p + at);
+    if (pooled(k)) k_pair_tasks<<<blocks, 256>>>(b->nrows[k], pair_pool(b->nrows[k]), k, b->tasks.p + at);
     else k_expand_tasks<<<blocks, 256>>>(b->nrows[k], first[k].p, cnt[k].p, k, splits(k), b->tasks.p + at);
     GPM_LAUNCH_CHECK();
     at += cnt_total[k];
@@ -1619,7 +1636,10 @@ int gpm_match_batch_create(gpm_graph *g, int nq, const gpm_query *const *queries
     if (factor && is_cycle4(queries[k], lc)) {
       CyclePlan cp;
       bool fits = false;
-      if ((s = cycle_plan(g, lc, queries[k], &cp, &b->cycle, &fits))) return bail(s);
+      // fewer wedges are walked, beside the other queries, before the four
+      // launches are through (R-MAT 12, 228 k wedges: 116 us walked, 94 us
+      // counted; R-MAT 14, 149 k: 107 and 129 us)
+      if ((s = cycle_plan(g, lc, queries[k], 200000, &cp, &b->cycle, &fits))) return bail(s);
       if (fits) {
         b->cycles.emplace_back(k, cp);
         continue;

@@ -96,9 +96,10 @@ struct CyclePlan {
 // Is q a 4-cycle whose labels all occur as partitions of lc?
 bool is_cycle4(const gpm_query *q, const LabelCsr *lc);
 // Chooses the opposite pair and makes room for the launch (*space grows, or is
-// created).  *fits = false: the counters would take too much memory, the
-// query has to be walked.
-int cycle_plan(gpm_graph *g, LabelCsr *lc, const gpm_query *q, CyclePlan *p, CycleSpace **space, bool *fits);
+// created).  *fits = false: fewer than min_wedges wedges, or the counters would
+// take too much memory; the query has to be walked.
+int cycle_plan(gpm_graph *g, LabelCsr *lc, const gpm_query *q, unsigned long long min_wedges, CyclePlan *p,
+               CycleSpace **space, bool *fits);
 // Launches only: the count is added to out[member ? member[root] : 0].
 int cycle_launch(const gpm_graph *g, const LabelCsr *lc, const CyclePlan &p, const CycleSpace *space,
                  const int32_t *member, unsigned long long *out, cudaStream_t st);

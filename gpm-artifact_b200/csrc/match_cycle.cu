@@ -334,7 +334,8 @@ bool is_cycle4(const gpm_query *q, const LabelCsr *lc) {
   return true;
 }
 
-int cycle_plan(gpm_graph *g, LabelCsr *lc, const gpm_query *q, CyclePlan *p, CycleSpace **space, bool *fits) {
+int cycle_plan(gpm_graph *g, LabelCsr *lc, const gpm_query *q, unsigned long long min_wedges, CyclePlan *p,
+               CycleSpace **space, bool *fits) {
   *fits = false;
   GPM_TRY(ensure_label_classes(g, lc));
   // the vertices around the cycle: 0, x, opposite, y
@@ -356,6 +357,7 @@ int cycle_plan(gpm_graph *g, LabelCsr *lc, const gpm_query *q, CyclePlan *p, Cyc
   unsigned long long h[2];
   GPM_CUDA(cudaMemcpy(h, w.p, sizeof h, cudaMemcpyDeviceToHost));
   const int pair = h[1] < h[0];
+  if (h[pair] < min_wedges) return GPM_OK;
   // the rarer label is the one with counters: fewer of them, most in shared memory
   const bool flip = size(l[pair]) < size(l[pair + 2]);
   p->la = flip ? l[pair + 2] : l[pair];
