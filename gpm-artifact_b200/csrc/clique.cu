@@ -875,7 +875,7 @@ static int cq_small_max(int k) {
 // Plan: task queues (heaviest first) and row slabs; the run is launches only.
 int clique_plan_build(CliquePlan *p, int64_t n, const int64_t *roff, const int32_t *radj, int max_deg, int k,
                       const int32_t *gid, unsigned long long *acc, int stride, int slot, cudaStream_t st,
-                      int warp_max) {
+                      int warp_max, int *cursors) {
   warp_max = std::max(1, std::min(warp_max, kCqWarpMax));
   p->n = n;
   p->roff = roff;
@@ -898,7 +898,11 @@ int clique_plan_build(CliquePlan *p, int64_t n, const int64_t *roff, const int32
   GPM_TRY(p->ctasks.reserve(n));
   GPM_TRY(p->wtasks.reserve(n));
   GPM_TRY(sizes.reserve(3));
-  GPM_TRY(p->counters.reserve(3));
+  p->cursors = cursors;
+  if (!cursors) {
+    GPM_TRY(p->counters.reserve(3));
+    p->cursors = p->counters.p;
+  }
   GPM_CUDA(cudaMemsetAsync(sizes.p, 0, 3 * sizeof(int), st));
   k_clique_tasks<<<grid_for(n), 256, 0, st>>>(n, roff, k, warp_max, cq_small_max(k), ckey.p, cval.p, wkey.p, wval.p,
                                               sizes.p);
@@ -958,9 +962,9 @@ int clique_plan_build(CliquePlan *p, int64_t n, const int64_t *roff, const int32
   return GPM_OK;
 }
 
-int clique_plan_run(CliquePlan *p, cudaStream_t st) {
+int clique_plan_run(CliquePlan *p, cudaStream_t st, bool zero) {
   if (p->n_cta + p->n_warp == 0) return GPM_OK;
-  GPM_CUDA(cudaMemsetAsync(p->counters.p, 0, 3 * sizeof(int), st));
+  if (zero) GPM_CUDA(cudaMemsetAsync(p->cursors, 0, 3 * sizeof(int), st));
   const CqGrids grids = cq_grids(p->k);
   const int nsmall = p->n_cta - p->n_big;
   const CqCore core{p->core.n_rows ? p->rowid.p : nullptr, p->core.rows.p, p->core.base, p->core.words};
@@ -974,18 +978,18 @@ int clique_plan_run(CliquePlan *p, cudaStream_t st) {
   cq_kernels(p->k, [&](auto small, auto big) {
     if (p->n_big > 0)
       big<<<p->big_grid, kCqBigThreads, kCqSmemBig, bst>>>(p->k, p->roff, p->radj, p->ctasks.p, p->n_big,
-                                                           p->counters.p, p->slabs.p, p->slab_words, core, p->gid,
+                                                           p->cursors, p->slabs.p, p->slab_words, core, p->gid,
                                                            p->acc, p->stride, p->slot);
     if (nsmall > 0)
       small<<<std::min(grids.small, nsmall), kCqSmallThreads, kCqSmemSmall, st>>>(
-          p->k, p->roff, p->radj, p->ctasks.p + p->n_big, nsmall, p->counters.p + 1, p->small_slabs.p, p->small_slab,
+          p->k, p->roff, p->radj, p->ctasks.p + p->n_big, nsmall, p->cursors + 1, p->small_slabs.p, p->small_slab,
           core, p->gid, p->acc, p->stride, p->slot);
   });
   GPM_LAUNCH_CHECK();
   if (bst != st) GPM_CUDA(cudaEventRecord(p->join, bst));
   if (p->n_warp > 0)
     k_clique_warp<<<std::min(grids.warp, (p->n_warp + 7) / 8), 256, 0, st>>>(
-        p->k, p->roff, p->radj, p->wtasks.p, p->n_warp, p->counters.p + 2, p->gid, p->acc, p->stride, p->slot);
+        p->k, p->roff, p->radj, p->wtasks.p, p->n_warp, p->cursors + 2, p->gid, p->acc, p->stride, p->slot);
   GPM_LAUNCH_CHECK();
   if (bst != st) GPM_CUDA(cudaStreamWaitEvent(st, p->join, 0));
   return GPM_OK;

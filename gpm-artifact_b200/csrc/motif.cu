@@ -649,6 +649,13 @@ static int dag_from_split(int64_t n, const int64_t *roff, const int64_t *split, 
   return GPM_OK;
 }
 
+// Work cursors behind the sums, zeroed with them: the triangle pass's (3), the
+// 4-cycle stage's (3) and the clique stage's (3), each in two words of acc.
+constexpr int kMotifCursors = 6;
+static int *te_cursors(MotifPlan *p) { return reinterpret_cast<int *>(p->acc.p + 8 * (size_t)p->in.ngraphs); }
+static int *c4_cursors(MotifPlan *p) { return te_cursors(p) + 4; }
+static int *k4_cursors(MotifPlan *p) { return te_cursors(p) + 8; }
+
 static int te_grid() {
   static PerDevice grid;
   return grid.get([] {
@@ -665,7 +672,7 @@ int motif_plan_build(const MotifInput &in, MotifPlan *p, cudaStream_t st) {
   const int64_t n = in.n;
   const int64_t *roff = in.roff;
   const int32_t *radj = in.radj;
-  GPM_TRY(p->acc.reserve(8 * (size_t)in.ngraphs));
+  GPM_TRY(p->acc.reserve(8 * (size_t)in.ngraphs + kMotifCursors));
   GPM_TRY(p->out.reserve(8 * (size_t)in.ngraphs));
   GPM_TRY(p->split.reserve(n));
   if (n > 0) k_split<<<grid_for(n), 256, 0, st>>>(n, roff, radj, p->split.p);
@@ -682,8 +689,6 @@ int motif_plan_build(const MotifInput &in, MotifPlan *p, cudaStream_t st) {
   DevBuf<unsigned long long> bb;
   GPM_TRY(bt.reserve(n));
   GPM_TRY(bb.reserve(n));
-  GPM_TRY(p->te_counters.reserve(3));
-  GPM_TRY(p->c4_counters.reserve(4));
   GPM_CUDA(cudaMemsetAsync(sizes.p, 0, 6 * sizeof(int), st));
   if (n > 0) {
     k_te_tasks<<<grid_for(n), 256, 0, st>>>(n, p->doff.p, std::min(in.te_cta_min, kTeWarpKeys), p->te_ct.p, p->te_wt.p, sizes.p);
@@ -749,7 +754,7 @@ int motif_plan_build(const MotifInput &in, MotifPlan *p, cudaStream_t st) {
     p->c4_grid = std::max(1, per_sm) * num_sms();
   }
   GPM_TRY(clique_plan_build(&p->k4, n, p->doff.p, p->dadj.p, p->dag_max, 4, in.gid, p->acc.p, 8, 5, st,
-                            in.cq_warp_max));
+                            in.cq_warp_max, k4_cursors(p)));
   GPM_CUDA(cudaStreamSynchronize(st));
   return GPM_OK;
 }
@@ -757,10 +762,9 @@ int motif_plan_build(const MotifInput &in, MotifPlan *p, cudaStream_t st) {
 // Triangles per edge, counted from zero.
 static int te_launch(MotifPlan *p, cudaStream_t st) {
   GPM_CUDA(cudaMemsetAsync(p->te.p, 0, sizeof(unsigned) * p->dadj.n, st));
-  GPM_CUDA(cudaMemsetAsync(p->te_counters.p, 0, 3 * sizeof(int), st));
   if (p->te_nc + p->te_nw + p->te_nl > 0)
     k_edge_tri<<<p->te_grid, 256, 0, st>>>(p->doff.p, p->dadj.p, p->te_ct.p, p->te_nc, p->te_wt.p, p->te_nw,
-                                           p->te_wt.p + (p->in.n - p->te_nl), p->te_nl, p->te_counters.p, p->te.p);
+                                           p->te_wt.p + (p->in.n - p->te_nl), p->te_nl, te_cursors(p), p->te.p);
   GPM_LAUNCH_CHECK();
   return GPM_OK;
 }
@@ -770,11 +774,11 @@ static int c4_launch(MotifPlan *p, cudaStream_t st) {
   const MotifInput &in = p->in;
   if (p->c4_nb > 0)
     k_c4_big<<<p->c4_big_grid, kC4BigThreads, kC4BigSmem, st>>>(
-        in.roff, p->split.p, in.radj, in.gid, in.gbase, p->c4_bt.p, p->c4_bb.p, p->c4_nb, p->c4_counters.p,
+        in.roff, p->split.p, in.radj, in.gid, in.gbase, p->c4_bt.p, p->c4_bb.p, p->c4_nb, c4_cursors(p),
         p->c4_cold.p, p->c4_cold_len, p->acc.p);
   if (p->c4_nc + p->c4_nw > 0)
     k_c4<<<p->c4_grid, 256, 0, st>>>(in.roff, p->split.p, in.radj, in.gid, in.gbase, p->c4_ct.p, p->c4_nc,
-                                     p->c4_wt.p, p->c4_nw, p->c4_counters.p, p->acc.p);
+                                     p->c4_wt.p, p->c4_nw, c4_cursors(p), p->acc.p);
   GPM_LAUNCH_CHECK();
   return GPM_OK;
 }
@@ -784,14 +788,14 @@ static int c4_launch(MotifPlan *p, cudaStream_t st) {
 int motif_plan_run(MotifPlan *p, cudaStream_t st) {
   const MotifInput &in = p->in;
   const int64_t n = in.n;
-  GPM_CUDA(cudaMemsetAsync(p->acc.p, 0, sizeof(unsigned long long) * 8 * in.ngraphs, st));
-  GPM_CUDA(cudaMemsetAsync(p->c4_counters.p, 0, 4 * sizeof(int), st));
+  // the sums, and behind them the cursors of all stages
+  GPM_CUDA(cudaMemsetAsync(p->acc.p, 0, sizeof(unsigned long long) * (8 * in.ngraphs + kMotifCursors), st));
   GPM_TRY(te_launch(p, st));
   if (n > 0)
     k_edge_sums<<<grid_for(n), 256, 0, st>>>(n, in.roff, p->doff.p, p->dadj.p, p->te.p, in.gid, p->acc.p);
   if (in.size == 4) {
     GPM_TRY(c4_launch(p, st));
-    GPM_TRY(clique_plan_run(&p->k4, st));
+    GPM_TRY(clique_plan_run(&p->k4, st, false));
   }
   k_motif_combine<<<std::max(1, (in.ngraphs + 255) / 256), 256, 0, st>>>(in.ngraphs, p->acc.p, p->out.p);
   GPM_LAUNCH_CHECK();
@@ -800,9 +804,10 @@ int motif_plan_run(MotifPlan *p, cudaStream_t st) {
 
 int motif_plan_run_stage(MotifPlan *p, int stage, cudaStream_t st) {
   if (stage == 0) {
+    GPM_CUDA(cudaMemsetAsync(te_cursors(p), 0, 4 * sizeof(int), st));
     GPM_TRY(te_launch(p, st));
   } else if (stage == 1) {
-    GPM_CUDA(cudaMemsetAsync(p->c4_counters.p, 0, 4 * sizeof(int), st));
+    GPM_CUDA(cudaMemsetAsync(c4_cursors(p), 0, 4 * sizeof(int), st));
     GPM_TRY(c4_launch(p, st));
   } else {
     GPM_TRY(clique_plan_run(&p->k4, st));

@@ -43,7 +43,8 @@ struct CliquePlan {
   unsigned long long *acc = nullptr;
   size_t slab_words = 0, small_slab = 0;  // words of half a slab (big, small CTAs)
   DevBuf<int32_t> ctasks, wtasks;
-  DevBuf<int> counters;
+  DevBuf<int> counters;    // the cursors, where the caller gave none
+  int *cursors = nullptr;  // 3
   DevBuf<uint32_t> slabs, small_slabs;
   DevBuf<int32_t> rowid;  // bitmap row of each vertex over the core (core.n_rows > 0)
   CoreRows core;
@@ -63,8 +64,9 @@ struct CliquePlan {
 };
 int clique_plan_build(CliquePlan *p, int64_t n, const int64_t *roff, const int32_t *radj, int max_deg, int k,
                       const int32_t *gid, unsigned long long *acc, int stride, int slot, cudaStream_t st,
-                      int warp_max = 64);
-int clique_plan_run(CliquePlan *p, cudaStream_t st);
+                      int warp_max = 64, int *cursors = nullptr);
+// zero == false: the caller has zeroed the plan's cursors
+int clique_plan_run(CliquePlan *p, cudaStream_t st, bool zero = true);
 
 // Motif pipeline split the same way; `acc` (scratch sums) and `out` are
 // owned by the plan, ngraphs x 8 each.  out per graph: [0] induced 2-paths,
@@ -81,7 +83,6 @@ struct MotifPlan {
   int te_nc = 0, te_nw = 0, te_nl = 0, c4_nc = 0, c4_nw = 0, c4_nb = 0, te_grid = 0, c4_grid = 0, c4_big_grid = 0;
   DevBuf<unsigned> c4_cold;  // cold counters of the giant tasks, c4_cold_len per CTA, zero between launches
   int64_t c4_cold_len = 0;
-  DevBuf<int> te_counters, c4_counters;
   CliquePlan k4;
   DevBuf<unsigned long long> acc, out;
 };

@@ -684,17 +684,21 @@ __global__ void k_partner_place(int64_t n, const int64_t *__restrict__ roff, con
     if (seg) pseg[lng ? poff[owner] + slot : poff[owner + 1] - 1 - slot] = sg;
   }
 }
-// The cursors taken apart: segments of each class, and the owner's work (keys
-// streamed plus one per segment)
+// The cursors taken apart: segments of each class, the owner's work (keys
+// streamed plus one per segment), and the sum of all work
 __global__ void k_place_counts(int64_t n, const unsigned long long *__restrict__ lcnt,
                                const unsigned long long *__restrict__ scnt, int32_t *__restrict__ plong,
-                               int32_t *__restrict__ pshort, unsigned long long *__restrict__ work) {
+                               int32_t *__restrict__ pshort, unsigned long long *__restrict__ work,
+                               unsigned long long *__restrict__ total) {
+  unsigned long long sum = 0;
   for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
     const unsigned long long l = lcnt[x], s = scnt[x];
     plong[x] = (int32_t)(uint32_t)l;
     pshort[x] = (int32_t)(uint32_t)s;
-    work[x] = (l >> 32) + (s >> 32) + (uint32_t)l + (uint32_t)s;
+    sum += work[x] = (l >> 32) + (s >> 32) + (uint32_t)l + (uint32_t)s;
   }
+  sum = warp_sum(sum);
+  if (lane_id() == 0 && sum) atomicAdd(total, sum);
 }
 // Dense core rows: rowid[v] = a row number when v has at least min_keys
 // keys >= core_base, else -1 (*nrows counts the rows)
@@ -785,21 +789,32 @@ __global__ void k_dense_tasks(int64_t n, const int64_t *__restrict__ roff, const
   }
 }
 
-// tasks: owners with partners, by their work
+// tasks: owners with partners, by their work.  Fixed schedule: an owner of at
+// most cta_min keys is a CTA task all the same when its work is more than
+// half a resident warp's share of the total (at least 1024): one warp would
+// hold up the count.  Without that rule / 4 shares / 1 share / half / a
+// quarter, us per count: R-MAT 14: 76, 29, 26, 26, 27; R-MAT 16: 120, 115, 68,
+// 58, 56; R-MAT 18: 224, 223, 173, 146, 140; R-MAT 20: 860, 844, 835, 828, 825;
+// R-MAT 22 unchanged; Chung-Lu 300,007 x 24: 154, 154, 156, 160, 165.
+constexpr unsigned long long kHeavyWork = 1024;
+constexpr int kHeavyShares = 2;
 __global__ void k_rank_tasks(int64_t n, const int64_t *__restrict__ roff, const int32_t *__restrict__ plong,
                              const int32_t *__restrict__ pshort,
                              const unsigned long long *__restrict__ work, int cta_min,
+                             const unsigned long long *__restrict__ total, int warps,
                              const uint8_t *__restrict__ cfg, const int32_t *__restrict__ pdense,
                              int32_t *__restrict__ donly, uint32_t *__restrict__ ckey,
                              int32_t *__restrict__ cval, uint32_t *__restrict__ wkey,
                              int32_t *__restrict__ wval, int *__restrict__ sizes) {
+  const unsigned long long heavy =
+      max(kHeavyWork, *total / (unsigned long long)(warps * kHeavyShares));
   for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
     if (plong[x] + pshort[x] == 0) {  // nothing to stream
       if (pdense && pdense[x]) donly[atomicAdd(&sizes[3], 1)] = (int32_t)x;  // dense segments only
       continue;
     }
     int64_t d = roff[x + 1] - roff[x];
-    if (cfg ? cfg[x] / 3 == 1 : d > cta_min) {
+    if (cfg ? cfg[x] / 3 == 1 : d > cta_min || work[x] > heavy) {
       int i = atomicAdd(&sizes[0], 1);
       ckey[i] = task_key(work[x]);
       cval[i] = (int32_t)x;
@@ -1290,6 +1305,15 @@ int core_rows_build(int64_t n, const int64_t *roff, const int32_t *radj, int64_t
   return GPM_OK;
 }
 
+static int rank_grid() {
+  static PerDevice grid;
+  return grid.get([] {
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tc_rank, 256, kRankSmem);
+    return std::max(1, per_sm) * num_sms();
+  });
+}
+
 int rank_plan_new(gpm_graph *g, int cta_min, int long_min, const uint8_t *cfg, cudaStream_t st, RankPlan **out) {
   GPM_TRY(ensure_rank_graph(g, st));
   bool fill = false;
@@ -1316,6 +1340,9 @@ int rank_plan_new(gpm_graph *g, int cta_min, int long_min, const uint8_t *cfg, c
   DevBuf<unsigned long long> lcnt, scnt;
   DevBuf<VertexInfo> info;
   if ((s = lcnt.reserve(n)) || (s = scnt.reserve(n)) || (s = info.reserve(n))) return bail(s);
+  DevBuf<unsigned long long> total;
+  if ((s = total.reserve(1))) return bail(s);
+  cudaMemsetAsync(total.p, 0, sizeof(unsigned long long), st);
   cudaMemsetAsync(lcnt.p, 0, sizeof(unsigned long long) * n, st);
   cudaMemsetAsync(scnt.p, 0, sizeof(unsigned long long) * n, st);
   if (g->rg->radj.n >= ((size_t)1 << 32)) return bail(fail(GPM_EUNSUPPORTED, "triangle plan: 2^32 keys or more"));
@@ -1343,7 +1370,7 @@ int rank_plan_new(gpm_graph *g, int cta_min, int long_min, const uint8_t *cfg, c
   k_partner_place<<<grid_for(keys), 256, 0, st>>>(n, roff, radj, ustart.p, info.p, fill ? g->rg->radj4.p : nullptr, g->rg->upward,
                                                long_min, cfg, p->poff.p, lcnt.p, scnt.p, p->pseg.p, p->core_base,
                                                p->row_words, dense_pct, p->pdense.p, sizes.p + 4);
-  k_place_counts<<<grid_for(n), 256, 0, st>>>(n, lcnt.p, scnt.p, p->plong.p, p->pshort.p, work.p);
+  k_place_counts<<<grid_for(n), 256, 0, st>>>(n, lcnt.p, scnt.p, p->plong.p, p->pshort.p, work.p, total.p);
   GPM_LAUNCH_CHECK();
   if (p->n_rows) {  // the dense segments moved out of the long ones
     DevBuf<int64_t> cnt;
@@ -1370,7 +1397,8 @@ int rank_plan_new(gpm_graph *g, int cta_min, int long_min, const uint8_t *cfg, c
     return bail(s);
   const int32_t *pdense = p->n_rows ? p->pdense.p : nullptr;
   if (pdense && (s = p->dense_only.reserve(n))) return bail(s);
-  k_rank_tasks<<<grid_for(n), 256, 0, st>>>(n, roff, p->plong.p, p->pshort.p, work.p, cta_min, cfg, pdense,
+  k_rank_tasks<<<grid_for(n), 256, 0, st>>>(n, roff, p->plong.p, p->pshort.p, work.p, cta_min, total.p, rank_grid() * kRWarps,
+                                            cfg, pdense,
                                             p->dense_only.p, ckey.p, cval.p, wkey.p, wval.p, sizes.p);
   if (pdense) {
     if ((s = dkey.reserve(n)) || (s = dval.reserve(n))) return bail(s);
@@ -1402,15 +1430,6 @@ int rank_plan_new(gpm_graph *g, int cta_min, int long_min, const uint8_t *cfg, c
   if (e != cudaSuccess) return bail(fail(GPM_ECUDA, std::string("rank plan: ") + cudaGetErrorString(e)));
   *out = p;
   return GPM_OK;
-}
-
-static int rank_grid() {
-  static PerDevice grid;
-  return grid.get([] {
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tc_rank, 256, kRankSmem);
-    return std::max(1, per_sm) * num_sms();
-  });
 }
 
 // Launch of a given plan; rec != nullptr selects the instrumented build.
