@@ -209,11 +209,18 @@ __global__ void __launch_bounds__(256) k_edge_tri(const int64_t *__restrict__ do
   }
   const int wid = threadIdx.x >> 5;
   const unsigned lane = threadIdx.x & 31;
+  // light tasks: dealt out in turn while a warp has few of them, else in runs
+  const int warps = gridDim.x * 8;
+  if (n_light <= 2 * kTaskRun * warps) {
+    for (int t = blockIdx.x * 8 + wid; t < n_light; t += warps)
+      te_warp_task(light_tasks[t], doff, dadj, te, T.warp[wid], lane);
+    n_light = 0;
+  }
   for (int light = 0; light < 2; ++light) {
     const int32_t *tasks = light ? light_tasks : warp_tasks;
     const int n = light ? n_light : n_warp;
     WarpTasks queue;
-    while (true) {
+    while (n > 0) {
       const int t = queue.next(&counters[1 + light], light ? 0 : n, lane);
       if (t >= n) break;
       te_warp_task(tasks[t], doff, dadj, te, T.warp[wid], lane);

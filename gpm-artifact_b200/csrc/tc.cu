@@ -522,6 +522,22 @@ static int lists_launch(gpm_graph *g, cudaStream_t st, unsigned long long *d_out
   return GPM_OK;
 }
 
+// Tiny graphs: a warp per stored edge, whatever the degrees; skewed ones up to
+// kTinySkewed entries where no plan is built at once.  Count / first count in
+// us, binary search, hash kernel, rank plan: Chung-Lu, 6,412 entries 7 / 20, 7 /
+// 39, 17 / 291; R-MAT 10, 10,504 entries 10 / 22, 25 / 52, 19 / 312; R-MAT 14,
+// 45,666 entries 19 / 30, 36 / 56, 22 / 386; R-MAT 12, 48,313 entries 27 / 37, 61 /
+// 91, 22 / 360.
+constexpr int64_t kTiny = 16384, kTinySkewed = 65536;
+// The count of a tiny graph, or of one with short lists alone, launched?
+static bool small_launch(gpm_graph *g, cudaStream_t st, unsigned long long *d_out, int *status) {
+  if (g->nnz <= 0) return false;
+  if (g->nnz <= kTiny) *status = tc_launch(g, GPM_TC_BSEARCH, st, d_out);
+  else if (g->max_deg <= kListDegree) *status = lists_launch(g, st, d_out);
+  else return false;
+  return true;
+}
+
 // gpm_tc's kernel.  The rank plan's repeated counts are the faster ones on
 // every graph of some size, but the plan has to be built first.  Microseconds
 // (hash count; rank count; its first count, plan included): R-MAT 14: 145, 83,
@@ -532,7 +548,9 @@ static int lists_launch(gpm_graph *g, cudaStream_t st, unsigned long long *d_out
 // within a factor of two, 5 ps each), and otherwise when the counts made on
 // this graph with the hash kernel have cost as much as the plan.
 static int tc_auto_launch(gpm_graph *g, cudaStream_t st, unsigned long long *d_out) {
-  if (g->nnz > 0 && g->max_deg <= kListDegree) return lists_launch(g, st, d_out);
+  int s = GPM_OK;
+  if (small_launch(g, st, d_out, &s)) return s;
+  if (g->nnz <= kTinySkewed) return tc_launch(g, GPM_TC_BSEARCH, st, d_out);
   if (!g->rank && g->nnz > 0) {
     const double hash_us = 10 + 5e-6 * (double)g->sum_deg2, plan_us = 300 + 2.5e-4 * (double)g->nnz;
     if (hash_us < 40 || g->hash_us + hash_us < plan_us) {
@@ -540,7 +558,7 @@ static int tc_auto_launch(gpm_graph *g, cudaStream_t st, unsigned long long *d_o
       return tc_launch(g, GPM_TC_HASH, st, d_out);
     }
   }
-  const int s = tc_launch(g, GPM_TC_BITMAP, st, d_out);
+  s = tc_launch(g, GPM_TC_BITMAP, st, d_out);
   if (s != GPM_ENOMEM && s != GPM_EUNSUPPORTED) return s;
   g->hash_us = -1e30;  // not tried again
   return tc_launch(g, GPM_TC_HASH, st, d_out);  // no room for the plan, or beyond its descriptors
@@ -555,7 +573,8 @@ extern "C" {
 int gpm_tc_async(gpm_graph *g, int variant, void *stream, uint64_t *d_out) {
   if (!g || !d_out) return fail(GPM_EINVAL, "gpm_tc_async: NULL argument");
   if (variant == GPM_TC_AUTO) {
-    if (g->nnz > 0 && g->max_deg <= kListDegree) return lists_launch(g, (cudaStream_t)stream, (unsigned long long *)d_out);
+    int s = GPM_OK;
+    if (small_launch(g, (cudaStream_t)stream, (unsigned long long *)d_out, &s)) return s;
     variant = GPM_TC_BITMAP;
   }
   if (variant == GPM_TC_LEARNED) return tc_learned_launch(g, (cudaStream_t)stream, (unsigned long long *)d_out);

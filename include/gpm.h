@@ -47,8 +47,8 @@ enum { GPM_V_CENTRIC = 0, GPM_E_CENTRIC = 1 };
 
 /* Triangle-count kernel variants (all return the same count). */
 enum {
-  GPM_TC_AUTO = 0,     /* engine's default: GPM_TC_BITMAP, or the two lists of each edge
-                          merged where every list is short                           */
+  GPM_TC_AUTO = 0,     /* engine's default: GPM_TC_BITMAP; tiny graphs GPM_TC_BSEARCH,
+                          the lists of each edge merged where every list is short    */
   GPM_TC_BSEARCH = 1,  /* warp per stored edge, binary search (TCSolver.cuh:27-59 shape) */
   GPM_TC_HASH = 2,     /* vertex tasks, shared-memory hash of N(u), hub/tail queues
                           with the fixed thresholds of tuning_schedules.cuh:196-197   */

@@ -11,6 +11,8 @@ pytestmark = pytest.mark.gpu
 
 GRAPHS = {
     "tiny": lambda: gpm.gen_er(40, 90, seed=1),
+    "rmat10": lambda: gpm.gen_rmat(10, 16, seed=2),
+    "rmat12": lambda: gpm.gen_rmat(12, 10, seed=2),
     "rmat13": lambda: gpm.gen_rmat(13, 16, seed=2),
     # more tail tasks than eight per resident warp
     "er200k": lambda: gpm.gen_er(200003, 1400000, seed=3),
