@@ -669,33 +669,118 @@ __global__ void k_match_pairs(WidePlan q, int64_t n, const int64_t *__restrict__
   }
 }
 
-// Label-partitioned copy of the lists: neighbours sorted by (label, id); loff
-// holds, per vertex, the L + 1 segment starts relative to off[v].
-__global__ void k_label_keys(int64_t nnz, const int32_t *__restrict__ adj, const int32_t *__restrict__ labels, int L,
-                             uint64_t *__restrict__ keys) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nnz; i += (int64_t)gridDim.x * blockDim.x) {
-    int32_t w = adj[i];
-    uint32_t l = L > 1 ? (uint32_t)labels[w] : 0u;
-    keys[i] = ((uint64_t)l << 32) | (uint32_t)w;
+// Label-partitioned copy of the lists: each list, sorted by id, reordered by
+// (label, id); loff holds, per vertex, the L + 1 segment starts relative to
+// off[v].  A stable partition: the entries' labels are counted, then every
+// entry goes to its label's next place.  A warp per list of up to kPartWarp
+// entries; longer ones (queued) are cut into one contiguous share per warp of
+// a CTA, whose counts are turned into places first.  (A segmented sort of
+// 64-bit (label, id) keys and a search of every segment start took 4.1 ms for
+// R-MAT 19.)
+constexpr int kPartWarp = 1024, kPartThreads = 512, kPartLabels = 64;
+
+// cnt[l] += entries of adj[s .. e) with label l, one warp
+__device__ __forceinline__ void part_count(const int32_t *__restrict__ adj, const int32_t *__restrict__ labels,
+                                           int64_t s, int64_t e, int32_t *cnt, unsigned lane) {
+  for (int64_t k = s + lane; k < e; k += 32) atomicAdd(&cnt[labels[adj[k]]], 1);
+  __syncwarp();
+}
+// the entries to out + at[label]++, in order, one warp
+__device__ __forceinline__ void part_place(const int32_t *__restrict__ adj, const int32_t *__restrict__ labels,
+                                           int64_t s, int64_t e, int32_t *at, int32_t *__restrict__ out,
+                                           unsigned lane) {
+  const unsigned below = (1u << lane) - 1u;
+  for (int64_t base = s; base < e; base += 32) {
+    const bool in = base + lane < e;
+    const int32_t w = in ? adj[base + lane] : 0;
+    const int l = in ? labels[w] : -1;
+    const unsigned same = __match_any_sync(0xffffffffu, l);
+    if (in) out[at[l] + __popc(same & below)] = w;
+    __syncwarp();
+    if (in && (same & below) == 0) at[l] += __popc(same);
+    __syncwarp();
   }
 }
-__global__ void k_label_offsets(int64_t n, const int64_t *__restrict__ off, const uint64_t *__restrict__ keys, int L,
-                                int32_t *__restrict__ ladj, int32_t *__restrict__ loff) {
+// cnt[0 .. L) -> exclusive prefix in place (L <= 64), segment starts to seg[0 .. L], one warp
+__device__ __forceinline__ void part_starts(int32_t *cnt, int L, int32_t *__restrict__ seg, unsigned lane) {
+  int carry = 0;
+  for (int b = 0; b < L; b += 32) {
+    const int l = b + (int)lane;
+    const int c = l < L ? cnt[l] : 0;
+    int inc = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, inc, o);
+      if ((int)lane >= o) inc += v;
+    }
+    if (l < L) {
+      cnt[l] = carry + inc - c;
+      seg[l] = carry + inc - c;
+    }
+    carry += __shfl_sync(0xffffffffu, inc, 31);
+  }
+  if (lane == 0) seg[L] = carry;
+  __syncwarp();
+}
+
+__global__ void __launch_bounds__(256) k_label_partition(int64_t n, const int64_t *__restrict__ off,
+                                                         const int32_t *__restrict__ adj,
+                                                         const int32_t *__restrict__ labels, int L,
+                                                         int32_t *__restrict__ ladj, int32_t *__restrict__ loff,
+                                                         int32_t *__restrict__ hubs, int *__restrict__ nhubs) {
+  __shared__ int32_t s_cnt[8][kPartLabels];
+  int32_t *cnt = s_cnt[threadIdx.x >> 5];
+  const unsigned lane = lane_id();
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const unsigned lane = lane_id();
   for (int64_t v = warp; v < n; v += nw) {
     const int64_t s = off[v], e = off[v + 1];
-    // segment start of label l = number of entries with label < l (sorted)
-    for (int l = lane; l <= L; l += 32) {
-      int64_t lo = s, hi = e;
-      while (lo < hi) {
-        int64_t mid = (lo + hi) >> 1;
-        if ((int64_t)(keys[mid] >> 32) < l) lo = mid + 1; else hi = mid;
-      }
-      loff[v * (L + 1) + l] = (int32_t)(lo - s);
+    if (e - s > kPartWarp) {
+      if (lane == 0) hubs[atomicAdd(nhubs, 1)] = (int32_t)v;
+      continue;
     }
-    for (int64_t k = s + lane; k < e; k += 32) ladj[k] = (int32_t)(keys[k] & 0xffffffffu);
+    for (int l = lane; l < L; l += 32) cnt[l] = 0;
+    __syncwarp();
+    part_count(adj, labels, s, e, cnt, lane);
+    part_starts(cnt, L, loff + v * (L + 1), lane);
+    part_place(adj, labels, s, e, cnt, ladj + s, lane);
+  }
+}
+__global__ void __launch_bounds__(kPartThreads) k_label_partition_hubs(const int32_t *__restrict__ hubs,
+                                                                       const int *__restrict__ nhubs,
+                                                                       const int64_t *__restrict__ off,
+                                                                       const int32_t *__restrict__ adj,
+                                                                       const int32_t *__restrict__ labels, int L,
+                                                                       int32_t *__restrict__ ladj,
+                                                                       int32_t *__restrict__ loff) {
+  constexpr int kW = kPartThreads / 32;
+  __shared__ int32_t s_cnt[kW][kPartLabels], s_sum[kPartLabels];
+  const int wid = threadIdx.x >> 5;
+  const unsigned lane = lane_id();
+  for (int h = blockIdx.x; h < *nhubs; h += gridDim.x) {
+    const int32_t v = hubs[h];
+    const int64_t s = off[v], e = off[v + 1], share = ((e - s + kW - 1) / kW + 31) & ~(int64_t)31;
+    const int64_t ws = min(e, s + wid * share), we = min(e, ws + share);
+    for (int l = lane; l < L; l += 32) s_cnt[wid][l] = 0;
+    __syncwarp();
+    part_count(adj, labels, ws, we, s_cnt[wid], lane);
+    __syncthreads();
+    for (int l = threadIdx.x; l < L; l += kPartThreads) {  // warps' places inside the label, the label's total
+      int run = 0;
+      for (int w = 0; w < kW; ++w) {
+        const int c = s_cnt[w][l];
+        s_cnt[w][l] = run;
+        run += c;
+      }
+      s_sum[l] = run;
+    }
+    __syncthreads();
+    if (wid == 0) part_starts(s_sum, L, loff + (int64_t)v * (L + 1), lane);
+    __syncthreads();
+    for (int l = lane; l < L; l += 32) s_cnt[wid][l] += s_sum[l];
+    __syncwarp();
+    part_place(adj, labels, ws, we, s_cnt[wid], ladj + s, lane);
+    __syncthreads();
   }
 }
 
@@ -861,10 +946,16 @@ __global__ void k_label_range(int64_t n, const int32_t *__restrict__ labels, int
 }
 
 __global__ void k_deg_hist(int64_t n, const int64_t *__restrict__ off, unsigned long long *__restrict__ h) {
+  __shared__ unsigned sh[65];
+  for (int i = threadIdx.x; i < 65; i += blockDim.x) sh[i] = 0u;
+  __syncthreads();
   for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
     const int64_t d = off[v + 1] - off[v];
-    atomicAdd(&h[d > 0 ? 64 - __clzll((unsigned long long)d) : 0], 1ull);  // bin b: 2^(b-1) <= d < 2^b
+    atomicAdd(&sh[d > 0 ? 64 - __clzll((unsigned long long)d) : 0], 1u);  // bin b: 2^(b-1) <= d < 2^b
   }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 65; i += blockDim.x)
+    if (sh[i]) atomicAdd(&h[i], (unsigned long long)sh[i]);
 }
 __global__ void k_hub_slots(int64_t n, const int64_t *__restrict__ off, int64_t dmin, int32_t *__restrict__ slot,
                             int *__restrict__ cnt) {
@@ -963,20 +1054,18 @@ static int ensure_label_csr(gpm_graph *g) {
     if ((s = lc->loff.reserve(1))) return bail(s);
     if (nnz > 0) cudaMemcpy(lc->ladj.p, g->adj.p, sizeof(int32_t) * nnz, cudaMemcpyDeviceToDevice);
   } else {
-    DevBuf<uint64_t> keys, sorted;
-    if ((s = lc->loff.reserve((size_t)n * (L + 1))) || (s = keys.reserve(nnz)) || (s = sorted.reserve(nnz)))
+    DevBuf<int32_t> hubs;
+    DevBuf<int> nhubs;
+    if ((s = lc->loff.reserve((size_t)n * (L + 1))) || (s = hubs.reserve(nnz / kPartWarp + 1)) ||
+        (s = nhubs.reserve(1)))
       return bail(s);
-    if (nnz > 0) {
-      k_label_keys<<<(int)std::min<int64_t>((nnz + 255) / 256, num_sms() * 16), 256>>>(nnz, g->adj.p, g->labels.p, L,
-                                                                                      keys.p);
-      size_t tmp = 0;
-      cub::DeviceSegmentedSort::SortKeys(nullptr, tmp, keys.p, sorted.p, (int)nnz, (int)n, g->off.p, g->off.p + 1);
-      DevBuf<char> t;
-      if ((s = t.reserve(tmp))) return bail(s);
-      cub::DeviceSegmentedSort::SortKeys(t.p, tmp, keys.p, sorted.p, (int)nnz, (int)n, g->off.p, g->off.p + 1);
-    }
-    k_label_offsets<<<(int)std::min<int64_t>((n * 32 + 255) / 256, num_sms() * 16), 256>>>(n, g->off.p, sorted.p, L,
-                                                                                          lc->ladj.p, lc->loff.p);
+    cudaMemset(nhubs.p, 0, sizeof(int));
+    k_label_partition<<<(int)std::min<int64_t>((n * 32 + 255) / 256, num_sms() * 16), 256>>>(
+        n, g->off.p, g->adj.p, g->labels.p, L, lc->ladj.p, lc->loff.p, hubs.p, nhubs.p);
+    k_label_partition_hubs<<<num_sms() * 4, kPartThreads>>>(hubs.p, nhubs.p, g->off.p, g->adj.p, g->labels.p, L,
+                                                            lc->ladj.p, lc->loff.p);
+    const cudaError_t le = cudaGetLastError();
+    if (le != cudaSuccess) return bail(fail(GPM_ECUDA, std::string("label partition: ") + cudaGetErrorString(le)));
   }
   if ((s = build_hub_index(g, lc))) return bail(s);
   cudaError_t e = cudaDeviceSynchronize();
