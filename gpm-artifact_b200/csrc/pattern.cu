@@ -70,30 +70,72 @@ __device__ __forceinline__ int wisect(const int32_t *a, int na, const int32_t *b
 #define DIFF(...) wdiff(__VA_ARGS__, lane)
 #define ISECT(...) wisect(__VA_ARGS__, lane)
 
-__global__ void __launch_bounds__(256) k_pattern(int p, int64_t nnz, const int64_t *__restrict__ off,
+// Heavy edges: both endpoints' lists together longer than `degree`.  Their
+// outer loop is shared out over `parts` warps, each of which builds the lists
+// for itself: an edge's cost grows with the cube of its degrees and more, and
+// one warp on the heaviest edge held up the whole count.  P7 walks common
+// neighbours alone, which are few, so its lists are what costs.  us per call,
+// one warp per edge / (degree, parts) = (48, 16) / (96, 16) / (192, 16), Chung-
+// Lu graphs: P5, 2,001 vertices 2918, 617, 715, 1764; P2, 801: 1745, 536, 1287,
+// 1868; P3, 801: 1556, 780, 1750, 1631; P6, 2,001: 859, 242, 265, 502; P8, 20,001:
+// 10164, 4681, 4464, 4646; P7, 4,099: 271, 324, 227, 179.
+struct HeavyRule {
+  int64_t degree;
+  int parts;
+};
+static HeavyRule heavy_rule(int p) { return p == 7 ? HeavyRule{192, 4} : HeavyRule{48, 16}; }
+__global__ void k_heavy_edges(HeavyRule rule, int64_t nnz, const int64_t *__restrict__ off, const int32_t *__restrict__ adj,
+                              const int32_t *__restrict__ src, int32_t *__restrict__ heavy,
+                              unsigned long long *__restrict__ nheavy) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nnz; e += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t v0 = src[e], v1 = adj[e];
+    if (off[v0 + 1] - off[v0] + off[v1 + 1] - off[v1] > rule.degree) heavy[atomicAdd(nheavy, 1ull)] = (int32_t)e;
+  }
+}
+
+// Pattern p on all edges that are not heavy (heavy == nullptr), or on the
+// heavy ones, whose (edge, part) pairs come from the cursor *next.
+__global__ void __launch_bounds__(256) k_pattern(int p, HeavyRule rule, int64_t nnz, const int64_t *__restrict__ off,
                                                  const int32_t *__restrict__ adj, const int32_t *__restrict__ src,
                                                  int32_t *__restrict__ scratch, int64_t maxd,
+                                                 const int32_t *__restrict__ heavy,
+                                                 const unsigned long long *__restrict__ nheavy,
+                                                 unsigned long long *__restrict__ next,
                                                  unsigned long long *__restrict__ out) {
   const unsigned lane = lane_id();
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   int32_t *A = scratch + warp * maxd * 5, *B = A + maxd, *C = B + maxd, *D = C + maxd, *E = D + maxd;
   unsigned long long c = 0;
-  for (int64_t e = warp; e < nnz; e += nw) {
+  const int step = heavy ? rule.parts : 1;
+  const int64_t tasks = heavy ? (int64_t)*nheavy * rule.parts : nnz;
+  for (int64_t t = warp; t < tasks; t += nw) {
+    int64_t e = t;
+    int part = 0;
+    if (heavy) {  // t counts the warp's own rounds here; the task comes from the cursor
+      unsigned long long q = 0;
+      if (lane == 0) q = atomicAdd(next, 1ull);
+      q = __shfl_sync(0xffffffffu, q, 0);
+      if (q >= (unsigned long long)tasks) break;
+      e = heavy[q / rule.parts];
+      part = (int)(q % rule.parts);
+      t = warp - nw;  // the cursor alone ends the loop
+    }
     const int32_t v0 = src[e], v1 = adj[e];
+    if (!heavy && off[v0 + 1] - off[v0] + off[v1 + 1] - off[v1] > rule.degree) continue;
     int nA, nB, nC, nD, nE;
     switch (p) {
       case 2:  // G2Miner_kernels.cuh:68-103
         nA = DIFF(NBR(v0), NBR(v1), kNoUb, A);
         nB = DIFF(NBR(v1), NBR(v0), kNoUb, B);
-        for (int i = 0; i < nB; ++i) {
+        for (int i = part; i < nB; i += step) {
           nC = DIFF(A, nA, NBR(B[i]), kNoUb, C);
           for (int j = 0; j < nC; ++j) c += DIFF(C, nC, NBR(C[j]), C[j], nullptr);
         }
         break;
       case 3:  // :126-157
         nA = DIFF(NBR(v0), NBR(v1), kNoUb, A);
-        for (int i = 0; i < nA; ++i) {
+        for (int i = part; i < nA; i += step) {
           nB = DIFF(A, nA, NBR(A[i]), A[i], B);
           for (int j = 0; j < nB; ++j) c += DIFF(B, nB, NBR(B[j]), B[j], nullptr);
         }
@@ -102,7 +144,7 @@ __global__ void __launch_bounds__(256) k_pattern(int p, int64_t nnz, const int64
         nA = DIFF(NBR(v0), NBR(v1), kNoUb, A);
         nB = DIFF(NBR(v1), NBR(v0), kNoUb, B);
         nC = ISECT(NBR(v0), NBR(v1), kNoUb, C);
-        for (int i = 0; i < nC; ++i) {
+        for (int i = part; i < nC; i += step) {
           nD = DIFF(A, nA, NBR(C[i]), kNoUb, D);
           nE = DIFF(B, nB, NBR(C[i]), kNoUb, E);
           for (int j = 0; j < nD; ++j) c += DIFF(E, nE, NBR(D[j]), kNoUb, nullptr);
@@ -111,7 +153,7 @@ __global__ void __launch_bounds__(256) k_pattern(int p, int64_t nnz, const int64
       case 6:  // :281-318
         nC = ISECT(NBR(v0), NBR(v1), kNoUb, C);
         nB = DIFF(NBR(v1), NBR(v0), kNoUb, B);
-        for (int i = 0; i < nC; ++i) {
+        for (int i = part; i < nC; i += step) {
           nD = DIFF(C, nC, NBR(C[i]), kNoUb, D);
           nE = DIFF(B, nB, NBR(C[i]), kNoUb, E);
           for (int j = 0; j < nD; ++j) c += DIFF(E, nE, NBR(D[j]), kNoUb, nullptr);
@@ -119,7 +161,7 @@ __global__ void __launch_bounds__(256) k_pattern(int p, int64_t nnz, const int64
         break;
       case 7:  // :339-371
         nC = ISECT(NBR(v0), NBR(v1), kNoUb, C);
-        for (int i = 0; i < nC; ++i) {
+        for (int i = part; i < nC; i += step) {
           nD = DIFF(C, nC, NBR(C[i]), C[i], D);
           for (int j = 0; j < nD; ++j) c += DIFF(D, nD, NBR(D[j]), D[j], nullptr);
         }
@@ -127,7 +169,7 @@ __global__ void __launch_bounds__(256) k_pattern(int p, int64_t nnz, const int64
       case 8:  // :394-430
         nC = ISECT(NBR(v0), NBR(v1), kNoUb, C);
         nB = DIFF(NBR(v1), NBR(v0), kNoUb, B);
-        for (int i = 0; i < nB; ++i) {
+        for (int i = part; i < nB; i += step) {
           nD = DIFF(C, nC, NBR(B[i]), kNoUb, D);
           for (int j = 0; j < nD; ++j) c += ISECT(D, nD, NBR(D[j]), D[j], nullptr);
         }
@@ -143,8 +185,8 @@ __global__ void __launch_bounds__(256) k_pattern(int p, int64_t nnz, const int64
 int pattern_enumerate(gpm_graph *g, int p, cudaStream_t st, uint64_t *result) {
   GPM_TRY(ensure_src(g, st));
   DevBuf<unsigned long long> d;
-  GPM_TRY(d.reserve(1));
-  GPM_CUDA(cudaMemsetAsync(d.p, 0, 8, st));
+  GPM_TRY(d.reserve(3));  // the count, the heavy edges, their cursor
+  GPM_CUDA(cudaMemsetAsync(d.p, 0, 24, st));
   const int64_t maxd = std::max(1, g->max_deg);
   // scratch: 5 lists of max degree per warp, capped at ~8 GB
   int64_t warps = (int64_t)num_sms() * 4 * 8;
@@ -153,8 +195,20 @@ int pattern_enumerate(gpm_graph *g, int p, cudaStream_t st, uint64_t *result) {
   DevBuf<int32_t> scratch;
   GPM_TRY(scratch.reserve((size_t)(warps * maxd * 5)));
   if (g->nnz > 0) {
-    k_pattern<<<(int)(warps / 8), 256, 0, st>>>(p, g->nnz, g->off.p, g->adj.p, g->src.p, scratch.p, maxd, d.p);
+    DevBuf<int32_t> heavy;
+    const HeavyRule rule = heavy_rule(p);
+    const bool some = 2 * maxd > rule.degree;
+    GPM_TRY(heavy.reserve(some ? g->nnz : 1));
+    if (some) {
+      k_heavy_edges<<<(int)std::min<int64_t>((g->nnz + 255) / 256, num_sms() * 8), 256, 0, st>>>(
+          rule, g->nnz, g->off.p, g->adj.p, g->src.p, heavy.p, d.p + 1);
+      k_pattern<<<(int)(warps / 8), 256, 0, st>>>(p, rule, g->nnz, g->off.p, g->adj.p, g->src.p, scratch.p, maxd, heavy.p,
+                                                  d.p + 1, d.p + 2, d.p);
+    }
+    k_pattern<<<(int)(warps / 8), 256, 0, st>>>(p, rule, g->nnz, g->off.p, g->adj.p, g->src.p, scratch.p, maxd, nullptr,
+                                                nullptr, nullptr, d.p);
     GPM_LAUNCH_CHECK();
+    GPM_CUDA(cudaStreamSynchronize(st));  // heavy is released here
   }
   unsigned long long h = 0;
   GPM_CUDA(cudaMemcpyAsync(&h, d.p, 8, cudaMemcpyDeviceToHost, st));
