@@ -509,12 +509,12 @@ def clique_workload(args, stream):
         avg = sum(ms) / len(ms)
         r = {"cliques": c, "value": c / (avg / 1e3), "ms_per_count": avg, "steps": reps,
              "ms_first_call": first[0],
-             "roofline": roofline(profiled(f"k_clique_local_rmat{W.CLIQUE_SCALE}",
+             "roofline": roofline(profiled(f"k_clique_rmat{W.CLIQUE_SCALE}",
                                            f"traffic_bytes_per_launch[k{k}]"), avg, hbm, peak_kind,
-                                  issue_active_pct=profiled(f"k_clique_local_rmat{W.CLIQUE_SCALE}",
+                                  issue_active_pct=profiled(f"k_clique_rmat{W.CLIQUE_SCALE}",
                                                             f"issue_active_pct[k{k}]"),
                                   note="bitset intersections in shared memory: issue-bound, DRAM only for "
-                                       "the graph (profiles/k_clique_local_rmat20.md)")}
+                                       "the graph (profiles/k_clique_rmat20.md)")}
         if k == 4:
             # the reference-shaped path: warp per stored edge, materialised
             # nested intersections (clique_4_edge_warp)
@@ -627,14 +627,13 @@ def motif_workload(args, stream):
         "e2e": {"value": total / (min(e2e_ms) / 1e3), "unit": "instances/s", "ms_per_step": min(e2e_ms),
                 "h2d_bytes_per_step": int(hsrc.numel() * 4 + hdst.numel() * 4),
                 "d2h_bytes_per_step": int(8 * 8 * ng)},
-        # the dominant stage's kernel, k_c4_big: its DRAM bytes and duration
-        # from one ncu capture of this batch (the stage time also holds k_c4)
-        "roofline": roofline(profiled("k_edge_tri_batch32", "traffic_bytes_per_launch[c4_big_batch256]"),
-                             profiled("k_edge_tri_batch32", "kernel_ms[c4_big_batch256]") or stages["four_cycles"],
+        # the dominant stage's kernel, k_c4_big, has been profiled on a smaller
+        # batch only, so no DRAM bytes of this one are given
+        "roofline": roofline(profiled("motif_batch48", "traffic_bytes_per_launch[c4_big_batch256]"),
+                             stages["four_cycles"],
                              hbm, peak_kind, kernel="k_c4_big (the 4-cycle stage's large tasks)",
-                             issue_active_pct=profiled("k_edge_tri_batch32", "issue_active_pct[edge_tri_batch32]"),
-                             note="issue- and latency-bound pipeline (profiles/k_edge_tri_batch32.md, "
-                                  "profiles/k_c4_big_chunglu200k.md)"),
+                             issue_active_pct=profiled("motif_batch48", "issue_active_pct[edge_tri_batch48]"),
+                             note="issue- and latency-bound pipeline (profiles/motif_batch48.md)"),
         "gpu_launches_timed": None,
     })
     if not args.no_cpu:
@@ -678,11 +677,10 @@ def match_workload(args, stream):
     res["untimed_queries"] = [q for q in queries if q not in todo]
     hbm, peak_kind = peaks()
     if "cycle4" in res["queries"]:
-        res["roofline"] = roofline(profiled("k_match_rmat21_cycle4", "traffic_bytes_per_launch[cycle4_rmat21]"),
-                                   res["queries"]["cycle4"]["ms"], hbm, peak_kind, kernel="k_match (4-cycle query)",
-                                   note="DRAM bytes of one ncu capture of this query on this graph: the "
-                                        "back-edge tests read adjacency-bitmap words and label-segment keys "
-                                        "at random (profiles/k_match_rmat21_cycle4.md)")
+        res["roofline"] = roofline(profiled("k_cycle_big_rmat19", "traffic_bytes_per_launch[cycle4_rmat21]"),
+                                   res["queries"]["cycle4"]["ms"], hbm, peak_kind, kernel="k_cycle_big (4-cycle query)",
+                                   note="2-hop walks over L2-resident lists into shared-memory counters: latency-bound "
+                                        "(profiles/k_cycle_big_rmat19.md, profiled at scale 19)")
     if todo:
         # the same queries counted together: one persistent launch over every
         # query's tasks, autotuned task split, CUDA-graph replay -- against
