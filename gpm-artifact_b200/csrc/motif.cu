@@ -355,6 +355,7 @@ __global__ void k_c4_tasks(int64_t n, const int64_t *__restrict__ roff, const in
         const int i = atomicAdd(&sizes[2], 1);
         big_tasks[i] = (int32_t)x;
         big_b[i] = b;
+        atomicMax(&sizes[3], (int)dx);
       } else if (b > (unsigned long long)warp_bound) {
         cta_tasks[atomicAdd(&sizes[0], 1)] = (int32_t)x;
       } else {
@@ -438,26 +439,25 @@ __global__ void __launch_bounds__(256) k_c4(const int64_t *__restrict__ roff, co
 // table of k_c4's holds (nearly every wedge ends at its own y).  Its counters
 // are indexed by y directly, a window of keys at a time, in shared memory --
 // 16-bit halves of 32-bit words while x has fewer than 65536 neighbours below
-// it, so no count can carry into the next key.  Ranks ascend with degree and y
-// lies below x, so the window just below x takes most wedges (R-MAT 18: 91 %
-// end within 50,000 of x, Chung-Lu 200,000: 61 %).  A task that spans more than
-// kC4Windows windows has shared counters for the first alone and counts the
-// `cold_len` keys below it in the CTA's own array in global memory.  Every
-// increment adds the counter's old value to the sum (C(c+1,2) - C(c,2) = c),
-// so no scan is needed.
-// The walk (wedge.cuh) clips each list to the window by binary search and takes
-// 1.2 G warp instructions for the 0.85 G wedges of R-MAT 18, where lane groups
-// with a cursor per list took 2.2 G (3.88 ms; 3.4 ms now; batch of 48
-// Chung-Lu graphs 13.95 -> 11.8 ms).  It is bound by the latency of the lists
-// and of the counters' old values at 48 warps per SM.  CTA shapes, R-MAT 18 /
-// batch: 2 x 768 threads, 100 KB each 3.4 / 11.8 ms; 1 x 1024, 200 KB 3.2 /
-// 14.5; 3 x 512, 66 KB 4.6 / 12.8; 4 x 384, 49 KB 6.4 / 14.4.  Windows: 8
-// against 4 at R-MAT 18 (six windows): 3.4 / 4.5 ms.
+// it, so no count can carry into the next key.  Every increment adds the
+// counter's old value to the sum (C(c+1,2) - C(c,2) = c), so no scan is needed.
+// The windows go down from x; a walk (wedge.cuh) leaves in `cursor` where each
+// list's part began, the next window's ends there and its start is near, so a
+// list is searched in full once per task.  Ranks ascend with degree and y lies
+// below x, so the window just below x takes most wedges (R-MAT 18: 91 % end
+// within 50,000 of x, Chung-Lu 200,000: 61 %), but the rest may span many: with
+// two full searches per list and window, and counters in global memory from
+// the ninth window on, motifs of R-MAT 18 / R-MAT 20 / the 256 Chung-Lu graphs
+// took 7.2 / 101 / 1320 ms, with cursors 6.2 / 39.6 / 698 ms (lane groups with
+// a cursor per list, 1024 threads and 200 KB: 11.8 / 70.7 / 806 ms, whole
+// pipelines).  It is bound by the latency of the lists and of the counters' old
+// values at 48 warps per SM.  CTA shapes, 48 Chung-Lu graphs / R-MAT 18 / 256
+// graphs: 2 x 768 threads, 100 KB each 21.3 / 6.22 / 698 ms; 1 x 1024, 200 KB
+// 24.1 / 6.41 / 700; 2 x 1024, 100 KB 21.5 / 6.35 / 719.
 constexpr int kC4BigThreads = 768, kC4BigPerSm = 2;
 constexpr int kC4HotWords = 25600;  // 100 KB per CTA
 constexpr int kC4BigSmem = kC4HotWords * 4;
-constexpr int kC4Windows = 8;
-constexpr int64_t kC4ColdBytes = 16ll << 30;  // most global memory for cold counters
+constexpr int64_t kC4CursorBytes = 4ll << 30;  // most global memory for cursors
 
 // Tasks whose bound is at most kC4HashMax count in an open-addressing table
 // over the same shared memory, slots of (key + 1, count) with 0 = empty.  The
@@ -490,11 +490,11 @@ __global__ void __launch_bounds__(kC4BigThreads, kC4BigPerSm)
     k_c4_big(const int64_t *__restrict__ roff, const int64_t *__restrict__ split, const int32_t *__restrict__ radj,
              const int32_t *__restrict__ gid, const int64_t *__restrict__ gbase, const int32_t *__restrict__ tasks,
              const unsigned long long *__restrict__ task_b, int n_tasks, int *__restrict__ counters,
-             unsigned *__restrict__ colds, int64_t cold_len, unsigned long long *__restrict__ acc) {
+             int *__restrict__ cursors, int cursor_len, unsigned long long *__restrict__ acc) {
   extern __shared__ __align__(16) unsigned hot[];
   __shared__ int s_task;
   __shared__ WedgeWalk s_walk;
-  unsigned *cold = colds + (int64_t)blockIdx.x * cold_len;
+  int *cursor = cursors + (int64_t)blockIdx.x * cursor_len;
   const unsigned lane = threadIdx.x & 31;
   int turn = 0;
   if (threadIdx.x == 0) s_walk.s[0].next = s_walk.s[0].nlong = 0;
@@ -513,8 +513,6 @@ __global__ void __launch_bounds__(kC4BigThreads, kC4BigPerSm)
     const int dx = (int)(split[x] - a0);
     const int sh = dx < 65536 ? 1 : 0;
     const unsigned mask = sh ? 0xffffu : 0xffffffffu;
-    // cold keys of this task
-    const int64_t cl = (int64_t)x - base <= (int64_t)kC4Windows * (kC4HotWords << sh) ? 0 : cold_len << sh;
     unsigned long long c = 0;
     if (W <= kC4HashMax) {
       cta_wedges(radj, dx, W, s_walk, &turn,
@@ -529,44 +527,38 @@ __global__ void __launch_bounds__(kC4BigThreads, kC4BigPerSm)
       __syncthreads();
     }
     for (int32_t hi = W <= kC4HashMax ? base : x; hi > base;) {
-      const int32_t hot0 = (int32_t)max((int64_t)base, (int64_t)hi - ((int64_t)kC4HotWords << sh));
-      const int32_t lo = (int32_t)max((int64_t)base, (int64_t)hot0 - cl);
-      // entries of N(a) in [lo, h) for the i-th neighbour a of x
-      auto part = [&](int h) {
-        return [=](int i, long long *st, int *len) {
-          const int32_t a = radj[a0 + i];
-          int64_t s = roff[a];
-          const int64_t e = first_at_least(radj, s, roff[a + 1], h);
-          if (lo > base) s = first_at_least(radj, s, e, lo);
-          *st = s;
-          *len = (int)(e - s);
-        };
-      };
-      cta_wedges(radj, dx, W, s_walk, &turn, part(hi), [&](int32_t y, long long, int) {
-        if (y >= hot0) {
-          const unsigned o = (unsigned)(y - hot0), s = (o & (unsigned)sh) << 4;
-          c += (atomicAdd(&hot[o >> sh], 1u << s) >> s) & mask;
-        } else {
-          const unsigned o = (unsigned)(y - lo), s = (o & (unsigned)sh) << 4;
-          c += (atomicAdd(&cold[o >> sh], 1u << s) >> s) & mask;
-        }
-      });
-      // back to zero: the hot words by a memset when the wedges are many, the
-      // rest by the same walk
-      const bool sweep = W * 4 >= (unsigned long long)kC4HotWords;
-      if (sweep) {
-        const int words = ((hi - hot0) >> sh) + 1;
-        uint4 *v = reinterpret_cast<uint4 *>(hot);
-        for (int i = threadIdx.x; 4 * i < words; i += blockDim.x)
-          if (i < kC4HotWords / 4) v[i] = make_uint4(0u, 0u, 0u, 0u);
-      }
-      if (!sweep || hot0 > lo)
-        cta_wedges(radj, dx, W, s_walk, &turn, part(sweep ? hot0 : hi), [&](int32_t y, long long, int) {
-          if (y >= hot0) hot[(unsigned)(y - hot0) >> sh] = 0u;
-          else cold[(unsigned)(y - lo) >> sh] = 0u;
-        });
-      else
-        __syncthreads();
+      const int32_t lo = (int32_t)max((int64_t)base, (int64_t)hi - ((int64_t)kC4HotWords << sh));
+      cta_wedges(radj, dx, W, s_walk, &turn,
+                 [&](int i, long long *st, int *len) {  // entries of N(a) in [lo, hi), a the i-th neighbour of x
+                   const int64_t s0 = roff[radj[a0 + i]];
+                   int64_t s = s0, e;
+                   if (hi < x && i < cursor_len) e = s0 + cursor[i];
+                   else e = first_at_least(radj, s0, roff[radj[a0 + i] + 1], hi);
+                   if (lo > base) {
+                     if (i < cursor_len) {  // back from e in doubling steps
+                       int64_t top = e, step = 1;
+                       while (s0 < top && __ldg(radj + max(s0, top - step)) >= lo) {
+                         top = max(s0, top - step);
+                         step *= 2;
+                       }
+                       s = first_at_least(radj, max(s0, top - step), top, lo);
+                       cursor[i] = (int)(s - s0);
+                     } else {
+                       s = first_at_least(radj, s0, e, lo);
+                     }
+                   }
+                   *st = s;
+                   *len = (int)(e - s);
+                 },
+                 [&](int32_t y, long long, int) {
+                   const unsigned o = (unsigned)(y - lo), s = (o & (unsigned)sh) << 4;
+                   c += (atomicAdd(&hot[o >> sh], 1u << s) >> s) & mask;
+                 });
+      const int words = ((hi - lo) >> sh) + 1;
+      uint4 *v = reinterpret_cast<uint4 *>(hot);
+      for (int i = threadIdx.x; 4 * i < words; i += blockDim.x)
+        if (i < kC4HotWords / 4) v[i] = make_uint4(0u, 0u, 0u, 0u);
+      __syncthreads();
       hi = lo;
     }
     c = warp_sum(c);
@@ -687,7 +679,7 @@ int motif_plan_build(const MotifInput &in, MotifPlan *p, cudaStream_t st) {
   GPM_TRY(p->te.reserve(p->dadj.n));
   // queues of the per-edge triangle pass and of the 4-cycle pass
   DevBuf<int> sizes;
-  GPM_TRY(sizes.reserve(6));
+  GPM_TRY(sizes.reserve(7));
   GPM_TRY(p->te_ct.reserve(n));
   GPM_TRY(p->te_wt.reserve(n));
   GPM_TRY(p->c4_ct.reserve(n));
@@ -696,7 +688,7 @@ int motif_plan_build(const MotifInput &in, MotifPlan *p, cudaStream_t st) {
   DevBuf<unsigned long long> bb;
   GPM_TRY(bt.reserve(n));
   GPM_TRY(bb.reserve(n));
-  GPM_CUDA(cudaMemsetAsync(sizes.p, 0, 6 * sizeof(int), st));
+  GPM_CUDA(cudaMemsetAsync(sizes.p, 0, 7 * sizeof(int), st));
   if (n > 0) {
     k_te_tasks<<<grid_for(n), 256, 0, st>>>(n, p->doff.p, std::min(in.te_cta_min, kTeWarpKeys), p->te_ct.p, p->te_wt.p, sizes.p);
     if (in.size == 4) {
@@ -710,7 +702,7 @@ int motif_plan_build(const MotifInput &in, MotifPlan *p, cudaStream_t st) {
                                                    p->c4_ct.p, p->c4_wt.p, bt.p, bb.p, sizes.p + 3);
     }
   }
-  int h[6];
+  int h[7];
   GPM_CUDA(cudaMemcpyAsync(h, sizes.p, sizeof h, cudaMemcpyDeviceToHost, st));
   GPM_CUDA(cudaStreamSynchronize(st));
   p->te_nc = h[0];
@@ -740,19 +732,16 @@ int motif_plan_build(const MotifInput &in, MotifPlan *p, cudaStream_t st) {
     GPM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_c4_big, kC4BigThreads, kC4BigSmem));
     p->c4_big_grid = std::max(1, per_sm) * num_sms();
     p->c4_big_grid = std::min(p->c4_big_grid, p->c4_nb);
-    // cold counters for every key below the shared ones of the largest member
-    // (none where all members span few windows), as far as memory goes (fewer:
-    // more passes over the lists)
-    size_t free_b = 0, total_b = 0;
-    GPM_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    int64_t room = std::min<int64_t>(kC4ColdBytes, (int64_t)(free_b / 4)) / 4 / p->c4_big_grid;
-    if (const char *e = getenv("GPM_C4_COLD_LEN")) room = std::min<int64_t>(room, std::max(0ll, atoll(e)));
-    p->c4_cold_len = in.max_graph_n <= (int64_t)kC4Windows * kC4HotWords ? 0 : std::min(room, in.max_graph_n);
-    while (p->c4_cold.reserve((size_t)p->c4_cold_len * p->c4_big_grid) != GPM_OK) {
-      if (p->c4_cold_len == 0) return GPM_ENOMEM;
-      p->c4_cold_len = p->c4_cold_len < 4096 ? 0 : p->c4_cold_len / 2;
+    // cursors for the longest task's neighbours, where some member spans two
+    // windows, as far as memory goes (the others search their whole list again)
+    int64_t len = in.max_graph_n <= kC4HotWords ? 0 : h[6];
+    if (const char *e = getenv("GPM_C4_CURSORS")) len = std::min<int64_t>(len, std::max(0ll, atoll(e)));
+    len = std::min(len, kC4CursorBytes / 4 / p->c4_big_grid);
+    while (p->c4_cursor.reserve((size_t)len * p->c4_big_grid) != GPM_OK) {
+      if (len == 0) return GPM_ENOMEM;
+      len = len < 4096 ? 0 : len / 2;
     }
-    GPM_CUDA(cudaMemsetAsync(p->c4_cold.p, 0, sizeof(unsigned) * (size_t)p->c4_cold_len * p->c4_big_grid, st));
+    p->c4_cursor_len = (int)len;
     GPM_CUDA(cudaStreamSynchronize(st));
   }
   {
@@ -782,7 +771,7 @@ static int c4_launch(MotifPlan *p, cudaStream_t st) {
   if (p->c4_nb > 0)
     k_c4_big<<<p->c4_big_grid, kC4BigThreads, kC4BigSmem, st>>>(
         in.roff, p->split.p, in.radj, in.gid, in.gbase, p->c4_bt.p, p->c4_bb.p, p->c4_nb, c4_cursors(p),
-        p->c4_cold.p, p->c4_cold_len, p->acc.p);
+        p->c4_cursor.p, p->c4_cursor_len, p->acc.p);
   if (p->c4_nc + p->c4_nw > 0)
     k_c4<<<p->c4_grid, 256, 0, st>>>(in.roff, p->split.p, in.radj, in.gid, in.gbase, p->c4_ct.p, p->c4_nc,
                                      p->c4_wt.p, p->c4_nw, c4_cursors(p), p->acc.p);

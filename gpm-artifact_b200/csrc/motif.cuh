@@ -81,8 +81,8 @@ struct MotifPlan {
   DevBuf<int32_t> te_ct, te_wt, c4_ct, c4_wt, c4_bt;
   DevBuf<unsigned long long> c4_bb;  // giant 4-cycle tasks and their 2-hop bounds, largest first
   int te_nc = 0, te_nw = 0, te_nl = 0, c4_nc = 0, c4_nw = 0, c4_nb = 0, te_grid = 0, c4_grid = 0, c4_big_grid = 0;
-  DevBuf<unsigned> c4_cold;  // cold counters of the giant tasks, c4_cold_len per CTA, zero between launches
-  int64_t c4_cold_len = 0;
+  DevBuf<int> c4_cursor;  // positions of the giant tasks' walks in their lists, c4_cursor_len per CTA
+  int c4_cursor_len = 0;
   CliquePlan k4;
   DevBuf<unsigned long long> acc, out;
 };

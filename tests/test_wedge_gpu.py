@@ -1,7 +1,7 @@
-"""4-cycle counters of the giant tasks: keys in shared memory, in the CTA's
-global array, and in further passes where that array is kept short, with 2-hop
-bounds down to a handful; and 4-cycle queries on classes larger than the shared
-counters.  Against the other kernels' counts."""
+"""4-cycle counters of the giant tasks: one window of keys and many, every list
+with a cursor, some and none, with 2-hop bounds down to a handful; and 4-cycle
+queries on classes larger than the shared counters.  Against the other
+kernels' counts."""
 import numpy as np
 import pytest
 
@@ -11,25 +11,25 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("graph", ["rmat", "cl", "star"])
-def test_cold_keys_and_passes(graph, monkeypatch):
+def test_windows_and_cursors(graph, monkeypatch):
     if graph == "rmat":
         n, s, d = gpm.gen_rmat(16, 4, seed=3)
     elif graph == "cl":
-        n, s, d = gpm.gen_chung_lu(600001, 2.2, 6.0, seed=4)  # more keys than eight windows
+        n, s, d = gpm.gen_chung_lu(600001, 2.2, 6.0, seed=4)  # a dozen windows
     else:  # two hubs over 70,000 common neighbours: 32-bit counters, one pair
         n = 300002
         s = np.concatenate([np.arange(70000), np.arange(70000)]).astype(np.int32)
         d = np.concatenate([np.full(70000, n - 2), np.full(70000, n - 1)]).astype(np.int32)
     want = None
-    for cold in (None, "0", "1000"):
+    for cursors in (None, "0", "1000"):
         for big in (None, "0"):
-            for name, value in (("GPM_C4_COLD_LEN", cold), ("GPM_C4_BIG_MIN", big)):
+            for name, value in (("GPM_C4_CURSORS", cursors), ("GPM_C4_BIG_MIN", big)):
                 monkeypatch.delenv(name, raising=False) if value is None else monkeypatch.setenv(name, value)
             g = gpm.Graph.from_edges(n, s, d)
             got = g.motif(4).tolist()
             assert got == g.motif(4).tolist()  # counters are left at zero
             want = want or got
-            assert got == want, (cold, big)
+            assert got == want, (cursors, big)
     if graph == "star":
         assert want[3] == 70000 * 69999 // 2
 
