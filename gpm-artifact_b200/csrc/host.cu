@@ -151,12 +151,20 @@ void *pool_get(size_t bytes, size_t *cap, int *dev) {
   return cudaMalloc(&p, want) == cudaSuccess ? p : nullptr;
 }
 
+// Waits for the work in flight on the current device the way cudaFree does: a
+// cudaDeviceSynchronize would fail, and end the capture, while any thread
+// captures a stream of the device.
+static bool pool_quiesce() {
+  void *p = nullptr;
+  if (cudaMalloc(&p, 256) == cudaSuccess) return cudaFree(p) == cudaSuccess;
+  cudaGetLastError();
+  return false;
+}
+
 void pool_put(void *p, size_t cap, int dev) {
   BlockPool &P = block_pool();
   int cur = -1;
-  // as with cudaFree, work in flight on the device ends first
-  if (dev >= 0 && dev < BlockPool::kDevices && cudaGetDevice(&cur) == cudaSuccess && cur == dev &&
-      cudaDeviceSynchronize() == cudaSuccess) {
+  if (dev >= 0 && dev < BlockPool::kDevices && cudaGetDevice(&cur) == cudaSuccess && cur == dev && pool_quiesce()) {
     std::lock_guard<std::mutex> lock(P.mu);
     if (P.bytes[dev] + cap <= BlockPool::kPoolBytes) {
       P.blocks[dev].emplace(cap, p);
