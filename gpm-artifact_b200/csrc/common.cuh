@@ -59,8 +59,8 @@ struct ArenaScope {
 // Every other allocation comes from a process-wide pool of freed blocks, per
 // device.  Freeing waits for the device, as cudaFree does, so a block in the
 // pool is idle and may go to any thread and stream; at most kPoolBytes are
-// kept per device, all of them are given back when an allocation fails or
-// plans are dropped, and larger remainders go straight to cudaFree.  (A first
+// kept per device, the longest idle make room for newer ones, and all are given
+// back when an allocation fails or plans are dropped.  (A first
 // triangle count on R-MAT 22 made 56 cudaMalloc and 37 cudaFree calls: 27 of
 // its 37 ms.)
 void *pool_get(size_t bytes, size_t *cap, int *dev);  // nullptr: out of memory (cudaGetLastError not cleared)

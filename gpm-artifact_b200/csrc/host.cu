@@ -90,8 +90,13 @@ struct BlockPool {
   static constexpr int kDevices = 64;
   static constexpr size_t kPoolBytes = (size_t)4 << 30;  // cached bytes per device
   std::mutex mu;
-  std::multimap<size_t, void *> blocks[kDevices];  // size -> idle block
+  struct Idle {
+    void *p;
+    uint64_t since;
+  };
+  std::multimap<size_t, Idle> blocks[kDevices];  // size -> idle block
   size_t bytes[kDevices] = {};
+  uint64_t clock = 0;
 };
 // never destroyed: buffers of static and thread-local objects may be freed
 // after the end of main
@@ -112,7 +117,7 @@ static void pool_trim_device(int dev) {
   std::vector<void *> gone;
   {
     std::lock_guard<std::mutex> lock(P.mu);
-    for (auto &b : P.blocks[dev]) gone.push_back(b.second);
+    for (auto &b : P.blocks[dev]) gone.push_back(b.second.p);
     P.blocks[dev].clear();
     P.bytes[dev] = 0;
   }
@@ -136,7 +141,7 @@ void *pool_get(size_t bytes, size_t *cap, int *dev) {
     auto &blocks = P.blocks[*dev];
     auto it = blocks.lower_bound(want);
     if (it != blocks.end() && it->first <= want + want / 4) {
-      p = it->second;
+      p = it->second.p;
       *cap = it->first;
       P.bytes[*dev] -= it->first;
       blocks.erase(it);
@@ -165,14 +170,28 @@ void pool_put(void *p, size_t cap, int dev) {
   BlockPool &P = block_pool();
   int cur = -1;
   if (dev >= 0 && dev < BlockPool::kDevices && cudaGetDevice(&cur) == cudaSuccess && cur == dev && pool_quiesce()) {
-    std::lock_guard<std::mutex> lock(P.mu);
-    if (P.bytes[dev] + cap <= BlockPool::kPoolBytes) {
-      P.blocks[dev].emplace(cap, p);
-      P.bytes[dev] += cap;
-      return;
+    std::vector<void *> gone;
+    {
+      std::lock_guard<std::mutex> lock(P.mu);
+      auto &blocks = P.blocks[dev];
+      if (cap <= BlockPool::kPoolBytes) {
+        // the longest idle make room: what earlier work left may fit nothing any more
+        while (P.bytes[dev] + cap > BlockPool::kPoolBytes) {
+          auto old = blocks.begin();
+          for (auto it = blocks.begin(); it != blocks.end(); ++it)
+            if (it->second.since < old->second.since) old = it;
+          P.bytes[dev] -= old->first;
+          gone.push_back(old->second.p);
+          blocks.erase(old);
+        }
+        blocks.emplace(cap, BlockPool::Idle{p, P.clock++});
+        P.bytes[dev] += cap;
+        p = nullptr;
+      }
     }
+    for (void *q : gone) cudaFree(q);
   }
-  cudaFree(p);
+  if (p) cudaFree(p);
 }
 
 int ensure_device() {
