@@ -59,6 +59,12 @@ struct CqCore {
 // 512-thread CTAs with kCqSmemBig, two per SM, and beyond that in a slab.
 constexpr size_t kCqSmemSmall = 44 * 1024, kCqSmemBig = 112 * 1024;
 constexpr int kCqSmallThreads = 256, kCqBigThreads = 512;
+// Cliques of other sizes than 4 and 5 walk a row's set in one warp while the
+// others wait at the end of the task: many small CTAs, with the slab for rows
+// past the small CTAs' shared memory, lose least (7-cliques of R-MAT 14 441 ->
+// 349 ms, 6-cliques of R-MAT 17 323 -> 304 ms against 512 threads and rows dealt in turn).
+__host__ __device__ constexpr size_t cq_smem_big(int k) { return k == 4 || k == 5 ? kCqSmemBig : kCqSmemSmall; }
+__host__ __device__ constexpr int cq_threads_big(int k) { return k == 4 || k == 5 ? kCqBigThreads : kCqSmallThreads; }
 
 static int grid_for(int64_t work, int block = 256) {
   int64_t g = (work + block - 1) / block;
@@ -670,8 +676,19 @@ __device__ unsigned long long clique_cta_task(int32_t u, int k, const int64_t *_
       __syncthreads();
     }
   } else {
-    // each lane accumulates the popcounts of its own words; the warp sum is the count
-    for (int i = wid; i < d; i += nw) c += warp_count_set(rows, W, wrow(rows, W, i, lane), k - 2, xs, lane);
+    // each lane accumulates the popcounts of its own words; the warp sum is the
+    // count.  Rows differ far in their work and the first hold most: taken one
+    // by one
+    __shared__ int s_row;
+    if (tid == 0) s_row = 0;
+    __syncthreads();
+    while (true) {
+      int i = 0;
+      if (lane == 0) i = atomicAdd(&s_row, 1);
+      i = __shfl_sync(0xffffffffu, i, 0);
+      if (i >= d) break;
+      c += warp_count_set(rows, W, wrow(rows, W, i, lane), k - 2, xs, lane);
+    }
   }
   __syncthreads();
   return c;
@@ -680,17 +697,17 @@ __device__ unsigned long long clique_cta_task(int32_t u, int k, const int64_t *_
 // CTA tasks [t0, t1) of the queue, heaviest first.  KM: 4, 5, or 0 for the
 // other clique sizes.  BIG: rows may be in the slab.
 template <int KM, bool BIG>
-__global__ void __launch_bounds__(BIG ? kCqBigThreads : kCqSmallThreads)
-    k_clique_cta(int k, const int64_t *__restrict__ roff, const int32_t *__restrict__ radj,
+__device__ __forceinline__ void
+    clique_cta(int k, const int64_t *__restrict__ roff, const int32_t *__restrict__ radj,
                  const int32_t *__restrict__ tasks, int ntasks, int *__restrict__ cursor, uint32_t *__restrict__ slabs,
                  size_t slab_half, CqCore core, const int32_t *__restrict__ gid, unsigned long long *__restrict__ acc,
                  int stride, int slot) {
   extern __shared__ __align__(16) uint32_t csm[];
   __shared__ int s_task;
-  __shared__ uint32_t sxs[KM == 0 ? (BIG ? kCqBigThreads : kCqSmallThreads) / 32 : 1][64];  // staged sets (wsum_pairs)
+  __shared__ uint32_t sxs[KM == 0 ? kCqSmallThreads / 32 : 1][64];  // staged sets (wsum_pairs)
   const int wid = threadIdx.x >> 5;
   const unsigned lane = threadIdx.x & 31;
-  constexpr size_t words = (BIG ? kCqSmemBig : kCqSmemSmall) / 4;
+  constexpr size_t words = (BIG ? cq_smem_big(KM) : kCqSmemSmall) / 4;
   uint32_t *slab = slabs + (size_t)blockIdx.x * 2 * slab_half;
   uint32_t *xs = sxs[KM == 0 ? wid : 0];
   while (true) {
@@ -708,6 +725,25 @@ __global__ void __launch_bounds__(BIG ? kCqBigThreads : kCqSmallThreads)
     c = warp_sum(c);
     if (lane == 0 && c) atomicAdd(&acc[(size_t)stride * (gid ? gid[u] : 0) + slot], c);
   }
+}
+
+template <int KM, bool BIG>
+__global__ void __launch_bounds__(BIG ? kCqBigThreads : kCqSmallThreads)
+    k_clique_cta(int k, const int64_t *__restrict__ roff, const int32_t *__restrict__ radj,
+                 const int32_t *__restrict__ tasks, int ntasks, int *__restrict__ cursor, uint32_t *__restrict__ slabs,
+                 size_t slab_half, CqCore core, const int32_t *__restrict__ gid, unsigned long long *__restrict__ acc,
+                 int stride, int slot) {
+  clique_cta<KM, BIG>(k, roff, radj, tasks, ntasks, cursor, slabs, slab_half, core, gid, acc, stride, slot);
+}
+// Cliques of other sizes than 4 and 5: five CTAs per SM, in place of the 32 and
+// 40 registers with spills that the compiler takes by itself.
+template <bool BIG>
+__global__ void __launch_bounds__(kCqSmallThreads, 5)
+    k_clique_any(int k, const int64_t *__restrict__ roff, const int32_t *__restrict__ radj,
+                 const int32_t *__restrict__ tasks, int ntasks, int *__restrict__ cursor, uint32_t *__restrict__ slabs,
+                 size_t slab_half, CqCore core, const int32_t *__restrict__ gid, unsigned long long *__restrict__ acc,
+                 int stride, int slot) {
+  clique_cta<0, BIG>(k, roff, radj, tasks, ntasks, cursor, slabs, slab_half, core, gid, acc, stride, slot);
 }
 
 __global__ void __launch_bounds__(256) k_clique_warp(int k, const int64_t *__restrict__ roff,
@@ -851,7 +887,7 @@ template <class F>
 static void cq_kernels(int k, F f) {
   if (k == 4) f(k_clique_cta<4, false>, k_clique_cta<4, true>);
   else if (k == 5) f(k_clique_cta<5, false>, k_clique_cta<5, true>);
-  else f(k_clique_cta<0, false>, k_clique_cta<0, true>);
+  else f(k_clique_any<false>, k_clique_any<true>);
 }
 
 struct CqGrids {
@@ -863,7 +899,7 @@ static CqGrids cq_grids(int k) {
   CqGrids g;
   cq_kernels(k, [&](auto s, auto b) {
     g.small = small[i].get([&] { return cq_grid(s, kCqSmallThreads, kCqSmemSmall); });
-    g.big = big[i].get([&] { return cq_grid(b, kCqBigThreads, kCqSmemBig); });
+    g.big = big[i].get([&] { return cq_grid(b, cq_threads_big(k), cq_smem_big(k)); });
   });
   g.warp = warp.get([] { return cq_grid(k_clique_warp, 256, 0); });
   return g;
@@ -951,7 +987,7 @@ int clique_plan_build(CliquePlan *p, int64_t n, const int64_t *roff, const int32
   }
   const CqLayout big = cq_layout(max_deg, k, kCqBigThreads / 32, true);
   const size_t comp_max = (size_t)max_deg * ((W + 3) & ~(size_t)3);
-  const bool spill = p->n_big && (big.total * 4 > kCqSmemBig || (k == 5 && comp_max > kCqBigThreads / 32 * cq_warp_words(1)));
+  const bool spill = p->n_big && (big.total * 4 > cq_smem_big(k) || (k == 5 && comp_max > kCqBigThreads / 32 * cq_warp_words(1)));
   p->slab_words = comp_max;
   GPM_TRY(p->slabs.reserve(spill ? 2 * p->slab_words * p->big_grid : 1));
   if (p->n_cta > p->n_big && k == 5) {
@@ -981,7 +1017,7 @@ int clique_plan_run(CliquePlan *p, cudaStream_t st, bool zero) {
   }
   cq_kernels(p->k, [&](auto small, auto big) {
     if (p->n_big > 0)
-      big<<<p->big_grid, kCqBigThreads, kCqSmemBig, bst>>>(p->k, p->roff, p->radj, p->ctasks.p, p->n_big,
+      big<<<p->big_grid, cq_threads_big(p->k), cq_smem_big(p->k), bst>>>(p->k, p->roff, p->radj, p->ctasks.p, p->n_big,
                                                            p->cursors, p->slabs.p, p->slab_words, core, p->gid,
                                                            p->acc, p->stride, p->slot);
     if (nsmall > 0)
