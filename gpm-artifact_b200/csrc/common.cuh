@@ -249,6 +249,7 @@ struct gpm_graph {
   gpm::DevBuf<int32_t> adj;     // nnz
   gpm::DevBuf<int32_t> labels;  // n (optional)
   gpm::DevBuf<int32_t> src;     // nnz, COO source of each stored entry (lazy)
+  bool src_filled = false;      // src has been filled, not only recorded into a capture
   gpm::TcPlan *tc = nullptr;    // cached triangle-count schedule (HASH)
   gpm::RankPlan *rank = nullptr; // cached schedule of the BITMAP path
   gpm::RankGraph *rg = nullptr;  // cached rank-relabelled copy
@@ -267,6 +268,8 @@ namespace gpm {
 int build_csr_device(gpm_graph *g, int64_t n, int64_t m, const int32_t *d_src,
                      const int32_t *d_dst, int symmetrize, cudaStream_t st);
 int ensure_src(gpm_graph *g, cudaStream_t st);
+bool src_ready(const gpm_graph *g);  // would ensure_src launch nothing?
+bool stream_capturing(cudaStream_t st);
 int compute_max_degree(gpm_graph *g, cudaStream_t st);
 void free_tc_plan(TcPlan *p);
 void free_rank_plan(RankPlan *p);

@@ -194,13 +194,28 @@ __global__ void k_fill_src(int64_t n, const int64_t *__restrict__ off, int32_t *
     for (int64_t e = off[u] + lane_id(); e < off[u + 1]; e += 32) src[e] = (int32_t)u;
 }
 
+bool stream_capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &c) != cudaSuccess) cudaGetLastError();
+  return c != cudaStreamCaptureStatusNone;
+}
+
+bool src_ready(const gpm_graph *g) { return g->src.p && g->src.n >= (size_t)g->nnz && g->src_filled; }
+
+// The sources are there for every stream once this has returned; inside a
+// capture the filling is part of the captured work and each replay's own, so
+// the next call outside of one fills them again.
 int ensure_src(gpm_graph *g, cudaStream_t st) {
-  if (g->src.p && g->src.n >= (size_t)g->nnz) return GPM_OK;
+  if (src_ready(g)) return GPM_OK;
+  g->src_filled = false;
   GPM_TRY(g->src.reserve(g->nnz));
   if (g->n > 0) {
     k_fill_src<<<grid_for(g->n * 32), 256, 0, st>>>(g->n, g->off.p, g->src.p);
     GPM_LAUNCH_CHECK();
   }
+  if (stream_capturing(st)) return GPM_OK;
+  GPM_CUDA(cudaStreamSynchronize(st));
+  g->src_filled = true;
   return GPM_OK;
 }
 

@@ -532,7 +532,9 @@ constexpr int64_t kTiny = 16384, kTinySkewed = 65536;
 // The count of a tiny graph, or of one with short lists alone, launched?
 static bool small_launch(gpm_graph *g, cudaStream_t st, unsigned long long *d_out, int *status) {
   if (g->nnz <= 0) return false;
-  if (g->nnz <= kTiny) *status = tc_launch(g, GPM_TC_BSEARCH, st, d_out);
+  // inside a capture only with the entries' sources there already: a count of
+  // the rank plan, which may be, needs no memory
+  if (g->nnz <= kTiny && (src_ready(g) || !stream_capturing(st))) *status = tc_launch(g, GPM_TC_BSEARCH, st, d_out);
   else if (g->max_deg <= kListDegree) *status = lists_launch(g, st, d_out);
   else return false;
   return true;
