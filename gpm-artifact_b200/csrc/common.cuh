@@ -259,7 +259,6 @@ struct gpm_graph {
   gpm::CliquePlan *clique[9] = {};                // cached k-clique schedules, by k
   gpm_sched *sched = nullptr;        // learned scheduler (not owned)
   gpm::DevBuf<uint64_t> result; // small device result scratch
-  gpm::DevBuf<int> tc_state;    // cursors and sum of the list-merging triangle count (tc.cu), zero between launches
   ~gpm_graph();
 };
 

@@ -325,33 +325,18 @@ __device__ __forceinline__ unsigned long long cta_sum(unsigned long long c) {
   return c;
 }
 
-// state: two cursors, the number of CTAs that have ended, and the sum, all
-// zero before the launch; the last CTA writes *out and leaves them zero, so a
-// repeated count is this launch alone (ER, 16,384 vertices: 26 us per count
-// before, with two memsets and one atomic per warp and task).
-struct HashState {
-  int cursor[2], done, pad;
-  unsigned long long sum;
-};
+// *out and the two cursors are zero before the launch.
 __global__ void __launch_bounds__(256) k_tc_hash(const int64_t *__restrict__ off,
                                                  const int32_t *__restrict__ adj,
                                                  const int32_t *__restrict__ cta_tasks, int n_cta,
                                                  const int32_t *__restrict__ warp_tasks, int n_warp,
-                                                 HashState *__restrict__ state, int even,
+                                                 int *__restrict__ cursors, int even,
                                                  unsigned long long *__restrict__ out) {
   extern __shared__ __align__(16) char smem[];
   __shared__ int s_task;
   const unsigned long long c =
-      cta_sum(hash_tasks(off, adj, cta_tasks, n_cta, warp_tasks, n_warp, state->cursor, even != 0, smem, &s_task));
-  if (threadIdx.x == 0) {
-    if (c) atomicAdd(&state->sum, c);
-    __threadfence();
-    if (atomicAdd(&state->done, 1) == (int)gridDim.x - 1) {
-      __threadfence();
-      *out = atomicExch(&state->sum, 0ull);
-      state->cursor[0] = state->cursor[1] = state->done = 0;
-    }
-  }
+      cta_sum(hash_tasks(off, adj, cta_tasks, n_cta, warp_tasks, n_warp, cursors, even != 0, smem, &s_task));
+  if (threadIdx.x == 0 && c) atomicAdd(out, c);
 }
 
 // ------------------------------------------------------------------ LISTS
@@ -359,14 +344,17 @@ __global__ void __launch_bounds__(256) k_tc_hash(const int64_t *__restrict__ off
 // lists, one or two sectors each.  No tables, queues or plan.  A warp takes
 // `span` consecutive vertices (a power of two up to 32, so that small graphs
 // fill the GPU), their edges end to end over its lanes.  Bound by the latency
-// of the merge's dependent loads, so only for the shortest lists.  ER, count /
-// first count in us, against hash kernel and rank plan: 16,384 x 16 (longest
-// list 15) 17 / 28, 17 / 44, 26 / 375; 100,003 x 20 (20) 71 / 83, 78 / 111, 82 /
-// 495; 10^6 x 12 (13) 160 / 173, 344 / 400, 345 / 1268.  But 10^6 x 32 (30) 952,
-// 920, 654, and Chung-Lu 100,001 x 8 (33) 114, 93, 52.
+// of the merge's dependent loads, so only for the shortest lists.  ER, count in
+// us against hash kernel and rank plan (first counts in brackets): 16,384 x 16
+// (longest list 15) 16 (28), 18 (44), 26 (375); 100,003 x 20 (20) 79 (88), 82
+// (111), 82 (495); 10^6 x 12 (13) 162 (175), 345 (400), 345 (1268).  But 10^6 x
+// 32 (30) 952, 920, 654, and Chung-Lu 100,001 x 8 (33) 114, 93, 52.  The sum goes
+// to *out by one atomic per CTA and *out is cleared by a memset before, 4 us of
+// the 79: a sum kept in the handle and cleared by the last CTA saved them, but
+// launches that overlap on two streams mixed theirs.
 constexpr int kListDegree = 24;  // longest list
 __global__ void __launch_bounds__(256) k_tc_lists(int64_t n, int span, const int64_t *__restrict__ off,
-                                                  const int32_t *__restrict__ adj, HashState *__restrict__ state,
+                                                  const int32_t *__restrict__ adj,
                                                   unsigned long long *__restrict__ out) {
   const int lane = (int)lane_id();
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -405,15 +393,7 @@ __global__ void __launch_bounds__(256) k_tc_lists(int64_t n, int span, const int
     }
   }
   c = cta_sum(c);
-  if (threadIdx.x == 0) {
-    if (c) atomicAdd(&state->sum, c);
-    __threadfence();
-    if (atomicAdd(&state->done, 1) == (int)gridDim.x - 1) {
-      __threadfence();
-      *out = atomicExch(&state->sum, 0ull);
-      state->done = 0;
-    }
-  }
+  if (threadIdx.x == 0 && c) atomicAdd(out, c);
 }
 
 // Task split by degree (the reference's USE_WARP / USE_CTA thresholds).
@@ -451,13 +431,11 @@ int tc_build_plan(gpm_graph *g, int warp_min, int cta_min, cudaStream_t st) {
   p->cta_min = cta_min;
   int64_t n = g->n;
   int s = GPM_OK;
-  static_assert(sizeof(HashState) == 6 * sizeof(int), "plan counters hold a HashState");
-  if ((s = p->cta_tasks.reserve(n)) || (s = p->warp_tasks.reserve(n)) || (s = p->counters.reserve(6)) ||
+  if ((s = p->cta_tasks.reserve(n)) || (s = p->warp_tasks.reserve(n)) || (s = p->counters.reserve(2)) ||
       (s = p->sizes.reserve(2))) {
     delete p;
     return s;
   }
-  cudaMemsetAsync(p->counters.p, 0, 6 * sizeof(int), st);
   cudaMemsetAsync(p->sizes.p, 0, 2 * sizeof(int), st);
   if (n > 0) {
     int grid = (int)std::min<int64_t>((n + 255) / 256, (int64_t)num_sms() * 8);
@@ -476,8 +454,8 @@ int tc_build_plan(gpm_graph *g, int warp_min, int cta_min, cudaStream_t st) {
   return GPM_OK;
 }
 
-int tc_launch(gpm_graph *g, int variant, cudaStream_t st, unsigned long long *d_out) {
-  if (variant != GPM_TC_HASH || g->nnz == 0) GPM_CUDA(cudaMemsetAsync(d_out, 0, sizeof(unsigned long long), st));
+int tc_launch(gpm_graph *g, int variant, cudaStream_t st, unsigned long long *d_out, int *cursors) {
+  if (!cursors) GPM_CUDA(cudaMemsetAsync(d_out, 0, sizeof(unsigned long long), st));
   if (g->nnz == 0) return GPM_OK;
   if (variant == GPM_TC_BSEARCH || variant == GPM_TC_MERGE) {
     GPM_TRY(ensure_src(g, st));
@@ -494,30 +472,30 @@ int tc_launch(gpm_graph *g, int variant, cudaStream_t st, unsigned long long *d_
     GPM_TRY(tc_build_plan(g, 2, 101, st));
     TcPlan *p = g->tc;
     if (p->cta_min - 1 > kWarpChunk) return fail(GPM_EINVAL, "warp tasks exceed the warp table");
+    if (!cursors) {
+      cursors = p->counters.p;
+      GPM_CUDA(cudaMemsetAsync(cursors, 0, 2 * sizeof(int), st));
+    }
     const int64_t blocks = (int64_t)p->n_cta + ((int64_t)p->n_warp + kWarps - 1) / kWarps;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(tc_hash_grid(), blocks));
     k_tc_hash<<<grid, 256, TC_SMEM, st>>>(g->off.p, g->adj.p, p->cta_tasks.p, p->n_cta, p->warp_tasks.p, p->n_warp,
-                                          reinterpret_cast<HashState *>(p->counters.p), g->max_deg <= kEvenDegree, d_out);
+                                          cursors, g->max_deg <= kEvenDegree, d_out);
     GPM_LAUNCH_CHECK();
     return GPM_OK;
   }
-  if (variant == GPM_TC_BITMAP) return rank_launch(g, st, d_out);
+  if (variant == GPM_TC_BITMAP) return rank_launch(g, st, d_out, cursors);
   return fail(GPM_EINVAL, "unknown triangle-count variant " + std::to_string(variant));
 }
 
+// *d_out is zero before the launch
 static int lists_launch(gpm_graph *g, cudaStream_t st, unsigned long long *d_out) {
-  if (!g->tc_state.p) {
-    GPM_TRY(g->tc_state.reserve(sizeof(HashState) / sizeof(int)));
-    GPM_CUDA(cudaMemsetAsync(g->tc_state.p, 0, sizeof(HashState), st));
-  }
   // one vertex per warp until all SMs have 32 warps, then more
   const int64_t warps = (int64_t)num_sms() * 32;
   int span = 1;
   while (span < 32 && (g->n + span - 1) / span > warps) span *= 2;
   const int64_t blocks = ((g->n + span - 1) / span + kWarps - 1) / kWarps;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(blocks, (int64_t)num_sms() * 32));
-  k_tc_lists<<<grid, 256, 0, st>>>(g->n, span, g->off.p, g->adj.p, reinterpret_cast<HashState *>(g->tc_state.p),
-                                   d_out);
+  k_tc_lists<<<grid, 256, 0, st>>>(g->n, span, g->off.p, g->adj.p, d_out);
   GPM_LAUNCH_CHECK();
   return GPM_OK;
 }
@@ -529,14 +507,21 @@ static int lists_launch(gpm_graph *g, cudaStream_t st, unsigned long long *d_out
 // 45,666 entries 19 / 30, 36 / 56, 22 / 386; R-MAT 12, 48,313 entries 27 / 37, 61 /
 // 91, 22 / 360.
 constexpr int64_t kTiny = 16384, kTinySkewed = 65536;
-// The count of a tiny graph, or of one with short lists alone, launched?
-static bool small_launch(gpm_graph *g, cudaStream_t st, unsigned long long *d_out, int *status) {
+// The count of a tiny graph, or of one with short lists alone, launched?  Both
+// kernels keep nothing between launches.  cursors: as tc_launch takes them.
+static bool small_launch(gpm_graph *g, cudaStream_t st, unsigned long long *d_out, int *cursors, int *status) {
   if (g->nnz <= 0) return false;
   // inside a capture only with the entries' sources there already: a count of
   // the rank plan, which may be, needs no memory
-  if (g->nnz <= kTiny && (src_ready(g) || !stream_capturing(st))) *status = tc_launch(g, GPM_TC_BSEARCH, st, d_out);
-  else if (g->max_deg <= kListDegree) *status = lists_launch(g, st, d_out);
-  else return false;
+  if (g->nnz <= kTiny && (src_ready(g) || !stream_capturing(st))) {
+    *status = tc_launch(g, GPM_TC_BSEARCH, st, d_out, cursors);
+    return true;
+  }
+  if (g->max_deg > kListDegree) return false;
+  if (!cursors && cudaMemsetAsync(d_out, 0, sizeof(unsigned long long), st) != cudaSuccess)
+    *status = fail(GPM_ECUDA, std::string("triangle count: ") + cudaGetErrorString(cudaGetLastError()));
+  else
+    *status = lists_launch(g, st, d_out);
   return true;
 }
 
@@ -549,21 +534,22 @@ static bool small_launch(gpm_graph *g, cudaStream_t st, unsigned long long *d_ou
 // clearly take longer than that (the sum of squared degrees follows its time
 // within a factor of two, 5 ps each), and otherwise when the counts made on
 // this graph with the hash kernel have cost as much as the plan.
-static int tc_auto_launch(gpm_graph *g, cudaStream_t st, unsigned long long *d_out) {
+// *d_out and the cursors are zero.
+static int tc_auto_launch(gpm_graph *g, cudaStream_t st, unsigned long long *d_out, int *cursors) {
   int s = GPM_OK;
-  if (small_launch(g, st, d_out, &s)) return s;
-  if (g->nnz <= kTinySkewed) return tc_launch(g, GPM_TC_BSEARCH, st, d_out);
+  if (small_launch(g, st, d_out, cursors, &s)) return s;
+  if (g->nnz <= kTinySkewed) return tc_launch(g, GPM_TC_BSEARCH, st, d_out, cursors);
   if (!g->rank && g->nnz > 0) {
     const double hash_us = 10 + 5e-6 * (double)g->sum_deg2, plan_us = 300 + 2.5e-4 * (double)g->nnz;
     if (hash_us < 40 || g->hash_us + hash_us < plan_us) {
       g->hash_us += hash_us;
-      return tc_launch(g, GPM_TC_HASH, st, d_out);
+      return tc_launch(g, GPM_TC_HASH, st, d_out, cursors);
     }
   }
-  s = tc_launch(g, GPM_TC_BITMAP, st, d_out);
+  s = tc_launch(g, GPM_TC_BITMAP, st, d_out, cursors);
   if (s != GPM_ENOMEM && s != GPM_EUNSUPPORTED) return s;
   g->hash_us = -1e30;  // not tried again
-  return tc_launch(g, GPM_TC_HASH, st, d_out);  // no room for the plan, or beyond its descriptors
+  return tc_launch(g, GPM_TC_HASH, st, d_out, cursors);  // no room for the plan, or beyond its descriptors
 }
 
 }  // namespace gpm
@@ -576,7 +562,7 @@ int gpm_tc_async(gpm_graph *g, int variant, void *stream, uint64_t *d_out) {
   if (!g || !d_out) return fail(GPM_EINVAL, "gpm_tc_async: NULL argument");
   if (variant == GPM_TC_AUTO) {
     int s = GPM_OK;
-    if (small_launch(g, (cudaStream_t)stream, (unsigned long long *)d_out, &s)) return s;
+    if (small_launch(g, (cudaStream_t)stream, (unsigned long long *)d_out, nullptr, &s)) return s;
     variant = GPM_TC_BITMAP;
   }
   if (variant == GPM_TC_LEARNED) return tc_learned_launch(g, (cudaStream_t)stream, (unsigned long long *)d_out);
@@ -587,7 +573,12 @@ int gpm_tc(gpm_graph *g, int mode, uint64_t *out) {
   if (!g || !out) return fail(GPM_EINVAL, "gpm_tc: NULL argument");
   if (mode != GPM_V_CENTRIC && mode != GPM_E_CENTRIC) return fail(GPM_EINVAL, "Wrong Calculation Mode.");
   GPM_TRY(g->result.reserve(8));
-  GPM_TRY(tc_auto_launch(g, 0, (unsigned long long *)g->result.p));
+  // The count and its work cursors, cleared together.  A synchronous count has
+  // cursors of its own: an asynchronous one of the same handle may be drawing
+  // tasks from the plan's on another stream.
+  static_assert(kTcCursors * sizeof(int) <= 7 * sizeof(uint64_t), "the result scratch holds the cursors");
+  GPM_CUDA(cudaMemsetAsync(g->result.p, 0, sizeof(uint64_t) + kTcCursors * sizeof(int), 0));
+  GPM_TRY(tc_auto_launch(g, 0, (unsigned long long *)g->result.p, reinterpret_cast<int *>(g->result.p + 1)));
   GPM_CUDA(cudaMemcpy(out, g->result.p, sizeof(uint64_t), cudaMemcpyDeviceToHost));
   return GPM_OK;
 }

@@ -1434,10 +1434,13 @@ int rank_plan_new(gpm_graph *g, int cta_min, int long_min, const uint8_t *cfg, c
 
 // Launch of a given plan; rec != nullptr selects the instrumented build.
 int rank_plan_launch(gpm_graph *g, RankPlan *p, cudaStream_t st, unsigned long long *d_out,
-                     unsigned long long *rec) {
-  GPM_CUDA(cudaMemsetAsync(d_out, 0, sizeof(unsigned long long), st));
+                     unsigned long long *rec, int *cursors) {
+  if (!cursors) GPM_CUDA(cudaMemsetAsync(d_out, 0, sizeof(unsigned long long), st));
   if (g->nnz == 0) return GPM_OK;
-  GPM_CUDA(cudaMemsetAsync(p->counters.p, 0, 4 * sizeof(int), st));
+  if (!cursors) {
+    cursors = p->counters.p;
+    GPM_CUDA(cudaMemsetAsync(cursors, 0, 4 * sizeof(int), st));
+  }
   if (p->n_dense) {  // forked onto the device's side stream, joined after the count kernel
     int s = GPM_OK;
     cudaStream_t side = dense_stream(&s);
@@ -1447,29 +1450,29 @@ int rank_plan_launch(gpm_graph *g, RankPlan *p, cudaStream_t st, unsigned long l
     k_tc_dense<<<p->dense_grid, 256, p->dense_smem, side>>>(g->rg->roff.p, g->rg->radj.p, p->doff.p, p->dseg.p,
                                                              p->dense_tasks.p, p->n_dense,
                                                              reinterpret_cast<const uint4 *>(p->rows.p),
-                                                             p->counters.p + 2, d_out);
+                                                             cursors + 2, d_out);
     GPM_LAUNCH_CHECK();
     GPM_CUDA(cudaEventRecord(p->join, side));
   }
   if (rec)
     k_tc_rank_t<true><<<rank_grid(), 256, kRankSmem, st>>>(
         g->rg->roff.p, g->rg->radj.p, g->rg->radj4.p, p->poff.p, p->pseg.p, p->plong.p, p->pshort.p, p->cta_tasks.p,
-        p->n_cta, p->warp_tasks.p, p->n_warp, p->counters.p, d_out, rec);
+        p->n_cta, p->warp_tasks.p, p->n_warp, cursors, d_out, rec);
   else
     k_tc_rank<<<rank_grid(), 256, kRankSmem, st>>>(g->rg->roff.p, g->rg->radj.p, g->rg->radj4.p, p->poff.p,
                                                    p->pseg.p, p->plong.p, p->pshort.p, p->cta_tasks.p, p->n_cta,
-                                                   p->warp_tasks.p, p->n_warp, p->counters.p, d_out, nullptr);
+                                                   p->warp_tasks.p, p->n_warp, cursors, d_out, nullptr);
   GPM_LAUNCH_CHECK();
   if (p->n_dense) GPM_CUDA(cudaStreamWaitEvent(st, p->join, 0));
   return GPM_OK;
 }
 
-int rank_launch(gpm_graph *g, cudaStream_t st, unsigned long long *d_out) {
+int rank_launch(gpm_graph *g, cudaStream_t st, unsigned long long *d_out, int *cursors) {
   if (g->nnz == 0) return cudaMemsetAsync(d_out, 0, 8, st) == cudaSuccess ? GPM_OK : GPM_ECUDA;
   // fixed schedule: owners with > kRankCtaMin keys go to a CTA, segments of
   // >= kRankLongMin keys are streamed by a half-warp
   GPM_TRY(rank_build_plan(g, kRankCtaMin, kRankLongMin, st));
-  return rank_plan_launch(g, g->rank, st, d_out, nullptr);
+  return rank_plan_launch(g, g->rank, st, d_out, nullptr, cursors);
 }
 
 // out[0] segments, out[1] keys in them, out[2] keys of the owners' lists

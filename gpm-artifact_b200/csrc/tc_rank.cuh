@@ -175,7 +175,7 @@ int ensure_rank_graph(gpm_graph *g, cudaStream_t st, const int32_t *gid = nullpt
 // g->adj is already on the device.
 int build_upward_rank_graph(gpm_graph *g, cudaStream_t st, const int64_t *h_off, const int32_t *h_adj);
 int rank_build_plan(gpm_graph *g, int cta_min, int long_min, cudaStream_t st);
-int rank_launch(gpm_graph *g, cudaStream_t st, unsigned long long *d_out);
+int rank_launch(gpm_graph *g, cudaStream_t st, unsigned long long *d_out, int *cursors = nullptr);
 // out[0..5]: segments, keys streamed from the key segments, owner-list keys,
 // owner tasks, dense segments, bitmap words ANDed for them (fixed plan)
 int rank_plan_stats(gpm_graph *g, uint64_t *out);
@@ -184,8 +184,9 @@ int rank_plan_stats(gpm_graph *g, uint64_t *out);
 // ({16, 64, 256}[cfg % 3]) instead of the fixed thresholds.
 int rank_plan_new(gpm_graph *g, int cta_min, int long_min, const uint8_t *cfg, cudaStream_t st, RankPlan **out);
 // rec != nullptr: instrumented run adding each owner's cost (active warp-cycles)
-// to rec[owner]; rec must be zeroed first
+// to rec[owner]; rec must be zeroed first.  cursors: as tc_launch takes them
+// (tc.cuh)
 int rank_plan_launch(gpm_graph *g, RankPlan *p, cudaStream_t st, unsigned long long *d_out,
-                     unsigned long long *rec);
+                     unsigned long long *rec, int *cursors = nullptr);
 
 }  // namespace gpm
