@@ -1025,13 +1025,12 @@ int clique_plan_run(CliquePlan *p, cudaStream_t st, bool zero) {
           p->k, p->roff, p->radj, p->ctasks.p + p->n_big, nsmall, p->cursors + 1, p->small_slabs.p, p->small_slab,
           core, p->gid, p->acc, p->stride, p->slot);
   });
-  GPM_LAUNCH_CHECK();
   if (bst != st) GPM_CUDA(cudaEventRecord(p->join, bst));
   if (p->n_warp > 0)
     k_clique_warp<<<std::min(grids.warp, (p->n_warp + 7) / 8), 256, 0, st>>>(
         p->k, p->roff, p->radj, p->wtasks.p, p->n_warp, p->cursors + 2, p->gid, p->acc, p->stride, p->slot);
+  if (bst != st) GPM_CUDA(cudaStreamWaitEvent(st, p->join, 0));  // joined whether or not the launches were accepted
   GPM_LAUNCH_CHECK();
-  if (bst != st) GPM_CUDA(cudaStreamWaitEvent(st, p->join, 0));
   return GPM_OK;
 }
 

@@ -55,8 +55,10 @@ struct CliquePlan {
   CliquePlan() = default;
   CliquePlan(const CliquePlan &) = delete;
   CliquePlan &operator=(const CliquePlan &) = delete;
+  // Nothing is waited for: the side stream's work is joined into the caller's
+  // stream (and waiting for an event that was last recorded inside a capture
+  // is an error)
   ~CliquePlan() {
-    if (join) cudaEventSynchronize(join);
     if (side) cudaStreamDestroy(side);
     if (fork) cudaEventDestroy(fork);
     if (join) cudaEventDestroy(join);

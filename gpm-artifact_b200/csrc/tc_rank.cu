@@ -1451,7 +1451,6 @@ int rank_plan_launch(gpm_graph *g, RankPlan *p, cudaStream_t st, unsigned long l
                                                              p->dense_tasks.p, p->n_dense,
                                                              reinterpret_cast<const uint4 *>(p->rows.p),
                                                              cursors + 2, d_out);
-    GPM_LAUNCH_CHECK();
     GPM_CUDA(cudaEventRecord(p->join, side));
   }
   if (rec)
@@ -1462,8 +1461,8 @@ int rank_plan_launch(gpm_graph *g, RankPlan *p, cudaStream_t st, unsigned long l
     k_tc_rank<<<rank_grid(), 256, kRankSmem, st>>>(g->rg->roff.p, g->rg->radj.p, g->rg->radj4.p, p->poff.p,
                                                    p->pseg.p, p->plong.p, p->pshort.p, p->cta_tasks.p, p->n_cta,
                                                    p->warp_tasks.p, p->n_warp, cursors, d_out, nullptr);
+  if (p->n_dense) GPM_CUDA(cudaStreamWaitEvent(st, p->join, 0));  // joined whether or not the launches were accepted
   GPM_LAUNCH_CHECK();
-  if (p->n_dense) GPM_CUDA(cudaStreamWaitEvent(st, p->join, 0));
   return GPM_OK;
 }
 

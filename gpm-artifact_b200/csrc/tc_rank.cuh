@@ -152,8 +152,8 @@ struct RankPlan {
   RankPlan() = default;
   RankPlan(const RankPlan &) = delete;
   RankPlan &operator=(const RankPlan &) = delete;
+  // nothing is waited for, as in ~CliquePlan (motif.cuh)
   ~RankPlan() {
-    if (join) cudaEventSynchronize(join);  // the side stream's last use of the buffers
     if (fork) cudaEventDestroy(fork);
     if (join) cudaEventDestroy(join);
   }
