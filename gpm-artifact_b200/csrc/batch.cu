@@ -64,6 +64,7 @@ static void drop_graph(gpm_batch *b) {
 }
 
 static void drop_plan(gpm_batch *b) {
+  DirectFree direct(b->g.foreign);
   drop_graph(b);
   delete b->plan;
   b->plan = nullptr;
@@ -313,6 +314,7 @@ int gpm_batch_stage_ms(gpm_batch *b, float *ms) {
 int gpm_batch_motif_async(gpm_batch *b, int use_graph, void *stream, uint64_t *d_out) {
   if (!b || !d_out) return fail(GPM_EINVAL, "gpm_batch_motif_async: NULL argument");
   cudaStream_t st = (cudaStream_t)stream;
+  b->g.foreign = b->g.foreign || foreign_stream(st);
   if (use_graph) {
     if (!b->exec) return fail(GPM_EINVAL, "call gpm_batch_motif once first (it captures the graph)");
     GPM_CUDA(cudaGraphLaunch(b->exec, st));
@@ -327,6 +329,7 @@ int gpm_batch_motif_async(gpm_batch *b, int use_graph, void *stream, uint64_t *d
 int gpm_batch_motif(gpm_batch *b, int use_graph, void *stream, uint64_t *out) {
   if (!b || !out) return fail(GPM_EINVAL, "gpm_batch_motif: NULL argument");
   cudaStream_t st = (cudaStream_t)stream;
+  b->g.foreign = b->g.foreign || foreign_stream(st);
   GPM_TRY(ensure_plan(b));
   if (use_graph) {
     GPM_TRY(ensure_graph(b));
@@ -340,6 +343,7 @@ int gpm_batch_motif(gpm_batch *b, int use_graph, void *stream, uint64_t *out) {
 }
 
 int gpm_batch_destroy(gpm_batch *b) {
+  DirectFree direct(b && b->g.foreign);
   delete b;
   return GPM_OK;
 }

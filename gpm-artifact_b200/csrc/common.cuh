@@ -56,9 +56,12 @@ struct ArenaScope {
   Arena *prev;
 };
 
-// Every other allocation comes from a process-wide pool of freed blocks, per
-// device.  Freeing waits for the device, as cudaFree does, so a block in the
-// pool is idle and may go to any thread and stream; at most kPoolBytes are
+// Every other allocation comes from a process-wide pool of idle blocks, per
+// device.  A block enters it only when no work can use it any more: the
+// library's own calls run on the legacy default stream, which is waited for
+// first; what a caller's stream, or a graph a caller has captured, may still use
+// is released inside a DirectFree scope and goes back to the driver at once.
+// So a block in the pool may go to any thread and stream.  At most kPoolBytes are
 // kept per device, the longest idle make room for newer ones, and all are given
 // back when an allocation fails or plans are dropped.  (A first
 // triangle count on R-MAT 22 made 56 cudaMalloc and 37 cudaFree calls: 27 of
@@ -66,6 +69,14 @@ struct ArenaScope {
 void *pool_get(size_t bytes, size_t *cap, int *dev);  // nullptr: out of memory (cudaGetLastError not cleared)
 void pool_put(void *p, size_t cap, int dev);
 void pool_trim();  // the current device's cached blocks back to the driver
+// While one with `on` is alive on a thread, the thread's releases bypass the pool.
+struct DirectFree {
+  explicit DirectFree(bool on);
+  ~DirectFree();
+  bool on;
+};
+// May work on st still run when the legacy default stream has been waited for?
+inline bool foreign_stream(cudaStream_t st) { return st != nullptr && st != cudaStreamLegacy; }
 
 // Owning device allocation; move-only.
 template <typename T>
@@ -245,6 +256,7 @@ struct gpm_graph {
   int oriented = 0;
   int relabeled = 0;
   int device = 0;
+  bool foreign = false;  // launched on a caller's stream: its memory is released directly (DirectFree)
   gpm::DevBuf<int64_t> off;     // n + 1
   gpm::DevBuf<int32_t> adj;     // nnz
   gpm::DevBuf<int32_t> labels;  // n (optional)

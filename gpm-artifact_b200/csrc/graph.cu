@@ -416,6 +416,7 @@ using namespace gpm;
 
 namespace gpm {
 void drop_plans(gpm_graph *g) {
+  DirectFree direct(g->foreign);
   g->hash_us = 0;
   free_tc_plan(g->tc);
   g->tc = nullptr;
@@ -571,6 +572,7 @@ int gpm_graph_generate(int kind, int64_t p0, int64_t p1, double a, double b, dou
 }
 
 int gpm_graph_destroy(gpm_graph *g) {
+  DirectFree direct(g && g->foreign);
   delete g;
   return GPM_OK;
 }
@@ -595,6 +597,7 @@ int gpm_graph_copy_csr(const gpm_graph *g, int64_t *offsets, int32_t *indices) {
 
 int gpm_graph_set_labels(gpm_graph *g, const int32_t *labels) {
   if (!g || !labels) return fail(GPM_EINVAL, "NULL argument");
+  DirectFree direct(g->foreign);
   GPM_TRY(g->labels.reserve(g->n));
   if (g->n > 0) GPM_CUDA(cudaMemcpy(g->labels.p, labels, sizeof(int32_t) * g->n, cudaMemcpyHostToDevice));
   free_label_csr(g->lcsr);  // the label partition follows the labels
@@ -604,6 +607,7 @@ int gpm_graph_set_labels(gpm_graph *g, const int32_t *labels) {
 
 int gpm_graph_orient(gpm_graph *g, int relabel) {
   if (!g) return fail(GPM_EINVAL, "NULL graph");
+  DirectFree direct(g->foreign);
   drop_plans(g);
   GPM_TRY(orient_on_stream(g, 0));
   if (relabel) GPM_TRY(relabel_device(g, 0));
@@ -614,6 +618,7 @@ int gpm_graph_orient(gpm_graph *g, int relabel) {
 
 int gpm_graph_relabel(gpm_graph *g) {
   if (!g) return fail(GPM_EINVAL, "NULL graph");
+  DirectFree direct(g->foreign);
   drop_plans(g);
   GPM_TRY(relabel_device(g, 0));
   GPM_TRY(compute_max_degree(g, 0));

@@ -17,6 +17,7 @@
 #include <limits>
 #include <map>
 #include <mutex>
+#include <new>
 #include <sstream>
 #include <string>
 #include <vector>
@@ -114,14 +115,13 @@ static size_t pool_size(size_t bytes) {
 
 static void pool_trim_device(int dev) {
   BlockPool &P = block_pool();
-  std::vector<void *> gone;
+  std::multimap<size_t, BlockPool::Idle> gone;
   {
     std::lock_guard<std::mutex> lock(P.mu);
-    for (auto &b : P.blocks[dev]) gone.push_back(b.second.p);
-    P.blocks[dev].clear();
+    gone.swap(P.blocks[dev]);
     P.bytes[dev] = 0;
   }
-  for (void *p : gone) cudaFree(p);
+  for (auto &b : gone) cudaFree(b.second.p);
 }
 
 void pool_trim() {
@@ -156,42 +156,59 @@ void *pool_get(size_t bytes, size_t *cap, int *dev) {
   return cudaMalloc(&p, want) == cudaSuccess ? p : nullptr;
 }
 
-// Waits for the work in flight on the current device the way cudaFree does: a
-// cudaDeviceSynchronize would fail, and end the capture, while any thread
-// captures a stream of the device.
+static thread_local int tl_direct = 0;
+DirectFree::DirectFree(bool o) : on(o) { tl_direct += on; }
+DirectFree::~DirectFree() { tl_direct -= on; }
+
+// Waits for the library's own work: it runs on the legacy default stream, side
+// streams are joined into that.  (Not for the device: cudaDeviceSynchronize
+// fails, and ends the capture, while any thread captures a stream.)
 static bool pool_quiesce() {
-  void *p = nullptr;
-  if (cudaMalloc(&p, 256) == cudaSuccess) return cudaFree(p) == cudaSuccess;
+  if (cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess) return true;
   cudaGetLastError();
   return false;
 }
 
-void pool_put(void *p, size_t cap, int dev) {
+// The longest idle block taken out, until `cap` more bytes fit; nullptr: they do.
+static void *pool_evict(BlockPool &P, int dev, size_t cap) {
+  auto &blocks = P.blocks[dev];
+  if (P.bytes[dev] + cap <= BlockPool::kPoolBytes || blocks.empty()) return nullptr;
+  auto old = blocks.begin();
+  for (auto it = blocks.begin(); it != blocks.end(); ++it)
+    if (it->second.since < old->second.since) old = it;
+  void *p = old->second.p;
+  P.bytes[dev] -= old->first;
+  blocks.erase(old);
+  return p;
+}
+
+// false: the block is not kept (called by destructors, so nothing is thrown)
+static bool pool_keep(void *p, size_t cap, int dev) {
   BlockPool &P = block_pool();
   int cur = -1;
-  if (dev >= 0 && dev < BlockPool::kDevices && cudaGetDevice(&cur) == cudaSuccess && cur == dev && pool_quiesce()) {
-    std::vector<void *> gone;
+  if (tl_direct || dev < 0 || dev >= BlockPool::kDevices || cap > BlockPool::kPoolBytes) return false;
+  if (cudaGetDevice(&cur) != cudaSuccess || cur != dev || !pool_quiesce()) return false;
+  while (true) {
+    void *gone = nullptr;
     {
       std::lock_guard<std::mutex> lock(P.mu);
-      auto &blocks = P.blocks[dev];
-      if (cap <= BlockPool::kPoolBytes) {
-        // the longest idle make room: what earlier work left may fit nothing any more
-        while (P.bytes[dev] + cap > BlockPool::kPoolBytes) {
-          auto old = blocks.begin();
-          for (auto it = blocks.begin(); it != blocks.end(); ++it)
-            if (it->second.since < old->second.since) old = it;
-          P.bytes[dev] -= old->first;
-          gone.push_back(old->second.p);
-          blocks.erase(old);
+      gone = pool_evict(P, dev, cap);
+      if (!gone) {
+        try {
+          P.blocks[dev].emplace(cap, BlockPool::Idle{p, P.clock++});
+        } catch (const std::bad_alloc &) {
+          return false;
         }
-        blocks.emplace(cap, BlockPool::Idle{p, P.clock++});
         P.bytes[dev] += cap;
-        p = nullptr;
+        return true;
       }
     }
-    for (void *q : gone) cudaFree(q);
+    cudaFree(gone);
   }
-  if (p) cudaFree(p);
+}
+
+void pool_put(void *p, size_t cap, int dev) {
+  if (!pool_keep(p, cap, dev)) cudaFree(p);
 }
 
 int ensure_device() {

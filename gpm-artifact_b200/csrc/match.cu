@@ -1375,6 +1375,7 @@ struct gpm_match_batch {
   int nq = 0, nm = 1;
   int qcap = 16;  // plan width of the launch: 16, or 64 when a query has more than 16 vertices
   bool weighted = false;  // some plan is factored (plan width 16 only)
+  bool foreign = false;   // as gpm_graph's
   std::vector<gpm::WidePlan> plans;
   // 4-cycle queries (their index) and the scratch they take one after another
   std::vector<std::pair<int, gpm::CyclePlan>> cycles;
@@ -1784,6 +1785,7 @@ int gpm_match_batch_create(gpm_graph *g, int nq, const gpm_query *const *queries
 
 int gpm_match_batch_autotune(gpm_match_batch *b, int64_t *span) {
   if (!b) return fail(GPM_EINVAL, "NULL batch");
+  DirectFree direct(b->foreign);
   static const int64_t cand[] = {0, 16384, 2048, 256};
   cudaEvent_t e0, e1;
   GPM_CUDA(cudaEventCreate(&e0));
@@ -1814,6 +1816,7 @@ int gpm_match_batch_autotune(gpm_match_batch *b, int64_t *span) {
 int gpm_match_batch_run_async(gpm_match_batch *b, int use_graph, void *stream, uint64_t *d_out) {
   if (!b || !d_out) return fail(GPM_EINVAL, "gpm_match_batch_run_async: NULL argument");
   cudaStream_t st = (cudaStream_t)stream;
+  if (foreign_stream(st)) b->foreign = b->g->foreign = true;
   GPM_TRY(batch_run(b, use_graph, st));
   GPM_CUDA(cudaMemcpyAsync(d_out, b->out.p, sizeof(unsigned long long) * b->nq * b->nm, cudaMemcpyDeviceToDevice, st));
   return GPM_OK;
@@ -1822,6 +1825,7 @@ int gpm_match_batch_run_async(gpm_match_batch *b, int use_graph, void *stream, u
 int gpm_match_batch_run(gpm_match_batch *b, int use_graph, void *stream, uint64_t *out) {
   if (!b || !out) return fail(GPM_EINVAL, "gpm_match_batch_run: NULL argument");
   cudaStream_t st = (cudaStream_t)stream;
+  if (foreign_stream(st)) b->foreign = b->g->foreign = true;
   GPM_TRY(batch_run(b, use_graph, st));
   GPM_CUDA(cudaMemcpyAsync(out, b->out.p, sizeof(unsigned long long) * b->nq * b->nm, cudaMemcpyDeviceToHost, st));
   GPM_CUDA(cudaStreamSynchronize(st));
@@ -1836,6 +1840,7 @@ int gpm_match_batch_info(const gpm_match_batch *b, int64_t *tasks, int64_t *span
 }
 
 int gpm_match_batch_destroy(gpm_match_batch *b) {
+  DirectFree direct(b && b->foreign);
   delete b;
   return GPM_OK;
 }

@@ -545,6 +545,7 @@ int gpm_sched_train(gpm_sched *s, int steps, float lr, double *final_loss) {
 int gpm_sched_attach(gpm_graph *g, gpm_sched *s) {
   if (!g) return fail(GPM_EINVAL, "NULL graph");
   if (s && !sched_live(s)) return fail(GPM_EINVAL, "gpm_sched_attach: not a live scheduler");
+  DirectFree direct(g->foreign);
   free_rank_plan(g->learned);
   g->learned = nullptr;
   g->sched = s;
@@ -603,6 +604,7 @@ int gpm_tc_set_schedule(gpm_graph *g, const uint8_t *cfg) {
   if (g->n) GPM_CUDA(cudaMemcpy(d.p, cfg, g->n, cudaMemcpyHostToDevice));
   RankPlan *p = nullptr;
   GPM_TRY(rank_plan_new(g, kRankCtaMin, kRankLongMin, d.p, 0, &p));
+  DirectFree direct(g->foreign);
   free_rank_plan(g->learned);
   g->learned = p;
   return GPM_OK;

@@ -560,6 +560,8 @@ extern "C" {
 
 int gpm_tc_async(gpm_graph *g, int variant, void *stream, uint64_t *d_out) {
   if (!g || !d_out) return fail(GPM_EINVAL, "gpm_tc_async: NULL argument");
+  g->foreign = g->foreign || foreign_stream((cudaStream_t)stream);
+  DirectFree direct(g->foreign);
   if (variant == GPM_TC_AUTO) {
     int s = GPM_OK;
     if (small_launch(g, (cudaStream_t)stream, (unsigned long long *)d_out, nullptr, &s)) return s;
