@@ -106,11 +106,12 @@ static BlockPool &block_pool() {
   return *p;
 }
 // sizes are rounded up by at most an eighth, so that blocks of nearly equal
-// requests serve one another
+// requests serve one another; blocks too large to be kept are not
 static size_t pool_size(size_t bytes) {
   size_t step = 512;
   while (step * 16 <= bytes) step *= 2;
-  return (bytes + step - 1) / step * step;
+  const size_t up = (bytes + step - 1) / step * step;
+  return up <= BlockPool::kPoolBytes ? up : bytes;
 }
 
 static void pool_trim_device(int dev) {
@@ -153,7 +154,11 @@ void *pool_get(size_t bytes, size_t *cap, int *dev) {
   if (!pooled) return nullptr;
   cudaGetLastError();
   pool_trim_device(*dev);
-  return cudaMalloc(&p, want) == cudaSuccess ? p : nullptr;
+  if (cudaMalloc(&p, want) == cudaSuccess) return p;
+  if (want == bytes) return nullptr;
+  cudaGetLastError();
+  *cap = bytes;  // the last of the memory: as asked for
+  return cudaMalloc(&p, bytes) == cudaSuccess ? p : nullptr;
 }
 
 static thread_local int tl_direct = 0;

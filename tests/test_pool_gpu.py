@@ -84,6 +84,27 @@ def test_bound():
     assert start - _free() < 64 * MIB
 
 
+@pytest.mark.parametrize("mib", [3100, 4400])
+def test_the_last_of_the_memory(mib):
+    """A buffer that fits, but not rounded up to a size of the pool's."""
+    import torch
+    g = gpm.Graph.from_edges(3, [0, 1], [1, 2], labels=[0, 0, 0])
+    q = gpm.Query(2, [0], [1], [0, 0])
+    assert g.match(q) == 4  # the label partition is there
+    buf = torch.empty(mib * MIB // 4, dtype=torch.int32)
+    _empty_pool()
+    torch.cuda.synchronize()
+    held = torch.empty(_free() - (mib + 64) * MIB, dtype=torch.uint8, device="cuda")
+    written = gpm.c_uint64()
+    try:
+        assert mib * MIB < _free() < (mib + 130) * MIB
+        gpm.check(gpm.lib.gpm_match_list(g.h, q.h, mib * MIB // 8, gpm.c_void_p(buf.data_ptr()), written))
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    assert written.value == 4
+
+
 def test_threads_and_streams():
     """Graphs built, counted on a stream of the thread's own, and closed, in
     several threads at once."""
