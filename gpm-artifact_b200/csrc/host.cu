@@ -270,6 +270,12 @@ int gpm_device_count(int *count) {
   return GPM_OK;
 }
 
+int gpm_trim(void) {
+  GPM_TRY(ensure_device());
+  pool_trim();
+  return GPM_OK;
+}
+
 // ------------------------------------------------------------------ readers
 // .mtx as the reference loader reads it (Loader::_load_mtx, io.h:84-139):
 // skip lines until one starts with a digit; three header integers; then a

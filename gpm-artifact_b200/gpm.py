@@ -43,6 +43,7 @@ _SIGS = {
     "gpm_last_error": ([], c_char_p),
     "gpm_abi_version": ([], c_int),
     "gpm_device_count": ([POINTER(c_int)], c_int),
+    "gpm_trim": ([], c_int),
     "gpm_read_mtx": ([c_char_p, POINTER(c_int64), POINTER(c_int64), _P, _P, c_int64, POINTER(c_int32)], c_int),
     "gpm_read_labels": ([c_char_p, c_int64, c_int32, _P], c_int),
     "gpm_read_tve": ([c_char_p, POINTER(c_int64), POINTER(c_int64), _P, _P, _P, c_int64], c_int),
@@ -139,6 +140,11 @@ def device_count() -> int:
     n = c_int(0)
     check(lib.gpm_device_count(ctypes.byref(n)))
     return n.value
+
+
+def trim() -> None:
+    """Gives the device memory kept idle for later calls back to the driver."""
+    check(lib.gpm_trim())
 
 
 # ---------------------------------------------------------------- host helpers

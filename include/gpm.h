@@ -85,6 +85,11 @@ const char *gpm_last_error(void);
 int gpm_abi_version(void);
 /* Number of visible CUDA devices (0 when none). */
 int gpm_device_count(int *count);
+/* Device memory that closed handles and finished calls leave idle is kept for
+ * later calls, at most 4 GiB per device.  gpm_trim gives the current device's
+ * back to the driver, for other users of the device; the engine does so by
+ * itself when an allocation of its own fails, and in gpm_graph_drop_plans. */
+int gpm_trim(void);
 
 /* ---- file formats (host only, no device needed) ------------------------- */
 /* Loader::_load_mtx, src/graph/io.h:84-139: skip lines until one starts with

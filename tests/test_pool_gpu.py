@@ -84,6 +84,21 @@ def test_bound():
     assert start - _free() < 64 * MIB
 
 
+def test_trim_without_a_handle():
+    import torch
+    gpm.trim()
+    torch.cuda.synchronize()
+    start = _free()
+    g = gpm.Graph.rmat(17, 16, seed=1).orient()
+    want = g.tc()
+    g.close()
+    assert start - _free() > 64 * MIB  # kept for the next graph
+    gpm.trim()
+    assert start - _free() < 32 * MIB
+    g = gpm.Graph.rmat(17, 16, seed=1).orient()
+    assert g.tc() == want
+
+
 @pytest.mark.parametrize("mib", [3100, 4400])
 def test_the_last_of_the_memory(mib):
     """A buffer that fits, but not rounded up to a size of the pool's."""
