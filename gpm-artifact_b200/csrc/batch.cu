@@ -33,6 +33,7 @@ struct gpm_batch {
   cudaStream_t cap = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
+  gpm::LaunchOrder order;  // the 4-cycle stage keeps positions in the lists (motif.cu)
   ~gpm_batch();
 };
 
@@ -125,6 +126,20 @@ static int ensure_graph(gpm_batch *b) {
   b->graph = graph;
   GPM_CUDA(cudaGraphInstantiate(&b->exec, b->graph, 0));
   return GPM_OK;
+}
+
+// One run of the pipeline on st and its counts to `out`, behind every earlier
+// run of the batch.
+static int run_ordered(gpm_batch *b, int use_graph, cudaStream_t st, uint64_t *out, cudaMemcpyKind kind) {
+  GPM_TRY(b->order.begin(st));
+  auto run = [&]() -> int {
+    if (use_graph) GPM_CUDA(cudaGraphLaunch(b->exec, st));
+    else GPM_TRY(motif_plan_run(b->plan, st));
+    GPM_CUDA(cudaMemcpyAsync(out, b->plan->out.p, sizeof(uint64_t) * 8 * b->ngraphs, kind, st));
+    return GPM_OK;
+  };
+  const int s = run(), e = b->order.end(st);
+  return s != GPM_OK ? s : e;
 }
 
 }  // namespace gpm
@@ -259,6 +274,7 @@ int gpm_batch_member_csr(const gpm_batch *b, int g, int64_t *offsets, int32_t *i
 
 int gpm_batch_autotune(gpm_batch *b, int *tuned) {
   if (!b) return fail(GPM_EINVAL, "NULL batch");
+  GPM_TRY(b->order.begin(0));
   static const int cand[3][4] = {{32, 64, 128, 128}, {64, 128, 256, 256}, {16, 32, 64, 64}};
   cudaEvent_t e0, e1;
   GPM_CUDA(cudaEventCreate(&e0));
@@ -295,6 +311,7 @@ int gpm_batch_autotune(gpm_batch *b, int *tuned) {
 
 int gpm_batch_stage_ms(gpm_batch *b, float *ms) {
   if (!b || !ms) return fail(GPM_EINVAL, "NULL argument");
+  GPM_TRY(b->order.begin(0));
   GPM_TRY(ensure_plan(b));
   cudaEvent_t e0, e1;
   GPM_CUDA(cudaEventCreate(&e0));
@@ -315,15 +332,9 @@ int gpm_batch_motif_async(gpm_batch *b, int use_graph, void *stream, uint64_t *d
   if (!b || !d_out) return fail(GPM_EINVAL, "gpm_batch_motif_async: NULL argument");
   cudaStream_t st = (cudaStream_t)stream;
   b->g.foreign = b->g.foreign || foreign_stream(st);
-  if (use_graph) {
-    if (!b->exec) return fail(GPM_EINVAL, "call gpm_batch_motif once first (it captures the graph)");
-    GPM_CUDA(cudaGraphLaunch(b->exec, st));
-  } else {
-    if (!b->plan) return fail(GPM_EINVAL, "call gpm_batch_motif once first (it builds the plan)");
-    GPM_TRY(motif_plan_run(b->plan, st));
-  }
-  GPM_CUDA(cudaMemcpyAsync(d_out, b->plan->out.p, sizeof(uint64_t) * 8 * b->ngraphs, cudaMemcpyDeviceToDevice, st));
-  return GPM_OK;
+  if (use_graph && !b->exec) return fail(GPM_EINVAL, "call gpm_batch_motif once first (it captures the graph)");
+  if (!b->plan) return fail(GPM_EINVAL, "call gpm_batch_motif once first (it builds the plan)");
+  return run_ordered(b, use_graph, st, d_out, cudaMemcpyDeviceToDevice);
 }
 
 int gpm_batch_motif(gpm_batch *b, int use_graph, void *stream, uint64_t *out) {
@@ -331,13 +342,8 @@ int gpm_batch_motif(gpm_batch *b, int use_graph, void *stream, uint64_t *out) {
   cudaStream_t st = (cudaStream_t)stream;
   b->g.foreign = b->g.foreign || foreign_stream(st);
   GPM_TRY(ensure_plan(b));
-  if (use_graph) {
-    GPM_TRY(ensure_graph(b));
-    GPM_CUDA(cudaGraphLaunch(b->exec, st));
-  } else {
-    GPM_TRY(motif_plan_run(b->plan, st));
-  }
-  GPM_CUDA(cudaMemcpyAsync(out, b->plan->out.p, sizeof(uint64_t) * 8 * b->ngraphs, cudaMemcpyDeviceToHost, st));
+  if (use_graph) GPM_TRY(ensure_graph(b));
+  GPM_TRY(run_ordered(b, use_graph, st, out, cudaMemcpyDeviceToHost));
   GPM_CUDA(cudaStreamSynchronize(st));
   return GPM_OK;
 }

@@ -138,6 +138,30 @@ struct DevBuf {
   }
 };
 
+// Orders the launches of one handle over all streams: scratch of its plan holds
+// positions and counters that two of them must not share.  A launch inside a
+// capture cannot wait for one outside of it and stays out of the order.
+bool stream_capturing(cudaStream_t st);
+struct LaunchOrder {
+  cudaEvent_t last = nullptr;  // behind the latest launch
+  LaunchOrder() = default;
+  LaunchOrder(const LaunchOrder &) = delete;
+  LaunchOrder &operator=(const LaunchOrder &) = delete;
+  ~LaunchOrder() {
+    if (last) cudaEventDestroy(last);
+  }
+  int begin(cudaStream_t st) {
+    if (last && !stream_capturing(st)) GPM_CUDA(cudaStreamWaitEvent(st, last, 0));
+    return GPM_OK;
+  }
+  int end(cudaStream_t st) {
+    if (stream_capturing(st)) return GPM_OK;
+    if (!last) GPM_CUDA(cudaEventCreateWithFlags(&last, cudaEventDisableTiming));
+    GPM_CUDA(cudaEventRecord(last, st));
+    return GPM_OK;
+  }
+};
+
 // ---------------------------------------------------------------- RNG
 // splitmix64 finaliser: a counter-based generator, so edge i of a seeded
 // graph is the same whichever thread (host or device) draws it.
@@ -280,7 +304,6 @@ int build_csr_device(gpm_graph *g, int64_t n, int64_t m, const int32_t *d_src,
                      const int32_t *d_dst, int symmetrize, cudaStream_t st);
 int ensure_src(gpm_graph *g, cudaStream_t st);
 bool src_ready(const gpm_graph *g);  // would ensure_src launch nothing?
-bool stream_capturing(cudaStream_t st);
 int compute_max_degree(gpm_graph *g, cudaStream_t st);
 void free_tc_plan(TcPlan *p);
 void free_rank_plan(RankPlan *p);

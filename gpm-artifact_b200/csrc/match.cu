@@ -1376,6 +1376,7 @@ struct gpm_match_batch {
   int qcap = 16;  // plan width of the launch: 16, or 64 when a query has more than 16 vertices
   bool weighted = false;  // some plan is factored (plan width 16 only)
   bool foreign = false;   // as gpm_graph's
+  gpm::LaunchOrder order;  // the 4-cycle counters are zero between launches (match_cycle.cu)
   std::vector<gpm::WidePlan> plans;
   // 4-cycle queries (their index) and the scratch they take one after another
   std::vector<std::pair<int, gpm::CyclePlan>> cycles;
@@ -1649,6 +1650,18 @@ static int batch_run(gpm_match_batch *b, int use_graph, cudaStream_t st) {
   return GPM_OK;
 }
 
+// One run on st and its counts to `out`, behind every earlier run of the batch.
+static int batch_run_ordered(gpm_match_batch *b, int use_graph, cudaStream_t st, uint64_t *out, cudaMemcpyKind kind) {
+  GPM_TRY(b->order.begin(st));
+  auto run = [&]() -> int {
+    GPM_TRY(batch_run(b, use_graph, st));
+    GPM_CUDA(cudaMemcpyAsync(out, b->out.p, sizeof(unsigned long long) * b->nq * b->nm, kind, st));
+    return GPM_OK;
+  };
+  const int s = run(), e = b->order.end(st);
+  return s != GPM_OK ? s : e;
+}
+
 }  // namespace gpm
 
 extern "C" {
@@ -1786,6 +1799,7 @@ int gpm_match_batch_create(gpm_graph *g, int nq, const gpm_query *const *queries
 int gpm_match_batch_autotune(gpm_match_batch *b, int64_t *span) {
   if (!b) return fail(GPM_EINVAL, "NULL batch");
   DirectFree direct(b->foreign);
+  GPM_TRY(b->order.begin(0));
   static const int64_t cand[] = {0, 16384, 2048, 256};
   cudaEvent_t e0, e1;
   GPM_CUDA(cudaEventCreate(&e0));
@@ -1817,17 +1831,14 @@ int gpm_match_batch_run_async(gpm_match_batch *b, int use_graph, void *stream, u
   if (!b || !d_out) return fail(GPM_EINVAL, "gpm_match_batch_run_async: NULL argument");
   cudaStream_t st = (cudaStream_t)stream;
   if (foreign_stream(st)) b->foreign = b->g->foreign = true;
-  GPM_TRY(batch_run(b, use_graph, st));
-  GPM_CUDA(cudaMemcpyAsync(d_out, b->out.p, sizeof(unsigned long long) * b->nq * b->nm, cudaMemcpyDeviceToDevice, st));
-  return GPM_OK;
+  return batch_run_ordered(b, use_graph, st, d_out, cudaMemcpyDeviceToDevice);
 }
 
 int gpm_match_batch_run(gpm_match_batch *b, int use_graph, void *stream, uint64_t *out) {
   if (!b || !out) return fail(GPM_EINVAL, "gpm_match_batch_run: NULL argument");
   cudaStream_t st = (cudaStream_t)stream;
   if (foreign_stream(st)) b->foreign = b->g->foreign = true;
-  GPM_TRY(batch_run(b, use_graph, st));
-  GPM_CUDA(cudaMemcpyAsync(out, b->out.p, sizeof(unsigned long long) * b->nq * b->nm, cudaMemcpyDeviceToHost, st));
+  GPM_TRY(batch_run_ordered(b, use_graph, st, out, cudaMemcpyDeviceToHost));
   GPM_CUDA(cudaStreamSynchronize(st));
   return GPM_OK;
 }

@@ -325,7 +325,10 @@ int gpm_batch_stage_ms(gpm_batch *b, float *ms);
  * call and replays it afterwards. */
 int gpm_batch_motif(gpm_batch *b, int use_graph, void *stream, uint64_t *out);
 /* The same into device memory d_out (8 * ngraphs uint64) without host
- * synchronisation; needs one gpm_batch_motif call before. */
+ * synchronisation; needs one gpm_batch_motif call before.  Runs of one batch on
+ * several streams follow one another.  A run recorded into a caller's own
+ * capture cannot be ordered so: its replays must not overlap other runs of the
+ * batch. */
 int gpm_batch_motif_async(gpm_batch *b, int use_graph, void *stream, uint64_t *d_out);
 int gpm_batch_destroy(gpm_batch *b);
 
@@ -372,7 +375,8 @@ int gpm_match_batch_autotune(gpm_match_batch *b, int64_t *span);
  * without member ids).  use_graph != 0 captures the launch into a CUDA graph
  * on the first call and replays it afterwards. */
 int gpm_match_batch_run(gpm_match_batch *b, int use_graph, void *stream, uint64_t *out);
-/* The same into device memory d_out without host synchronisation. */
+/* The same into device memory d_out without host synchronisation; ordered as
+ * gpm_batch_motif_async. */
 int gpm_match_batch_run_async(gpm_match_batch *b, int use_graph, void *stream, uint64_t *d_out);
 /* Tasks in the launch and the current split span. */
 int gpm_match_batch_info(const gpm_match_batch *b, int64_t *tasks, int64_t *span);
