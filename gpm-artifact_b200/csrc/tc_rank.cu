@@ -544,9 +544,8 @@ __device__ __forceinline__ int64_t upper_bound_key(const int32_t *__restrict__ a
 // (start, len) and the smallest and largest key of it, its first 16-byte row
 // in radj4, and its core bitmap row (-1: none).
 struct __align__(32) VertexInfo {
-  uint32_t start;
-  int32_t len, kmin, kmax, row4, rowid;
-  int32_t pad[2];
+  int64_t start;
+  int32_t len, kmin, kmax, row4, rowid, pad;
 };
 __global__ void k_vertex_info(int64_t n, const int64_t *__restrict__ roff, const int32_t *__restrict__ radj,
                               const int64_t *__restrict__ roff4, const int32_t *__restrict__ rowid,
@@ -554,13 +553,13 @@ __global__ void k_vertex_info(int64_t n, const int64_t *__restrict__ roff, const
   for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
     const int64_t s = roff[v], e = roff[v + 1];
     VertexInfo f;
-    f.start = (uint32_t)s;
+    f.start = s;
     f.len = (int32_t)(e - s);
     f.kmin = e > s ? radj[s] : 0;
     f.kmax = e > s ? radj[e - 1] : 0;
     f.row4 = (int32_t)(roff4[v] >> 2);
     f.rowid = rowid ? rowid[v] : -1;
-    f.pad[0] = f.pad[1] = 0;
+    f.pad = 0;
     info[v] = f;
   }
 }
@@ -573,7 +572,8 @@ __global__ void k_vertex_info(int64_t n, const int64_t *__restrict__ roff, const
 // [poff[x], poff[x+1]) -- one slot per incident edge, so it always fits --
 // long segments from the front (cursor lcnt[x]), short ones from the back
 // (cursor scnt[x]), as ranges of radj4; a cursor's upper half adds up the keys
-// that will be streamed.  With radj4 non-null the pass also copies each list u
+// that will be streamed, in units of 2^work_shift: a list is streamed at most
+// twice for one owner, so 2^work_shift is 1 for fewer than 2^31 stored keys.  With radj4 non-null the pass also copies each list u
 // into it (with its INT32_MAX padding).  upward: every list holds only ids
 // above its vertex, so when u owns the edge, min N(u) <= v < every id of N(v)
 // and the lower search is skipped.
@@ -596,7 +596,7 @@ __global__ void k_partner_place(int64_t n, const int64_t *__restrict__ roff, con
                                 const uint8_t *__restrict__ cfg, const int64_t *__restrict__ poff,
                                 unsigned long long *__restrict__ lcnt, unsigned long long *__restrict__ scnt,
                                 Seg *__restrict__ pseg, int32_t core_base, int row_words, int dense_pct,
-                                int32_t *__restrict__ pdense, int *__restrict__ too_long) {
+                                int32_t *__restrict__ pdense, int *__restrict__ too_long, int work_shift) {
   const unsigned lane = lane_id(), below = (1u << lane) - 1u;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -629,7 +629,7 @@ __global__ void k_partner_place(int64_t n, const int64_t *__restrict__ roff, con
       const VertexInfo U = info[u], V = info[v];
       if (radj4) {
         int32_t *row = radj4 + 4 * (int64_t)U.row4;
-        const int at = (int)(k - (int64_t)U.start);
+        const int at = (int)(k - U.start);
         row[at] = v;
         if (at == U.len - 1)
           for (int i = U.len; i & 3; ++i) row[i] = INT32_MAX;
@@ -653,7 +653,7 @@ __global__ void k_partner_place(int64_t n, const int64_t *__restrict__ roff, con
           if (P.rowid >= 0 && kmin >= core_base &&
               100 * len >= (int64_t)dense_pct * core_and_words(kmin, kmax))
             row = (int64_t)P.rowid * (row_words >> 2) + (((kmin & ~127) - core_base) >> 7);
-          units = row >= 0 ? 0u : (unsigned)len;
+          units = row >= 0 ? 0u : (unsigned)(len >> work_shift);
           lng = row >= 0 || len >= owner_long_min(cfg, owner, long_min);
           const int64_t lo4 = lo - ps;  // the same keys in radj4
           if (len >= (1 << 29)) *too_long = 1;  // no 8-byte descriptor for it
@@ -689,13 +689,13 @@ __global__ void k_partner_place(int64_t n, const int64_t *__restrict__ roff, con
 __global__ void k_place_counts(int64_t n, const unsigned long long *__restrict__ lcnt,
                                const unsigned long long *__restrict__ scnt, int32_t *__restrict__ plong,
                                int32_t *__restrict__ pshort, unsigned long long *__restrict__ work,
-                               unsigned long long *__restrict__ total) {
+                               unsigned long long *__restrict__ total, int work_shift) {
   unsigned long long sum = 0;
   for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
     const unsigned long long l = lcnt[x], s = scnt[x];
     plong[x] = (int32_t)(uint32_t)l;
     pshort[x] = (int32_t)(uint32_t)s;
-    sum += work[x] = (l >> 32) + (s >> 32) + (uint32_t)l + (uint32_t)s;
+    sum += work[x] = (((l >> 32) + (s >> 32)) << work_shift) + (uint32_t)l + (uint32_t)s;
   }
   sum = warp_sum(sum);
   if (lane_id() == 0 && sum) atomicAdd(total, sum);
@@ -1345,7 +1345,6 @@ int rank_plan_new(gpm_graph *g, int cta_min, int long_min, const uint8_t *cfg, c
   cudaMemsetAsync(total.p, 0, sizeof(unsigned long long), st);
   cudaMemsetAsync(lcnt.p, 0, sizeof(unsigned long long) * n, st);
   cudaMemsetAsync(scnt.p, 0, sizeof(unsigned long long) * n, st);
-  if (g->rg->radj.n >= ((size_t)1 << 32)) return bail(fail(GPM_EUNSUPPORTED, "triangle plan: 2^32 keys or more"));
   // 8-byte segment descriptors address radj4 by 16-byte rows in 31 bits
   if ((int64_t)(g->rg->radj4.n / 4) >= ((int64_t)1 << 31))
     return bail(fail(GPM_EUNSUPPORTED, "triangle plan: more than 2^33 padded keys"));
@@ -1364,13 +1363,15 @@ int rank_plan_new(gpm_graph *g, int cta_min, int long_min, const uint8_t *cfg, c
   cudaMemsetAsync(sizes.p, 0, 5 * sizeof(int), st);
   k_vertex_info<<<grid_for(n), 256, 0, st>>>(n, roff, radj, g->rg->roff4.p, p->n_rows ? rowid.p : nullptr, info.p);
   const int64_t keys = (int64_t)g->rg->radj.n;
+  int work_shift = 0;
+  while ((2 * keys) >> work_shift >= (1ll << 32)) ++work_shift;
   DevBuf<int32_t> ustart;
   if ((s = ustart.reserve((keys + 31) / 32))) return bail(s);
   k_chunk_starts<<<grid_for(n), 256, 0, st>>>(n, roff, ustart.p);
   k_partner_place<<<grid_for(keys), 256, 0, st>>>(n, roff, radj, ustart.p, info.p, fill ? g->rg->radj4.p : nullptr, g->rg->upward,
                                                long_min, cfg, p->poff.p, lcnt.p, scnt.p, p->pseg.p, p->core_base,
-                                               p->row_words, dense_pct, p->pdense.p, sizes.p + 4);
-  k_place_counts<<<grid_for(n), 256, 0, st>>>(n, lcnt.p, scnt.p, p->plong.p, p->pshort.p, work.p, total.p);
+                                               p->row_words, dense_pct, p->pdense.p, sizes.p + 4, work_shift);
+  k_place_counts<<<grid_for(n), 256, 0, st>>>(n, lcnt.p, scnt.p, p->plong.p, p->pshort.p, work.p, total.p, work_shift);
   GPM_LAUNCH_CHECK();
   if (p->n_rows) {  // the dense segments moved out of the long ones
     DevBuf<int64_t> cnt;
