@@ -85,11 +85,11 @@ struct HeavyRule {
 };
 static HeavyRule heavy_rule(int p) { return p == 7 ? HeavyRule{192, 4} : HeavyRule{48, 16}; }
 __global__ void k_heavy_edges(HeavyRule rule, int64_t nnz, const int64_t *__restrict__ off, const int32_t *__restrict__ adj,
-                              const int32_t *__restrict__ src, int32_t *__restrict__ heavy,
+                              const int32_t *__restrict__ src, uint32_t *__restrict__ heavy,
                               unsigned long long *__restrict__ nheavy) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nnz; e += (int64_t)gridDim.x * blockDim.x) {
     const int32_t v0 = src[e], v1 = adj[e];
-    if (off[v0 + 1] - off[v0] + off[v1 + 1] - off[v1] > rule.degree) heavy[atomicAdd(nheavy, 1ull)] = (int32_t)e;
+    if (off[v0 + 1] - off[v0] + off[v1 + 1] - off[v1] > rule.degree) heavy[atomicAdd(nheavy, 1ull)] = (uint32_t)e;
   }
 }
 
@@ -98,7 +98,7 @@ __global__ void k_heavy_edges(HeavyRule rule, int64_t nnz, const int64_t *__rest
 __global__ void __launch_bounds__(256) k_pattern(int p, HeavyRule rule, int64_t nnz, const int64_t *__restrict__ off,
                                                  const int32_t *__restrict__ adj, const int32_t *__restrict__ src,
                                                  int32_t *__restrict__ scratch, int64_t maxd,
-                                                 const int32_t *__restrict__ heavy,
+                                                 const uint32_t *__restrict__ heavy,
                                                  const unsigned long long *__restrict__ nheavy,
                                                  unsigned long long *__restrict__ next,
                                                  unsigned long long *__restrict__ out) {
@@ -195,8 +195,9 @@ int pattern_enumerate(gpm_graph *g, int p, cudaStream_t st, uint64_t *result) {
   DevBuf<int32_t> scratch;
   GPM_TRY(scratch.reserve((size_t)(warps * maxd * 5)));
   if (g->nnz > 0) {
-    DevBuf<int32_t> heavy;
-    const HeavyRule rule = heavy_rule(p);
+    DevBuf<uint32_t> heavy;
+    HeavyRule rule = heavy_rule(p);
+    if (g->nnz >= (1ll << 32)) rule.degree = INT64_MAX;  // edges are listed by 32-bit numbers
     const bool some = 2 * maxd > rule.degree;
     GPM_TRY(heavy.reserve(some ? g->nnz : 1));
     if (some) {
