@@ -60,11 +60,18 @@ struct CqCore {
 constexpr size_t kCqSmemSmall = 44 * 1024, kCqSmemBig = 112 * 1024;
 constexpr int kCqSmallThreads = 256, kCqBigThreads = 512;
 // Cliques of other sizes than 4 and 5 walk a row's set in one warp while the
-// others wait at the end of the task: many small CTAs, with the slab for rows
-// past the small CTAs' shared memory, lose least (7-cliques of R-MAT 14 441 ->
-// 349 ms, 6-cliques of R-MAT 17 323 -> 304 ms against 512 threads and rows dealt in turn).
-__host__ __device__ constexpr size_t cq_smem_big(int k) { return k == 4 || k == 5 ? kCqSmemBig : kCqSmemSmall; }
-__host__ __device__ constexpr int cq_threads_big(int k) { return k == 4 || k == 5 ? kCqBigThreads : kCqSmallThreads; }
+// others of its CTA wait at the end of the task, so they run in 256-thread
+// CTAs (k_clique_any), rows past kCqSmemAny in the slab.  The heaviest tasks end
+// the count: few CTAs per SM finish each of them sooner, and the warp tasks run
+// beside them on the caller's stream and fill what they leave.  ms with 5 / 4 / 3 / 2
+// CTAs per SM (the warp tasks inside the same kernel), in brackets 3 as it is:
+// R-MAT 16, k = 6: 117 / 116 / 108 / 130 (108), R-MAT 17, k = 6: 300 / 292 / 301 / 372 (300),
+// R-MAT 14, k = 7: 300 / 302 / 289 / 280 (289), Chung-Lu 300,001, k = 6: 0.58 / 0.66 /
+// 0.81 / - (0.53).  (4 and 5 CTAs, the warp tasks after them: R-MAT 16 119, R-MAT 14
+// 360; 5 CTAs on rows from a binary search: 108, 294, 328, 0.83.)
+constexpr size_t kCqSmemAny = 40 * 1024;
+constexpr int kCqAnyThreads = 256, kCqAnyPerSm = 3;
+__host__ __device__ constexpr bool cq_any(int k) { return k != 4 && k != 5; }
 
 static int grid_for(int64_t work, int block = 256) {
   int64_t g = (work + block - 1) / block;
@@ -694,22 +701,17 @@ __device__ unsigned long long clique_cta_task(int32_t u, int k, const int64_t *_
   return c;
 }
 
-// CTA tasks [t0, t1) of the queue, heaviest first.  KM: 4, 5, or 0 for the
-// other clique sizes.  BIG: rows may be in the slab.
-template <int KM, bool BIG>
-__device__ __forceinline__ void
-    clique_cta(int k, const int64_t *__restrict__ roff, const int32_t *__restrict__ radj,
-                 const int32_t *__restrict__ tasks, int ntasks, int *__restrict__ cursor, uint32_t *__restrict__ slabs,
-                 size_t slab_half, CqCore core, const int32_t *__restrict__ gid, unsigned long long *__restrict__ acc,
-                 int stride, int slot) {
-  extern __shared__ __align__(16) uint32_t csm[];
+// The CTA tasks of a queue, heaviest first, in WORDS words of shared memory.
+// KM: 4, 5, or 0 for the other clique sizes.  SLAB: rows that do not fit are in
+// the CTA's slab.
+template <int KM, bool SLAB, size_t WORDS>
+__device__ __forceinline__ void clique_cta(int k, const int64_t *__restrict__ roff, const int32_t *__restrict__ radj,
+                                           const int32_t *__restrict__ tasks, int ntasks, int *__restrict__ cursor,
+                                           uint32_t *smem, uint32_t *slab, size_t slab_half, const CqCore &core,
+                                           uint32_t *xs, const int32_t *__restrict__ gid,
+                                           unsigned long long *__restrict__ acc, int stride, int slot) {
   __shared__ int s_task;
-  __shared__ uint32_t sxs[KM == 0 ? kCqSmallThreads / 32 : 1][64];  // staged sets (wsum_pairs)
-  const int wid = threadIdx.x >> 5;
   const unsigned lane = threadIdx.x & 31;
-  constexpr size_t words = (BIG ? cq_smem_big(KM) : kCqSmemSmall) / 4;
-  uint32_t *slab = slabs + (size_t)blockIdx.x * 2 * slab_half;
-  uint32_t *xs = sxs[KM == 0 ? wid : 0];
   while (true) {
     if (threadIdx.x == 0) s_task = atomicAdd(cursor, 1);
     __syncthreads();
@@ -718,10 +720,10 @@ __device__ __forceinline__ void
     if (t >= ntasks) break;
     const int32_t u = tasks[t];
     unsigned long long c;
-    if (BIG && cq_layout((int)(roff[u + 1] - roff[u]), k, kCqBigThreads / 32, true).total > words)
-      c = clique_cta_task<KM, false>(u, k, roff, radj, csm, slab, slab_half, core, xs);
+    if (SLAB && cq_layout((int)(roff[u + 1] - roff[u]), k, blockDim.x / 32, true).total > WORDS)
+      c = clique_cta_task<KM, false>(u, k, roff, radj, smem, slab, slab_half, core, xs);
     else
-      c = clique_cta_task<KM, true>(u, k, roff, radj, csm, slab, slab_half, core, xs);
+      c = clique_cta_task<KM, true>(u, k, roff, radj, smem, slab, slab_half, core, xs);
     c = warp_sum(c);
     if (lane == 0 && c) atomicAdd(&acc[(size_t)stride * (gid ? gid[u] : 0) + slot], c);
   }
@@ -733,17 +735,10 @@ __global__ void __launch_bounds__(BIG ? kCqBigThreads : kCqSmallThreads)
                  const int32_t *__restrict__ tasks, int ntasks, int *__restrict__ cursor, uint32_t *__restrict__ slabs,
                  size_t slab_half, CqCore core, const int32_t *__restrict__ gid, unsigned long long *__restrict__ acc,
                  int stride, int slot) {
-  clique_cta<KM, BIG>(k, roff, radj, tasks, ntasks, cursor, slabs, slab_half, core, gid, acc, stride, slot);
-}
-// Cliques of other sizes than 4 and 5: five CTAs per SM, in place of the 32 and
-// 40 registers with spills that the compiler takes by itself.
-template <bool BIG>
-__global__ void __launch_bounds__(kCqSmallThreads, 5)
-    k_clique_any(int k, const int64_t *__restrict__ roff, const int32_t *__restrict__ radj,
-                 const int32_t *__restrict__ tasks, int ntasks, int *__restrict__ cursor, uint32_t *__restrict__ slabs,
-                 size_t slab_half, CqCore core, const int32_t *__restrict__ gid, unsigned long long *__restrict__ acc,
-                 int stride, int slot) {
-  clique_cta<0, BIG>(k, roff, radj, tasks, ntasks, cursor, slabs, slab_half, core, gid, acc, stride, slot);
+  extern __shared__ __align__(16) uint32_t csm[];
+  clique_cta<KM, BIG, (BIG ? kCqSmemBig : kCqSmemSmall) / 4>(k, roff, radj, tasks, ntasks, cursor, csm,
+                                                             slabs + (size_t)blockIdx.x * 2 * slab_half, slab_half,
+                                                             core, nullptr, gid, acc, stride, slot);
 }
 
 __global__ void __launch_bounds__(256) k_clique_warp(int k, const int64_t *__restrict__ roff,
@@ -764,6 +759,19 @@ __global__ void __launch_bounds__(256) k_clique_warp(int k, const int64_t *__res
     unsigned long long c = warp_sum(clique_warp_task(u, k, roff, radj, sm[threadIdx.x >> 5]));
     if (lane == 0 && c) atomicAdd(&acc[(size_t)stride * (gid ? gid[u] : 0) + slot], c);
   }
+}
+
+// CTA tasks of cliques of other sizes than 4 and 5.
+__global__ void __launch_bounds__(kCqAnyThreads, 4)  // 48 registers, no spills
+    k_clique_any(int k, const int64_t *__restrict__ roff, const int32_t *__restrict__ radj,
+                 const int32_t *__restrict__ tasks, int ntasks, int *__restrict__ cursor, uint32_t *__restrict__ slabs,
+                 size_t slab_words, CqCore core, const int32_t *__restrict__ gid, unsigned long long *__restrict__ acc,
+                 int stride, int slot) {
+  extern __shared__ __align__(16) uint32_t csm[];
+  __shared__ uint32_t sxs[kCqAnyThreads / 32][64];  // staged sets (wsum_pairs)
+  clique_cta<0, true, kCqSmemAny / 4>(k, roff, radj, tasks, ntasks, cursor, csm,
+                                      slabs + (size_t)blockIdx.x * slab_words, 0, core, sxs[threadIdx.x >> 5], gid, acc,
+                                      stride, slot);
 }
 
 __global__ void k_clique_tasks(int64_t n, const int64_t *__restrict__ roff, int k, int warp_max, int small_max,
@@ -882,25 +890,28 @@ static int cq_grid(K kernel, int threads, size_t smem) {
   return std::max(1, per_sm) * num_sms();
 }
 
-// The kernels of clique size k: f(small CTA kernel, big CTA kernel).
+// The kernels of clique size 4 or 5: f(small CTA kernel, big CTA kernel).
 template <class F>
 static void cq_kernels(int k, F f) {
   if (k == 4) f(k_clique_cta<4, false>, k_clique_cta<4, true>);
-  else if (k == 5) f(k_clique_cta<5, false>, k_clique_cta<5, true>);
-  else f(k_clique_any<false>, k_clique_any<true>);
+  else f(k_clique_cta<5, false>, k_clique_cta<5, true>);
 }
 
 struct CqGrids {
-  int small, big, warp;
+  int small, big, warp;  // of the other sizes: small = 0, big = k_clique_any's
 };
 static CqGrids cq_grids(int k) {
-  static PerDevice small[3], big[3], warp;
-  const int i = k == 4 ? 0 : k == 5 ? 1 : 2;
+  static PerDevice small[2], big[2], warp, any;
   CqGrids g;
-  cq_kernels(k, [&](auto s, auto b) {
-    g.small = small[i].get([&] { return cq_grid(s, kCqSmallThreads, kCqSmemSmall); });
-    g.big = big[i].get([&] { return cq_grid(b, cq_threads_big(k), cq_smem_big(k)); });
-  });
+  if (cq_any(k)) {
+    g.small = 0;
+    g.big = any.get([] { return std::min(cq_grid(k_clique_any, kCqAnyThreads, kCqSmemAny), kCqAnyPerSm * num_sms()); });
+  } else {
+    cq_kernels(k, [&](auto s, auto b) {
+      g.small = small[k - 4].get([&] { return cq_grid(s, kCqSmallThreads, kCqSmemSmall); });
+      g.big = big[k - 4].get([&] { return cq_grid(b, kCqBigThreads, kCqSmemBig); });
+    });
+  }
   g.warp = warp.get([] { return cq_grid(k_clique_warp, 256, 0); });
   return g;
 }
@@ -973,10 +984,11 @@ int clique_plan_build(CliquePlan *p, int64_t n, const int64_t *roff, const int32
     if (s == GPM_ENOMEM) p->core = CoreRows();  // counted without them
     else GPM_TRY(s);
   }
-  // per-CTA slabs of the big CTAs: rows, and compacted rows, that do not fit
+  // per-CTA slabs: rows, and for the big CTAs compacted rows, that do not fit
   // in shared memory
   const size_t W = (size_t)(max_deg + 31) / 32;
   const CqGrids grids = cq_grids(k);
+  if (cq_any(k)) p->n_big = p->n_cta;
   p->big_grid = std::max(1, std::min(grids.big, p->n_big));
   if (p->n_big > 0 && p->n_big < p->n_cta + p->n_warp && !p->side &&
       (cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking) != cudaSuccess ||
@@ -985,11 +997,12 @@ int clique_plan_build(CliquePlan *p, int64_t n, const int64_t *roff, const int32
     cudaGetLastError();
     return fail(GPM_ECUDA, "clique plan: side stream");
   }
-  const CqLayout big = cq_layout(max_deg, k, kCqBigThreads / 32, true);
+  const CqLayout big = cq_layout(max_deg, k, (cq_any(k) ? kCqAnyThreads : kCqBigThreads) / 32, true);
   const size_t comp_max = (size_t)max_deg * ((W + 3) & ~(size_t)3);
-  const bool spill = p->n_big && (big.total * 4 > cq_smem_big(k) || (k == 5 && comp_max > kCqBigThreads / 32 * cq_warp_words(1)));
+  const bool spill = p->n_big && (big.total * 4 > (cq_any(k) ? kCqSmemAny : kCqSmemBig) ||
+                                  (k == 5 && comp_max > kCqBigThreads / 32 * cq_warp_words(1)));
   p->slab_words = comp_max;
-  GPM_TRY(p->slabs.reserve(spill ? 2 * p->slab_words * p->big_grid : 1));
+  GPM_TRY(p->slabs.reserve(spill ? (cq_any(k) ? 1 : 2) * p->slab_words * p->big_grid : 1));
   if (p->n_cta > p->n_big && k == 5) {
     // small CTAs: compacted rows beyond the warps' buffers
     const int sd = std::min(max_deg, cq_small_max(k));
@@ -1015,16 +1028,23 @@ int clique_plan_run(CliquePlan *p, cudaStream_t st, bool zero) {
     GPM_CUDA(cudaEventRecord(p->fork, st));
     GPM_CUDA(cudaStreamWaitEvent(bst, p->fork, 0));
   }
-  cq_kernels(p->k, [&](auto small, auto big) {
+  if (cq_any(p->k)) {
     if (p->n_big > 0)
-      big<<<p->big_grid, cq_threads_big(p->k), cq_smem_big(p->k), bst>>>(p->k, p->roff, p->radj, p->ctasks.p, p->n_big,
-                                                           p->cursors, p->slabs.p, p->slab_words, core, p->gid,
-                                                           p->acc, p->stride, p->slot);
-    if (nsmall > 0)
-      small<<<std::min(grids.small, nsmall), kCqSmallThreads, kCqSmemSmall, st>>>(
-          p->k, p->roff, p->radj, p->ctasks.p + p->n_big, nsmall, p->cursors + 1, p->small_slabs.p, p->small_slab,
-          core, p->gid, p->acc, p->stride, p->slot);
-  });
+      k_clique_any<<<p->big_grid, kCqAnyThreads, kCqSmemAny, bst>>>(p->k, p->roff, p->radj, p->ctasks.p, p->n_big,
+                                                                    p->cursors, p->slabs.p, p->slab_words, core,
+                                                                    p->gid, p->acc, p->stride, p->slot);
+  } else {
+    cq_kernels(p->k, [&](auto small, auto big) {
+      if (p->n_big > 0)
+        big<<<p->big_grid, kCqBigThreads, kCqSmemBig, bst>>>(p->k, p->roff, p->radj, p->ctasks.p, p->n_big, p->cursors,
+                                                             p->slabs.p, p->slab_words, core, p->gid, p->acc,
+                                                             p->stride, p->slot);
+      if (nsmall > 0)
+        small<<<std::min(grids.small, nsmall), kCqSmallThreads, kCqSmemSmall, st>>>(
+            p->k, p->roff, p->radj, p->ctasks.p + p->n_big, nsmall, p->cursors + 1, p->small_slabs.p, p->small_slab,
+            core, p->gid, p->acc, p->stride, p->slot);
+    });
+  }
   if (bst != st) GPM_CUDA(cudaEventRecord(p->join, bst));
   if (p->n_warp > 0)
     k_clique_warp<<<std::min(grids.warp, (p->n_warp + 7) / 8), 256, 0, st>>>(
