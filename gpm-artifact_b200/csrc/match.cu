@@ -1225,7 +1225,9 @@ static int extend_rows(const WidePlan &plan, const MatchGraph &G, DevBuf<int32_t
     if (bytes > budget) break;
     DevBuf<int32_t> next;
     if (nn) {
-      GPM_TRY(next.reserve((size_t)nn * (*t + 1)));
+      const int s = next.reserve((size_t)nn * (*t + 1));
+      if (s == GPM_ENOMEM) break;  // walked from the rows there are
+      GPM_TRY(s);
       GPM_CUDA(cudaMemset(cnt.p, 0, 8));
       k_extend_rows<<<blocks, 256>>>(plan, G, *rows, *nrows, *t, next.p, nn, cnt.p);
       GPM_LAUNCH_CHECK();

@@ -1,0 +1,45 @@
+"""Counts whose faster way needs scratch that cannot be had: they take the way
+that does without it."""
+import contextlib
+
+import numpy as np
+import pytest
+
+import gpm
+
+pytestmark = pytest.mark.gpu
+
+MIB = 1 << 20
+
+
+@contextlib.contextmanager
+def _left(mib):
+    """All device memory but about `mib` MiB taken."""
+    import torch
+    gpm.trim()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    held = torch.empty(torch.cuda.mem_get_info()[0] - mib * MIB, dtype=torch.uint8, device="cuda")
+    try:
+        assert torch.cuda.mem_get_info()[0] < (mib + 4) * MIB
+        yield
+    finally:
+        del held
+        torch.cuda.empty_cache()
+
+
+def test_rows_that_cannot_be_extended():
+    """One root, 30 hubs, 100,000 leaves under each hub, one vertex under all
+    leaves: 30 pairs, whose extension takes 36 MB."""
+    hubs, leaves = 30, 100000
+    n = 1 + hubs + leaves + 1
+    leaf = np.arange(1 + hubs, 1 + hubs + leaves)
+    s = np.concatenate([np.zeros(hubs), np.repeat(np.arange(1, 1 + hubs), leaves), leaf]).astype(np.int32)
+    d = np.concatenate([np.arange(1, 1 + hubs), np.tile(leaf, hubs), np.full(leaves, n - 1)]).astype(np.int32)
+    lab = np.full(n, 2, np.int32)
+    lab[0], lab[1:1 + hubs], lab[n - 1] = 0, 1, 3
+    g = gpm.Graph.from_edges(n, s, d, labels=lab)
+    q = gpm.Query(4, [0, 1, 2], [1, 2, 3], [0, 1, 2, 3])
+    assert g.match(q, limit=1 << 40) == hubs * leaves
+    with _left(20):
+        assert g.match(q, limit=1 << 40) == hubs * leaves
