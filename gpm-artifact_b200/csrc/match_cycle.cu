@@ -337,7 +337,9 @@ bool is_cycle4(const gpm_query *q, const LabelCsr *lc) {
 int cycle_plan(gpm_graph *g, LabelCsr *lc, const gpm_query *q, unsigned long long min_wedges, CyclePlan *p,
                CycleSpace **space, bool *fits) {
   *fits = false;
-  GPM_TRY(ensure_label_classes(g, lc));
+  const int classes = ensure_label_classes(g, lc);
+  if (classes == GPM_ENOMEM) return GPM_OK;
+  GPM_TRY(classes);
   // the vertices around the cycle: 0, x, opposite, y
   const int x = __builtin_ctzll(q->adjmask[0]), y = 63 - __builtin_clzll(q->adjmask[0]), o = 6 - x - y;
   const int32_t l[4] = {q->labels[0], q->labels[x], q->labels[o], q->labels[y]};

@@ -28,6 +28,16 @@ def _left(mib):
         torch.cuda.empty_cache()
 
 
+def test_cycle_query_without_label_classes():
+    g = gpm.Graph.rmat(19, 16, seed=3)
+    g.set_labels(np.where(np.arange(1 << 19) % 4096 == 0, 1, 0).astype(np.int32) + (np.arange(1 << 19) % 4096 == 1) * 2)
+    q = gpm.Query(4, [0, 1, 2, 3], [1, 2, 3, 0], [1, 2, 1, 2])
+    want = g.match(q, limit=1 << 40)  # walked
+    with _left(48):
+        assert g.match(q) == want
+    assert g.match(q) == want
+
+
 def test_rows_that_cannot_be_extended():
     """One root, 30 hubs, 100,000 leaves under each hub, one vertex under all
     leaves: 30 pairs, whose extension takes 36 MB."""
