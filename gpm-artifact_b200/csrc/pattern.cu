@@ -198,8 +198,15 @@ int pattern_enumerate(gpm_graph *g, int p, cudaStream_t st, uint64_t *result) {
     DevBuf<uint32_t> heavy;
     HeavyRule rule = heavy_rule(p);
     if (g->nnz >= (1ll << 32)) rule.degree = INT64_MAX;  // edges are listed by 32-bit numbers
-    const bool some = 2 * maxd > rule.degree;
-    GPM_TRY(heavy.reserve(some ? g->nnz : 1));
+    bool some = 2 * maxd > rule.degree;
+    if (some) {
+      const int s = heavy.reserve(g->nnz);
+      if (s != GPM_OK && s != GPM_ENOMEM) return s;
+      if (s == GPM_ENOMEM) {  // no room for the list: a warp per edge, heavy or not
+        some = false;
+        rule.degree = INT64_MAX;
+      }
+    }
     if (some) {
       k_heavy_edges<<<(int)std::min<int64_t>((g->nnz + 255) / 256, num_sms() * 8), 256, 0, st>>>(
           rule, g->nnz, g->off.p, g->adj.p, g->src.p, heavy.p, d.p + 1);

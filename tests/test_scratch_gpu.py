@@ -53,3 +53,12 @@ def test_rows_that_cannot_be_extended():
     assert g.match(q, limit=1 << 40) == hubs * leaves
     with _left(20):
         assert g.match(q, limit=1 << 40) == hubs * leaves
+
+
+def test_heavy_edges_without_their_list():
+    g = gpm.Graph.generate(1, 200000, 13000000, seed=5)
+    assert g.info().max_degree * 2 > 192
+    want = g.pattern("P7")
+    with _left(40):
+        got = g.pattern("P7")
+    assert got[0] == want[0] > 0 and got[1].tolist() == want[1].tolist()
