@@ -515,7 +515,8 @@ __device__ __forceinline__ unsigned cq_pairs(const uint32_t *comp, int stride, i
 }
 
 // One vertex task on a CTA.  SM: the rows are in shared memory (smem), else in
-// the CTA's slab (two halves of slab_half words: rows, compacted rows).  Each
+// the CTA's slab (two halves of slab_half words: rows, compacted rows; without rows the
+// first half holds the compacted ones).  Each
 // thread returns its part of the count.
 template <int KM, bool SM>
 __device__ unsigned long long clique_cta_task(int32_t u, int k, const int64_t *__restrict__ roff,
@@ -669,7 +670,7 @@ __device__ unsigned long long clique_cta_task(int32_t u, int k, const int64_t *_
       __syncthreads();
       const int m = s_heavy, strips = (m + 31) >> 5, stride = (strips + 3) & ~3;
       // the slab holds what the warps' buffers have no room for
-      uint32_t *comp = (size_t)m * stride <= lay.comp_words ? smem + lay.comp : slab + slab_half;
+      uint32_t *comp = (size_t)m * stride <= lay.comp_words ? smem + lay.comp : slab + (SM ? 0 : slab_half);
       for (int r = wid; r < strips; r += nw) cq_compact(rows, ri, W, xl, m, 32 * r, mv, comp, stride, lane);
       __syncthreads();
       // (r <= w, four column words from 4 (w / 4) on): small w first, they have most columns
@@ -737,7 +738,7 @@ __global__ void __launch_bounds__(BIG ? kCqBigThreads : kCqSmallThreads)
                  int stride, int slot) {
   extern __shared__ __align__(16) uint32_t csm[];
   clique_cta<KM, BIG, (BIG ? kCqSmemBig : kCqSmemSmall) / 4>(k, roff, radj, tasks, ntasks, cursor, csm,
-                                                             slabs + (size_t)blockIdx.x * 2 * slab_half, slab_half,
+                                                             slabs + (size_t)blockIdx.x * (BIG ? 2 : 1) * slab_half, slab_half,
                                                              core, nullptr, gid, acc, stride, slot);
 }
 
@@ -976,14 +977,6 @@ int clique_plan_build(CliquePlan *p, int64_t n, const int64_t *roff, const int32
   p->n_cta = h[0];
   p->n_warp = h[1];
   p->n_big = h[2];
-  if (p->n_cta > 0) {
-    int64_t nkeys = 0;
-    GPM_CUDA(cudaMemcpyAsync(&nkeys, roff + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    GPM_CUDA(cudaStreamSynchronize(st));
-    const int s = core_rows_build(n, roff, radj, nkeys, kCqCore, kCqCoreMin, p->rowid, &p->core, st);
-    if (s == GPM_ENOMEM) p->core = CoreRows();  // counted without them
-    else GPM_TRY(s);
-  }
   // per-CTA slabs: rows, and for the big CTAs compacted rows, that do not fit
   // in shared memory
   const size_t W = (size_t)(max_deg + 31) / 32;
@@ -1002,14 +995,33 @@ int clique_plan_build(CliquePlan *p, int64_t n, const int64_t *roff, const int32
   const bool spill = p->n_big && (big.total * 4 > (cq_any(k) ? kCqSmemAny : kCqSmemBig) ||
                                   (k == 5 && comp_max > kCqBigThreads / 32 * cq_warp_words(1)));
   p->slab_words = comp_max;
-  GPM_TRY(p->slabs.reserve(spill ? (cq_any(k) ? 1 : 2) * p->slab_words * p->big_grid : 1));
-  if (p->n_cta > p->n_big && k == 5) {
-    // small CTAs: compacted rows beyond the warps' buffers
-    const int sd = std::min(max_deg, cq_small_max(k));
-    p->small_slab = (size_t)sd * (((sd + 31) / 32 + 3) & ~3);
-    GPM_TRY(p->small_slabs.reserve(2 * p->small_slab * grids.small));
-  } else {
-    GPM_TRY(p->small_slabs.reserve(1));
+  // a grid of half the CTAs where their slabs find no memory
+  auto reserve = [](DevBuf<uint32_t> &buf, size_t per_cta, int *grid) -> int {
+    while (true) {
+      const int s = buf.reserve(std::max<size_t>(1, per_cta * *grid));
+      if (s != GPM_ENOMEM || *grid == 1) return s;
+      *grid /= 2;
+    }
+  };
+  GPM_TRY(reserve(p->slabs, spill ? (cq_any(k) ? 1 : 2) * p->slab_words : 0, &p->big_grid));
+  p->small_grid = std::max(1, std::min(grids.small, p->n_cta - p->n_big));
+  // small CTAs: compacted rows beyond the warps' buffers
+  const int sd = std::min(max_deg, cq_small_max(k)), sw = (sd + 31) / 32;
+  p->small_slab = (size_t)sd * ((sw + 3) & ~3);
+  const bool small_spill = p->n_cta > p->n_big && k == 5 && p->small_slab > kCqSmallThreads / 32 * cq_warp_words(1);
+  GPM_TRY(reserve(p->small_slabs, small_spill ? p->small_slab : 0, &p->small_grid));
+  // the bitmaps last: what cannot do without memory comes first
+  if (p->n_cta > 0) {
+    int64_t nkeys = 0;
+    GPM_CUDA(cudaMemcpyAsync(&nkeys, roff + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    GPM_CUDA(cudaStreamSynchronize(st));
+    const int s = core_rows_build(n, roff, radj, nkeys, kCqCore, kCqCoreMin, p->rowid, &p->core, st);
+    if (s == GPM_ENOMEM) {  // counted without them
+      p->core = CoreRows();
+      p->rowid.reset();
+    } else {
+      GPM_TRY(s);
+    }
   }
   GPM_CUDA(cudaStreamSynchronize(st));
   return GPM_OK;
@@ -1040,7 +1052,7 @@ int clique_plan_run(CliquePlan *p, cudaStream_t st, bool zero) {
                                                              p->slabs.p, p->slab_words, core, p->gid, p->acc,
                                                              p->stride, p->slot);
       if (nsmall > 0)
-        small<<<std::min(grids.small, nsmall), kCqSmallThreads, kCqSmemSmall, st>>>(
+        small<<<p->small_grid, kCqSmallThreads, kCqSmemSmall, st>>>(
             p->k, p->roff, p->radj, p->ctasks.p + p->n_big, nsmall, p->cursors + 1, p->small_slabs.p, p->small_slab,
             core, p->gid, p->acc, p->stride, p->slot);
     });

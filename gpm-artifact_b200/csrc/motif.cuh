@@ -38,10 +38,10 @@ struct CliquePlan {
   const int64_t *roff = nullptr;
   const int32_t *radj = nullptr;
   int k = 0, stride = 0, slot = 0, n_cta = 0, n_warp = 0;
-  int n_big = 0, big_grid = 0;  // the first n_big CTA tasks take the large CTAs
+  int n_big = 0, big_grid = 0, small_grid = 0;  // the first n_big CTA tasks take the large CTAs
   const int32_t *gid = nullptr;
   unsigned long long *acc = nullptr;
-  size_t slab_words = 0, small_slab = 0;  // words of half a slab (big, small CTAs)
+  size_t slab_words = 0, small_slab = 0;  // words of half a big CTA's slab, of a small CTA's
   DevBuf<int32_t> ctasks, wtasks;
   DevBuf<int> counters;    // the cursors, where the caller gave none
   int *cursors = nullptr;  // 3

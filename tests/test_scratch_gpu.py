@@ -62,3 +62,14 @@ def test_heavy_edges_without_their_list():
     with _left(40):
         got = g.pattern("P7")
     assert got[0] == want[0] > 0 and got[1].tolist() == want[1].tolist()
+
+
+@pytest.mark.parametrize("k,scale,levels", [(3, 20, range(230, 310, 10)), (5, 18, range(44, 90, 6)), (4, 20, range(150, 310, 20))])
+def test_cliques_with_little_memory(k, scale, levels):
+    """Room for the rows' slabs, but not for the hubs' bitmaps beside them."""
+    g = gpm.Graph.rmat(scale, 16, seed=4).orient()
+    want = g.clique(k)
+    for mib in levels:
+        g.drop_plans()
+        with _left(mib):
+            assert g.clique(k) == want, mib
