@@ -451,29 +451,38 @@ __global__ void __launch_bounds__(256) k_c4(const int64_t *__restrict__ roff, co
 // took 7.2 / 101 / 1320 ms, with cursors 6.2 / 39.6 / 698 ms (lane groups with
 // a cursor per list, 1024 threads and 200 KB: 11.8 / 70.7 / 806 ms, whole
 // pipelines).  It is bound by the latency of the lists and of the counters' old
-// values at 48 warps per SM.  CTA shapes, 48 Chung-Lu graphs / R-MAT 18 / 256
-// graphs: 2 x 768 threads, 100 KB each 21.3 / 6.22 / 698 ms; 1 x 1024, 200 KB
-// 24.1 / 6.41 / 700; 2 x 1024, 100 KB 21.5 / 6.35 / 719.
-constexpr int kC4BigThreads = 768, kC4BigPerSm = 2;
-constexpr int kC4HotWords = 25600;  // 100 KB per CTA
-constexpr int kC4BigSmem = kC4HotWords * 4;
+// values at 32 to 48 warps per SM.  Two CTAs per SM and windows of 51,200 keys
+// while every member has at most kC4WideMin vertices, one CTA and windows of
+// 102,400 keys beyond: members that span many windows pay for each with a walk
+// over all lists (two searches each).  ms narrow / wide, Chung-Lu of exponent 2.8 and
+// mean degree 64: 150,001 vertices 3.38 / 3.84, 250,001 6.48 / 6.87, 400,001 12.25 /
+// 11.97, 600,001 22.1 / 20.5, 10^6 47.8 / 40.7; R-MAT 18 6.1 / 6.4, R-MAT 20 39.4 /
+// 39.1.  (2 x 1024 threads with 100 KB each: R-MAT 20 41.6, 10^6 vertices 52.0.)
+template <int THREADS, int PER_SM, int WORDS>
+struct C4Shape {
+  static constexpr int kThreads = THREADS, kPerSm = PER_SM, kWords = WORDS, kSmem = 4 * WORDS;
+  // Tasks whose bound is at most kHashMax count in an open-addressing table
+  // over the same shared memory, slots of (key + 1, count) with 0 = empty.  The
+  // bound caps the distinct keys below the slot count, so every probe ends.
+  static constexpr unsigned kHashSlots = WORDS / 2;
+  static constexpr unsigned long long kHashMax = kHashSlots * 6 / 10;
+};
+using C4Narrow = C4Shape<768, 2, 25600>;
+using C4Wide = C4Shape<1024, 1, 51200>;
+constexpr int64_t kC4WideMin = 400000;
 constexpr int64_t kC4CursorBytes = 4ll << 30;  // most global memory for cursors
 
-// Tasks whose bound is at most kC4HashMax count in an open-addressing table
-// over the same shared memory, slots of (key + 1, count) with 0 = empty.  The
-// bound caps the distinct keys below the slot count, so every probe ends.
-constexpr unsigned kC4HashSlots = kC4HotWords / 2;
-constexpr unsigned long long kC4HashMax = kC4HashSlots * 6 / 10;
+template <unsigned SLOTS>
 __device__ __forceinline__ unsigned c4_hash_add(unsigned *cw, unsigned key1) {
-  unsigned h = (unsigned)(((unsigned long long)(key1 * 2654435761u) * kC4HashSlots) >> 32);
-  for (unsigned p = 0; p < kC4HashSlots; ++p) {
+  unsigned h = (unsigned)(((unsigned long long)(key1 * 2654435761u) * SLOTS) >> 32);
+  for (unsigned p = 0; p < SLOTS; ++p) {
     unsigned cur = cw[2 * h];
     if (cur == 0u) {
       cur = atomicCAS(&cw[2 * h], 0u, key1);
       if (cur == 0u) cur = key1;
     }
     if (cur == key1) return atomicAdd(&cw[2 * h + 1], 1u);
-    if (++h == kC4HashSlots) h = 0;
+    if (++h == SLOTS) h = 0;
   }
   return 0u;
 }
@@ -486,11 +495,14 @@ __device__ __forceinline__ int64_t first_at_least(const int32_t *__restrict__ a,
   return lo;
 }
 
-__global__ void __launch_bounds__(kC4BigThreads, kC4BigPerSm)
+// hash_max: at most S::kHashMax
+template <class S>
+__global__ void __launch_bounds__(S::kThreads, S::kPerSm)
     k_c4_big(const int64_t *__restrict__ roff, const int64_t *__restrict__ split, const int32_t *__restrict__ radj,
              const int32_t *__restrict__ gid, const int64_t *__restrict__ gbase, const int32_t *__restrict__ tasks,
              const unsigned long long *__restrict__ task_b, int n_tasks, int *__restrict__ counters,
-             int *__restrict__ cursors, int cursor_len, unsigned long long *__restrict__ acc) {
+             int *__restrict__ cursors, int cursor_len, unsigned long long hash_max,
+             unsigned long long *__restrict__ acc) {
   extern __shared__ __align__(16) unsigned hot[];
   __shared__ int s_task;
   __shared__ WedgeWalk s_walk;
@@ -498,7 +510,7 @@ __global__ void __launch_bounds__(kC4BigThreads, kC4BigPerSm)
   const unsigned lane = threadIdx.x & 31;
   int turn = 0;
   if (threadIdx.x == 0) s_walk.s[0].next = s_walk.s[0].nlong = 0;
-  for (int i = threadIdx.x; i < kC4HotWords; i += blockDim.x) hot[i] = 0u;
+  for (int i = threadIdx.x; i < S::kWords; i += blockDim.x) hot[i] = 0u;
   while (true) {
     if (threadIdx.x == 0) s_task = atomicAdd(&counters[2], 1);
     __syncthreads();
@@ -514,20 +526,20 @@ __global__ void __launch_bounds__(kC4BigThreads, kC4BigPerSm)
     const int sh = dx < 65536 ? 1 : 0;
     const unsigned mask = sh ? 0xffffu : 0xffffffffu;
     unsigned long long c = 0;
-    if (W <= kC4HashMax) {
+    if (W <= hash_max) {
       cta_wedges(radj, dx, W, s_walk, &turn,
                  [&](int i, long long *st, int *len) {
                    const int32_t a = radj[a0 + i];
                    *st = roff[a];
                    *len = (int)(first_at_least(radj, *st, roff[a + 1], x) - *st);
                  },
-                 [&](int32_t y, long long, int) { c += c4_hash_add(hot, (unsigned)(y - base) + 1u); });
+                 [&](int32_t y, long long, int) { c += c4_hash_add<S::kHashSlots>(hot, (unsigned)(y - base) + 1u); });
       uint4 *v = reinterpret_cast<uint4 *>(hot);
-      for (int i = threadIdx.x; i < kC4HotWords / 4; i += blockDim.x) v[i] = make_uint4(0u, 0u, 0u, 0u);
+      for (int i = threadIdx.x; i < S::kWords / 4; i += blockDim.x) v[i] = make_uint4(0u, 0u, 0u, 0u);
       __syncthreads();
     }
-    for (int32_t hi = W <= kC4HashMax ? base : x; hi > base;) {
-      const int32_t lo = (int32_t)max((int64_t)base, (int64_t)hi - ((int64_t)kC4HotWords << sh));
+    for (int32_t hi = W <= hash_max ? base : x; hi > base;) {
+      const int32_t lo = (int32_t)max((int64_t)base, (int64_t)hi - ((int64_t)S::kWords << sh));
       cta_wedges(radj, dx, W, s_walk, &turn,
                  [&](int i, long long *st, int *len) {  // entries of N(a) in [lo, hi), a the i-th neighbour of x
                    const int64_t s0 = roff[radj[a0 + i]];
@@ -557,7 +569,7 @@ __global__ void __launch_bounds__(kC4BigThreads, kC4BigPerSm)
       const int words = ((hi - lo) >> sh) + 1;
       uint4 *v = reinterpret_cast<uint4 *>(hot);
       for (int i = threadIdx.x; 4 * i < words; i += blockDim.x)
-        if (i < kC4HotWords / 4) v[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (i < S::kWords / 4) v[i] = make_uint4(0u, 0u, 0u, 0u);
       __syncthreads();
       hi = lo;
     }
@@ -655,6 +667,12 @@ static int *te_cursors(MotifPlan *p) { return reinterpret_cast<int *>(p->acc.p +
 static int *c4_cursors(MotifPlan *p) { return te_cursors(p) + 4; }
 static int *k4_cursors(MotifPlan *p) { return te_cursors(p) + 8; }
 
+// f(C4Narrow{}) or f(C4Wide{})
+template <class F>
+static int c4_shape(int64_t max_graph_n, F f) {
+  return max_graph_n > kC4WideMin ? f(C4Wide{}) : f(C4Narrow{});
+}
+
 static int te_grid() {
   static PerDevice grid;
   return grid.get([] {
@@ -727,14 +745,24 @@ int motif_plan_build(const MotifInput &in, MotifPlan *p, cudaStream_t st) {
     GPM_TRY(t.reserve(tmp));
     GPM_CUDA(cub::DeviceRadixSort::SortPairsDescending(t.p, tmp, bb.p, p->c4_bb.p, bt.p, p->c4_bt.p, p->c4_nb, 0,
                                                        64, st));
-    GPM_CUDA(cudaFuncSetAttribute(k_c4_big, cudaFuncAttributeMaxDynamicSharedMemorySize, kC4BigSmem));
-    int per_sm = 0;
-    GPM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_c4_big, kC4BigThreads, kC4BigSmem));
-    p->c4_big_grid = std::max(1, per_sm) * num_sms();
+    int words = 0;
+    GPM_TRY(c4_shape(in.max_graph_n, [&](auto shape) -> int {
+      using S = decltype(shape);
+      words = S::kWords;
+      p->c4_hash_max = S::kHashMax;
+      GPM_CUDA(cudaFuncSetAttribute(k_c4_big<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem));
+      int per_sm = 0;
+      GPM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_c4_big<S>, S::kThreads, S::kSmem));
+      p->c4_big_grid = std::max(1, per_sm) * num_sms();
+      return GPM_OK;
+    }));
+    // tests send small tasks through the windows
+    if (const char *e = getenv("GPM_C4_HASH_MAX"))
+      p->c4_hash_max = std::min<unsigned long long>(p->c4_hash_max, std::max(0ll, atoll(e)));
     p->c4_big_grid = std::min(p->c4_big_grid, p->c4_nb);
     // cursors for the longest task's neighbours, where some member spans two
     // windows, as far as memory goes (the others search their whole list again)
-    int64_t len = in.max_graph_n <= kC4HotWords ? 0 : h[6];
+    int64_t len = in.max_graph_n <= words ? 0 : h[6];
     if (const char *e = getenv("GPM_C4_CURSORS")) len = std::min<int64_t>(len, std::max(0ll, atoll(e)));
     len = std::min(len, kC4CursorBytes / 4 / p->c4_big_grid);
     while (p->c4_cursor.reserve((size_t)len * p->c4_big_grid) != GPM_OK) {
@@ -769,9 +797,13 @@ static int te_launch(MotifPlan *p, cudaStream_t st) {
 static int c4_launch(MotifPlan *p, cudaStream_t st) {
   const MotifInput &in = p->in;
   if (p->c4_nb > 0)
-    k_c4_big<<<p->c4_big_grid, kC4BigThreads, kC4BigSmem, st>>>(
-        in.roff, p->split.p, in.radj, in.gid, in.gbase, p->c4_bt.p, p->c4_bb.p, p->c4_nb, c4_cursors(p),
-        p->c4_cursor.p, p->c4_cursor_len, p->acc.p);
+    GPM_TRY(c4_shape(in.max_graph_n, [&](auto shape) -> int {
+      using S = decltype(shape);
+      k_c4_big<S><<<p->c4_big_grid, S::kThreads, S::kSmem, st>>>(
+          in.roff, p->split.p, in.radj, in.gid, in.gbase, p->c4_bt.p, p->c4_bb.p, p->c4_nb, c4_cursors(p),
+          p->c4_cursor.p, p->c4_cursor_len, p->c4_hash_max, p->acc.p);
+      return GPM_OK;
+    }));
   if (p->c4_nc + p->c4_nw > 0)
     k_c4<<<p->c4_grid, 256, 0, st>>>(in.roff, p->split.p, in.radj, in.gid, in.gbase, p->c4_ct.p, p->c4_nc,
                                      p->c4_wt.p, p->c4_nw, c4_cursors(p), p->acc.p);

@@ -85,6 +85,7 @@ struct MotifPlan {
   int te_nc = 0, te_nw = 0, te_nl = 0, c4_nc = 0, c4_nw = 0, c4_nb = 0, te_grid = 0, c4_grid = 0, c4_big_grid = 0;
   DevBuf<int> c4_cursor;  // positions of the giant tasks' walks in their lists, c4_cursor_len per CTA
   int c4_cursor_len = 0;
+  unsigned long long c4_hash_max = 0;  // giant tasks up to this bound count in a hash table
   CliquePlan k4;
   DevBuf<unsigned long long> acc, out;
 };
