@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(256, GPM_TC_RANK_MIN_BLOCKS)
                 const Seg *__restrict__ pseg,
                 const int32_t *__restrict__ plong, const int32_t *__restrict__ pshort,
                 const int32_t *__restrict__ cta_tasks, int n_cta,
-                const int32_t *__restrict__ warp_tasks, int n_warp, int *__restrict__ counters,
+                const int32_t *__restrict__ warp_tasks, int n_warp, int lone, int *__restrict__ counters,
                 unsigned long long *__restrict__ out, unsigned long long *__restrict__ rec) {
   extern __shared__ __align__(16) uint32_t rsm[];
   __shared__ int s_task;
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(256, GPM_TC_RANK_MIN_BLOCKS)
   uint32_t *region = rsm + wid * kWarpWords;
   WarpTasks queue;
   while (true) {
-    const int t = queue.next(&counters[1], gridDim.x * kRWarps * 8, lane);
+    const int t = queue.next(&counters[1], lone, lane);
     if (t >= n_warp) break;
     const int32_t x = warp_tasks[t];
     c += owner_task<false, REC>(x, roff, radj, radj4, poff, pseg, plong, pshort, region, kWarpWords,
@@ -798,6 +798,13 @@ __global__ void k_dense_tasks(int64_t n, const int64_t *__restrict__ roff, const
 // R-MAT 22 unchanged; Chung-Lu 300,007 x 24: 154, 154, 156, 160, 165.
 constexpr unsigned long long kHeavyWork = 1024;
 constexpr int kHeavyShares = 2;
+// Warp tasks of more than kLoneWork keys come from the cursor one at a time, the
+// rest in runs (WarpTasks): a run of heavy ones ends the count late.  All come
+// alone where that is most of them, or where a warp has few.  us per count, all
+// alone / runs behind the first eight per warp / so: ER 200,003 x 64: 425, 485,
+// 425; ER 100,003 x 64: 219, 230, 219; ER 600,007 x 40: 555, 493, 495; ER 300,007 x
+// 30: 232, 191, 191; R-MAT 21: 945, 898, 895; R-MAT 22: 5013, 4830, 4835.
+constexpr unsigned long long kLoneWork = 384;
 __global__ void k_rank_tasks(int64_t n, const int64_t *__restrict__ roff, const int32_t *__restrict__ plong,
                              const int32_t *__restrict__ pshort,
                              const unsigned long long *__restrict__ work, int cta_min,
@@ -822,6 +829,7 @@ __global__ void k_rank_tasks(int64_t n, const int64_t *__restrict__ roff, const 
       int i = atomicAdd(&sizes[1], 1);
       wkey[i] = task_key(work[x]);
       wval[i] = (int32_t)x;
+      if (work[x] > kLoneWork) atomicAdd(&sizes[5], 1);
     }
   }
 }
@@ -1357,10 +1365,11 @@ int rank_plan_new(gpm_graph *g, int cta_min, int long_min, const uint8_t *cfg, c
     cudaMemsetAsync(p->pdense.p, 0, sizeof(int32_t) * n, st);
   }
   // sizes: [0] CTA tasks, [1] warp tasks, [2] dense tasks, [3] dense-only
-  // owners, [4] a segment too long for its descriptor
+  // owners, [4] a segment too long for its descriptor, [5] warp tasks of
+  // more than kLoneWork keys
   DevBuf<int> sizes;
-  if ((s = sizes.reserve(5))) return bail(s);
-  cudaMemsetAsync(sizes.p, 0, 5 * sizeof(int), st);
+  if ((s = sizes.reserve(6))) return bail(s);
+  cudaMemsetAsync(sizes.p, 0, 6 * sizeof(int), st);
   k_vertex_info<<<grid_for(n), 256, 0, st>>>(n, roff, radj, g->rg->roff4.p, p->n_rows ? rowid.p : nullptr, info.p);
   const int64_t keys = (int64_t)g->rg->radj.n;
   int work_shift = 0;
@@ -1405,13 +1414,16 @@ int rank_plan_new(gpm_graph *g, int cta_min, int long_min, const uint8_t *cfg, c
     if ((s = dkey.reserve(n)) || (s = dval.reserve(n))) return bail(s);
     k_dense_tasks<<<grid_for(n), 256, 0, st>>>(n, roff, radj, pdense, dkey.p, dval.p, sizes.p + 2);
   }
-  int h[5] = {0, 0, 0, 0, 0};
+  int h[6] = {0, 0, 0, 0, 0, 0};
   cudaMemcpyAsync(h, sizes.p, sizeof h, cudaMemcpyDeviceToHost, st);
   cudaError_t e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return bail(fail(GPM_ECUDA, std::string("rank plan: ") + cudaGetErrorString(e)));
   if (h[4]) return bail(fail(GPM_EUNSUPPORTED, "triangle plan: a partner segment of 2^29 keys or more"));
   p->n_cta = h[0];
   p->n_warp = h[1];
+  const int64_t warps = (int64_t)rank_grid() * kRWarps;
+  const bool alone = p->n_warp <= 2 * kTaskRun * warps || h[5] > p->n_warp / 2;
+  p->n_lone = alone ? p->n_warp : (int)std::max<int64_t>(h[5], kTaskRun * warps);
   p->n_dense = h[2];
   p->n_dense_only = h[3];
   if (p->n_dense && (s = p->dense_tasks.reserve(p->n_dense))) return bail(s);
@@ -1457,11 +1469,11 @@ int rank_plan_launch(gpm_graph *g, RankPlan *p, cudaStream_t st, unsigned long l
   if (rec)
     k_tc_rank_t<true><<<rank_grid(), 256, kRankSmem, st>>>(
         g->rg->roff.p, g->rg->radj.p, g->rg->radj4.p, p->poff.p, p->pseg.p, p->plong.p, p->pshort.p, p->cta_tasks.p,
-        p->n_cta, p->warp_tasks.p, p->n_warp, cursors, d_out, rec);
+        p->n_cta, p->warp_tasks.p, p->n_warp, p->n_lone, cursors, d_out, rec);
   else
     k_tc_rank<<<rank_grid(), 256, kRankSmem, st>>>(g->rg->roff.p, g->rg->radj.p, g->rg->radj4.p, p->poff.p,
                                                    p->pseg.p, p->plong.p, p->pshort.p, p->cta_tasks.p, p->n_cta,
-                                                   p->warp_tasks.p, p->n_warp, cursors, d_out, nullptr);
+                                                   p->warp_tasks.p, p->n_warp, p->n_lone, cursors, d_out, nullptr);
   if (p->n_dense) GPM_CUDA(cudaStreamWaitEvent(st, p->join, 0));  // joined whether or not the launches were accepted
   GPM_LAUNCH_CHECK();
   return GPM_OK;

@@ -132,6 +132,7 @@ __host__ __device__ __forceinline__ int core_clear_words(int32_t kmin, int32_t k
 struct RankPlan {
   int cta_min = 0, long_min = 0;
   int n_cta = 0, n_warp = 0;
+  int n_lone = 0;                 // warp tasks handed out one at a time, the heaviest
   int32_t core_base = INT32_MAX;  // INT32_MAX: no dense core
   int row_words = 0;              // multiple of 4
   int64_t n_rows = 0;
