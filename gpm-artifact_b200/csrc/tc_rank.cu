@@ -791,12 +791,13 @@ __global__ void k_dense_tasks(int64_t n, const int64_t *__restrict__ roff, const
 
 // tasks: owners with partners, by their work.  Fixed schedule: an owner of at
 // most cta_min keys is a CTA task all the same when its work is more than
-// half a resident warp's share of the total (at least 1024): one warp would
-// hold up the count.  Without that rule / 4 shares / 1 share / half / a
+// half a resident warp's share of the total (at least 1024, and four times the
+// mean: where tasks are alike a CTA each only costs barriers, ER 10,007 x 64 30.7 ->
+// 29.0 us, R-MAT 18 204 -> 193): one warp would hold up the count.  Without that rule / 4 shares / 1 share / half / a
 // quarter, us per count: R-MAT 14: 76, 29, 26, 26, 27; R-MAT 16: 120, 115, 68,
 // 58, 56; R-MAT 18: 224, 223, 173, 146, 140; R-MAT 20: 860, 844, 835, 828, 825;
 // R-MAT 22 unchanged; Chung-Lu 300,007 x 24: 154, 154, 156, 160, 165.
-constexpr unsigned long long kHeavyWork = 1024;
+constexpr unsigned long long kHeavyWork = 1024, kHeavyMeans = 4;
 constexpr int kHeavyShares = 2;
 // Warp tasks of more than kLoneWork keys come from the cursor one at a time, the
 // rest in runs (WarpTasks): a run of heavy ones ends the count late.  All come
@@ -814,7 +815,7 @@ __global__ void k_rank_tasks(int64_t n, const int64_t *__restrict__ roff, const 
                              int32_t *__restrict__ cval, uint32_t *__restrict__ wkey,
                              int32_t *__restrict__ wval, int *__restrict__ sizes) {
   const unsigned long long heavy =
-      max(kHeavyWork, *total / (unsigned long long)(warps * kHeavyShares));
+      max(max(kHeavyWork, kHeavyMeans * (*total / (unsigned long long)n)), *total / (unsigned long long)(warps * kHeavyShares));
   for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
     if (plong[x] + pshort[x] == 0) {  // nothing to stream
       if (pdense && pdense[x]) donly[atomicAdd(&sizes[3], 1)] = (int32_t)x;  // dense segments only
