@@ -139,26 +139,39 @@ struct DevBuf {
 };
 
 // Orders the launches of one handle over all streams: scratch of its plan holds
-// positions and counters that two of them must not share.  A launch inside a
-// capture cannot wait for one outside of it and stays out of the order.
+// positions and counters that two of them must not share.  The legacy default
+// stream orders its own launches (two event calls per launch cost 4 us of host
+// time).  A launch inside a capture cannot wait for one outside of it and
+// stays out of the order.
 bool stream_capturing(cudaStream_t st);
 struct LaunchOrder {
-  cudaEvent_t last = nullptr;  // behind the latest launch
+  cudaEvent_t event = nullptr;
+  enum { kNone, kLegacy, kEvent } last = kNone;  // where the latest launch went: kEvent, `event` is behind it
   LaunchOrder() = default;
   LaunchOrder(const LaunchOrder &) = delete;
   LaunchOrder &operator=(const LaunchOrder &) = delete;
   ~LaunchOrder() {
-    if (last) cudaEventDestroy(last);
+    if (event) cudaEventDestroy(event);
+  }
+  int record(cudaStream_t st) {
+    if (!event) GPM_CUDA(cudaEventCreateWithFlags(&event, cudaEventDisableTiming));
+    GPM_CUDA(cudaEventRecord(event, st));
+    last = kEvent;
+    return GPM_OK;
   }
   int begin(cudaStream_t st) {
-    if (last && !stream_capturing(st)) GPM_CUDA(cudaStreamWaitEvent(st, last, 0));
+    const bool foreign = foreign_stream(st);
+    if (last == kNone || (last == kLegacy && !foreign) || stream_capturing(st)) return GPM_OK;
+    if (last == kLegacy) GPM_TRY(record(cudaStreamLegacy));
+    GPM_CUDA(cudaStreamWaitEvent(st, event, 0));
     return GPM_OK;
   }
   int end(cudaStream_t st) {
-    if (stream_capturing(st)) return GPM_OK;
-    if (!last) GPM_CUDA(cudaEventCreateWithFlags(&last, cudaEventDisableTiming));
-    GPM_CUDA(cudaEventRecord(last, st));
-    return GPM_OK;
+    if (!foreign_stream(st)) {
+      last = kLegacy;
+      return GPM_OK;
+    }
+    return stream_capturing(st) ? GPM_OK : record(st);
   }
 };
 

@@ -10,9 +10,11 @@ import gpm
 pytestmark = pytest.mark.gpu
 
 
-def _overlap(run_async, want):
+def _overlap(run_async, want, legacy=False):
     import torch
     streams = [torch.cuda.Stream() for _ in range(3)]
+    if legacy:  # the legacy default stream between two others
+        streams[1] = torch.cuda.default_stream()
     out = torch.zeros(12, want.size, dtype=torch.int64, device="cuda")
     for r in range(4):
         out.fill_(-1)
@@ -29,6 +31,7 @@ def test_motif_batch():
     want = b.motif(use_graph=False)
     assert (want == b.motif(use_graph=True)).all() and want[:, 5].all()
     _overlap(b.motif_async, want)
+    _overlap(b.motif_async, want, legacy=True)
     assert (want == b.motif(use_graph=False)).all()
 
 
@@ -42,4 +45,5 @@ def test_match_batch():
     assert want[:, 0].tolist() == [g.match(q) for q in qs] and want.all()
     assert (want == b.run(use_graph=True)).all()
     _overlap(b.run_async, want)
+    _overlap(b.run_async, want, legacy=True)
     assert (want == b.run(use_graph=False)).all()
