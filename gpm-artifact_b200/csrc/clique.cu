@@ -71,6 +71,7 @@ constexpr int kCqSmallThreads = 256, kCqBigThreads = 512;
 // 360; 5 CTAs on rows from a binary search: 108, 294, 328, 0.83.)
 constexpr size_t kCqSmemAny = 40 * 1024;
 constexpr int kCqAnyThreads = 256, kCqAnyPerSm = 3;
+constexpr int kCqFewPerSm = 5;  // CTAs of k_clique_warp per SM where each warp gets few tasks
 __host__ __device__ constexpr bool cq_any(int k) { return k != 4 && k != 5; }
 
 static int grid_for(int64_t work, int block = 256) {
@@ -1058,8 +1059,12 @@ int clique_plan_run(CliquePlan *p, cudaStream_t st, bool zero) {
     });
   }
   if (bst != st) GPM_CUDA(cudaEventRecord(p->join, bst));
+  // few tasks per warp: fewer warps meet less often at the cursor (us at eight /
+  // five CTAs per SM, k = 4: ER 100,003 x 4, 24,000 tasks 54 / 46, ER 10,007 x 16
+  // 36 / 33; but ER 100,003 x 32, 100,000 tasks 118 / 142)
+  const int warp_grid = p->n_warp <= 4 * 8 * grids.warp ? std::min(grids.warp, kCqFewPerSm * num_sms()) : grids.warp;
   if (p->n_warp > 0)
-    k_clique_warp<<<std::min(grids.warp, (p->n_warp + 7) / 8), 256, 0, st>>>(
+    k_clique_warp<<<std::min(warp_grid, (p->n_warp + 7) / 8), 256, 0, st>>>(
         p->k, p->roff, p->radj, p->wtasks.p, p->n_warp, p->cursors + 2, p->gid, p->acc, p->stride, p->slot);
   if (bst != st) GPM_CUDA(cudaStreamWaitEvent(st, p->join, 0));  // joined whether or not the launches were accepted
   GPM_LAUNCH_CHECK();
