@@ -78,11 +78,19 @@ __device__ __forceinline__ int wisect(const int32_t *a, int na, const int32_t *b
 // one warp per edge / (degree, parts) = (48, 16) / (96, 16) / (192, 16), Chung-
 // Lu graphs: P5, 2,001 vertices 2918, 617, 715, 1764; P2, 801: 1745, 536, 1287,
 // 1868; P3, 801: 1556, 780, 1750, 1631; P6, 2,001: 859, 242, 265, 502; P8, 20,001:
-// 10164, 4681, 4464, 4646; P7, 4,099: 271, 324, 227, 179.
+// 10164, 4681, 4464, 4646; P7, 4,099: 271, 324, 227, 179.  P7 at 192 with 1 / 4 / 8 / 16
+// parts: Chung-Lu 4,099 x 9 203, 129, 120, 115, 20,001 x 9 612, 377, 457, 715, 3,001 x 30
+// 893, 503, 524, 677.
 struct HeavyRule {
   int64_t degree;
   int parts;
 };
+// And longer than kHeavyMean times the edges' mean: where all edges are alike, the
+// parts build the same lists for nothing.  us, start of the sharing / without /
+// with that bound: complete graph of 300, P2 1145, 7010, 559, P5 15051, 22810, 14832; ER
+// 3,000 x 30, P6 781, 1079, 187; R-MAT 10 P6 57798, 4208, 5093 (bounds of 1.5 and 2
+// times the mean: 5444, 10714).
+constexpr double kHeavyMean = 1.25;
 static HeavyRule heavy_rule(int p) { return p == 7 ? HeavyRule{192, 4} : HeavyRule{48, 16}; }
 __global__ void k_heavy_edges(HeavyRule rule, int64_t nnz, const int64_t *__restrict__ off, const int32_t *__restrict__ adj,
                               const int32_t *__restrict__ src, uint32_t *__restrict__ heavy,
@@ -197,6 +205,10 @@ int pattern_enumerate(gpm_graph *g, int p, cudaStream_t st, uint64_t *result) {
   if (g->nnz > 0) {
     DevBuf<uint32_t> heavy;
     HeavyRule rule = heavy_rule(p);
+    // nor are edges heavy that are like most others: the graph's heavy ones
+    // are what holds up the count
+    const double mean = 2.0 * (double)g->sum_deg2 / (double)g->nnz;  // of an edge's two list lengths
+    rule.degree = std::max<int64_t>(rule.degree, (int64_t)(kHeavyMean * mean));
     if (g->nnz >= (1ll << 32)) rule.degree = INT64_MAX;  // edges are listed by 32-bit numbers
     bool some = 2 * maxd > rule.degree;
     if (some) {
