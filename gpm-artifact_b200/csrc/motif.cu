@@ -232,18 +232,21 @@ __global__ void __launch_bounds__(256) k_edge_tri(const int64_t *__restrict__ do
 // acc[g*8 + 0] S, 1 A4 = sum (da-1)(db-1), 2 A1 = sum t, 3 A2 = sum C(t,2),
 // 4 A3 = sum t(da+db-4), 5 K4, 6 C4, 7 sum C(d,2)
 //
-// A warp takes a run of consecutive blocks of 32 vertices, whose upward edges
+// A warp takes a run of consecutive blocks of up to 32 vertices, whose upward edges
 // are consecutive too, keeps its sums in registers and adds them to the graph's
 // totals when the run or the graph ends: one set of atomics per vertex, all on
 // the same few words, took 1.87 ms for a batch of 2.2 M vertices and 35 M
 // edges.
-__global__ void k_edge_sums(int64_t n, const int64_t *__restrict__ roff, const int64_t *__restrict__ doff,
+// span: vertices per block, a power of two up to 32, fewer where 32 each would
+// leave SMs without a warp (complete graph of 300 vertices: 304 us in blocks of
+// 32, 15 so).
+__global__ void k_edge_sums(int64_t n, int span, const int64_t *__restrict__ roff, const int64_t *__restrict__ doff,
                             const int32_t *__restrict__ dadj, const unsigned *__restrict__ te,
                             const int32_t *__restrict__ gid, unsigned long long *__restrict__ acc) {
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const unsigned lane = lane_id();
-  const int64_t blocks = (n + 31) / 32, run = (blocks + nw - 1) / nw;
+  const int64_t blocks = (n + span - 1) / span, run = (blocks + nw - 1) / nw;
   unsigned long long s = 0, c2 = 0, a4 = 0, a1 = 0, a2 = 0, a3 = 0;
   int g = -1;
   auto flush = [&]() {
@@ -258,8 +261,8 @@ __global__ void k_edge_sums(int64_t n, const int64_t *__restrict__ roff, const i
     s = c2 = a4 = a1 = a2 = a3 = 0;
   };
   for (int64_t b = warp * run; b < min(blocks, (warp + 1) * run); ++b) {
-    const int64_t x = b * 32 + lane;
-    const bool in = x < n;
+    const int64_t x = b * span + lane;
+    const bool in = (int)lane < span && x < n;
     const unsigned long long da = in ? (unsigned long long)(roff[x + 1] - roff[x]) : 0ull;
     const int64_t e0 = in ? doff[x] : 0, e1 = in ? doff[x + 1] : INT64_MAX;
     const int gx = in ? graph_of(gid, x) : -1;
@@ -819,8 +822,10 @@ int motif_plan_run(MotifPlan *p, cudaStream_t st) {
   // the sums, and behind them the cursors of all stages
   GPM_CUDA(cudaMemsetAsync(p->acc.p, 0, sizeof(unsigned long long) * (8 * in.ngraphs + kMotifCursors), st));
   GPM_TRY(te_launch(p, st));
+  int span = 1;
+  while (span < 32 && n / span > (int64_t)num_sms() * 32) span *= 2;
   if (n > 0)
-    k_edge_sums<<<grid_for(n), 256, 0, st>>>(n, in.roff, p->doff.p, p->dadj.p, p->te.p, in.gid, p->acc.p);
+    k_edge_sums<<<grid_for((n + span - 1) / span * 32), 256, 0, st>>>(n, span, in.roff, p->doff.p, p->dadj.p, p->te.p, in.gid, p->acc.p);
   if (in.size == 4) {
     GPM_TRY(c4_launch(p, st));
     GPM_TRY(clique_plan_run(&p->k4, st, false));
