@@ -90,22 +90,24 @@ __device__ __forceinline__ unsigned long long wedge_bound(const CycleArgs &A, in
 }
 
 // Roots with wedges on both sides into the queue of their size; a warp takes
-// 32 roots and queues them with one atomic per queue.  Roots come in descending
-// degree order, so a warp takes every (nroots / 32)-th of them: 32 neighbours
+// up to 32 roots and queues them with one atomic per queue -- fewer where there
+// are too few for all SMs, since it takes them one after another (a query with
+// 3,671 roots, ER 10,007 x 64: 128 us with 32 each, 79 so).  Roots come in
+// descending degree order, so a warp takes every (nroots / per)-th of them: neighbours
 // would give all hubs to a few warps (R-MAT 19, labels 0 0 3 1: 1.3-2.1 ms; the
 // whole call 5.6 ms then, 3.4 ms now).  The side with fewer
 // wedges is the one that is counted (its counters are written and cleared).
-__global__ void k_cycle_split(CycleArgs A, const int32_t *__restrict__ roots, int64_t nroots, int2 *__restrict__ small,
+__global__ void k_cycle_split(CycleArgs A, const int32_t *__restrict__ roots, int64_t nroots, int per, int2 *__restrict__ small,
                               int4 *__restrict__ big, int *__restrict__ sizes) {
   const unsigned lane = lane_id();
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const bool same = A.lb == A.ld;
-  const int64_t groups = (nroots + 31) / 32;
+  const int64_t groups = (nroots + per - 1) / per;
   for (int64_t r0 = warp; r0 < groups; r0 += nw) {
     int4 mine = make_int4(0, 0, 0, 0);
     int which = 0;  // 1 small, 2 big
-    for (int j = 0; j < 32 && r0 + j * groups < nroots; ++j) {
+    for (int j = 0; j < per && r0 + j * groups < nroots; ++j) {
       const int32_t v = roots[r0 + j * groups];
       const unsigned long long wb = wedge_bound(A, v, A.lb, lane), wd = same ? wb : wedge_bound(A, v, A.ld, lane);
       if ((int)lane == j && min(wb, wd) > 0) {
@@ -152,8 +154,11 @@ __global__ void __launch_bounds__(kSmallWarps * 32)
   for (int i = lane; i < kSmallSlots; i += 32) tab[i] = make_int2(-1, 0);
   __syncwarp();
   WarpTasks queue;
+  // runs only where the warps have many tasks each: the first are the heaviest
+  // (the same query 79 us in runs, 42 so; R-MAT 14, labels 0 1 2 3 202, 91)
+  const int lone = n <= 2 * kTaskRun * (int)gridDim.x * kSmallWarps ? n : 0;
   while (true) {
-    const int t = queue.next(&sizes[2], 0, lane);
+    const int t = queue.next(&sizes[2], lone, lane);
     if (t >= n) break;
     const int2 task = tasks[t];
     const int32_t self = A.skip_root ? A.lrank[task.x] : -1;
@@ -408,8 +413,9 @@ int cycle_launch(const gpm_graph *g, const LabelCsr *lc, const CyclePlan &p, con
   if (nroots == 0) return GPM_OK;
   const CycleArgs A{g->off.p, lc->ladj.p, lc->loff.p, lc->lrk.p, lc->lrank.p, lc->L, p.lb, p.lc, p.ld, p.la == p.lc};
   GPM_CUDA(cudaMemsetAsync(s->sizes.p, 0, 4 * sizeof(int), st));
-  k_cycle_split<<<blocks_for(nroots), 256, 0, st>>>(A, lc->lorder.p + lc->lstart[p.la], nroots, s->small.p, s->big.p,
-                                                    s->sizes.p);
+  const int per = (int)std::min<int64_t>(32, std::max<int64_t>(1, nroots / ((int64_t)num_sms() * 32)));
+  k_cycle_split<<<blocks_for((nroots + per - 1) / per * 32), 256, 0, st>>>(A, lc->lorder.p + lc->lstart[p.la], nroots,
+                                                                           per, s->small.p, s->big.p, s->sizes.p);
   k_cycle_big<<<s->grid, kBigThreads, kHot * sizeof(unsigned), st>>>(A, s->big.p, s->sizes.p, s->tail.p, s->tail_len,
                                                                      member, out);
   k_cycle_small<<<num_sms() * 6, kSmallWarps * 32, 0, st>>>(A, s->small.p, s->sizes.p, member, out);
