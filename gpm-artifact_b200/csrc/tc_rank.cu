@@ -814,8 +814,9 @@ __global__ void k_rank_tasks(int64_t n, const int64_t *__restrict__ roff, const 
                              int32_t *__restrict__ donly, uint32_t *__restrict__ ckey,
                              int32_t *__restrict__ cval, uint32_t *__restrict__ wkey,
                              int32_t *__restrict__ wval, int *__restrict__ sizes) {
+  const unsigned long long mean = n >= warps ? *total / (unsigned long long)n : 0;  // fewer owners: the heaviest is the time
   const unsigned long long heavy =
-      max(max(kHeavyWork, kHeavyMeans * (*total / (unsigned long long)n)), *total / (unsigned long long)(warps * kHeavyShares));
+      max(max(kHeavyWork, kHeavyMeans * mean), *total / (unsigned long long)(warps * kHeavyShares));
   for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
     if (plong[x] + pshort[x] == 0) {  // nothing to stream
       if (pdense && pdense[x]) donly[atomicAdd(&sizes[3], 1)] = (int32_t)x;  // dense segments only
