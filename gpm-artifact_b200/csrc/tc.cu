@@ -280,6 +280,11 @@ __device__ unsigned long long warp_task(int32_t u, const int64_t *__restrict__ o
 // of kTaskRun otherwise (ER, 10^6 vertices of mean degree 12: 621 -> 339 us).
 // Uneven tasks come one at a time: R-MAT 16 took 688 us in runs, 463 singly.
 constexpr int kEvenDegree = 48;
+// ... nor has a task more than kEvenMean entries on average: heavier ones end the
+// count late in runs (us singly / so, ER of mean out-degree 8, 10, 12, 16: 100,003
+// vertices 76 / 66, 79 / 80, 81 / 94, 107 / 127; 200,003: 140 / 107, 142 / 132, 148 / 160,
+// 195 / 217).
+constexpr int64_t kEvenMean = 10;
 __device__ __forceinline__ unsigned long long hash_tasks(const int64_t *__restrict__ off,
                                                          const int32_t *__restrict__ adj,
                                                          const int32_t *__restrict__ cta_tasks, int n_cta,
@@ -476,10 +481,11 @@ int tc_launch(gpm_graph *g, int variant, cudaStream_t st, unsigned long long *d_
       cursors = p->counters.p;
       GPM_CUDA(cudaMemsetAsync(cursors, 0, 2 * sizeof(int), st));
     }
+    const bool even = g->max_deg <= kEvenDegree && g->nnz <= kEvenMean * ((int64_t)p->n_cta + p->n_warp);
     const int64_t blocks = (int64_t)p->n_cta + ((int64_t)p->n_warp + kWarps - 1) / kWarps;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(tc_hash_grid(), blocks));
     k_tc_hash<<<grid, 256, TC_SMEM, st>>>(g->off.p, g->adj.p, p->cta_tasks.p, p->n_cta, p->warp_tasks.p, p->n_warp,
-                                          cursors, g->max_deg <= kEvenDegree, d_out);
+                                          cursors, even, d_out);
     GPM_LAUNCH_CHECK();
     return GPM_OK;
   }
