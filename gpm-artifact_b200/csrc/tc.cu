@@ -284,7 +284,7 @@ constexpr int kEvenDegree = 48;
 // count late in runs (us singly / so, ER of mean out-degree 8, 10, 12, 16: 100,003
 // vertices 76 / 66, 79 / 80, 81 / 94, 107 / 127; 200,003: 140 / 107, 142 / 132, 148 / 160,
 // 195 / 217).
-constexpr int64_t kEvenMean = 10;
+constexpr int64_t kEvenMean = 11;
 __device__ __forceinline__ unsigned long long hash_tasks(const int64_t *__restrict__ off,
                                                          const int32_t *__restrict__ adj,
                                                          const int32_t *__restrict__ cta_tasks, int n_cta,
