@@ -544,8 +544,13 @@ __device__ __forceinline__ int64_t upper_bound_key(const int32_t *__restrict__ a
 // (start, len) and the smallest and largest key of it, its first 16-byte row
 // in radj4, and its core bitmap row (-1: none).
 struct __align__(32) VertexInfo {
-  int64_t start;
-  int32_t len, kmin, kmax, row4, rowid, pad;
+  uint32_t start_lo;  // the low half first: fewer than 2^31 keys need no other
+  int32_t len, kmin, kmax, row4, rowid;
+  uint32_t start_hi, pad;
+  template <bool WIDE>
+  __device__ __forceinline__ int64_t start() const {
+    return WIDE ? (int64_t)(((uint64_t)start_hi << 32) | start_lo) : (int64_t)start_lo;
+  }
 };
 __global__ void k_vertex_info(int64_t n, const int64_t *__restrict__ roff, const int32_t *__restrict__ radj,
                               const int64_t *__restrict__ roff4, const int32_t *__restrict__ rowid,
@@ -553,7 +558,8 @@ __global__ void k_vertex_info(int64_t n, const int64_t *__restrict__ roff, const
   for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
     const int64_t s = roff[v], e = roff[v + 1];
     VertexInfo f;
-    f.start = s;
+    f.start_lo = (uint32_t)s;
+    f.start_hi = (uint32_t)((uint64_t)s >> 32);
     f.len = (int32_t)(e - s);
     f.kmin = e > s ? radj[s] : 0;
     f.kmax = e > s ? radj[e - 1] : 0;
@@ -590,6 +596,9 @@ __global__ void k_chunk_starts(int64_t n, const int64_t *__restrict__ roff, int3
   for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x)
     for (int64_t c = (roff[u] + 31) >> 5; 32 * c < roff[u + 1]; ++c) ustart[c] = (int32_t)u;
 }
+// WIDE: 2^31 stored keys or more.  (Without it list starts take half the registers:
+// 32 in place of 40, R-MAT 20 from the host 5.06 -> 5.02 ms.)
+template <bool WIDE>
 __global__ void k_partner_place(int64_t n, const int64_t *__restrict__ roff, const int32_t *__restrict__ radj,
                                 const int32_t *__restrict__ ustart, const VertexInfo *__restrict__ info,
                                 int32_t *__restrict__ radj4, int upward, int long_min,
@@ -629,7 +638,7 @@ __global__ void k_partner_place(int64_t n, const int64_t *__restrict__ roff, con
       const VertexInfo U = info[u], V = info[v];
       if (radj4) {
         int32_t *row = radj4 + 4 * (int64_t)U.row4;
-        const int at = (int)(k - U.start);
+        const int at = (int)(k - U.start<WIDE>());
         row[at] = v;
         if (at == U.len - 1)
           for (int i = U.len; i & 3; ++i) row[i] = INT32_MAX;
@@ -639,7 +648,7 @@ __global__ void k_partner_place(int64_t n, const int64_t *__restrict__ roff, con
       const int32_t kmin = own_u ? U.kmin : V.kmin, kmax = own_u ? U.kmax : V.kmax;
       const VertexInfo P = own_u ? V : U;
       if ((own_u ? U.len : V.len) >= 2 && P.len > 0) {
-        const int64_t ps = P.start, pe = ps + P.len;
+        const int64_t ps = P.start<WIDE>(), pe = ps + P.len;
         // upward: when v owns the edge, every id of N(u) up to v sits at or
         // before slot k, and min N(v) > v, so the search starts past k
         const int64_t lo = upward && own_u ? ps : lower_bound_key(radj, upward ? k + 1 : ps, pe, kmin);
@@ -653,7 +662,7 @@ __global__ void k_partner_place(int64_t n, const int64_t *__restrict__ roff, con
           if (P.rowid >= 0 && kmin >= core_base &&
               100 * len >= (int64_t)dense_pct * core_and_words(kmin, kmax))
             row = (int64_t)P.rowid * (row_words >> 2) + (((kmin & ~127) - core_base) >> 7);
-          units = row >= 0 ? 0u : (unsigned)(len >> work_shift);
+          units = row >= 0 ? 0u : (unsigned)(len >> (WIDE ? work_shift : 0));
           lng = row >= 0 || len >= owner_long_min(cfg, owner, long_min);
           const int64_t lo4 = lo - ps;  // the same keys in radj4
           if (len >= (1 << 29)) *too_long = 1;  // no 8-byte descriptor for it
@@ -814,6 +823,7 @@ __global__ void k_rank_tasks(int64_t n, const int64_t *__restrict__ roff, const 
                              int32_t *__restrict__ donly, uint32_t *__restrict__ ckey,
                              int32_t *__restrict__ cval, uint32_t *__restrict__ wkey,
                              int32_t *__restrict__ wval, int *__restrict__ sizes) {
+  int lone = 0;
   const unsigned long long mean = n >= warps ? *total / (unsigned long long)n : 0;  // fewer owners: the heaviest is the time
   const unsigned long long heavy =
       max(max(kHeavyWork, kHeavyMeans * mean), *total / (unsigned long long)(warps * kHeavyShares));
@@ -831,9 +841,11 @@ __global__ void k_rank_tasks(int64_t n, const int64_t *__restrict__ roff, const 
       int i = atomicAdd(&sizes[1], 1);
       wkey[i] = task_key(work[x]);
       wval[i] = (int32_t)x;
-      if (work[x] > kLoneWork) atomicAdd(&sizes[5], 1);
+      lone += work[x] > kLoneWork;
     }
   }
+  lone = warp_sum(lone);
+  if (lane_id() == 0 && lone) atomicAdd(&sizes[5], lone);
 }
 
 void free_rank_plan(RankPlan *p) { delete p; }
@@ -1379,7 +1391,7 @@ int rank_plan_new(gpm_graph *g, int cta_min, int long_min, const uint8_t *cfg, c
   DevBuf<int32_t> ustart;
   if ((s = ustart.reserve((keys + 31) / 32))) return bail(s);
   k_chunk_starts<<<grid_for(n), 256, 0, st>>>(n, roff, ustart.p);
-  k_partner_place<<<grid_for(keys), 256, 0, st>>>(n, roff, radj, ustart.p, info.p, fill ? g->rg->radj4.p : nullptr, g->rg->upward,
+  (work_shift ? k_partner_place<true> : k_partner_place<false>)<<<grid_for(keys), 256, 0, st>>>(n, roff, radj, ustart.p, info.p, fill ? g->rg->radj4.p : nullptr, g->rg->upward,
                                                long_min, cfg, p->poff.p, lcnt.p, scnt.p, p->pseg.p, p->core_base,
                                                p->row_words, dense_pct, p->pdense.p, sizes.p + 4, work_shift);
   k_place_counts<<<grid_for(n), 256, 0, st>>>(n, lcnt.p, scnt.p, p->plong.p, p->pshort.p, work.p, total.p, work_shift);
