@@ -627,13 +627,12 @@ def motif_workload(args, stream):
         "e2e": {"value": total / (min(e2e_ms) / 1e3), "unit": "instances/s", "ms_per_step": min(e2e_ms),
                 "h2d_bytes_per_step": int(hsrc.numel() * 4 + hdst.numel() * 4),
                 "d2h_bytes_per_step": int(8 * 8 * ng)},
-        # the dominant stage's kernel, k_c4_big, has been profiled on a smaller
-        # batch only, so no DRAM bytes of this one are given
+        # the dominant stage's kernel; its issue rate is that of a smaller batch
         "roofline": roofline(profiled("motif_batch48", "traffic_bytes_per_launch[c4_big_batch256]"),
                              stages["four_cycles"],
                              hbm, peak_kind, kernel="k_c4_big (the 4-cycle stage's large tasks)",
-                             issue_active_pct=profiled("motif_batch48", "issue_active_pct[edge_tri_batch48]"),
-                             note="issue- and latency-bound pipeline (profiles/motif_batch48.md)"),
+                             issue_active_pct=profiled("motif_batch48", "issue_active_pct[c4_big_batch48]"),
+                             note="latency of lists and shared counters (profiles/motif_batch48.md)"),
         "gpu_launches_timed": None,
     })
     if not args.no_cpu:

@@ -86,7 +86,7 @@ def run_one(d, name, timeout):
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--scales", default="16,18,21")
-    ap.add_argument("--workdir", default=os.path.join(ROOT, "_work", "ceci"))
+    ap.add_argument("--workdir", required=True, help="where the runs' inputs and outputs go")
     ap.add_argument("--timeout", type=float, default=7200)
     ap.add_argument("--jobs", type=int, default=4)
     ap.add_argument("--queries", default="21:triangle,cycle4,diamond",
