@@ -520,7 +520,10 @@ __device__ __forceinline__ unsigned long long match_task(const QueryPlanT<Q> &q,
 #define GPM_MATCH_MIN_BLOCKS 6
 #endif
 #ifndef GPM_MATCH_WGT_BLOCKS
-#define GPM_MATCH_WGT_BLOCKS 4  // factored plans
+// factored plans.  Houses of R-MAT 16, 15 and 15 (other labels) with 3 / 4 / 5 / 6:
+// 5.46 5.49 4.93 4.72, 1.80 1.80 1.62 1.62, 0.79 0.79 0.72 0.73 ms; diamonds,
+// 5-cycles and tailed triangles are the same with each
+#define GPM_MATCH_WGT_BLOCKS 4
 #endif
 // Candidate rows of the wide kernels (Q > kNarrowQ): Q rows of 32 ids per
 // warp in dynamic shared memory (64 KB per CTA at Q = 64).
@@ -859,13 +862,16 @@ static int plan_query(const gpm_query *q, const std::vector<int64_t> &label_freq
 // position; the number of images they can take is a set size that multiplies
 // the count, so the embeddings that differ only there are never walked one by
 // one.  (The diamond query becomes, per edge, two set sizes.  R-MAT 17, a
-// batch of a triangle, a diamond, a house and a 4-cycle: 1.67 s walked, 14.8
+// batch of a triangle, a diamond, a house and a 4-cycle: 1.67 s walked, 14
 // ms with the sets and match_cycle.cu's 4-cycles.)  Every choice of such
 // vertices and of a root is compared with the plan at hand by the number of
 // partial embeddings and of entries scanned that an average graph with these
 // label frequencies would give: each position multiplies by the mean label
 // segment (walks meet hubs, hence kSkew times the mean) and each further back
-// edge by kClose.
+// edge by kClose.  Both are rough: what matters is that they are not low, since a
+// wide set is then walked where it could be a size.  kSkew 1 / 4 / 16, ms: house
+// R-MAT 16 189, 5.5, 5.5, R-MAT 14 2.97, 2.97, 0.68, diamond R-MAT 17 1.21, 0.40,
+// 0.40; kClose 0.02 / 0.1 / 0.5: 190, 5.5, 5.5, 2.98, 2.97, 0.68, 1.21, 0.40, 0.41.
 static void factor_query(const gpm_query *q, const std::vector<int64_t> &label_freq, int64_t n, int64_t nnz,
                          WidePlan *p) {
   const int nq = q->n;

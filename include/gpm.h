@@ -47,8 +47,10 @@ enum { GPM_V_CENTRIC = 0, GPM_E_CENTRIC = 1 };
 
 /* Triangle-count kernel variants (all return the same count). */
 enum {
-  GPM_TC_AUTO = 0,     /* engine's default: GPM_TC_BITMAP; tiny graphs GPM_TC_BSEARCH,
-                          the lists of each edge merged where every list is short    */
+  GPM_TC_AUTO = 0,     /* engine's default.  gpm_tc_async: GPM_TC_BSEARCH up to 16,384
+                          stored entries, the two lists of each edge merged where no
+                          list is longer than 24, else GPM_TC_BITMAP.
+                          gpm_tc_host_csr: always GPM_TC_BITMAP                        */
   GPM_TC_BSEARCH = 1,  /* warp per stored edge, binary search (TCSolver.cuh:27-59 shape) */
   GPM_TC_HASH = 2,     /* vertex tasks, shared-memory hash of N(u), hub/tail queues
                           with the fixed thresholds of tuning_schedules.cuh:196-197   */
@@ -189,12 +191,17 @@ int gpm_graph_work(gpm_graph *g, uint64_t *wedge_work, uint64_t *pair_work);
  * |N(u) & N(v)|.  On an oriented graph this is the triangle count (the
  * reference's Engine::RunTC orients first, src/Engine.h:47-56).
  * mode: GPM_V_CENTRIC or GPM_E_CENTRIC, the reference's two kernels; both
- * give the same count, and both run the kernel that suits the graph: the
- * GPM_TC_HASH kernel for small graphs and first counts, GPM_TC_BITMAP once its
- * plan pays (src/TCSolver.cuh chooses by mode alone). */
+ * give the same count, and both run the kernel that suits the graph
+ * (src/TCSolver.cuh chooses by mode alone): GPM_TC_BSEARCH up to 16,384 stored
+ * entries, the merging kernel of GPM_TC_AUTO where no list is longer than 24,
+ * GPM_TC_BSEARCH up to 65,536 entries, and above that GPM_TC_HASH for light
+ * graphs and first counts, GPM_TC_BITMAP once its plan pays.  The call has
+ * work cursors of its own, so it may overlap asynchronous counts of g. */
 int gpm_tc(gpm_graph *g, int mode, uint64_t *out);
 /* Explicit variant, asynchronous: writes the count to device memory d_out
- * (8 bytes) on stream; no host synchronisation; capturable. */
+ * (8 bytes) on stream; no host synchronisation; capturable.  Counts of one
+ * handle by GPM_TC_HASH, GPM_TC_BITMAP or GPM_TC_LEARNED share the handle's
+ * work cursors: where they run on several streams, the caller orders them. */
 int gpm_tc_async(gpm_graph *g, int variant, void *stream, uint64_t *d_out);
 /* End to end from host memory: upload a symmetric CSR (sorted,
  * duplicate-free), orient on the device, count, return the count.  This is

@@ -2,7 +2,7 @@
 graphs, as a golden fixture.
 
     python tests/golden/make_ceci_config_golden.py [--scales 16,18,21] [--queries 21:triangle,cycle4,diamond]
-                                                   [--workdir DIR] [--timeout 7200] [--jobs 4]
+                                                   --workdir DIR [--timeout 7200] [--jobs 4]
 
 sub_ceci is built from the reference's sources into oracle/_ref/myceci
 (`make -C oracle ref`).  For each R-MAT scale (edge factor 16, seed 3, 8
